@@ -1,19 +1,25 @@
-// k_tail.cu -- the tail rounds of an MSB Multilinear / InnerProduct proof in
-// one thread block.
+// k_tail.cu -- the last rounds of a Multilinear / InnerProduct proof in one
+// thread block or one thread-block cluster.
 //
 // Once a prover's tables are small, a round costs far more in kernel
 // boundaries (launch, grid-wide ticket, a lone last block running the
 // transcript) than in arithmetic.  The tail kernel loads the tables into
 // shared memory once (base tables embedded when the field is Fp3), then per
-// round: folds in place with the previous challenge (new = lo + (hi - lo) r,
-// reference src/inner_product_sumcheck.rs:143-176 and
-// src/multilinear_sumcheck.rs:132-178), accumulates the round polynomial of
-// the folded tables on the fly (the same quadruple scheme as the fused
-// kernels), reduces across the block, and runs the transcript step (wire
-// values, hook bytes, challenge squeeze) in warp 0.  After the
-// last round the folded tables go back to global memory so that finalize /
-// final_value and the post-state accessors see exactly what the per-round
-// path would leave.  A batch launches one block per instance.
+// round: folds with the previous challenge (new = lo + (hi - lo) r, reference
+// src/inner_product_sumcheck.rs:143-176 and
+// src/multilinear_sumcheck.rs:132-178), sums the round polynomial of the
+// folded tables, and runs the transcript step (wire values, hook bytes,
+// challenge squeeze) in warp 0.  After the last round the folded tables go
+// back to global memory so that finalize / final_value and the post-state
+// accessors see exactly what the per-round path would leave.  A batch
+// launches one block per instance.
+//
+// What bounds it is one warp's latency: of about 5.5 us a round (InnerProduct
+// over Fp3), 2.6 are the Keccak permutation, the rest the chain fold ->
+// barrier -> sums -> barrier -> absorb, squeeze, reduce -> barrier.  n = 12:
+// 110.8 us when a thread carried whole quadruples and the words were summed
+// with shuffles, 74.8 in one block as split below, 66.6 in a cluster (whose
+// two barriers a round cost less than the first rounds' folds on one SM).
 #include "round_common.cuh"
 
 #include <atomic>
@@ -21,21 +27,16 @@
 
 namespace effsc {
 
-template <int FW>
-__device__ __forceinline__ F3 sm_ld(const u64* sm, u64 L, int t, u64 i) {
-    F3 r;
-    r.c0 = sm[(u64)(t * FW) * L + i];
-    if (FW == 3) { r.c1 = sm[(u64)(t * 3 + 1) * L + i]; r.c2 = sm[(u64)(t * 3 + 2) * L + i]; }
-    else { r.c1 = r.c2 = 0; }
-    return r;
-}
-template <int FW>
-__device__ __forceinline__ void sm_st(u64* sm, u64 L, int t, u64 i, const F3& v) {
-    sm[(u64)(t * FW) * L + i] = v.c0;
-    if (FW == 3) { sm[(u64)(t * 3 + 1) * L + i] = v.c1; sm[(u64)(t * 3 + 2) * L + i] = v.c2; }
-}
-
-constexpr int TAIL_TPB = 512;
+// How a round is split.  A late round is one block's latency, not its
+// throughput: a few dozen entries, every step waiting for the one before.  So
+// no thread carries a whole quadruple (36 products in a row): a fold with
+// fewer entries than threads gives each thread one component of one folded
+// entry (three products into one sum), the round polynomial gives each warp
+// one row of products (a_k times b_0, b_1, b_2) of one of its two values, and
+// a warp's sum takes three integer warp reductions (redux on 22-bit pieces)
+// instead of five shuffle-and-add levels per word.  The challenge is left in
+// shared memory together with its multiples by W.
+constexpr int TAIL_TPB = 768;        // 24 warps: a multiple of the 6 components of two Fp3 values
 constexpr int TAIL_NW = TAIL_TPB / 32;
 
 // Index i of a table of 2^lg entries with its lg bits reversed.  An LSB
@@ -43,229 +44,386 @@ constexpr int TAIL_NW = TAIL_TPB / 32;
 // folds (p, p + L/2) -> p, in place, with entry j of every later length at
 // the reversed position again; so the LSB tail is the MSB tail on a
 // bit-reversed layout, reversed back when the tables are written out.
-__device__ __forceinline__ u64 tail_rev(u64 i, u32 lg) { return lg ? (u64)(__brev((u32)i) >> (32 - lg)) : 0; }
-__device__ __forceinline__ u32 tail_lg(u64 n) { return n > 1 ? 63 - __clzll(n) : 0; }
+__device__ __forceinline__ u32 tail_rev(u32 i, u32 lg) { return lg ? __brev(i) >> (32 - lg) : 0; }
+__device__ __forceinline__ u32 tail_lg(u32 n) { return n > 1 ? 31 - __clz(n) : 0; }
 
-// Shared state of a tail block: block partials, round totals, challenge,
-// squeeze scratch, and (cluster kernel, CTA 0) the partials of every CTA.
-constexpr int TAIL_NW3 = 12;
 constexpr int TAIL_MAX_CS = 16;
+// Shared state of a tail block.
 struct TailShared {
-    u64 red[TAIL_NW][TAIL_NW3];
-    u64 tot[TAIL_NW3];
-    u64 chal[3];
+    uint4 part[3 * TAIL_NW];           // the warps' sums, in 22-bit pieces
+    u64 chal[5];                       // W r1, W r2, r0, r1, r2 of the last challenge r
+    u64 tot[6];                        // wire values, component c of value e at 3 e + c
+    u64 raw[3];
     __align__(8) uint8_t scr[64];
-    u64 cred[TAIL_MAX_CS][TAIL_NW3];
+    u64 cred[TAIL_MAX_CS][6];          // (cluster kernel, CTA 0) every CTA's sums
 };
 
-// Fold (pairs q, q+2Q and q+Q, q+3Q of the quarter length Q) and accumulate
-// the round polynomial of the folded tables; `put` stores the folded pair.
-template <int POL, int FW, class Put>
-__device__ __forceinline__ void tail_fold_eval(const u64* smb, u64 stride, u64 len, const u64* chal,
-                                               Policy<POL, FW == 3 ? (1u << Policy<POL, 0>::NT) - 1 : 0>& acc, Put put) {
-    constexpr int NT = Policy<POL, 0>::NT;
-    constexpr bool E = FW == 3;
-    const Mul3 m = mul3_prepare<E>(f3_make(chal[0], chal[1], chal[2]));
-    const u64 Q = len >> 2;
-    F3 lo[NT], hi[NT];
-    for (u64 q = threadIdx.x; q < Q; q += TAIL_TPB) {
-#pragma unroll
-        for (int t = 0; t < NT; t++) {
-            F3 x0 = sm_ld<FW>(smb, stride, t, q), x1 = sm_ld<FW>(smb, stride, t, q + Q);
-            F3 x2 = sm_ld<FW>(smb, stride, t, q + 2 * Q), x3 = sm_ld<FW>(smb, stride, t, q + 3 * Q);
-            lo[t] = f3_fold<E, E>(x0, x2, m);
-            hi[t] = f3_fold<E, E>(x1, x3, m);
-            put(t, q, Q, lo[t], hi[t]);
-        }
-        acc.pair(lo, hi);
-    }
+// Where a tail's tables are: component c of table t, entry i at
+// sm[(t FW + c) stride + off + i].  A fold writes the half of its rows that
+// the table does not occupy (off alternates between 0 and stride / 2), so
+// that threads may share an entry; only a table that fills its rows is
+// folded in place, by one thread per entry.
+struct TailTab {
+    u64* sm;
+    u32 stride, off, len;
+};
+
+// Sum of a warp's canonical values as three sums of 22-bit pieces (50 cycles
+// for the three; five levels of shuffles and modular adds take 300).
+__device__ __forceinline__ uint4 warp_sum_pieces(u64 v) {
+    uint4 p;
+    p.x = __reduce_add_sync(0xffffffffu, (u32)v & 0x3FFFFFu);
+    p.y = __reduce_add_sync(0xffffffffu, (u32)(v >> 22) & 0x3FFFFFu);
+    p.z = __reduce_add_sync(0xffffffffu, (u32)(v >> 44));
+    p.w = 0;
+    return p;
+}
+// x + y 2^22 + z 2^44 mod p (x, y, z < 2^32).
+__device__ __forceinline__ u64 join_pieces(const uint4& p) {
+    const u64 t = (u64)p.z << 44, lo = (u64)p.x + ((u64)p.y << 22) + t;
+    return gl_reduce_limbs((u32)lo, (u32)(lo >> 32), (p.z >> 20) + (lo < t ? 1u : 0u), 0, 0);
 }
 
-// Block reduction of the round polynomial into sh.tot (lanes < NW3 of warp 0).
-template <int NRAW>
-__device__ __forceinline__ void tail_block_reduce(F3* raw, bool active, TailShared& sh) {
-    constexpr int NW3 = 3 * NRAW;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (active) {
+// Component c of lo + (hi - lo) r; ch = the prepared challenge.
+template <int FW>
+__device__ __forceinline__ u64 tail_fold_comp(const u64* row0, u32 stride, u32 j, u32 half, int c, const u64* ch) {
+    AccF<FOLD_FORM> s;
+    s.from(row0[c * stride + j]);
+    // c0 = d0 r0 + d1 W r2 + d2 W r1, c1 = d0 r1 + d1 r0 + d2 W r2, c2 = d0 r2 + d1 r1 + d2 r0
+    u64 d[FW];
 #pragma unroll
-        for (int off = 16; off; off >>= 1) {
+    for (int k = 0; k < FW; k++) d[k] = gl_sub(row0[k * stride + j + half], row0[k * stride + j]);
 #pragma unroll
-            for (int i = 0; i < NRAW; i++) {
-                raw[i].c0 = gl_add(raw[i].c0, __shfl_down_sync(0xffffffffu, raw[i].c0, off));
-                raw[i].c1 = gl_add(raw[i].c1, __shfl_down_sync(0xffffffffu, raw[i].c1, off));
-                raw[i].c2 = gl_add(raw[i].c2, __shfl_down_sync(0xffffffffu, raw[i].c2, off));
+    for (int k = 0; k < FW; k++) s.mac(d[k], ch[2 + c - k]);
+    return s.reduce();
+}
+
+// Fold every table (pairs j, j + len/2).  `base`: the entries' components 1
+// and 2 are zero (tables given in Fp, Fp3 challenges).  put(t, c, j, value)
+// sees the folded entries too.  In place when out == T.off.
+template <int NT, int FW, class Put>
+__device__ __forceinline__ void tail_fold(const TailTab& T, u32 out, bool base, const u64* ch, Put put) {
+    const u32 half = T.len >> 1;
+    if (FW == 3 && (out == T.off || NT * half >= TAIL_TPB)) {
+        // a whole entry per thread
+        Mul3 m;
+        m.w1 = ch[0]; m.w2 = ch[1]; m.m0 = ch[2]; m.m1 = ch[3]; m.m2 = ch[4];
+        for (u32 i = threadIdx.x; i < NT * half; i += TAIL_TPB) {
+            const int t = NT > 1 && i >= half ? 1 : 0;
+            const u32 j = i - t * half;
+            const u64* row = T.sm + t * 3 * T.stride + T.off;
+            u64* dst = T.sm + t * 3 * T.stride + out;
+            F3 lo, hi, v;
+            lo.c0 = row[j]; hi.c0 = row[j + half];
+            if (base) {
+                lo.c1 = lo.c2 = hi.c1 = hi.c2 = 0;
+                v = f3_fold<false, true>(lo, hi, m);
+            } else {
+                lo.c1 = row[T.stride + j]; lo.c2 = row[2 * T.stride + j];
+                hi.c1 = row[T.stride + j + half]; hi.c2 = row[2 * T.stride + j + half];
+                v = f3_fold<true, true>(lo, hi, m);
             }
+            dst[j] = v.c0; dst[T.stride + j] = v.c1; dst[2 * T.stride + j] = v.c2;
+            put(t, 0, j, v.c0); put(t, 1, j, v.c1); put(t, 2, j, v.c2);
         }
+        return;
     }
-    if (lane == 0) {
-#pragma unroll
-        for (int i = 0; i < NRAW; i++) { sh.red[warp][3 * i] = raw[i].c0; sh.red[warp][3 * i + 1] = raw[i].c1; sh.red[warp][3 * i + 2] = raw[i].c2; }
-    }
-    __syncthreads();
-    if (warp == 0 && lane < NW3) {
-        u64 v = 0;
-#pragma unroll
-        for (int q = 0; q < TAIL_NW; q++) v = gl_add(v, sh.red[q][lane]);
-        sh.tot[lane] = v;
+    // one component of one entry per thread and step, j fastest
+    const u32 lg = tail_lg(half);
+    for (u32 i = threadIdx.x; i < NT * FW * half; i += TAIL_TPB) {
+        const u32 r = i >> lg;                        // t FW + c
+        const int t = NT > 1 && r >= FW ? 1 : 0, c = (int)r - t * FW;
+        const u32 j = i & (half - 1);
+        const u64 v = tail_fold_comp<FW>(T.sm + t * FW * T.stride + T.off, T.stride, j, half, c, ch);
+        T.sm[r * T.stride + out + j] = v;
+        put(t, c, j, v);
     }
 }
 
-// Transcript step of round k in warp 0 (src/runner.rs:39-55): send the wire
-// values in sh.tot, absorb the hook, squeeze the challenge into sh.chal and
-// record both in the proof.
-template <int POL>
-__device__ __forceinline__ void tail_transcript(WarpTx& w, const TailArgs& a, u32 k, TailShared& sh) {
-    constexpr int NWIRE = POL == POL_ML ? 1 : 2;
-    const int lane = threadIdx.x & 31;
-    tx_send_elems(w, lane, sh.tot, NWIRE);
-    if (a.hook_len) {
-        const uint8_t* hk = a.hook;
-        if (((w.pos & 7) == 0 || w.squeezing) && (a.hook_len & 7) == 0 && ((uintptr_t)hk & 7) == 0) {
-            const u64* hw = (const u64*)hk;
-            tx_absorb_words(w, lane, a.hook_len >> 3, [&](u32 i) -> u64 { return hw[i]; });
-        } else {
-            tx_absorb(w, lane, a.hook_len, [&](u32 i) -> uint8_t { return hk[i]; });
-        }
-    }
-    tx_challenge(w, lane, sh.chal, sh.scr);
-    if (lane < 3 * NWIRE) a.proof_wire[(u64)k * 3 * NWIRE + lane] = sh.tot[lane];
-    if (lane < 3) a.proof_chal[(u64)k * 3 + lane] = sh.chal[lane];
-}
-
-// After the last round: store the transcript state, apply the runner's
-// finalize fold, write the read-back entries and the folded tables.
+// The warps' work on the round polynomial, NWIRE values of FW components:
+//   InnerProduct: q0 = sum a_lo b_lo, qinf = sum (a_hi - a_lo)(b_hi - b_lo)
+//   (src/provers/inner_product.rs:94-103); Multilinear: the wire is
+//   s0 = sum lo alone (src/provers/multilinear.rs:52-61).
+// The warps divide into roles with WPR warps each, slot s of a role taking the
+// entries 32 s + lane, + 32 WPR, ...:
+//   TERM  (IP over Fp3, at most 32 pairs) one product: x_k y_m of value
+//         `which`, m = (c - k) mod 3, its y times W where the index wraps;
+//   ROW   (IP over Fp3) x_k with all three y_m;
+//   VALUE (Fp, or Fp3 before base tables' first fold) a whole value; ML over
+//         Fp3: one component of it.
+// Every sum goes to sh.part, those of a wire word next to each other, wire word `word` is the sum of its TERMS x slots entries.
 template <int POL, int FW>
-__device__ __forceinline__ void tail_finish(u64* smb, u64 stride, u64 len, const TailArgs& a, WarpTx& w, TailShared& sh) {
+struct TailRoles {
+    static constexpr int NWIRE = POL == POL_ML ? 1 : 2;
+    static constexpr int N = NWIRE * FW;                  // wire words
+    static constexpr bool ROWS = POL == POL_IP && FW == 3;
+    static constexpr int WPR = TAIL_NW / N, WPR_BASE = TAIL_NW / NWIRE;
+};
+
+// A round's sums over the current tables into sh.part; returns how many
+// slots of each role held entries.
+template <int POL, int FW>
+__device__ __forceinline__ u32 tail_eval(const TailTab& T, bool base, TailShared& sh) {
+    using R = TailRoles<POL, FW>;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const u32 half = T.len > 1 ? T.len >> 1 : 1;         // a single entry feeds h(0) alone
+    const u64* a = T.sm + T.off;
+    const u64* b = a + FW * T.stride;
+    if (R::ROWS && !base && half <= 32) {
+        // TERM
+        const int word = warp / 3, k = warp - 3 * word, which = word >= 3, c = word - 3 * which;
+        if (word < 6) {
+            const int m = c - k + (k > c ? 3 : 0);
+            u64 v = 0;
+            if (lane < (int)half && (T.len > 1 || !which)) {
+                const u64 *pa = a + k * T.stride + lane, *pb = b + m * T.stride + lane;
+                u64 x = pa[0], y = pb[0];
+                if (which) { x = gl_sub(pa[half], x); y = gl_sub(pb[half], y); }
+                if (k > c) y = gl_mul_w(y);
+                v = gl_mul(x, y);
+            }
+            __syncwarp();
+            const uint4 p = warp_sum_pieces(v);
+            if (lane == 0) sh.part[warp] = p;
+        }
+        return 1;
+    }
+    const u32 wpr = base ? R::WPR_BASE : R::WPR;
+    const u32 role = base ? warp / R::WPR_BASE : warp / R::WPR, slot = warp - role * wpr;
+    const u32 slots = min(wpr, (half + 31) >> 5);
+    if (slot >= slots) return slots;
+    const u32 j0 = slot * 32 + lane, step = 32 * wpr;
+    if (R::ROWS && !base) {
+        const u32 which = role >= 3, k = role - 3 * which;
+        AccF<0> s[3];
+#pragma unroll
+        for (int o = 0; o < 3; o++) s[o].zero();
+        const u64* ak = a + k * T.stride;
+        for (u32 j = j0; j < half; j += step) {
+            u64 x = ak[j], y[3];
+#pragma unroll
+            for (int o = 0; o < 3; o++) y[o] = b[o * T.stride + j];
+            if (which) {
+                x = gl_sub(ak[j + half], x);
+#pragma unroll
+                for (int o = 0; o < 3; o++) y[o] = gl_sub(b[o * T.stride + j + half], y[o]);
+            }
+#pragma unroll
+            for (int o = 0; o < 3; o++) s[o].mac(x, y[o]);
+        }
+#pragma unroll
+        for (int o = 0; o < 3; o++) {
+            const bool wrap = k + o >= 3;
+            u64 v = s[o].reduce();
+            if (wrap) v = gl_mul_w(v);
+            const uint4 p = warp_sum_pieces(v);
+            // wire word 3 which + (k + o) mod 3, its term k
+            if (lane == 0) sh.part[((3 * which + k + o - (wrap ? 3 : 0)) * 3 + k) * slots + slot] = p;
+        }
+        return slots;
+    }
+    Acc s = acc_zero();
+    for (u32 j = j0; j < half; j += step) {
+        if (POL == POL_ML) {
+            acc_add64(s, a[role * T.stride + j]);
+        } else {
+            u64 x = a[j], y = b[j];
+            if (role) {
+                x = T.len > 1 ? gl_sub(a[j + half], x) : 0;
+                y = T.len > 1 ? gl_sub(b[j + half], y) : 0;
+            }
+            acc_mac(s, x, y);
+        }
+    }
+    const uint4 p = warp_sum_pieces(acc_reduce(s));
+    if (lane == 0) sh.part[role * slots + slot] = p;
+    return slots;
+}
+// Wire word (which FW + c) from sh.part, in that lane; 0 in the others.
+template <int POL, int FW>
+__device__ __forceinline__ u64 tail_total(const TailShared& sh, int lane, bool base, u32 slots) {
+    using R = TailRoles<POL, FW>;
+    u64 v = 0;
+    if (lane < R::N && !(base && lane % FW)) {
+        const u32 n = R::ROWS && !base ? 3 * slots : slots;
+        const uint4* q = sh.part + (base ? lane / FW : lane) * n;
+        uint4 s = q[0];
+        for (u32 i = 1; i < n; i++) {
+            const uint4 p = q[i];
+            s.x += p.x; s.y += p.y; s.z += p.z;
+        }
+        v = join_pieces(s);
+    }
+    __syncwarp();
+    return v;
+}
+
+// The transcript of a tail, in warp 0: its state and, per lane, the words
+// that every round absorbs after the wire values (the hook, the padding).
+struct TailTx {
+    WarpTx w;
+    u64 fixed;
+    bool fast;        // wire, hook and padding fit one block, in whole words
+};
+template <int NW>
+__device__ __forceinline__ void tail_tx_init(TailTx& x, const TailArgs& a, int lane) {
+    x.w = tx_load((const DevTranscript*)a.tx, lane);
+    x.fast = (a.hook_len & 7) == 0 && ((uintptr_t)a.hook & 7) == 0 && 8 * NW + a.hook_len < TX_RATE;
+    x.fixed = 0;
+    if (x.fast) {
+        const int hw = (int)(a.hook_len >> 3);
+        if (lane >= NW && lane < NW + hw) x.fixed = ((const u64*)a.hook)[lane - NW];
+        if (lane == NW + hw) x.fixed ^= 0x06;
+        if (lane == TX_RATE / 8 - 1) x.fixed ^= 0x80ULL << 56;
+    }
+}
+// The transcript step of a round (src/runner.rs:39-55): send the wire values
+// (word i of them in lane i), absorb the hook, squeeze the challenge into
+// sh.chal, prepared.  After the first round the transcript is always at a
+// squeeze, so the wire, the hook and the padding make one block of whole
+// words: one xor per lane, the permutation, and the challenge straight from
+// the lanes that hold it.
+template <int POL, int FW>
+__device__ __forceinline__ void tail_transcript(TailTx& x, u64 wire, const TailArgs& a, TailShared& sh) {
+    constexpr int NWIRE = TailRoles<POL, FW>::NWIRE, NW = TailRoles<POL, FW>::N;
+    const int lane = threadIdx.x & 31;
+    if (lane < NW) sh.tot[FW == 3 ? lane : 3 * lane] = wire;
+    u64 r;
+    __syncwarp();
+    if (x.fast && x.w.squeezing) {
+        x.w.a ^= x.fixed ^ wire;
+        keccak_f_warp(x.w.a, lane);
+        x.w.pos = 16 * FW;
+        const u64 lo = shfl64(x.w.a, (2 * lane) & 31), hi = shfl64(x.w.a, (2 * lane + 1) & 31);
+        r = lane < FW ? gl_reduce128(lo, hi) : 0;
+    } else {
+        tx_send_elems(x.w, lane, sh.tot, NWIRE);
+        if (a.hook_len) {
+            const uint8_t* hk = a.hook;
+            tx_absorb(x.w, lane, a.hook_len, [&](u32 i) -> uint8_t { return hk[i]; });
+        }
+        tx_challenge(x.w, lane, sh.raw, sh.scr);
+        r = lane < 3 ? sh.raw[lane] : 0;
+    }
+    if (lane < 3) sh.chal[2 + lane] = r;
+    if (FW == 3 && (lane == 1 || lane == 2)) sh.chal[lane - 1] = gl_mul_w(r);
+}
+// Round k's wire values and challenge into the proof, by the last warp after
+// the barrier that publishes them (the next round changes them two barriers
+// later).
+template <int POL, int FW>
+__device__ __forceinline__ void tail_record(const TailArgs& a, u32 k, const TailShared& sh) {
+    constexpr u32 NW3 = 3 * TailRoles<POL, FW>::NWIRE;
+    const u32 i = threadIdx.x - (TAIL_TPB - 32);
+    if (i < NW3) a.proof_wire[k * NW3 + i] = FW == 3 || i % 3 == 0 ? sh.tot[i] : 0;
+    else if (i >= 8 && i < 11) a.proof_chal[3 * k + i - 8] = sh.chal[i - 6];
+}
+
+// The challenge before the first round, prepared (or zeros).
+template <int FW>
+__device__ __forceinline__ void tail_first_challenge(const TailArgs& a, TailShared& sh) {
+    if (threadIdx.x < 3) {
+        const u64 r = a.first_fold ? a.chal_in[threadIdx.x] : 0;
+        sh.chal[2 + threadIdx.x] = r;
+        if (threadIdx.x) sh.chal[threadIdx.x - 1] = gl_mul_w(r);
+    }
+}
+
+// The next fold's destination: the half of the rows the table is not in.
+__device__ __forceinline__ u32 tail_next_off(const TailTab& T) {
+    return T.len == T.stride ? T.off : T.off ? 0 : T.stride >> 1;
+}
+
+// Rounds k0 .. a.nrounds-1 in one block, then the transcript state, the
+// runner's finalize fold, the read-back entries and the folded tables.
+template <int POL, int FW>
+__device__ __forceinline__ void tail_loop(TailTab T, u32 k0, bool fold, bool base, const TailArgs& a, TailTx& x,
+                                          TailShared& sh) {
     constexpr int NT = Policy<POL, 0>::NT;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (warp == 0) tx_store((DevTranscript*)a.tx, w, lane);
-    if (a.final_fold && len >= 2) {
+    for (u32 k = k0; k < a.nrounds; k++) {
+        if (fold) {
+            const u32 out = tail_next_off(T);
+            tail_fold<NT, FW>(T, out, base, sh.chal, [](int, int, u32, u64) {});
+            T.off = out;
+            T.len >>= 1;
+            base = false;
+            __syncthreads();
+        }
+        const u32 slots = tail_eval<POL, FW>(T, base, sh);
+        __syncthreads();
+        if (warp == 0) tail_transcript<POL, FW>(x, tail_total<POL, FW>(sh, lane, base, slots), a, sh);
+        __syncthreads();
+        tail_record<POL, FW>(a, k, sh);
+        fold = true;
+    }
+    if (warp == 0) tx_store((DevTranscript*)a.tx, x.w, lane);
+    if (a.final_fold && T.len >= 2) {
         // SumcheckProver::finalize with the last challenge: one MSB fold
         // (src/inner_product_sumcheck.rs:143-176, src/multilinear_sumcheck.rs:132-178)
-        constexpr bool E = FW == 3;
-        const Mul3 m = mul3_prepare<E>(f3_make(sh.chal[0], sh.chal[1], sh.chal[2]));
-        const u64 half = len >> 1;
-        for (u64 j = threadIdx.x; j < half; j += TAIL_TPB)
-#pragma unroll
-            for (int t = 0; t < NT; t++)
-                sm_st<FW>(smb, stride, t, j, f3_fold<E, E>(sm_ld<FW>(smb, stride, t, j), sm_ld<FW>(smb, stride, t, j + half), m));
+        const u32 out = tail_next_off(T);
+        tail_fold<NT, FW>(T, out, base, sh.chal, [](int, int, u32, u64) {});
+        T.off = out;
+        T.len >>= 1;
         __syncthreads();
-        len = half;
     }
     if (a.first_out && threadIdx.x < 12) {
         const int t = threadIdx.x / 3, c = threadIdx.x % 3;
-        a.first_out[threadIdx.x] = (t < NT && c < FW) ? smb[(u64)(t * FW + c) * stride] : 0;
+        a.first_out[threadIdx.x] = (t < NT && c < FW) ? T.sm[(t * FW + c) * T.stride + T.off] : 0;
     }
     // write back the tables after the last fold (LSB: from the reversed layout)
     if (a.out[0][0]) {
-        const u32 lg = tail_lg(len);
+        const u32 lg = tail_lg(T.len);
         for (int t = 0; t < NT; t++)
             for (int c = 0; c < FW; c++) {
-                const u64* src = smb + (u64)(t * FW + c) * stride;
+                const u64* src = T.sm + (t * FW + c) * T.stride + T.off;
                 u64* dst = a.out[t][c];
-                for (u64 i = threadIdx.x; i < len; i += TAIL_TPB) dst[i] = src[a.lsb ? tail_rev(i, lg) : i];
+                for (u32 i = threadIdx.x; i < T.len; i += TAIL_TPB) dst[i] = src[a.lsb ? tail_rev(i, lg) : i];
             }
     }
 }
 
-// Rounds k0 .. a.nrounds-1 in one block on tables of length `len` at smb
-// (table t, component c, element i at smb[(t*FW + c)*stride + i]); then the
-// folded tables go back to global memory and the transcript state is stored.
+// One block: rows of the starting length.  Warp 0 keeps the transcript state
+// in registers for the whole tail.
 template <int POL, int FW>
-__device__ void tail_loop(u64* smb, u64 stride, u64 len, u32 k0, bool fold, const TailArgs& a, WarpTx& w,
-                          TailShared& sh) {
-    constexpr int NT = Policy<POL, 0>::NT;
-    constexpr u32 MF = FW == 3 ? (1u << NT) - 1 : 0;
-    using P = Policy<POL, MF>;
-    const int warp = threadIdx.x >> 5;
-    for (u32 k = k0; k < a.nrounds; k++) {
-        // warps without entries this round skip the arithmetic and the
-        // reduction of their (zero) sums; every warp reaches both barriers
-        const u64 nwork = fold ? (len >> 2) : len == 1 ? 1 : (len >> 1);
-        const bool active = (u64)warp * 32 < nwork;
-        P acc;
-        F3 raw[P::NRAW];
-#pragma unroll
-        for (int i = 0; i < P::NRAW; i++) raw[i] = f3_zero();
-        if (active) {
-            acc.init();
-            F3 lo[NT], hi[NT];
-            if (fold) {
-                tail_fold_eval<POL, FW>(smb, stride, len, sh.chal, acc, [&](int t, u64 q, u64 Q, const F3& l, const F3& h) {
-                    sm_st<FW>(smb, stride, t, q, l);
-                    sm_st<FW>(smb, stride, t, q + Q, h);
-                });
-            } else if (len == 1) {
-                if (threadIdx.x == 0) {
-#pragma unroll
-                    for (int t = 0; t < NT; t++) lo[t] = sm_ld<FW>(smb, stride, t, 0);
-                    acc.single(lo);
-                }
-            } else {
-                const u64 half = len >> 1;
-                for (u64 j = threadIdx.x; j < half; j += TAIL_TPB) {
-#pragma unroll
-                    for (int t = 0; t < NT; t++) { lo[t] = sm_ld<FW>(smb, stride, t, j); hi[t] = sm_ld<FW>(smb, stride, t, j + half); }
-                    acc.pair(lo, hi);
-                }
-            }
-            acc.result(raw);
-        }
-        if (fold) len >>= 1;
-        tail_block_reduce<P::NRAW>(raw, active, sh);
-        if (warp == 0) {
-            __syncwarp();
-            tail_transcript<POL>(w, a, k, sh);
-        }
-        __syncthreads();
-        fold = true;
-    }
-    tail_finish<POL, FW>(smb, stride, len, a, w, sh);
-}
-
-// Shared-memory layout: table t, component c, element i at sm[(t*FW + c)*L0 + i]
-// with L0 the starting length (rows keep their stride as the tables shrink).
-// Warp 0 keeps the transcript state in registers for the whole tail and the
-// challenge stays in shared memory, so a round costs one block reduction and
-// one transcript step.
-template <int POL, int FW>
-__device__ void tail_body(const TailArgs& a) {
+__device__ __forceinline__ void tail_body(const TailArgs& a) {
     extern __shared__ __align__(16) u64 sm[];
     constexpr int NT = Policy<POL, 0>::NT;
     __shared__ TailShared sh;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const u64 L0 = a.L;
-    const u32 lg0 = tail_lg(L0);
+    const u32 L0 = (u32)a.L, lg0 = tail_lg(L0);
     for (int t = 0; t < NT; t++)
         for (int c = 0; c < FW; c++) {
             const u64* src = (c == 0 || ((a.in_ext >> t) & 1u)) ? a.in[t][c] : nullptr;
-            u64* dst = sm + (u64)(t * FW + c) * L0;
-            for (u64 i = threadIdx.x; i < L0; i += TAIL_TPB) dst[a.lsb ? tail_rev(i, lg0) : i] = src ? src[i] : 0;
+            u64* dst = sm + (t * FW + c) * L0;
+            for (u32 i = threadIdx.x; i < L0; i += TAIL_TPB) dst[a.lsb ? tail_rev(i, lg0) : i] = src ? src[i] : 0;
         }
-    if (threadIdx.x < 3) sh.chal[threadIdx.x] = a.first_fold ? a.chal_in[threadIdx.x] : 0;
-    WarpTx w;
-    if (warp == 0) w = tx_load((const DevTranscript*)a.tx, lane);
+    tail_first_challenge<FW>(a, sh);
+    TailTx x;
+    if (warp == 0) tail_tx_init<TailRoles<POL, FW>::N>(x, a, lane);
     __syncthreads();
-    tail_loop<POL, FW>(sm, L0, L0, 0, a.first_fold != 0, a, w, sh);
+    TailTab T{sm, L0, 0, L0};
+    tail_loop<POL, FW>(T, 0, a.first_fold != 0, FW == 3 && a.in_ext == 0, a, x, sh);
 }
 
 // ---- cluster tail ---------------------------------------------------------
-// Tables up to CS times one block's capacity: a thread-block cluster of CS
-// CTAs holds them in distributed shared memory, CTA c the groups of G = 16
-// consecutive entries whose group index is c mod CS: entry k with
-// (k / G) mod CS = c at local index (k / (G CS)) G + k mod G.  The slices
-// load as whole 128-byte lines, and MSB pairs (k, k + L/2) are local pairs
-// (j, j + L/(2 CS)) while L/2 is a multiple of G CS, so each CTA folds and
-// evaluates its slice exactly as the one-block tail does; the CTAs' sums meet in CTA 0 (distributed
-// shared memory stores), which runs the transcript step and writes the
-// challenge back into every CTA.  After log2(CS) + 1 rounds the last fold
-// writes the table (now half a slice long) straight into CTA 0, which
-// finishes the proof alone.  Every CTA passes the same 1 + 2 (log2(CS) + 1)
-// cluster barriers.
-constexpr u64 CL_G = 16;
+// Tables up to CS times one block's capacity, and smaller ones whose first
+// rounds are worth sharing: a thread-block cluster of CS CTAs holds them in
+// distributed shared memory.  MSB: CTA c holds the groups of G consecutive
+// entries whose group index is c mod CS: entry k with (k / G) mod CS = c at
+// local index (k / (G CS)) G + k mod G; the slices load as whole sectors
+// (G = 16: lines), and pairs (k, k + L/2) are local pairs (j, j + L/(2 CS))
+// while L/2 is a multiple of G CS.  LSB: CTA c holds the entries c Ll ..
+// (c + 1) Ll - 1 bit-reversed among themselves, so its first log2(Ll) folds
+// are local too.  Each CTA folds and evaluates its slice exactly as the
+// one-block tail does; the CTAs' sums meet in CTA 0 (distributed shared
+// memory stores), which runs the transcript step and writes the challenge
+// back into every CTA.  Fold log2(CS) + 1 also writes the table (now half a
+// slice long) into CTA 0's free half, which finishes the proof alone.  Every
+// CTA passes the same cluster barriers, two per round.
 // Global index of local entry j of CTA c.
-__device__ __forceinline__ u64 cl_global(u64 j, u32 c, u32 cs_log) {
-    return (((j / CL_G) << cs_log) + c) * CL_G + (j % CL_G);
+__device__ __forceinline__ u32 cl_global(u32 j, u32 c, u32 cs_log, u32 g_log) {
+    return ((((j >> g_log) << cs_log) + c) << g_log) + (j & ((1u << g_log) - 1));
 }
 __device__ __forceinline__ u32 cluster_rank() {
     u32 r;
@@ -282,160 +440,84 @@ __device__ __forceinline__ void dsmem_st(const void* p, u32 rank, u64 v) {
     asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(remote), "l"(v) : "memory");
 }
 
-// The H = log2(CS) + 1 cluster rounds of k_tail_cluster as separate loops
-// (Multilinear: its cheap rounds measured faster this way, with CTA 0 going
-// on in tail_loop, than in the one loop InnerProduct uses: n = 20, 168
-// against 178 us per proof); the last fold hands the table to CTA 0.
 template <int POL, int FW>
-__device__ __forceinline__ void tail_cluster_rounds(u64* sm, u64 Ll, u64& len, u32 cs_log, u32 rank, const TailArgs& a,
-                                                    WarpTx& w, TailShared& sh) {
-    constexpr int NT = Policy<POL, 0>::NT;
-    constexpr u32 MF = FW == 3 ? (1u << NT) - 1 : 0;
-    using P = Policy<POL, MF>;
-    constexpr int NW3 = 3 * P::NRAW;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const u32 CS = 1u << cs_log, H = cs_log + 1;
-    for (u32 k = 0; k < H; k++) {
-        const u64 ll = len >> cs_log;      // slice length this round (>= 4)
-        const bool last = k + 1 == H;
-        P acc;
-        acc.init();
-        F3 raw[P::NRAW];
-        if (!last) {
-            tail_fold_eval<POL, FW>(sm, Ll, ll, sh.chal, acc, [&](int t, u64 q, u64 Q, const F3& l, const F3& h) {
-                sm_st<FW>(sm, Ll, t, q, l);
-                sm_st<FW>(sm, Ll, t, q + Q, h);
-            });
-        } else {
-            // the folded table (L0 / 2^H = Ll / 2 entries) goes to CTA 0's
-            // rows from offset Ll / 2 on, at its global index
-            tail_fold_eval<POL, FW>(sm, Ll, ll, sh.chal, acc, [&](int t, u64 q, u64 Q, const F3& l, const F3& h) {
-                const u64 g_lo = cl_global(q, rank, cs_log), g_hi = cl_global(q + Q, rank, cs_log);
-                u64* row = sm + (u64)(t * FW) * Ll + Ll / 2;
-                dsmem_st(row + g_lo, 0, l.c0);
-                dsmem_st(row + g_hi, 0, h.c0);
-                if (FW == 3) {
-                    dsmem_st(row + Ll + g_lo, 0, l.c1);
-                    dsmem_st(row + Ll + g_hi, 0, h.c1);
-                    dsmem_st(row + 2 * Ll + g_lo, 0, l.c2);
-                    dsmem_st(row + 2 * Ll + g_hi, 0, h.c2);
-                }
-            });
-        }
-        acc.result(raw);
-        len >>= 1;
-        tail_block_reduce<P::NRAW>(raw, true, sh);
-        if (warp == 0 && lane < NW3) dsmem_st(&sh.cred[rank][lane], 0, sh.tot[lane]);
-        cluster_sync_all();   // all CTAs' sums (and in the last round the table) are in CTA 0
-        if (rank == 0 && warp == 0) {
-            if (lane < NW3) {
-                u64 v = 0;
-                for (u32 c = 0; c < CS; c++) v = gl_add(v, sh.cred[c][lane]);
-                sh.tot[lane] = v;
-            }
-            __syncwarp();
-            tail_transcript<POL>(w, a, k, sh);
-            __syncwarp();
-            if (lane >= 1 && (u32)lane < CS)
-                for (int c = 0; c < 3; c++) dsmem_st(&sh.chal[c], (u32)lane, sh.chal[c]);
-        }
-        cluster_sync_all();   // the challenge is in every CTA
-    }
-}
-
-template <int POL, int FW>
-__global__ void __launch_bounds__(TAIL_TPB, 1) k_tail_cluster(TailArgs a, u32 cs_log) {
+__global__ void __launch_bounds__(TAIL_TPB, 1) k_tail_cluster(TailArgs a, u32 cs_log, u32 g_log) {
     extern __shared__ __align__(16) u64 sm[];
     constexpr int NT = Policy<POL, 0>::NT;
-    constexpr u32 MF = FW == 3 ? (1u << NT) - 1 : 0;
-    using P = Policy<POL, MF>;
-    constexpr int NW3 = 3 * P::NRAW;
+    constexpr int NW = TailRoles<POL, FW>::N;
     __shared__ TailShared sh;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const u32 CS = 1u << cs_log, rank = cluster_rank();
-    const u64 L0 = a.L, Ll = L0 >> cs_log;   // slice length (row stride)
+    const u32 Ll = (u32)(a.L >> cs_log);     // slice length (row stride)
+    const u32 lgl = tail_lg(Ll);
     // this CTA's slice; base tables are embedded when the field is Fp3
     for (int t = 0; t < NT; t++)
         for (int c = 0; c < FW; c++) {
             const u64* src = (c == 0 || ((a.in_ext >> t) & 1u)) ? a.in[t][c] : nullptr;
-            u64* dst = sm + (u64)(t * FW + c) * Ll;
-            for (u64 j = threadIdx.x; j < Ll; j += TAIL_TPB) dst[j] = src ? src[cl_global(j, rank, cs_log)] : 0;
+            u64* dst = sm + (t * FW + c) * Ll;
+            if (a.lsb)
+                for (u32 j = threadIdx.x; j < Ll; j += TAIL_TPB) dst[tail_rev(j, lgl)] = src ? src[rank * Ll + j] : 0;
+            else
+                for (u32 j = threadIdx.x; j < Ll; j += TAIL_TPB) dst[j] = src ? src[cl_global(j, rank, cs_log, g_log)] : 0;
         }
-    if (threadIdx.x < 3) sh.chal[threadIdx.x] = a.chal_in[threadIdx.x];
-    WarpTx w;
-    if (rank == 0 && warp == 0) w = tx_load((const DevTranscript*)a.tx, lane);
+    tail_first_challenge<FW>(a, sh);
+    TailTx x;
+    if (rank == 0 && warp == 0) tail_tx_init<NW>(x, a, lane);
     cluster_sync_all();   // every CTA is running before any remote store
-    // InnerProduct: every round runs the same loop body, the cluster rounds
-    // (k < H) and CTA 0's rounds after them -- one copy of the fold,
-    // reduction and transcript code, already in the SM's instruction cache
-    // when CTA 0 goes on alone (a separate copy measured ~15 us for CTA 0's
-    // first round against ~3 us for the next ones; n = 26: 0.170 -> 0.156 ms
-    // for the tail).
-    const u32 H = cs_log + 1;
-    u64 len = L0;
-    if constexpr (POL != POL_IP) {
-        tail_cluster_rounds<POL, FW>(sm, Ll, len, cs_log, rank, a, w, sh);
-        if (rank != 0) return;    // no remote access to this CTA follows
-        tail_loop<POL, FW>(sm + Ll / 2, Ll, len, H, true, a, w, sh);
-    } else {
-        for (u32 k = 0; k < a.nrounds; k++) {
-            const bool cl = k < H;             // a cluster round: every CTA
-            if (!cl && rank != 0) break;       // the others are done (no remote access to them follows)
-            const bool handoff = k + 1 == H;   // the fold goes to CTA 0's rows
-            u64* smb = cl ? sm : sm + Ll / 2;  // CTA 0 continues on rows from offset Ll / 2
-            const u64 ll = cl ? len >> cs_log : len;   // entries per row this round (>= 4 in cluster rounds)
-            const bool active = (u64)warp * 32 < (ll >> 2);
-            P acc;
-            F3 raw[P::NRAW];
-    #pragma unroll
-            for (int i = 0; i < P::NRAW; i++) raw[i] = f3_zero();
-            if (active) {
-                acc.init();
-                tail_fold_eval<POL, FW>(smb, Ll, ll, sh.chal, acc, [&](int t, u64 q, u64 Q, const F3& l, const F3& h) {
-                    if (!handoff) {
-                        sm_st<FW>(smb, Ll, t, q, l);
-                        sm_st<FW>(smb, Ll, t, q + Q, h);
-                        return;
-                    }
-                    // the folded table (L0 / 2^H = Ll / 2 entries) goes to CTA
-                    // 0's rows from offset Ll / 2 on, at its global index
-                    const u64 g_lo = cl_global(q, rank, cs_log), g_hi = cl_global(q + Q, rank, cs_log);
-                    u64* row = sm + (u64)(t * FW) * Ll + Ll / 2;
-                    dsmem_st(row + g_lo, 0, l.c0);
-                    dsmem_st(row + g_hi, 0, h.c0);
-                    if (FW == 3) {
-                        dsmem_st(row + Ll + g_lo, 0, l.c1);
-                        dsmem_st(row + Ll + g_hi, 0, h.c1);
-                        dsmem_st(row + 2 * Ll + g_lo, 0, l.c2);
-                        dsmem_st(row + 2 * Ll + g_hi, 0, h.c2);
-                    }
+    TailTab T{sm, Ll, 0, Ll};
+    bool base = FW == 3 && a.in_ext == 0, fold = a.first_fold != 0;
+    u32 gather = 0, left = cs_log + 1;       // folds to the hand-over
+    u32 k = 0;
+    for (; left; k++) {
+        if (fold) {
+            u32 out = tail_next_off(T);
+            if (--left) {
+                tail_fold<NT, FW>(T, out, base, sh.chal, [](int, int, u32, u64) {});
+            } else {
+                // the whole folded table goes to the free half of CTA 0's rows,
+                // at its global (LSB: globally bit-reversed) index; the slice
+                // itself is folded next to its source, into the half that holds
+                // it (Ll / CS entries there, half of that written, CS >= 4)
+                gather = out;
+                out = T.off + T.len;
+                const u32 rrev = tail_rev(rank, cs_log);
+                tail_fold<NT, FW>(T, out, base, sh.chal, [&](int t, int c, u32 j, u64 v) {
+                    const u32 g = a.lsb ? (j << cs_log) + rrev : cl_global(j, rank, cs_log, g_log);
+                    dsmem_st(sm + (t * FW + c) * Ll + gather + g, 0, v);
                 });
-                acc.result(raw);
             }
-            len >>= 1;
-            tail_block_reduce<P::NRAW>(raw, active, sh);
-            if (cl) {
-                if (warp == 0 && lane < NW3) dsmem_st(&sh.cred[rank][lane], 0, sh.tot[lane]);
-                cluster_sync_all();   // all CTAs' sums (and after the hand-off the table) are in CTA 0
-            }
-            if (rank == 0 && warp == 0) {
-                if (cl && lane < NW3) {
-                    u64 v = 0;
-                    for (u32 c = 0; c < CS; c++) v = gl_add(v, sh.cred[c][lane]);
-                    sh.tot[lane] = v;
-                }
-                __syncwarp();
-                tail_transcript<POL>(w, a, k, sh);
-                __syncwarp();
-                if (cl && lane >= 1 && (u32)lane < CS)
-                    for (int c = 0; c < 3; c++) dsmem_st(&sh.chal[c], (u32)lane, sh.chal[c]);
-            }
-            if (cl) cluster_sync_all();   // the challenge is in every CTA
-            else __syncthreads();
+            T.off = out;
+            T.len >>= 1;
+            base = false;
+            __syncthreads();
         }
-        if (rank != 0) return;
-        tail_finish<POL, FW>(sm + Ll / 2, Ll, len, a, w, sh);
+        fold = true;
+        const u32 slots = tail_eval<POL, FW>(T, base, sh);
+        __syncthreads();
+        if (warp == 0) {
+            const u64 v = tail_total<POL, FW>(sh, lane, base, slots);
+            if (lane < NW) dsmem_st(&sh.cred[rank][lane], 0, v);
+        }
+        cluster_sync_all();   // all CTAs' sums (and at the hand-over the table) are in CTA 0
+        if (rank == 0 && warp == 0) {
+            u64 wire = 0;
+            if (lane < NW) {
+                Acc v = acc_zero();
+                for (u32 c = 0; c < CS; c++) acc_add64(v, sh.cred[c][lane]);
+                wire = acc_reduce(v);
+            }
+            tail_transcript<POL, FW>(x, wire, a, sh);
+            __syncwarp();
+            if (lane >= 1 && (u32)lane < CS)
+                for (int c = 0; c < 5; c++) dsmem_st(&sh.chal[c], (u32)lane, sh.chal[c]);
+        }
+        cluster_sync_all();   // the challenge is in every CTA
+        if (rank == 0) tail_record<POL, FW>(a, k, sh);
     }
+    if (rank != 0) return;    // no remote access to this CTA follows
+    T.off = gather;
+    T.len = Ll >> 1;
+    tail_loop<POL, FW>(T, k, true, false, a, x, sh);
 }
 
 template <int POL, int FW>
@@ -468,7 +550,7 @@ static bool tail_inst(const TailArgs* dev_args, const TailArgs* one, u32 n, u64 
 }
 
 template <int POL, int FW>
-static bool tail_cluster_inst(const TailArgs& a, u32 cs_log, cudaStream_t s) {
+static bool tail_cluster_inst(const TailArgs& a, u32 cs_log, u32 g_log, cudaStream_t s) {
     const u32 CS = 1u << cs_log;
     const size_t bytes = (size_t)pol_ntables(POL) * FW * (a.L >> cs_log) * sizeof(u64);
     if (bytes > TAIL_SMEM_CAP || CS > (u32)TAIL_MAX_CS) return false;
@@ -486,7 +568,7 @@ static bool tail_cluster_inst(const TailArgs& a, u32 cs_log, cudaStream_t s) {
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_tail_cluster<POL, FW>, a, cs_log) == cudaSuccess;
+    return cudaLaunchKernelEx(&cfg, k_tail_cluster<POL, FW>, a, cs_log, g_log) == cudaSuccess;
 }
 
 // Largest cluster the device runs for the cluster tail (8 or 16 CTAs of
@@ -524,14 +606,35 @@ u32 tail_cluster_max(void) {
     return (u32)v;
 }
 
-bool launch_tail_cluster(int pol, int fw, const TailArgs& a, u32 cs_log, cudaStream_t s) {
+bool launch_tail_cluster(int pol, int fw, const TailArgs& a, u32 cs_log, u32 g_log, cudaStream_t s) {
     switch (pol * 4 + fw) {
-    case POL_ML * 4 + 1: return tail_cluster_inst<POL_ML, 1>(a, cs_log, s);
-    case POL_ML * 4 + 3: return tail_cluster_inst<POL_ML, 3>(a, cs_log, s);
-    case POL_IP * 4 + 1: return tail_cluster_inst<POL_IP, 1>(a, cs_log, s);
-    case POL_IP * 4 + 3: return tail_cluster_inst<POL_IP, 3>(a, cs_log, s);
+    case POL_ML * 4 + 1: return tail_cluster_inst<POL_ML, 1>(a, cs_log, g_log, s);
+    case POL_ML * 4 + 3: return tail_cluster_inst<POL_ML, 3>(a, cs_log, g_log, s);
+    case POL_IP * 4 + 1: return tail_cluster_inst<POL_IP, 1>(a, cs_log, g_log, s);
+    case POL_IP * 4 + 3: return tail_cluster_inst<POL_IP, 3>(a, cs_log, g_log, s);
     default: return false;
     }
+}
+
+// The split of a tail over a cluster: as many CTAs as the device runs and the
+// slices allow (at least 4), groups of 16 entries where the pairs stay in
+// their CTA to the hand-over, else of 4 (which also leaves LSB slices of
+// at least 4 entries there).
+bool tail_cluster_split(int pol, int fw, u64 L, u32 rounds, bool first_fold, u32* cs_log, u32* g_log) {
+    if (L < TAIL_CLUSTER_MIN || (L & (L - 1)) || L > (1u << 30)) return false;
+    const u64 cap = tail_max_len(pol, fw, TAIL_SMEM_CAP);
+    for (u32 lg = 4; lg >= 2; lg--) {
+        const u64 cs = 1ull << lg;
+        if (cs > tail_cluster_max() || L / cs > cap) continue;
+        const u64 last = L >> (lg + 2);          // half of the table handed over
+        if (last % (4 * cs) != 0) continue;
+        const u32 folds = rounds - (first_fold ? 0 : 1);
+        if (rounds < 1 || folds < lg + 1 || folds >= 63 || (L >> folds) < 2) continue;
+        *cs_log = lg;
+        *g_log = last % (16 * cs) == 0 ? 4 : 2;
+        return true;
+    }
+    return false;
 }
 
 bool launch_tail(int pol, int fw, const TailArgs* dev_args, const TailArgs* one, u32 n, u64 smem_len, cudaStream_t s) {

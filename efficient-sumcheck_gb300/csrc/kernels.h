@@ -176,8 +176,11 @@ constexpr u64 TAIL_SMEM_CAP = 200 * 1024;
 // One block per TailArgs; `smem_len` = largest L among them.
 bool launch_tail(int pol, int fw, const TailArgs* dev_args, const TailArgs* one, u32 n, u64 smem_len, cudaStream_t s);
 // Cluster tail: 2^cs_log CTAs hold a table of a.L entries (a.L >> cs_log per
-// CTA within TAIL_SMEM_CAP); needs a.first_fold = 1 and a.nrounds > cs_log + 1.
-bool launch_tail_cluster(int pol, int fw, const TailArgs& a, u32 cs_log, cudaStream_t s);
+// CTA within TAIL_SMEM_CAP) in groups of 2^g_log; needs cs_log + 1 folds.
+bool launch_tail_cluster(int pol, int fw, const TailArgs& a, u32 cs_log, u32 g_log, cudaStream_t s);
+// Whether (and how) `rounds` rounds on tables of L entries run that way.
+constexpr u64 TAIL_CLUSTER_MIN = 1 << 11;
+bool tail_cluster_split(int pol, int fw, u64 L, u32 rounds, bool first_fold, u32* cs_log, u32* g_log);
 // Largest cluster size the device runs for it (16, 8 or 0).
 u32 tail_cluster_max(void);
 

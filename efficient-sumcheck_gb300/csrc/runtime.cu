@@ -632,28 +632,26 @@ bool tail_ok(const effsc_prover* P, size_t r, size_t num_rounds, const Chal& ch)
     return folds < 63 && (L >> folds) >= 2;
 }
 
-// cluster tail: the same tables up to tail_cluster_max() times one block's
-// capacity, entered mid-proof (a challenge to fold with), with at least
-// log2(CS) + 1 rounds left; *cs_log = log2(CS), CS = L / capacity.
-bool cluster_tail_ok(const effsc_prover* P, size_t r, size_t num_rounds, const Chal& ch, u32* cs_log) {
-    // the tail's provers, MSB (the slices need MSB pairs)
-    if (tail_pol(P) < 0 || P->order != EFFSC_MSB || !P->tail_len) return false;
-    if (r >= num_rounds || !ch.has || !ch.dev) return false;
+// cluster tail: the same tables, up to tail_cluster_max() times one block's
+// capacity, in a thread-block cluster (tail_cluster_split chooses it).
+struct ClusterSplit {
+    u32 cs_log = 0, g_log = 0;
+};
+bool cluster_tail_ok(const effsc_prover* P, size_t r, size_t num_rounds, const Chal& ch, ClusterSplit* cl) {
+    if (tail_pol(P) < 0 || !P->tail_len) return false;
+    if (r >= num_rounds || num_rounds - r >= 63 || (ch.has && !ch.dev)) return false;
     const size_t L = P->t[0].len;
     for (int i = 1; i < P->ntab; i++)
         if (P->t[i].len != L) return false;
-    if (!is_pow2(L) || L > P->tail_len) return false;
-    const int fw = P->field == EFFSC_FP3 ? 3 : 1;
-    const size_t cap = (size_t)tail_max_len(tail_pol(P), fw, TAIL_SMEM_CAP);
-    if (L <= cap) return false;
-    const size_t cs = L / cap, csmax = tail_cluster_max();
-    if (cs > csmax || cs < 2 || cap < 32 * cs) return false;   // slices of whole 16-entry groups
-    u32 lg = 0;
-    while (((size_t)1 << lg) < cs) lg++;
-    const size_t rounds = num_rounds - r;
-    if (rounds < lg + 1 || rounds >= 63 || (L >> rounds) < 2) return false;
-    *cs_log = lg;
-    return true;
+    if (L > P->tail_len) return false;
+    return tail_cluster_split(tail_pol(P), P->field == EFFSC_FP3 ? 3 : 1, L, (u32)(num_rounds - r), ch.has, &cl->cs_log,
+                              &cl->g_log);
+}
+// Whether a whole proof runs in one tail launch: the two-pass starts leave it.
+bool whole_in_tail(const effsc_prover* P, size_t num_rounds) {
+    Chal none;
+    ClusterSplit cl;
+    return tail_ok(P, 0, num_rounds, none) || cluster_tail_ok(P, 0, num_rounds, none, &cl);
 }
 
 // Rounds r .. r + *nr - 1 of effsc_prove in one cooperative launch
@@ -674,9 +672,9 @@ bool persist_ok(const effsc_prover* P, size_t r, size_t num_rounds, const Chal& 
             if ((uintptr_t)T.bufs[T.cur].p[c] & 15) return false;
     }
     size_t lim = P->tail_len ? std::min<size_t>(P->tail_len, (size_t)tail_max_len(POL_IP, 3, TAIL_SMEM_CAP)) : 0;
-    // MSB: stop where the cluster tail takes over (tables of up to
+    // stop where the cluster tail takes over (tables of up to
     // tail_cluster_max() times the one-block capacity)
-    if (lim && P->order == EFFSC_MSB && tail_cluster_max() >= 2) {
+    if (lim && tail_cluster_max() >= 4) {
         const size_t cl = lim * tail_cluster_max();
         if (cl <= P->tail_len) lim = cl;
     }
@@ -735,7 +733,7 @@ int do_persist(effsc_prover* P, size_t r, size_t nr, const Chal& ch, size_t hook
 
 // fin: the tail also runs the runner's finalize (the last challenge's fold)
 // and writes the tables' first entries to `first` (the proof read-back).
-int do_tail(effsc_prover* P, size_t r, size_t num_rounds, const Chal& ch, const TxIO& tx, bool dry, u32 cs_log = 0,
+int do_tail(effsc_prover* P, size_t r, size_t num_rounds, const Chal& ch, const TxIO& tx, bool dry, ClusterSplit cl = {},
             bool fin = false, u64* first = nullptr) {
     const int pol = tail_pol(P), fw = P->field == EFFSC_FP3 ? 3 : 1, nt = P->ntab;
     const size_t L = P->t[0].len, rounds = num_rounds - r, folds = rounds - (ch.has ? 0 : 1) + (fin ? 1 : 0);
@@ -768,7 +766,7 @@ int do_tail(effsc_prover* P, size_t r, size_t num_rounds, const Chal& ch, const 
         }
     }
     if (!dry) {
-        if (cs_log) TRY(timed_launch(P->ctx->stream, "tail_cluster", bytes, [&] { return launch_tail_cluster(pol, fw, ta, cs_log, P->ctx->stream); }));
+        if (cl.cs_log) TRY(timed_launch(P->ctx->stream, "tail_cluster", bytes, [&] { return launch_tail_cluster(pol, fw, ta, cl.cs_log, cl.g_log, P->ctx->stream); }));
         else TRY(timed_launch(P->ctx->stream, "tail", bytes, [&] { return launch_tail(pol, fw, nullptr, &ta, 1, L, P->ctx->stream); }));
     }
     if (folds)
@@ -850,8 +848,7 @@ bool fuse_first_ok(const effsc_prover* P, size_t num_rounds) {
     if (P->order == EFFSC_LSB)
         for (int i = 0; i < 2; i++)
             if (((uintptr_t)P->t[i].bufs[0].p[0] & 15) != 0) return false;
-    Chal none;
-    return !tail_ok(P, 0, num_rounds, none);
+    return !whole_in_tail(P, num_rounds);
 }
 
 // Rounds 0-3 in two passes (k_ip012.cu) from num_vars = 14 on (below, the
@@ -1031,13 +1028,7 @@ bool ml_first_ok(const effsc_prover* P, size_t num_rounds) {
     if (!P->fuse_first || P->kind != EFFSC_ML || P->order != EFFSC_MSB || num_rounds < 3) return false;
     const Table& T = P->t[0];
     if (T.ext || T.cur != 0 || !is_pow2(T.len) || T.len < 8) return false;
-    Chal none;
-    if (tail_ok(P, 0, num_rounds, none)) return false;
-    // a table the cluster tail takes from round 1 on runs faster that way
-    // (measured: n = 18 over Fp)
-    const int fw = P->field == EFFSC_FP3 ? 3 : 1;
-    const size_t cap = (size_t)tail_max_len(POL_ML, fw, TAIL_SMEM_CAP) * std::max<u32>(1, tail_cluster_max());
-    return T.len > cap || T.len > P->tail_len;
+    return !whole_in_tail(P, num_rounds);
 }
 
 int do_ml_first(effsc_prover* P, const TxIO& tx0, const TxIO& tx2, const u64* chals, bool dry) {
@@ -1264,7 +1255,11 @@ int do_eqf_left(effsc_prover* P, const TxIO& tx, bool dry) {
         ta.hook_len = tx.hook_len;
         ta.proof_wire = tx.proof_wire;
         ta.proof_chal = tx.proof_chal;
-        TRY(timed_launch(s, "tail", 2 * rows * wbytes(out_ext), [&] { return launch_tail(POL_IP, fw, nullptr, &ta, 1, rows, s); }));
+        ClusterSplit cl;
+        const bool clus = tail_cluster_split(POL_IP, fw, rows, (u32)vl, false, &cl.cs_log, &cl.g_log);
+        TRY(timed_launch(s, clus ? "tail_cluster" : "tail", 2 * rows * wbytes(out_ext), [&] {
+            return clus ? launch_tail_cluster(POL_IP, fw, ta, cl.cs_log, cl.g_log, s) : launch_tail(POL_IP, fw, nullptr, &ta, 1, rows, s);
+        }));
         // eq weights of r_0 .. r_{v_l-2} (MSB order), then the weighted row sum of p
         launch_build_eq(P->d_chals, (u32)(vl - 1), fw == 3, Ew, Ew + rows2, Ew + 2 * rows2, s);
         g_launches++;
@@ -2426,9 +2421,11 @@ int effsc_prove(effsc_prover* P, size_t num_rounds, effsc_transcript* T, const u
             tx.proof_chal = P->d_chals + 3 * r;
             tx.chal_next = nullptr;
             // the tail runs the remaining rounds, the runner's finalize and
-            // the read-back gather in its one launch
-            if (tail_ok(P, r, num_rounds, ch)) {
-                TRY(do_tail(P, r, num_rounds, ch, tx, dry, 0, true, P->d_first));
+            // the read-back gather in its one launch, in a cluster where its
+            // first rounds are worth sharing
+            ClusterSplit cl;
+            if (cluster_tail_ok(P, r, num_rounds, ch, &cl) || tail_ok(P, r, num_rounds, ch)) {
+                TRY(do_tail(P, r, num_rounds, ch, tx, dry, cl, true, P->d_first));
                 tail_done = true;
                 break;
             }
@@ -2442,12 +2439,6 @@ int effsc_prove(effsc_prover* P, size_t num_rounds, effsc_transcript* T, const u
                 TRY(do_persist(P, r, nr, ch, hook_len, dry));
                 r += nr - 1;
                 continue;
-            }
-            u32 cs_log = 0;
-            if (cluster_tail_ok(P, r, num_rounds, ch, &cs_log)) {
-                TRY(do_tail(P, r, num_rounds, ch, tx, dry, cs_log, true, P->d_first));
-                tail_done = true;
-                break;
             }
             TRY(do_round(P, ch, tx, dry));
         }
