@@ -19,7 +19,9 @@
 // accumulates 26 base-field sums, each one product per octet
 // (ip012_sums), and the last block interpolates all three rounds' wire
 // values at the challenges as it runs the three transcript steps
-// (finalize_ip012).  The second pass folds every octet with r0, r1, r2 at
+// (finalize_ip012).  Tables that are 16-byte aligned take the sums from the
+// tensor cores (k_gram.cu); this form of the first pass is for the others.
+// The second pass folds every octet with r0, r1, r2 at
 // once -- the multilinear form sum_s D_s prod_{i in s} r_i with D_s the
 // octet's finite differences, 7 base x Fp3 products per component --
 // writes the Fp3 tables of length L/8 and evaluates round 3 on them.
@@ -191,17 +193,6 @@ __device__ __forceinline__ void ip012_reduce_and_finalize(const Acc (&s)[IP012_G
         if (threadIdx.x == 0) *a.counter = 0;
     }
     __syncthreads();
-    if (a.acc_mode != ACC_NONE) {
-        // one chunk of the tables: carry the sums to the next chunk's launch
-        if (threadIdx.x < IP012_WORDS) {
-            const u64 v = s_tot[threadIdx.x];
-            if (a.acc_mode == ACC_FIRST) a.acc[threadIdx.x] = v;
-            else if (a.acc_mode == ACC_MID) a.acc[threadIdx.x] = gl_add(a.acc[threadIdx.x], v);
-            else s_tot[threadIdx.x] = gl_add(a.acc[threadIdx.x], v);
-        }
-        if (a.acc_mode != ACC_LAST) return;
-        __syncthreads();
-    }
     if (warp == 0) finalize_ip012(s_tot, a);
 }
 
@@ -402,143 +393,6 @@ __device__ __forceinline__ void ip3x_body(const RoundArgs& a, u32 bid, u32 nb) {
     F3 raw[2];
     acc.result(raw);
     reduce_and_finalize_seg<2>(raw, a, POL_IP, nb, bid);
-}
-
-// ---------------------------------------------------------------------------
-// Staged passes: tiles of both tables stream into S shared-memory stages by
-// bulk copies (cp.async.bulk, the stage's mbarrier counting the bytes);
-// waits are bounded by the global timer (1 s: the block records a timeout,
-// drains its copies in flight and stops); the last warp to finish reading a
-// stage refills it with the block's tile S iterations ahead.  Bytes in
-// flight then no longer depend on registers per thread.
-// ---------------------------------------------------------------------------
-template <int S>
-struct StageRing {
-    u64 bar[S];
-    u32 reads_done[S];
-    u32 issued[S];
-};
-template <int S, class Issue>
-__device__ __forceinline__ void ring_start(StageRing<S>& R, u32 ntiles, Issue issue) {
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < S; s++) {
-            mbar_init(&R.bar[s], 1);
-            R.reads_done[s] = 0;
-            R.issued[s] = 0;
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        for (int s = 0; s < S; s++) {
-            const u32 tile = blockIdx.x + s * gridDim.x;
-            if (tile < ntiles) { issue(tile, s); R.issued[s]++; }
-        }
-    }
-    __syncthreads();
-}
-// The warp has read the stage of its i-th tile; the last warp refills it.
-template <int S, class Issue>
-__device__ __forceinline__ void ring_release(StageRing<S>& R, u32 i, u32 ntiles, Issue issue) {
-    __syncwarp();
-    if ((threadIdx.x & 31) == 0) {
-        const int s = i % S;
-        __threadfence_block();
-        if (atomicAdd(&R.reads_done[s], 1u) == NWARP - 1) {
-            atomicExch(&R.reads_done[s], 0u);
-            const u32 nt = blockIdx.x + (i + S) * gridDim.x;
-            if (nt < ntiles) {
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                issue(nt, s);
-                R.issued[s]++;
-            }
-        }
-    }
-}
-// After a timed-out wait at iteration i: wait (bounded) for every copy still
-// in flight (stage s has completed the phases of the tiles before i and holds
-// issued[s] minus those), then record the timeout.
-template <int S>
-__device__ __forceinline__ void ring_drain(StageRing<S>& R, u32 i, u32* status) {
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < S; s++)
-            for (u32 ph = i / S + (s < (int)(i % S) ? 1u : 0u); ph < R.issued[s]; ph++)
-                mbar_wait_bounded(&R.bar[s], ph & 1u);
-        if (status) *(volatile u32*)status = EFFSC_STATUS_TIMEOUT;
-    }
-}
-
-constexpr int IP012_TQ = 256;    // octets per tile of the first pass (two per thread)
-constexpr int IP012_S = 3;       // its stages: 3 x 32 KB
-constexpr int IP012_STAGE_WORDS = 2 * 8 * IP012_TQ;
-constexpr int IP012_SMEM = IP012_S * IP012_STAGE_WORDS * 8;
-
-// Pass 1, staged.  Tile = IP012_TQ octets; a stage holds, per table, the
-// tile's 8 entries of each octet (MSB: 8 chunks, one per j, of TQ words; LSB:
-// the 8 TQ consecutive entries).  Warps 0..3 accumulate sums 0..13, warps
-// 4..7 sums 14..25, both from the same stage; each thread takes TQ / 128
-// octets of a tile, so the stage wait and release are paid once per two
-// octets.
-template <bool LSB>
-__device__ __forceinline__ void ip012_staged_body(const RoundArgs& a, u32 ntiles) {
-    extern __shared__ __align__(128) u64 stg[];
-    __shared__ StageRing<IP012_S> R;
-    constexpr int TQ = IP012_TQ, S = IP012_S, SW = IP012_STAGE_WORDS;
-    const u64 O = a.L >> 3;
-    const u64* X[2] = {a.t[0].in[0], a.t[1].in[0]};
-    auto issue = [&](u32 tile, int s) {
-        mbar_expect_tx(&R.bar[s], (u32)(SW * 8));
-        u64* dst = stg + (size_t)s * SW;
-        tile += a.tile0;
-#pragma unroll
-        for (int t = 0; t < 2; t++) {
-            if (LSB) {
-                tma_load_1d(dst + t * 8 * TQ, X[t] + (u64)tile * 8 * TQ, 8 * TQ * 8, &R.bar[s]);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-                    tma_load_1d(dst + (t * 8 + j) * TQ, X[t] + j * O + (u64)tile * TQ, TQ * 8, &R.bar[s]);
-            }
-        }
-    };
-    ring_start<S>(R, ntiles, issue);
-    constexpr int HALF = TPB / 2, PER = TQ / HALF;
-    static_assert(TQ % HALF == 0, "a tile holds whole rows of octets for a warp group");
-    const int group = threadIdx.x >= HALF;
-    Acc sums[IP012_G1];
-#pragma unroll
-    for (int i = 0; i < IP012_G1; i++) sums[i] = acc_zero();
-    bool abort = false;
-    u32 i = 0;
-    for (u32 tile = blockIdx.x; tile < ntiles; tile += gridDim.x, i++) {
-        if (!mbar_wait_bounded(&R.bar[i % S], (i / S) & 1u)) { abort = true; break; }
-        const u64* st_ = stg + (size_t)(i % S) * SW;
-#pragma unroll
-        for (int h = 0; h < PER; h++) {
-            const int ml = (threadIdx.x & (HALF - 1)) + h * HALF;
-            u64 x[8], y[8];
-            if (LSB) {
-                const ulonglong2* px = (const ulonglong2*)(st_ + 8 * ml);
-                const ulonglong2* py = (const ulonglong2*)(st_ + 8 * TQ + 8 * ml);
-                const ulonglong2 a01 = px[0], a23 = px[1], a45 = px[2], a67 = px[3];
-                const ulonglong2 b01 = py[0], b23 = py[1], b45 = py[2], b67 = py[3];
-                x[0] = a01.x; x[4] = a01.y; x[2] = a23.x; x[6] = a23.y; x[1] = a45.x; x[5] = a45.y; x[3] = a67.x; x[7] = a67.y;
-                y[0] = b01.x; y[4] = b01.y; y[2] = b23.x; y[6] = b23.y; y[1] = b45.x; y[5] = b45.y; y[3] = b67.x; y[7] = b67.y;
-            } else {
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    x[j] = st_[j * TQ + ml];
-                    y[j] = st_[(8 + j) * TQ + ml];
-                }
-            }
-            // the stage is free once the tile's last octets are in registers
-            if (h == PER - 1) ring_release<S>(R, i, ntiles, issue);
-            if (group == 0) ip012_sums<0>(sums, x, y);
-            else ip012_sums<1>(sums, x, y);
-        }
-    }
-    if (__syncthreads_or(abort)) {
-        ring_drain<S>(R, i, a.status);
-        return;
-    }
-    ip012_reduce_and_finalize(sums, group, a, gridDim.x, blockIdx.x);
 }
 
 }  // namespace effsc

@@ -275,12 +275,14 @@ bool launch_ip012(bool lsb, const RoundArgs& a, int grid, cudaStream_t s);
 // for the second pass.
 bool launch_ip012_mirror(bool lsb, const RoundArgs& a, int grid, cudaStream_t s);
 bool launch_ip3x(bool lsb, const RoundArgs& a, int grid, cudaStream_t s);
-// The first pass with the tables streamed through shared memory by bulk
-// copies: ntiles = (L/8) / ip012_tile_octets() tiles; device-memory tables,
-// 16-byte aligned; at most two blocks per SM for the partials.  (The second
-// pass keeps direct loads: staged, it measured slower.)
-bool launch_ip012_staged(bool lsb, const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s);
-u32 ip012_tile_octets(void);
+// The first pass on the tensor cores (k_gram.cu): tiles a.tile0 ..
+// a.tile0 + ntiles - 1 of gram_tile_octets() octets, tables 16-byte aligned
+// (a.t[i].in[0]; with `mirror` also the device buffers a.t[i].out[0], to which
+// the words are copied).  At most gram_max_tiles() tiles per block; partials
+// of 64 words per block.
+bool launch_ip_gram(bool lsb, bool mirror, const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s);
+u32 gram_tile_octets(void);
+u32 gram_max_tiles(void);
 // Consecutive InnerProduct rounds over Fp3 tables in one cooperative launch
 // (k_persist.cu): round k of the launch folds tables of length L0 >> k with
 // the previous challenge and evaluates; the last block to reach the grid

@@ -887,7 +887,7 @@ bool mirror_ok(effsc_prover* P, size_t L) {
 bool upload_chunks_ok(const effsc_prover* P, size_t L) {
     if (P->order != EFFSC_MSB) return false;
     const size_t O = L / 8;
-    if (O % ((size_t)UPLOAD_CHUNKS * ip012_tile_octets()) != 0) return false;
+    if (O % ((size_t)UPLOAD_CHUNKS * gram_tile_octets()) != 0) return false;
     for (int i = 0; i < 2; i++) {
         cudaPointerAttributes at;
         if (cudaPointerGetAttributes(&at, P->t[i].bufs[0].p[0]) != cudaSuccess) { cudaGetLastError(); return false; }
@@ -896,30 +896,53 @@ bool upload_chunks_ok(const effsc_prover* P, size_t L) {
     return true;
 }
 
+// The first pass on the tensor cores (k_gram.cu) over tiles lo .. lo + n - 1:
+// one launch while a block's accumulators hold its tiles, else several, the
+// sums carried from one to the next.
+bool gram_ok(const effsc_prover* P, size_t L, const RoundArgs& a) {
+    uintptr_t bits = 0;
+    for (int i = 0; i < 2; i++) bits |= (uintptr_t)a.t[i].in[0] | (uintptr_t)a.t[i].out[0];
+    return (bits & 15) == 0 && (L / 8) % gram_tile_octets() == 0 && L / 8 / gram_tile_octets() < (1u << 31);
+}
+int gram_pass(effsc_prover* P, RoundArgs a, bool mirror, size_t lo, size_t n, bool first, bool last, const char* name) {
+    cudaStream_t s = P->ctx->stream;
+    const int sms = max_grid() / 8;
+    const size_t most = (size_t)sms * gram_max_tiles();
+    for (size_t at = 0; at < n; at += most) {
+        const size_t cnt = std::min(most, n - at);
+        const bool f = first && at == 0, l = last && at + cnt == n;
+        a.tile0 = (u32)(lo + at);
+        a.acc_mode = f && l ? ACC_NONE : f ? ACC_FIRST : l ? ACC_LAST : ACC_MID;
+        TRY(timed_launch(s, name, 16 * 8 * (uint64_t)cnt * gram_tile_octets(), [&] {
+            return launch_ip_gram(P->order == EFFSC_LSB, mirror, a, (u32)cnt, (int)std::min<size_t>(cnt, sms), s);
+        }));
+    }
+    return EFFSC_OK;
+}
+int need_acc(effsc_prover* P) {
+    if (!P->d_acc) CK(cudaMallocAsync((void**)&P->d_acc, 32 * sizeof(u64), P->ctx->stream));
+    return EFFSC_OK;
+}
+
 int chunked_first_pass(effsc_prover* P, RoundArgs a, const int* mi, bool dry) {
     cudaStream_t s = P->ctx->stream;
     const size_t L = P->t[0].len, O = L / 8, CW = O / UPLOAD_CHUNKS;
     if (!P->copy_stream) CK(cudaStreamCreateWithFlags(&P->copy_stream, cudaStreamNonBlocking));
     for (cudaEvent_t& e : P->chunk_ev)
         if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    if (!P->d_acc) CK(cudaMallocAsync((void**)&P->d_acc, 32 * sizeof(u64), s));
     if (dry) return EFFSC_OK;
     // the copies start after the stream's earlier work (the buffers' allocation)
     CK(cudaEventRecord(P->chunk_ev[UPLOAD_CHUNKS], s));
     CK(cudaStreamWaitEvent(P->copy_stream, P->chunk_ev[UPLOAD_CHUNKS], 0));
-    const u32 ct = (u32)(CW / ip012_tile_octets());
-    const int g = std::min<int>((int)ct, (max_grid() / 8) * 2);
+    const size_t ct = CW / gram_tile_octets();
     for (int i = 0; i < 2; i++) a.t[i].in[0] = P->t[i].bufs[mi[i]].p[0];
-    a.acc = P->d_acc;
     for (int c = 0; c < UPLOAD_CHUNKS; c++) {
         for (int i = 0; i < 2; i++)
             CK(cudaMemcpy2DAsync(P->t[i].bufs[mi[i]].p[0] + c * CW, O * sizeof(u64), P->t[i].bufs[0].p[0] + c * CW,
                                  O * sizeof(u64), CW * sizeof(u64), 8, cudaMemcpyHostToDevice, P->copy_stream));
         CK(cudaEventRecord(P->chunk_ev[c], P->copy_stream));
         CK(cudaStreamWaitEvent(s, P->chunk_ev[c], 0));
-        a.tile0 = (u32)c * ct;
-        a.acc_mode = c == 0 ? ACC_FIRST : c == UPLOAD_CHUNKS - 1 ? ACC_LAST : ACC_MID;
-        TRY(timed_launch(s, "ip_rounds_0_2_chunked", 16 * (uint64_t)CW * 8, [&] { return launch_ip012_staged(false, a, ct, g, s); }));
+        TRY(gram_pass(P, a, false, (size_t)c * ct, ct, c == 0, c == UPLOAD_CHUNKS - 1, "ip_rounds_0_2_chunked"));
     }
     return EFFSC_OK;
 }
@@ -931,23 +954,7 @@ int do_fuse3(effsc_prover* P, const TxIO& tx0, const TxIO& tx3, const u64* chals
     a.tx = tx0;
     a.L = L;
     for (int i = 0; i < 2; i++) set_in(a, i, P->t[i]);
-    // First pass, MSB: staged through shared memory for device tables
-    // (16-byte aligned, as the allocator gives).  LSB keeps direct loads: a
-    // thread's octet is 64 contiguous bytes, and reading those from a staged
-    // tile conflicts on the shared-memory banks (measured slower: 0.51 against
-    // 0.40 ms at n = 26).  A block takes 128 octets per step; one wave of two
-    // blocks per SM at most (the partials hold 32 words for each).  The
-    // second pass reads directly in both orders (staged, MSB measured 0.447
-    // against 0.36 ms at n = 26).
-    bool staged = !lsb;
-    for (int i = 0; i < 2; i++) {
-        const Buf& b0 = P->t[i].bufs[0];
-        staged &= !b0.host && ((uintptr_t)b0.p[0] & 15) == 0;
-    }
-    const u32 nt1 = (u32)((L / 8) / ip012_tile_octets());
-    staged &= nt1 >= 1 && (L / 8) % ip012_tile_octets() == 0;
     const int two_per_sm = (max_grid() / 8) * 2;
-    const int g1 = staged ? std::min<int>((int)nt1, two_per_sm) : std::min<int>(grid_for(L / 8, 2), two_per_sm);
     // Tables in host memory: when the device has room, the first pass also
     // copies them into device buffers (the mirror), so they cross the host
     // link once and the second pass reads HBM.
@@ -957,12 +964,17 @@ int do_fuse3(effsc_prover* P, const TxIO& tx0, const TxIO& tx3, const u64* chals
             TRY(out_buffer(P, P->t[i], false, L, false, &mi[i]));
             a.t[i].out[0] = P->t[i].bufs[mi[i]].p[0];
         }
-    if (mi[0] >= 0 && upload_chunks_ok(P, L)) {
+    TRY(need_acc(P));
+    a.acc = P->d_acc;
+    const bool gram = gram_ok(P, L, a);
+    if (mi[0] >= 0 && gram && upload_chunks_ok(P, L)) {
         TRY(chunked_first_pass(P, a, mi, dry));
+    } else if (!dry && gram) {
+        TRY(gram_pass(P, a, mi[0] >= 0, 0, L / 8 / gram_tile_octets(), true, true, mi[0] >= 0 ? "ip_rounds_0_2_from_host" : "ip_rounds_0_2"));
     } else if (!dry) {
+        const int g1 = std::min<int>(grid_for(L / 8, 2), two_per_sm);
         TRY(timed_launch(P->ctx->stream, mi[0] >= 0 ? "ip_rounds_0_2_from_host" : "ip_rounds_0_2", 16 * (uint64_t)L, [&] {
-            if (mi[0] >= 0) return launch_ip012_mirror(lsb, a, g1, P->ctx->stream);
-            return staged ? launch_ip012_staged(lsb, a, nt1, g1, P->ctx->stream) : launch_ip012(lsb, a, g1, P->ctx->stream);
+            return mi[0] >= 0 ? launch_ip012_mirror(lsb, a, g1, P->ctx->stream) : launch_ip012(lsb, a, g1, P->ctx->stream);
         }));
     }
     if (mi[0] >= 0)
