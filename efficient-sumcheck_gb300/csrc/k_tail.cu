@@ -258,53 +258,24 @@ __device__ __forceinline__ u64 tail_total(const TailShared& sh, int lane, bool b
     return v;
 }
 
-// The transcript of a tail, in warp 0: its state and, per lane, the words
-// that every round absorbs after the wire values (the hook, the padding).
+// The transcript of a tail, in warp 0.
 struct TailTx {
     WarpTx w;
-    u64 fixed;
-    bool fast;        // wire, hook and padding fit one block, in whole words
+    TxStream s;
 };
 template <int NW>
 __device__ __forceinline__ void tail_tx_init(TailTx& x, const TailArgs& a, int lane) {
     x.w = tx_load((const DevTranscript*)a.tx, lane);
-    x.fast = (a.hook_len & 7) == 0 && ((uintptr_t)a.hook & 7) == 0 && 8 * NW + a.hook_len < TX_RATE;
-    x.fixed = 0;
-    if (x.fast) {
-        const int hw = (int)(a.hook_len >> 3);
-        if (lane >= NW && lane < NW + hw) x.fixed = ((const u64*)a.hook)[lane - NW];
-        if (lane == NW + hw) x.fixed ^= 0x06;
-        if (lane == TX_RATE / 8 - 1) x.fixed ^= 0x80ULL << 56;
-    }
+    x.s = tx_stream<NW>(a.hook, a.hook_len, lane);
 }
-// The transcript step of a round (src/runner.rs:39-55): send the wire values
-// (word i of them in lane i), absorb the hook, squeeze the challenge into
-// sh.chal, prepared.  After the first round the transcript is always at a
-// squeeze, so the wire, the hook and the padding make one block of whole
-// words: one xor per lane, the permutation, and the challenge straight from
-// the lanes that hold it.
+// The transcript step of a round: send the wire values (word i of them in
+// lane i), absorb the hook, squeeze the challenge into sh.chal, prepared.
 template <int POL, int FW>
 __device__ __forceinline__ void tail_transcript(TailTx& x, u64 wire, const TailArgs& a, TailShared& sh) {
-    constexpr int NWIRE = TailRoles<POL, FW>::NWIRE, NW = TailRoles<POL, FW>::N;
+    constexpr int NW = TailRoles<POL, FW>::N;
     const int lane = threadIdx.x & 31;
     if (lane < NW) sh.tot[FW == 3 ? lane : 3 * lane] = wire;
-    u64 r;
-    __syncwarp();
-    if (x.fast && x.w.squeezing) {
-        x.w.a ^= x.fixed ^ wire;
-        keccak_f_warp(x.w.a, lane);
-        x.w.pos = 16 * FW;
-        const u64 lo = shfl64(x.w.a, (2 * lane) & 31), hi = shfl64(x.w.a, (2 * lane + 1) & 31);
-        r = lane < FW ? gl_reduce128(lo, hi) : 0;
-    } else {
-        tx_send_elems(x.w, lane, sh.tot, NWIRE);
-        if (a.hook_len) {
-            const uint8_t* hk = a.hook;
-            tx_absorb(x.w, lane, a.hook_len, [&](u32 i) -> uint8_t { return hk[i]; });
-        }
-        tx_challenge(x.w, lane, sh.raw, sh.scr);
-        r = lane < 3 ? sh.raw[lane] : 0;
-    }
+    const u64 r = tx_step<NW, FW>(x.w, x.s, wire, a.hook, a.hook_len, lane, sh.tot, sh.raw, sh.scr);
     if (lane < 3) sh.chal[2 + lane] = r;
     if (FW == 3 && (lane == 1 || lane == 2)) sh.chal[lane - 1] = gl_mul_w(r);
 }

@@ -275,14 +275,18 @@ bool launch_ip012(bool lsb, const RoundArgs& a, int grid, cudaStream_t s);
 // for the second pass.
 bool launch_ip012_mirror(bool lsb, const RoundArgs& a, int grid, cudaStream_t s);
 bool launch_ip3x(bool lsb, const RoundArgs& a, int grid, cudaStream_t s);
-// The first pass on the tensor cores (k_gram.cu): tiles a.tile0 ..
-// a.tile0 + ntiles - 1 of gram_tile_octets() octets, tables 16-byte aligned
-// (a.t[i].in[0]; with `mirror` also the device buffers a.t[i].out[0], to which
-// the words are copied).  At most gram_max_tiles() tiles per block; partials
-// of 64 words per block.
-bool launch_ip_gram(bool lsb, bool mirror, const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s);
-u32 gram_tile_octets(void);
+// InnerProduct rounds 0 .. nv (nv = 3 or 4) in two passes on the tensor cores,
+// tables 16-byte aligned.  First pass (k_gram.cu): rounds 0 .. nv - 1 from
+// tiles a.tile0 .. a.tile0 + ntiles - 1 of TC_TILE_ITEMS groups of 2^nv
+// entries, at most gram_max_tiles() per block (with `mirror` the words are
+// also copied to the device buffers a.t[i].out[0]); partials of 4^nv words per
+// block, a.acc of as many.  Second pass (k_tcfold.cu): the fold with r_0 ..
+// r_{nv-1} (a.chal_ptr: 3 nv words) and round nv, over all
+// (L >> nv) / TC_TILE_ITEMS tiles.
+constexpr u32 TC_TILE_ITEMS = 128;
+bool launch_ip_gram(bool lsb, int nv, bool mirror, const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s);
 u32 gram_max_tiles(void);
+bool launch_tc_fold(bool lsb, int nv, const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s);
 // Consecutive InnerProduct rounds over Fp3 tables in one cooperative launch
 // (k_persist.cu): round k of the launch folds tables of length L0 >> k with
 // the previous challenge and evaluates; the last block to reach the grid

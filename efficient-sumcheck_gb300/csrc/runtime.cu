@@ -877,34 +877,22 @@ bool mirror_ok(effsc_prover* P, size_t L) {
     return P->mirror == 1;
 }
 
-// Pinned host tables of an MSB prover with room on the device: upload them
-// in UPLOAD_CHUNKS chunks of whole octets (octets m in [c O/C, (c+1) O/C),
-// one 2-D copy per table: eight rows of O/C entries at stride O) on a copy
-// stream, and run the first pass on each chunk as soon as it has arrived,
-// carrying the 26 sums from chunk to chunk; the last chunk's launch
-// finalises rounds 0-2.  The copy engines then set the pace and all but the
-// last chunk's pass hide behind the transfer.
-bool upload_chunks_ok(const effsc_prover* P, size_t L) {
-    if (P->order != EFFSC_MSB) return false;
-    const size_t O = L / 8;
-    if (O % ((size_t)UPLOAD_CHUNKS * gram_tile_octets()) != 0) return false;
-    for (int i = 0; i < 2; i++) {
-        cudaPointerAttributes at;
-        if (cudaPointerGetAttributes(&at, P->t[i].bufs[0].p[0]) != cudaSuccess) { cudaGetLastError(); return false; }
-        if (at.type != cudaMemoryTypeHost) return false;   // pageable: the kernel reads it in place
-    }
-    return true;
-}
-
-// The first pass on the tensor cores (k_gram.cu) over tiles lo .. lo + n - 1:
-// one launch while a block's accumulators hold its tiles, else several, the
-// sums carried from one to the next.
-bool gram_ok(const effsc_prover* P, size_t L, const RoundArgs& a) {
+// The tensor-core start takes every two-pass start whose tables it can load
+// 16 bytes at a time: rounds 0-4 when the proof has them (one pass over the
+// tables fewer bytes of folded tables: 2 x 24 L/16 instead of 2 x 24 L/8),
+// else rounds 0-3.  0: the general form (k_ip012.cu, rounds 0-3).
+int tc_rounds(size_t L, size_t num_rounds, const RoundArgs& a) {
     uintptr_t bits = 0;
     for (int i = 0; i < 2; i++) bits |= (uintptr_t)a.t[i].in[0] | (uintptr_t)a.t[i].out[0];
-    return (bits & 15) == 0 && (L / 8) % gram_tile_octets() == 0 && L / 8 / gram_tile_octets() < (1u << 31);
+    const int nv = num_rounds >= 5 ? 4 : 3;
+    const size_t items = L >> nv;
+    if ((bits & 15) || items % TC_TILE_ITEMS || items / TC_TILE_ITEMS >= (1u << 31)) return 0;
+    return nv;
 }
-int gram_pass(effsc_prover* P, RoundArgs a, bool mirror, size_t lo, size_t n, bool first, bool last, const char* name) {
+// The first pass over tiles lo .. lo + n - 1: one launch while a block's
+// accumulators hold its tiles, else several, the sums carried from one to the
+// next.
+int gram_pass(effsc_prover* P, RoundArgs a, int nv, bool mirror, size_t lo, size_t n, bool first, bool last, const char* name) {
     cudaStream_t s = P->ctx->stream;
     const int sms = max_grid() / 8;
     const size_t most = (size_t)sms * gram_max_tiles();
@@ -913,20 +901,34 @@ int gram_pass(effsc_prover* P, RoundArgs a, bool mirror, size_t lo, size_t n, bo
         const bool f = first && at == 0, l = last && at + cnt == n;
         a.tile0 = (u32)(lo + at);
         a.acc_mode = f && l ? ACC_NONE : f ? ACC_FIRST : l ? ACC_LAST : ACC_MID;
-        TRY(timed_launch(s, name, 16 * 8 * (uint64_t)cnt * gram_tile_octets(), [&] {
-            return launch_ip_gram(P->order == EFFSC_LSB, mirror, a, (u32)cnt, (int)std::min<size_t>(cnt, sms), s);
+        TRY(timed_launch(s, name, (uint64_t)cnt * TC_TILE_ITEMS * (16u << nv), [&] {
+            return launch_ip_gram(P->order == EFFSC_LSB, nv, mirror, a, (u32)cnt, (int)std::min<size_t>(cnt, sms), s);
         }));
     }
     return EFFSC_OK;
 }
-int need_acc(effsc_prover* P) {
-    if (!P->d_acc) CK(cudaMallocAsync((void**)&P->d_acc, 32 * sizeof(u64), P->ctx->stream));
-    return EFFSC_OK;
+
+// Pinned host tables of an MSB prover with room on the device: upload them
+// in UPLOAD_CHUNKS chunks of whole groups (groups m in [c N/C, (c+1) N/C) of
+// N = L / 2^nv, one 2-D copy per table: 2^nv rows of N/C entries at stride N)
+// on a copy stream, and run the first pass on each chunk as soon as it has
+// arrived, carrying the sums from chunk to chunk; the last chunk's launch
+// runs the rounds.  The copy engines then set the pace and all but the last
+// chunk's pass hide behind the transfer.
+bool upload_chunks_ok(const effsc_prover* P, size_t items) {
+    if (P->order != EFFSC_MSB) return false;
+    if (items % ((size_t)UPLOAD_CHUNKS * TC_TILE_ITEMS) != 0) return false;
+    for (int i = 0; i < 2; i++) {
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, P->t[i].bufs[0].p[0]) != cudaSuccess) { cudaGetLastError(); return false; }
+        if (at.type != cudaMemoryTypeHost) return false;   // pageable: the kernel reads it in place
+    }
+    return true;
 }
 
-int chunked_first_pass(effsc_prover* P, RoundArgs a, const int* mi, bool dry) {
+int chunked_first_pass(effsc_prover* P, RoundArgs a, int nv, const int* mi, bool dry) {
     cudaStream_t s = P->ctx->stream;
-    const size_t L = P->t[0].len, O = L / 8, CW = O / UPLOAD_CHUNKS;
+    const size_t N = P->t[0].len >> nv, CW = N / UPLOAD_CHUNKS, ct = CW / TC_TILE_ITEMS;
     if (!P->copy_stream) CK(cudaStreamCreateWithFlags(&P->copy_stream, cudaStreamNonBlocking));
     for (cudaEvent_t& e : P->chunk_ev)
         if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -934,27 +936,27 @@ int chunked_first_pass(effsc_prover* P, RoundArgs a, const int* mi, bool dry) {
     // the copies start after the stream's earlier work (the buffers' allocation)
     CK(cudaEventRecord(P->chunk_ev[UPLOAD_CHUNKS], s));
     CK(cudaStreamWaitEvent(P->copy_stream, P->chunk_ev[UPLOAD_CHUNKS], 0));
-    const size_t ct = CW / gram_tile_octets();
     for (int i = 0; i < 2; i++) a.t[i].in[0] = P->t[i].bufs[mi[i]].p[0];
     for (int c = 0; c < UPLOAD_CHUNKS; c++) {
         for (int i = 0; i < 2; i++)
-            CK(cudaMemcpy2DAsync(P->t[i].bufs[mi[i]].p[0] + c * CW, O * sizeof(u64), P->t[i].bufs[0].p[0] + c * CW,
-                                 O * sizeof(u64), CW * sizeof(u64), 8, cudaMemcpyHostToDevice, P->copy_stream));
+            CK(cudaMemcpy2DAsync(P->t[i].bufs[mi[i]].p[0] + c * CW, N * sizeof(u64), P->t[i].bufs[0].p[0] + c * CW,
+                                 N * sizeof(u64), CW * sizeof(u64), (size_t)1 << nv, cudaMemcpyHostToDevice, P->copy_stream));
         CK(cudaEventRecord(P->chunk_ev[c], P->copy_stream));
         CK(cudaStreamWaitEvent(s, P->chunk_ev[c], 0));
-        TRY(gram_pass(P, a, false, (size_t)c * ct, ct, c == 0, c == UPLOAD_CHUNKS - 1, "ip_rounds_0_2_chunked"));
+        TRY(gram_pass(P, a, nv, false, (size_t)c * ct, ct, c == 0, c == UPLOAD_CHUNKS - 1, "ip_first_rounds_chunked"));
     }
     return EFFSC_OK;
 }
 
-int do_fuse3(effsc_prover* P, const TxIO& tx0, const TxIO& tx3, const u64* chals, bool dry) {
+// The two-pass start: *done = the rounds it ran (4 or 5).
+int do_fuse3(effsc_prover* P, size_t num_rounds, const TxIO& tx0, const u64* chals, size_t* done, bool dry) {
     const size_t L = P->t[0].len;
     const bool lsb = P->order == EFFSC_LSB;
     RoundArgs a = base_args(P);
     a.tx = tx0;
     a.L = L;
     for (int i = 0; i < 2; i++) set_in(a, i, P->t[i]);
-    const int two_per_sm = (max_grid() / 8) * 2;
+    const int sms = max_grid() / 8, two_per_sm = sms * 2;
     // Tables in host memory: when the device has room, the first pass also
     // copies them into device buffers (the mirror), so they cross the host
     // link once and the second pass reads HBM.
@@ -964,43 +966,48 @@ int do_fuse3(effsc_prover* P, const TxIO& tx0, const TxIO& tx3, const u64* chals
             TRY(out_buffer(P, P->t[i], false, L, false, &mi[i]));
             a.t[i].out[0] = P->t[i].bufs[mi[i]].p[0];
         }
-    TRY(need_acc(P));
-    a.acc = P->d_acc;
-    const bool gram = gram_ok(P, L, a);
-    if (mi[0] >= 0 && gram && upload_chunks_ok(P, L)) {
-        TRY(chunked_first_pass(P, a, mi, dry));
-    } else if (!dry && gram) {
-        TRY(gram_pass(P, a, mi[0] >= 0, 0, L / 8 / gram_tile_octets(), true, true, mi[0] >= 0 ? "ip_rounds_0_2_from_host" : "ip_rounds_0_2"));
+    const bool mirror = mi[0] >= 0;
+    const int tc = tc_rounds(L, num_rounds, a), nv = tc ? tc : 3;
+    const char* name = mirror ? "ip_first_rounds_from_host" : "ip_first_rounds";
+    if (tc) {
+        if (!P->d_acc) CK(cudaMallocAsync((void**)&P->d_acc, 256 * sizeof(u64), P->ctx->stream));
+        a.acc = P->d_acc;
+        if (mirror && upload_chunks_ok(P, L >> nv)) TRY(chunked_first_pass(P, a, nv, mi, dry));
+        else if (!dry) TRY(gram_pass(P, a, nv, mirror, 0, (L >> nv) / TC_TILE_ITEMS, true, true, name));
     } else if (!dry) {
         const int g1 = std::min<int>(grid_for(L / 8, 2), two_per_sm);
-        TRY(timed_launch(P->ctx->stream, mi[0] >= 0 ? "ip_rounds_0_2_from_host" : "ip_rounds_0_2", 16 * (uint64_t)L, [&] {
-            return mi[0] >= 0 ? launch_ip012_mirror(lsb, a, g1, P->ctx->stream) : launch_ip012(lsb, a, g1, P->ctx->stream);
+        TRY(timed_launch(P->ctx->stream, name, 16 * (uint64_t)L, [&] {
+            return mirror ? launch_ip012_mirror(lsb, a, g1, P->ctx->stream) : launch_ip012(lsb, a, g1, P->ctx->stream);
         }));
     }
-    if (mi[0] >= 0)
+    if (mirror)
         for (int i = 0; i < 2; i++) P->t[i].cur = mi[i];
+    const size_t N = L >> nv;
     int bi[2];
-    for (int i = 0; i < 2; i++) TRY(out_buffer(P, P->t[i], true, L / 8, true, &bi[i]));
+    for (int i = 0; i < 2; i++) TRY(out_buffer(P, P->t[i], true, N, true, &bi[i]));
     RoundArgs b = base_args(P);
-    b.tx = tx3;
+    b.tx = tx0;
+    b.tx.proof_wire = tx0.proof_wire + (size_t)nv * 6;
+    b.tx.proof_chal = tx0.proof_chal + (size_t)nv * 3;
     b.L = L;
     b.chal_ptr = chals;
     for (int i = 0; i < 2; i++) {
         set_in(b, i, P->t[i]);
         set_out(b, i, P->t[i].bufs[bi[i]]);
     }
-    // one wave (two blocks per SM, the kernel's residency): n = 26 measured
-    // 0.369 against 0.377 ms (MSB) and 0.350 against 0.364 ms (LSB) for four
-    // waves of blocks
-    if (!dry) TRY(timed_launch(P->ctx->stream, "ip_round_3_triple_fold", 16 * (uint64_t)L + 6 * (uint64_t)L, [&] {
-        return launch_ip3x(lsb, b, std::min<int>(grid_for(L / 16), two_per_sm), P->ctx->stream);
+    // the general form: one wave (two blocks per SM, the kernel's residency)
+    if (!dry) TRY(timed_launch(P->ctx->stream, "ip_fold_and_round", 16 * (uint64_t)L + 48 * (uint64_t)N, [&] {
+        if (!tc) return launch_ip3x(lsb, b, std::min<int>(grid_for(L / 16), two_per_sm), P->ctx->stream);
+        const size_t tiles = N / TC_TILE_ITEMS;
+        return launch_tc_fold(lsb, nv, b, (u32)tiles, (int)std::min<size_t>(tiles, sms), P->ctx->stream);
     }));
     for (int i = 0; i < 2; i++) {
         Table& T = P->t[i];
         T.cur = bi[i];
-        T.len = L / 8;
+        T.len = N;
         T.ext = true;
     }
+    *done = nv + 1;
     return EFFSC_OK;
 }
 
@@ -1584,7 +1591,8 @@ int final_value(effsc_prover* P, HF* out) {
 
 int prover_common_init(effsc_prover* P) {
     cudaStream_t s = P->ctx->stream;
-    CK(cudaMallocAsync((void**)&P->partials, (size_t)max_grid() * 12 * sizeof(u64), s));
+    // 12 words per block of the round kernels, 256 per SM of the tensor-core passes
+    CK(cudaMallocAsync((void**)&P->partials, (size_t)max_grid() * 32 * sizeof(u64), s));
     CK(cudaMallocAsync((void**)&P->counter, 2 * sizeof(u32), s));
     CK(cudaMemsetAsync(P->counter, 0, 2 * sizeof(u32), s));
     P->h_res = (u64*)pinned_get(P->ctx, 16 * sizeof(u64));
@@ -2347,18 +2355,14 @@ int effsc_prove(effsc_prover* P, size_t num_rounds, effsc_transcript* T, const u
         size_t r0 = 0;
         bool tail_done = false;
         if (fuse3_ok(P, num_rounds)) {
-            TxIO t0, t3;
+            TxIO t0;
             memset(&t0, 0, sizeof t0);
             t0.tx = P->d_tx;
             t0.hook = P->d_hook;
             t0.hook_len = (u32)hook_len;
-            t3 = t0;
             t0.proof_wire = P->d_wire;
             t0.proof_chal = P->d_chals;
-            t3.proof_wire = P->d_wire + (size_t)3 * 3 * d;
-            t3.proof_chal = P->d_chals + 3 * 3;
-            TRY(do_fuse3(P, t0, t3, P->d_chals, dry));
-            r0 = 4;
+            TRY(do_fuse3(P, num_rounds, t0, P->d_chals, &r0, dry));
         } else if (coef3_first_ok(P, num_rounds)) {
             TxIO t0, t2;
             memset(&t0, 0, sizeof t0);

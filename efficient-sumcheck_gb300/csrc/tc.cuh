@@ -20,12 +20,10 @@ __device__ __forceinline__ uint4 digits_of(u64 v) {
 // 128-byte rows with the 128-byte swizzle: chunk c of row r.
 __device__ __forceinline__ u32 swz128(u32 row, u32 chunk) { return row * 128 + ((chunk ^ (row & 7)) << 4); }
 
-// Shared-memory matrix descriptor: start address, both strides (bytes between
-// 8-row groups / between 128-byte wide atoms; the operands here are one atom
-// wide, so only one is used), 128-byte swizzle.
-__device__ __forceinline__ u64 tc_desc(u32 addr, u32 stride) {
-    const u64 s = stride >> 4;
-    return (u64)((addr & 0x3FFFF) >> 4) | (s << 16) | (s << 32) | (1ULL << 46) | (2ULL << 61);
+// Shared-memory matrix descriptor with the 128-byte swizzle: start address,
+// bytes between 128-byte wide atoms, bytes between 8-row groups of an atom.
+__device__ __forceinline__ u64 tc_desc(u32 addr, u32 atoms, u32 groups) {
+    return (u64)((addr & 0x3FFFF) >> 4) | ((u64)(atoms >> 4) << 16) | ((u64)(groups >> 4) << 32) | (1ULL << 46) | (2ULL << 61);
 }
 // Instruction descriptor of kind::f8f6f4, e4m3 x e4m3 -> f32 (mn: both
 // operands stored with the M / N index contiguous, else K).
@@ -51,20 +49,77 @@ __device__ __forceinline__ void tc_dealloc(u32 addr, u32 cols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// 16 columns of this warp's 32 tensor-memory lanes.
+// 16 columns of this warp's 32 tensor-memory lanes: issue, and wait for every
+// load issued (the registers pass through the wait, so that nothing reads
+// them before it).
 __device__ __forceinline__ void tc_ld16(float (&f)[16], u32 addr) {
-    u32 r[16];
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]), "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]),
+                   "=f"(f[8]), "=f"(f[9]), "=f"(f[10]), "=f"(f[11]), "=f"(f[12]), "=f"(f[13]), "=f"(f[14]), "=f"(f[15])
                  : "r"(addr));
-#pragma unroll
-    for (int i = 0; i < 16; i++) f[i] = __uint_as_float(r[i]);
 }
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tc_wait_ld(float (&f)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+f"(f[0]), "+f"(f[1]), "+f"(f[2]), "+f"(f[3]), "+f"(f[4]), "+f"(f[5]), "+f"(f[6]), "+f"(f[7]),
+                   "+f"(f[8]), "+f"(f[9]), "+f"(f[10]), "+f"(f[11]), "+f"(f[12]), "+f"(f[13]), "+f"(f[14]), "+f"(f[15])
+                 :: "memory");
+}
 __device__ __forceinline__ void mbar_arrive(u64* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+
+// ---------------------------------------------------------------------------
+// Tiles of digit rows.  A tile is 128 items (groups of 2^NV table entries
+// that one entry of the NV times folded table comes from) of two tables, an
+// item a row of 16 x 2^NV digit bytes: one atom of [128 rows][128 bytes] per
+// 8 values.  Rows 32 g + 16 h + p: item x = 16 g + .. of half h, the halves
+// being the two items of a folded pair.  MSB: value v of item m is entry
+// v N + m, halves m0 + x and m0 + x + H; LSB: value el of item o is entry
+// o 2^NV + el, halves the items 2 x and 2 x + 1 of m0 .. m0 + 127.
+// A unit is 16 bytes per lane of one warp; its two words are two items of one
+// value (MSB) or two values of one item (LSB).  The row order within a half
+// keeps the digit stores free of bank conflicts.
+template <bool LSB, int NV>
+struct TcTile {
+    static constexpr int VALS = 1 << NV, ATOMS = VALS / 8;
+    static constexpr u32 ATOM = 128 * 128, BYTES = 2 * ATOMS * ATOM;
+    static constexpr int UNITS = 4 * VALS;
+    static constexpr int LPI = VALS / 2, IPU = 32 / LPI;     // LSB: lanes per item, items per unit
+    __device__ __forceinline__ static int table(int unit) { return unit / (2 * VALS); }
+    __device__ __forceinline__ static u64 word(int unit, int lane, u64 m0, u64 H, u64 N) {
+        const int u = unit % (2 * VALS);
+        if (LSB) return (m0 + u * IPU + lane / LPI) * VALS + 2 * (lane % LPI);
+        return (u64)(u >> 1) * N + m0 + (u & 1) * H + 2 * lane;
+    }
+    __device__ __forceinline__ static void store(char* stage, int unit, int lane, const ulonglong2& v) {
+        const int u = unit % (2 * VALS);
+        char* base = stage + table(unit) * ATOMS * ATOM;
+        if (LSB) {
+            const u32 o = u * IPU + lane / LPI, h = o & 1, k = o >> 1, q = lane % LPI;
+            const u32 row = 32 * (k >> 4) + 16 * h + ((k & 15) ^ h);
+            // NV = 4: a quarter warp stores one row's 16 chunks in two turns,
+            // even ones of the first atom with odd ones of the second
+            const u32 sel = NV == 4 ? q >> 2 : 0;
+            base += (q >> 2) * ATOM;
+            *(uint4*)(base + swz128(row, (2 * q + sel) & 7)) = digits_of(sel ? v.y : v.x);
+            *(uint4*)(base + swz128(row, (2 * q + 1 - sel) & 7)) = digits_of(sel ? v.x : v.y);
+        } else {
+            const u32 val = u >> 1, row = 32 * (lane >> 3) + 16 * (u & 1) + (lane & 7);
+            base += (val >> 3) * ATOM;
+            *(uint4*)(base + swz128(row, val & 7)) = digits_of(v.x);
+            *(uint4*)(base + swz128(row + 8, val & 7)) = digits_of(v.y);
+        }
+    }
+    // Row 32 g + lane: which entry of the folded table (m0, H as above), and
+    // the lane of the pair's other half.
+    __device__ __forceinline__ static u64 entry(int g, int lane, u64 m0, u64 H) {
+        const int h = lane >> 4, p = lane & 15;
+        if (LSB) return m0 + 2 * (16 * g + (p ^ h)) + h;
+        return m0 + 16 * g + 2 * (p & 7) + (p >> 3) + h * H;
+    }
+    static constexpr int PARTNER = LSB ? 17 : 16;
+};
 
 }  // namespace effsc
