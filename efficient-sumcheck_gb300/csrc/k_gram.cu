@@ -29,8 +29,10 @@
 // (256 bytes written, 256 read by the MMAs) and 2 on the tensor core (NV = 4:
 // twice that), where the tables take 5.8 cycles to arrive.
 // Measured, n = 26: rounds 0-2 in 310 us on the integer pipes, 215 us here
-// with NV = 3, rounds 0-3 in 236 us with NV = 4 (4.5 TB/s; ~30 us of it the
-// last block's reduction and the four transcript steps).
+// with NV = 3, rounds 0-3 in 236 us with NV = 4 (~30 us of it the last block's
+// reduction and the four transcript steps) and 210 us with each tile asked into
+// L2 two tiles before its register loads (four ahead 216, eight 241) and
+// streaming loads.
 #include "ip012.cuh"
 #include "tc.cuh"
 
@@ -222,7 +224,7 @@ __global__ void __launch_bounds__(GR_TPB, 1) k_ip_gram(RoundArgs a, u32 ntiles) 
         for (int q = 0; q < AHEAD; q++)
             if ((u32)q < mine)
 #pragma unroll
-                for (int u = 0; u < UPW; u++) v[q][u] = *(const ulonglong2*)(X + word(q, u));
+                for (int u = 0; u < UPW; u++) v[q][u] = __ldcs((const ulonglong2*)(X + word(q, u)));
         for (u32 i0 = 0; i0 < mine && !abort; i0 += AHEAD) {
 #pragma unroll
             for (int q = 0; q < AHEAD; q++) {
@@ -237,7 +239,10 @@ __global__ void __launch_bounds__(GR_TPB, 1) k_ip_gram(RoundArgs a, u32 ntiles) 
                     for (int u = 0; u < UPW; u++) *(ulonglong2*)(M + word(i, u)) = v[q][u];
                 if (i + AHEAD < mine)
 #pragma unroll
-                    for (int u = 0; u < UPW; u++) v[q][u] = *(const ulonglong2*)(X + word(i + AHEAD, u));
+                    for (int u = 0; u < UPW; u++) v[q][u] = __ldcs((const ulonglong2*)(X + word(i + AHEAD, u)));
+                if (lane == 0 && i + AHEAD + TC_PREFETCH < mine)
+#pragma unroll
+                    for (int u = 0; u < UPW; u++) l2_prefetch(X + word(i + AHEAD + TC_PREFETCH, u), 512);
                 fence_async_shared();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sh.full[s]);

@@ -23,7 +23,10 @@
 //
 // Measured, n = 26: the triple fold and round 3 on the integer pipes 373 us
 // (and round 4 another 120); the fourfold fold and round 4 here 280 us
-// (4.6 TB/s).  Whole proof 1038 -> 857 us; LSB n = 24 458 -> 416.
+// (4.6 TB/s), 274 with tiles asked into L2 ahead.  Whole proof 1038 -> 857 us; LSB
+// n = 24 458 -> 416.  Not faster: a third group of epilogue warps (284 us, at
+// fewer registers), a third tile in registers (spills, 356), tensor-memory
+// loads one component ahead, streaming stores.
 #include "tc.cuh"
 
 #include <atomic>
@@ -162,7 +165,7 @@ __global__ void __launch_bounds__(TF_TPB, 1) k_tc_fold(RoundArgs a, u32 ntiles) 
         for (int q = 0; q < AHEAD; q++)
             if ((u32)q < mine)
 #pragma unroll
-                for (int u = 0; u < UPW; u++) v[q][u] = *(const ulonglong2*)(X + word(q, u));
+                for (int u = 0; u < UPW; u++) v[q][u] = __ldcs((const ulonglong2*)(X + word(q, u)));
         for (u32 i0 = 0; i0 < mine && !abort; i0 += AHEAD) {
 #pragma unroll
             for (int q = 0; q < AHEAD; q++) {
@@ -174,7 +177,10 @@ __global__ void __launch_bounds__(TF_TPB, 1) k_tc_fold(RoundArgs a, u32 ntiles) 
                 for (int u = 0; u < UPW; u++) Tile::store(stages + s * Tile::BYTES, warp * UPW + u, lane, v[q][u]);
                 if (i + AHEAD < mine)
 #pragma unroll
-                    for (int u = 0; u < UPW; u++) v[q][u] = *(const ulonglong2*)(X + word(i + AHEAD, u));
+                    for (int u = 0; u < UPW; u++) v[q][u] = __ldcs((const ulonglong2*)(X + word(i + AHEAD, u)));
+                if (lane == 0 && i + AHEAD + TC_PREFETCH < mine)
+#pragma unroll
+                    for (int u = 0; u < UPW; u++) l2_prefetch(X + word(i + AHEAD + TC_PREFETCH, u), 512);
                 fence_async_shared();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sh.full[s]);

@@ -67,6 +67,11 @@ __device__ __forceinline__ void tc_wait_ld(float (&f)[16]) {
 __device__ __forceinline__ void mbar_arrive(u64* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// Tiles ahead of the register loads that a unit's 512 bytes are asked into L2.
+constexpr int TC_PREFETCH = 2;
+__device__ __forceinline__ void l2_prefetch(const void* p, u32 bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 
