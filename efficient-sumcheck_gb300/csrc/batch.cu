@@ -1,7 +1,9 @@
 // batch.cu -- many independent Multilinear / InnerProduct (MSB) provers of
 // uneven size proved together: one kernel launch per step for every instance
 // still in its multi-block rounds (k_serve_step: each instance's segment runs
-// its own round, or the two-pass start of an InnerProduct proof over Fp3),
+// its own round), two launches before them for the tensor-core start of every
+// InnerProduct instance over Fp3 large enough for it (rounds 0-4, k_gram.cu and
+// k_tcfold.cu; smaller ones take the two-pass start of rounds 0-2 as steps),
 // one launch of the one-block tail kernel for every instance's last rounds,
 // one launch for all final folds; each instance keeps its own grid reduction
 // and Keccak transcript, and the whole protocol is captured once as a CUDA
@@ -56,6 +58,10 @@ struct effsc_batch {
     TailArgs* d_tail = nullptr;
     u32 n_tail = 0;
     u64 tail_smem_len = 0;
+    u32 n_tc = 0, tc_grid = 0;             // the tensor-core start's two launches
+    TcSeg* d_tc_segs = nullptr;
+    RoundArgs* d_tc_args = nullptr;        // n_tc of the first pass, then n_tc of the second
+    u64* d_tc_partials = nullptr;
     u32 rounds_planned = 0;                // step launches before the tail
     std::vector<size_t> seg_off, seg_cnt;  // per step into d_segs / d_args
     std::vector<u32> grid;                 // blocks per step
@@ -78,6 +84,9 @@ struct effsc_batch {
 
 namespace {
 
+// A table's share of the pool: tables start on 128-byte lines.
+size_t table_words(size_t w) { return (w + 15) / 16 * 16; }
+
 int deg_of(const effsc_batch* b) { return b->kind == EFFSC_ML ? 1 : 2; }
 
 void free_schedule(effsc_batch* b) {
@@ -88,6 +97,11 @@ void free_schedule(effsc_batch* b) {
     if (b->d_ext) cudaFreeAsync(b->d_ext, s);
     if (b->d_partials) cudaFreeAsync(b->d_partials, s);
     if (b->d_tail) cudaFreeAsync(b->d_tail, s);
+    if (b->d_tc_segs) cudaFreeAsync(b->d_tc_segs, s);
+    if (b->d_tc_args) cudaFreeAsync(b->d_tc_args, s);
+    if (b->d_tc_partials) cudaFreeAsync(b->d_tc_partials, s);
+    b->d_tc_segs = nullptr; b->d_tc_args = nullptr; b->d_tc_partials = nullptr;
+    b->n_tc = 0;
     b->d_tail = nullptr;
     b->n_tail = 0;
     b->d_segs = nullptr; b->d_args = nullptr; b->d_fin_args = nullptr; b->d_ext = nullptr; b->d_partials = nullptr;
@@ -110,18 +124,58 @@ int plan(effsc_batch* b) {
         if (tail_log < 2) b->tail_r0[i] = n_i;
         else b->tail_r0[i] = n_i <= tail_log ? 0 : n_i - tail_log + 1;
     }
+    // The tensor-core start: InnerProduct instances over Fp3 whose rounds 0-4
+    // are all multi-block, largest first (a block per SM at a time: the small
+    // ones fill the end).
+    std::vector<char> tc(b->n, 0);
+    std::vector<size_t> tc_order;
+    for (size_t i = 0; i < b->n; i++) {
+        tc[i] = b->kind == EFFSC_IP && F3W == 3 && b->tail_r0[i] >= 5 && b->nv[i] >= TC_MIN_LOG;
+        if (tc[i]) tc_order.push_back(i);
+    }
+    std::stable_sort(tc_order.begin(), tc_order.end(), [&](size_t x, size_t y) { return b->nv[x] > b->nv[y]; });
+    std::vector<TcSeg> tc_segs;
+    std::vector<RoundArgs> tc_args(2 * tc_order.size());
+    u32 tc_grid = 0;
+    u64 tc_total = 0;
+    for (size_t i : tc_order) tc_total += (1ULL << (b->nv[i] - 4)) / TC_TILE_ITEMS;
+    const u64 tc_per_block = tc_many_tiles(tc_total);
+    for (size_t k = 0; k < tc_order.size(); k++) {
+        const size_t i = tc_order[k];
+        const u64 tiles = (1ULL << (b->nv[i] - 4)) / TC_TILE_ITEMS;
+        const u64 nb = (tiles + tc_per_block - 1) / tc_per_block;
+        tc_segs.push_back({tc_grid, (u32)nb, (u32)tiles, 0});
+        for (int pass = 0; pass < 2; pass++) {
+            RoundArgs& a = tc_args[k + pass * tc_order.size()];
+            memset(&a, 0, sizeof a);
+            const u32 r = pass ? 4 : 0;
+            for (int t = 0; t < 2; t++) {
+                a.t[t].in[0] = b->in[i * 2 + t];
+                if (pass) for (int c = 0; c < 3; c++) a.t[t].out[c] = b->work[i * 2 + t] + c * (1ULL << (b->nv[i] - 1));
+            }
+            a.L = 1ULL << b->nv[i];
+            a.chal_ptr = b->d_chal + 3 * b->round_off[i];
+            a.counter = b->d_counters + i;
+            a.status = b->d_status;
+            a.tx.tx = b->d_tx + i;
+            a.tx.proof_wire = b->d_wire + 6 * (b->round_off[i] + r);
+            a.tx.proof_chal = b->d_chal + 3 * (b->round_off[i] + r);
+        }
+        tc_grid += (u32)nb;
+    }
     // steps: one launch each.  An InnerProduct instance over Fp3 whose first
     // three rounds are all multi-block takes two steps for them (ip01.cuh:
     // rounds 0-1, then round 2 with the double fold); every other round is
     // one step.  Step s of instance i runs round s, or for the two-pass
-    // start: rounds 0-1 (s = 0), round 2 (s = 1), round s + 1 (s >= 2).
+    // start: rounds 0-1 (s = 0), round 2 (s = 1), round s + 1 (s >= 2), and
+    // after the tensor-core start round s + 5.
     const int maxb = max_grid();
     std::vector<char> two(b->n, 0);
     std::vector<u32> nsteps(b->n, 0);
     u32 S = 0;
     for (size_t i = 0; i < b->n; i++) {
-        two[i] = b->kind == EFFSC_IP && F3W == 3 && b->tail_r0[i] >= 3;
-        nsteps[i] = two[i] ? b->tail_r0[i] - 1 : b->tail_r0[i];
+        two[i] = !tc[i] && b->kind == EFFSC_IP && F3W == 3 && b->tail_r0[i] >= 3;
+        nsteps[i] = tc[i] ? b->tail_r0[i] - 5 : two[i] ? b->tail_r0[i] - 1 : b->tail_r0[i];
         S = std::max<u32>(S, nsteps[i]);
     }
     std::vector<ServeSeg> segs;
@@ -158,7 +212,7 @@ int plan(effsc_batch* b) {
                 a.chal_ptr = st ? b->d_chal + 3 * b->round_off[i] : nullptr;
                 a.chal2_ptr = st ? b->d_chal + 3 * (b->round_off[i] + 1) : nullptr;
             } else {
-                r = two[i] ? st + 1 : st;
+                r = tc[i] ? st + 5 : two[i] ? st + 1 : st;
                 L = r == 0 ? (1ULL << n_i) : (1ULL << (n_i - r + 1));
                 work = r == 0 ? L / 2 : L / 4;
                 phase = r == 0 ? SERVE_EVAL : (r == 1 || F3W == 1) ? SERVE_FOLD_BASE : SERVE_FOLD_EXT;
@@ -244,6 +298,17 @@ int plan(effsc_batch* b) {
     }
     cudaStream_t s = b->stream;
     BCK(cudaMallocAsync((void**)&b->d_partials, max_blocks * 12 * sizeof(u64), s));
+    b->n_tc = (u32)tc_segs.size();
+    b->tc_grid = tc_grid;
+    if (b->n_tc) {
+        BCK(cudaMallocAsync((void**)&b->d_tc_partials, (size_t)tc_grid * 256 * sizeof(u64), s));
+        for (size_t k = 0; k < tc_args.size(); k++)
+            tc_args[k].partials = b->d_tc_partials + (size_t)tc_segs[k % tc_segs.size()].first_block * 256;
+        BCK(cudaMallocAsync((void**)&b->d_tc_segs, tc_segs.size() * sizeof(TcSeg), s));
+        BCK(cudaMallocAsync((void**)&b->d_tc_args, tc_args.size() * sizeof(RoundArgs), s));
+        BCK(cudaMemcpyAsync(b->d_tc_segs, tc_segs.data(), tc_segs.size() * sizeof(TcSeg), cudaMemcpyHostToDevice, s));
+        BCK(cudaMemcpyAsync(b->d_tc_args, tc_args.data(), tc_args.size() * sizeof(RoundArgs), cudaMemcpyHostToDevice, s));
+    }
     b->n_tail = (u32)tails.size();
     if (!tails.empty()) {
         BCK(cudaMallocAsync((void**)&b->d_tail, tails.size() * sizeof(TailArgs), s));
@@ -265,6 +330,12 @@ int plan(effsc_batch* b) {
 }
 
 int launch_protocol(effsc_batch* b, uint64_t* kernels) {
+    if (b->n_tc) {
+        if (!launch_ip_gram_many(b->d_tc_segs, b->n_tc, b->d_tc_args, b->tc_grid, b->stream) ||
+            !launch_tc_fold_many(b->d_tc_segs, b->n_tc, b->d_tc_args + b->n_tc, b->tc_grid, b->stream))
+            return effsc_set_error(EFFSC_CUDA_ERROR, "tensor-core start launch");
+        *kernels += 2;
+    }
     for (u32 st = 0; st < b->rounds_planned; st++) {
         if (!b->seg_cnt[st]) continue;
         launch_serve_step(b->d_segs + b->seg_off[st], (u32)b->seg_cnt[st], b->d_args + b->seg_off[st], b->grid[st],
@@ -318,7 +389,7 @@ int effsc_batch_create(effsc_ctx* ctx, int kind, int field, size_t n_inst, const
     const int F3W = field == EFFSC_FP3 ? 3 : 1;
     // one pool: inputs (2^n words per table) then work buffers (F3W * 2^(n-1))
     size_t words = 0;
-    for (size_t i = 0; i < n_inst; i++) words += (size_t)b->ntab * ((1ULL << b->nv[i]) + F3W * (1ULL << (b->nv[i] - 1)));
+    for (size_t i = 0; i < n_inst; i++) words += (size_t)b->ntab * (table_words(1ULL << b->nv[i]) + table_words(F3W * (1ULL << (b->nv[i] - 1))));
     cudaStream_t s = b->stream;
     auto bail = [&](int rc) { effsc_batch_destroy(b); return rc; };
     cudaError_t e = cudaMallocAsync((void**)&b->pool, words * sizeof(u64), s);
@@ -330,9 +401,9 @@ int effsc_batch_create(effsc_ctx* ctx, int kind, int field, size_t n_inst, const
         for (int t = 0; t < b->ntab; t++) {
             const size_t L = 1ULL << b->nv[i];
             b->in[i * b->ntab + t] = b->pool + off;
-            off += L;
+            off += table_words(L);
             b->work[i * b->ntab + t] = b->pool + off;
-            off += F3W * (L / 2);
+            off += table_words(F3W * (L / 2));
         }
     for (size_t i = 0; i < n_inst; i++)
         for (int t = 0; t < b->ntab; t++) {

@@ -36,8 +36,6 @@
 #include "ip012.cuh"
 #include "tc.cuh"
 
-#include <atomic>
-
 namespace effsc {
 
 constexpr int GR_LW = 16;                     // loading warps
@@ -184,9 +182,9 @@ __device__ __noinline__ void gram_rounds(typename Gram<LSB, NV>::Shared& sh, con
 
 // MIRROR: the tables are in host memory; every word loaded is also written
 // to the device buffers a.t[i].out[0] for the second pass.
+// Block bid of nb takes the tiles bid, bid + nb, ...
 template <bool LSB, int NV, bool MIRROR>
-__global__ void __launch_bounds__(GR_TPB, 1) k_ip_gram(RoundArgs a, u32 ntiles) {
-    chain_enter();
+__device__ __forceinline__ void gram_body(const RoundArgs& a, u32 ntiles, u32 bid, u32 nb) {
     using GT = Gram<LSB, NV>;
     using Tile = TcTile<LSB, NV>;
     constexpr int S = GT::S, UPW = GT::UPW, AHEAD = GT::AHEAD, V = GT::V;
@@ -208,8 +206,8 @@ __global__ void __launch_bounds__(GR_TPB, 1) k_ip_gram(RoundArgs a, u32 ntiles) 
     __syncthreads();
     tc_fence_after();
     const u32 tmem = sh.tmem;
-    const u32 G = gridDim.x;
-    const u32 mine = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / G + 1 : 0;   // this block's tiles
+    const u32 G = nb;
+    const u32 mine = bid < ntiles ? (ntiles - 1 - bid) / G + 1 : 0;   // this block's tiles
     bool abort = false;
     if (warp < GR_LW) {
         const u64 N = a.L >> NV;
@@ -217,7 +215,7 @@ __global__ void __launch_bounds__(GR_TPB, 1) k_ip_gram(RoundArgs a, u32 ntiles) 
         const u64* X = a.t[t].in[0];
         u64* M = MIRROR ? a.t[t].out[0] : nullptr;
         auto word = [&](u32 i, int u) {
-            return Tile::word(warp * UPW + u, lane, (a.tile0 + blockIdx.x + (u64)i * G) * 128, 64, N);
+            return Tile::word(warp * UPW + u, lane, (a.tile0 + bid + (u64)i * G) * 128, 64, N);
         };
         ulonglong2 v[AHEAD][UPW];
 #pragma unroll
@@ -281,9 +279,8 @@ __global__ void __launch_bounds__(GR_TPB, 1) k_ip_gram(RoundArgs a, u32 ntiles) 
         return;
     }
     // the blocks' sums: the last block adds them up
-    const u32 nb = gridDim.x;
     if (nb > 1) {
-        for (int i = threadIdx.x; i < V * V; i += GR_TPB) a.partials[(u64)blockIdx.x * V * V + i] = sh.g[i];
+        for (int i = threadIdx.x; i < V * V; i += GR_TPB) a.partials[(u64)bid * V * V + i] = sh.g[i];
         __threadfence();
         __syncthreads();
         if (threadIdx.x == 0) sh.last = atomicAdd(a.counter, 1u) == nb - 1;
@@ -325,21 +322,38 @@ __global__ void __launch_bounds__(GR_TPB, 1) k_ip_gram(RoundArgs a, u32 ntiles) 
     if (warp == 0) gram_rounds<LSB, NV>(sh, a);
 }
 
+template <bool LSB, int NV, bool MIRROR>
+__global__ void __launch_bounds__(GR_TPB, 1) k_ip_gram(RoundArgs a, u32 ntiles) {
+    chain_enter();
+    gram_body<LSB, NV, MIRROR>(a, ntiles, blockIdx.x, gridDim.x);
+}
+// The passes of many MSB proofs in one launch.
+__global__ void __launch_bounds__(GR_TPB, 1) k_ip_gram_many(const TcSeg* segs, u32 nsegs, const RoundArgs* args) {
+    __shared__ __align__(16) RoundArgs sa;
+    const TcSeg sg = tc_segment(segs, nsegs, args, sa);
+    gram_body<false, 4, false>(sa, sg.ntiles, blockIdx.x - sg.first_block, sg.nblocks);
+}
+
 u32 gram_max_tiles(void) { return GR_MAX_TILES; }
+u32 tc_many_tiles(u64 total) {
+    const u64 blocks = (u64)(max_grid() / 8) * 5 / 2;
+    const u64 t = (total + blocks - 1) / blocks;
+    return (u32)(t < 16 ? 16 : t > GR_MAX_TILES ? GR_MAX_TILES : t);
+}
 
 template <bool LSB, int NV, bool MIRROR>
 static bool gram_inst(const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s) {
     constexpr u32 SMEM = Gram<LSB, NV>::SMEM;
     static std::atomic<uint64_t> configured{0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return false;
-    const uint64_t bit = 1ull << (dev & 63);
-    if (!(configured.load() & bit)) {
-        if (cudaFuncSetAttribute(k_ip_gram<LSB, NV, MIRROR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) != cudaSuccess)
-            return false;
-        configured.fetch_or(bit);
-    }
+    if (!tc_allow_smem(k_ip_gram<LSB, NV, MIRROR>, SMEM, configured)) return false;
     return launch_chain(k_ip_gram<LSB, NV, MIRROR>, grid, GR_TPB, SMEM, s, a, ntiles);
+}
+bool launch_ip_gram_many(const TcSeg* segs, u32 nsegs, const RoundArgs* args, u32 grid, cudaStream_t s) {
+    constexpr u32 SMEM = Gram<false, 4>::SMEM;
+    static std::atomic<uint64_t> configured{0};
+    if (!tc_allow_smem(k_ip_gram_many, SMEM, configured)) return false;
+    k_ip_gram_many<<<grid, GR_TPB, SMEM, s>>>(segs, nsegs, args);
+    return true;
 }
 bool launch_ip_gram(bool lsb, int nv, bool mirror, const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s) {
     switch ((nv << 2) + (lsb ? 2 : 0) + (mirror ? 1 : 0)) {

@@ -29,8 +29,6 @@
 // loads one component ahead, streaming stores.
 #include "tc.cuh"
 
-#include <atomic>
-
 namespace effsc {
 
 constexpr int TF_LW = 16;                     // loading warps
@@ -98,9 +96,9 @@ __device__ __forceinline__ u64 join_digits(const float (&f)[16]) {
     return reduce96(lo32(lo), c1, c2);
 }
 
+// Block bid of nb takes the tiles bid, bid + nb, ...
 template <bool LSB, int NV>
-__global__ void __launch_bounds__(TF_TPB, 1) k_tc_fold(RoundArgs a, u32 ntiles) {
-    chain_enter();
+__device__ __forceinline__ void tc_fold_body(const RoundArgs& a, u32 ntiles, u32 bid, u32 nb) {
     using FT = TcFold<LSB, NV>;
     using Tile = TcTile<LSB, NV>;
     constexpr int S = FT::S, UPW = FT::UPW, AHEAD = FT::AHEAD, V = FT::V;
@@ -147,8 +145,8 @@ __global__ void __launch_bounds__(TF_TPB, 1) k_tc_fold(RoundArgs a, u32 ntiles) 
     __syncthreads();
     tc_fence_after();
     const u32 tmem = sh.tmem;
-    const u32 G = gridDim.x;
-    const u32 mine = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / G + 1 : 0;
+    const u32 G = nb;
+    const u32 mine = bid < ntiles ? (ntiles - 1 - bid) / G + 1 : 0;
     const u64 N = a.L >> NV, H = N >> 1;
     bool abort = false;
     ProdAcc<true, true> acc;
@@ -157,7 +155,7 @@ __global__ void __launch_bounds__(TF_TPB, 1) k_tc_fold(RoundArgs a, u32 ntiles) 
         const int t = Tile::table(warp * UPW);
         const u64* X = a.t[t].in[0];
         auto word = [&](u32 i, int u) {
-            const u64 tile = blockIdx.x + (u64)i * G;
+            const u64 tile = bid + (u64)i * G;
             return Tile::word(warp * UPW + u, lane, tile * (LSB ? 128 : 64), H, N);
         };
         ulonglong2 v[AHEAD][UPW];
@@ -219,7 +217,7 @@ __global__ void __launch_bounds__(TF_TPB, 1) k_tc_fold(RoundArgs a, u32 ntiles) 
             const u32 b = i % TF_BUFS;
             if (!mbar_wait_bounded(&sh.tfull[b], (i / TF_BUFS) & 1u)) { abort = true; break; }
             tc_fence_after();
-            const u64 m = Tile::entry(quad, lane, (blockIdx.x + (u64)i * G) * (LSB ? 128 : 64), H);
+            const u64 m = Tile::entry(quad, lane, (bid + (u64)i * G) * (LSB ? 128 : 64), H);
             F3 x[2];
 #pragma unroll
             for (int t = 0; t < 2; t++) {
@@ -270,13 +268,12 @@ __global__ void __launch_bounds__(TF_TPB, 1) k_tc_fold(RoundArgs a, u32 ntiles) 
         if (threadIdx.x == 0 && a.status) *(volatile u32*)a.status = EFFSC_STATUS_TIMEOUT;
         return;
     }
-    const u32 nb = gridDim.x;
     if (threadIdx.x < 6) {
         u64 s = 0;
 #pragma unroll
         for (int w = 0; w < 4 * TF_EG; w++) s = gl_add(s, (&sh.red[w][0][0])[threadIdx.x]);
         if (nb == 1) sh.tot[threadIdx.x] = s;
-        else a.partials[(u64)blockIdx.x * 6 + threadIdx.x] = s;
+        else a.partials[(u64)bid * 6 + threadIdx.x] = s;
     }
     if (nb > 1) {
         __threadfence();
@@ -303,17 +300,30 @@ __global__ void __launch_bounds__(TF_TPB, 1) k_tc_fold(RoundArgs a, u32 ntiles) 
 }
 
 template <bool LSB, int NV>
+__global__ void __launch_bounds__(TF_TPB, 1) k_tc_fold(RoundArgs a, u32 ntiles) {
+    chain_enter();
+    tc_fold_body<LSB, NV>(a, ntiles, blockIdx.x, gridDim.x);
+}
+// The passes of many MSB proofs in one launch.
+__global__ void __launch_bounds__(TF_TPB, 1) k_tc_fold_many(const TcSeg* segs, u32 nsegs, const RoundArgs* args) {
+    __shared__ __align__(16) RoundArgs sa;
+    const TcSeg sg = tc_segment(segs, nsegs, args, sa);
+    tc_fold_body<false, 4>(sa, sg.ntiles, blockIdx.x - sg.first_block, sg.nblocks);
+}
+
+template <bool LSB, int NV>
 static bool fold_inst(const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s) {
     constexpr u32 SMEM = TcFold<LSB, NV>::SMEM;
     static std::atomic<uint64_t> configured{0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return false;
-    const uint64_t bit = 1ull << (dev & 63);
-    if (!(configured.load() & bit)) {
-        if (cudaFuncSetAttribute(k_tc_fold<LSB, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) != cudaSuccess) return false;
-        configured.fetch_or(bit);
-    }
+    if (!tc_allow_smem(k_tc_fold<LSB, NV>, SMEM, configured)) return false;
     return launch_chain(k_tc_fold<LSB, NV>, grid, TF_TPB, SMEM, s, a, ntiles);
+}
+bool launch_tc_fold_many(const TcSeg* segs, u32 nsegs, const RoundArgs* args, u32 grid, cudaStream_t s) {
+    constexpr u32 SMEM = TcFold<false, 4>::SMEM;
+    static std::atomic<uint64_t> configured{0};
+    if (!tc_allow_smem(k_tc_fold_many, SMEM, configured)) return false;
+    k_tc_fold_many<<<grid, TF_TPB, SMEM, s>>>(segs, nsegs, args);
+    return true;
 }
 bool launch_tc_fold(bool lsb, int nv, const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s) {
     if (nv == 3) return lsb ? fold_inst<true, 3>(a, ntiles, grid, s) : fold_inst<false, 3>(a, ntiles, grid, s);

@@ -287,6 +287,21 @@ constexpr u32 TC_TILE_ITEMS = 128;
 bool launch_ip_gram(bool lsb, int nv, bool mirror, const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s);
 u32 gram_max_tiles(void);
 bool launch_tc_fold(bool lsb, int nv, const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s);
+// The same passes (MSB, nv = 4) of many proofs in one launch each: segment k
+// has nblocks blocks for the ntiles = (L >> 4) / TC_TILE_ITEMS tiles of
+// args[k] (at most gram_max_tiles() per block).
+struct TcSeg {
+    u32 first_block, nblocks, ntiles, reserved;
+};
+bool launch_ip_gram_many(const TcSeg* segs, u32 nsegs, const RoundArgs* args, u32 grid, cudaStream_t s);
+bool launch_tc_fold_many(const TcSeg* segs, u32 nsegs, const RoundArgs* args, u32 grid, cudaStream_t s);
+// Tiles per block of a launch over `total` tiles.  A block's fixed cost (setup,
+// reading its accumulators out, its partial sums) is about ten tiles' time and
+// an SM runs one block at a time, so two and a half waves of blocks: 128
+// proofs of 10..22 variables measured 1764 us a cohort at 64 tiles per block
+// (five waves), 1725 at 128, 1975 at 256.
+u32 tc_many_tiles(u64 total);
+constexpr u32 TC_MIN_LOG = 14;        // smallest table (entries, log2) they take
 // Consecutive InnerProduct rounds over Fp3 tables in one cooperative launch
 // (k_persist.cu): round k of the launch folds tables of length L0 >> k with
 // the previous challenge and evaluates; the last block to reach the grid

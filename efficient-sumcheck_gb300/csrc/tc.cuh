@@ -11,6 +11,8 @@
 #pragma once
 #include "round_common.cuh"
 
+#include <atomic>
+
 namespace effsc {
 
 __device__ __forceinline__ uint4 digits_of(u64 v) {
@@ -126,5 +128,39 @@ struct TcTile {
     }
     static constexpr int PARTNER = LSB ? 17 : 16;
 };
+
+// This block's segment of a launch over many proofs, its arguments in `sa`.
+__device__ __forceinline__ TcSeg tc_segment(const TcSeg* segs, u32 nsegs, const RoundArgs* args, RoundArgs& sa) {
+    __shared__ u32 s_k;
+    if (threadIdx.x == 0) {
+        u32 lo = 0, hi = nsegs - 1;
+        while (lo < hi) {
+            const u32 mid = (lo + hi + 1) >> 1;
+            if (segs[mid].first_block <= blockIdx.x) lo = mid; else hi = mid - 1;
+        }
+        s_k = lo;
+    }
+    __syncthreads();
+    const u32 k = s_k;
+    const u32* src = (const u32*)(args + k);
+    u32* dst = (u32*)&sa;
+    for (u32 w = threadIdx.x; w < sizeof(RoundArgs) / 4; w += blockDim.x) dst[w] = src[w];
+    __syncthreads();
+    return segs[k];
+}
+
+// The dynamic shared-memory limit is a per-device function attribute: set
+// once per device (one bit each), safe when threads race to set it.
+template <class K>
+inline bool tc_allow_smem(K kernel, u32 bytes, std::atomic<uint64_t>& configured) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const uint64_t bit = 1ull << (dev & 63);
+    if (!(configured.load() & bit)) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return false;
+        configured.fetch_or(bit);
+    }
+    return true;
+}
 
 }  // namespace effsc

@@ -87,3 +87,17 @@ def test_unaligned_and_pinned(E, lsb):
     pinned = [torch.from_numpy(t.view(np.int64)).pin_memory() for t in tabs]
     p = cls.from_host([t.numpy().view(np.uint64) for t in pinned])
     assert same(p.prove(n, E.Transcript.keccak(E.FP3, b"gram"), use_graph=False), want)
+
+
+@pytest.mark.parametrize("tail", [None, 0, 64])
+def test_batch_start(E, tail):
+    """A cohort whose larger instances share the two tensor-core launches
+    (one and several blocks each; tables behind odd-sized neighbours)."""
+    nv = [1, 14, 16, 3, 17, 15, 2, 19, 13, 18, 16]
+    tabs = [tables(v, "uniform", 50 + i) for i, v in enumerate(nv)]
+    b = E.Batch(E.IP, nv, tables=tabs)
+    b.set_tail(tail)
+    for rep in range(2):
+        proofs = b.prove([E.Transcript.keccak(E.FP3, b"gram") for _ in nv], use_graph=rep == 1)
+        for pf, t, v in zip(proofs, tabs, nv):
+            assert same(pf, oracle_proof(t, O.MSB, v)), v
