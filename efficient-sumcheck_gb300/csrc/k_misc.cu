@@ -156,13 +156,23 @@ void launch_join_aos(const u64* c0, const u64* c1, const u64* c2, u64 n, int nco
     k_join_aos<<<g, 256, 0, s>>>(c0, c1, c2, n, ncomp, aos, to_mont);
 }
 
+// dst[0..n) = src[0..n), src in device or GPU-readable host memory; bound by
+// the host link, 16 bytes a load where both ends allow it.
 __global__ void k_copy(const u64* src, u64* dst, u64 n) {
-    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) dst[i] = src[i];
+    const u64 tid = (u64)blockIdx.x * blockDim.x + threadIdx.x, stride = (u64)gridDim.x * blockDim.x;
+    u64 done = 0;
+    if ((((uintptr_t)src | (uintptr_t)dst) & 15) == 0) {
+        const u64 n2 = n >> 1;
+#pragma unroll 4
+        for (u64 i = tid; i < n2; i += stride) ((ulonglong2*)dst)[i] = __ldcs((const ulonglong2*)src + i);
+        done = n2 * 2;
+    }
+    for (u64 i = done + tid; i < n; i += stride) dst[i] = __ldcs(src + i);
 }
 void launch_copy(const u64* src, u64* dst, u64 n, cudaStream_t s) {
     if (!n) return;
-    u64 blocks = (n + 255) / 256;
-    int g = (int)(blocks < (u64)max_grid() * 2 ? blocks : (u64)max_grid() * 2);
+    u64 blocks = (n / 2 + 255) / 256;
+    int g = (int)(blocks < (u64)max_grid() * 2 ? (blocks ? blocks : 1) : (u64)max_grid() * 2);
     k_copy<<<g, 256, 0, s>>>(src, dst, n);
 }
 __global__ void k_fill(u64* dst, u64 n, u64 v) {

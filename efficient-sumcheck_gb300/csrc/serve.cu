@@ -41,6 +41,7 @@ void effsc_internal_tx_state(const effsc_transcript* t, void* out);
 int effsc_internal_ctx_device(const effsc_ctx* c);
 cudaStream_t effsc_internal_ctx_stream(const effsc_ctx* c);
 uint64_t effsc_internal_add_launches(uint64_t k);
+cudaError_t effsc_internal_upload(int device, u64* dst, const uint64_t* host, size_t words, cudaStream_t s, bool* in_place);
 
 #define SCK(call)                                                                                           \
     do {                                                                                                    \
@@ -60,6 +61,7 @@ constexpr int SERVE_INFLIGHT = 4;        // steps queued ahead of the GPU
 constexpr u32 MAX_ROUNDS = 34;
 constexpr size_t RES_WORDS = MAX_ROUNDS * 6 + MAX_ROUNDS * 3 + 3;   // wire | chal | final
 constexpr size_t TX_WORDS = (sizeof(DevTranscript) + 7) / 8;
+static_assert(sizeof(TcSeg) == sizeof(ServeSeg), "staged in the same array");
 
 double now_s() {
     using namespace std::chrono;
@@ -80,6 +82,8 @@ struct Req {
     u64* res = nullptr;    // RES_WORDS proof words | transcript | counter
     u32 round = 0;         // next round (n: finalize)
     bool two_pass = false; // InnerProduct over Fp3, n >= 3: rounds 0-2 in two steps (ip01.cuh)
+    bool tc = false;       // InnerProduct over Fp3, n >= TC_MIN_LOG: rounds 0-3, then round 4 with the
+                           // fourfold fold, on the tensor cores (k_gram.cu, k_tcfold.cu)
     bool in_tail = false;  // the remaining rounds are running in a tail launch
     cudaEvent_t tail_ev = nullptr;
     cudaEvent_t up_ev = nullptr;   // host tables: their upload on the lane's upload stream
@@ -139,6 +143,8 @@ struct Lane {
     ServeSeg* d_segs = nullptr;
     RoundArgs* d_args = nullptr;
     u64* d_partials = nullptr;
+    u64* d_tc_partials = nullptr;   // from the pool, grown in the lane stream's order
+    u32 tc_blocks = 0;
 };
 
 struct effsc_server {
@@ -239,6 +245,7 @@ int join_uploaded(effsc_server* s, Lane& ln, Lane::Stage& st, u32* ntx, std::vec
 
 int admit(effsc_server* s, Lane& ln, Lane::Stage& st, u32* ntx, std::vector<Req*>& fresh) {
     cudaStream_t cs = ln.stream;
+    bool pageable = false;
     TRYS(join_uploaded(s, ln, st, ntx, fresh));
     while (!ln.queue.empty() && s->n_active < s->max_active) {
         Req* r = ln.queue.front();
@@ -266,9 +273,11 @@ int admit(effsc_server* s, Lane& ln, Lane::Stage& st, u32* ntx, std::vector<Req*
             SCK(cudaEventRecord(e, cs));
             SCK(cudaStreamWaitEvent(ln.up_stream, e, 0));
             s->free_events.push_back(e);
-            for (int t = 0; t < r->ntab; t++)
-                SCK(cudaMemcpyAsync(r->in(t), r->htab[t], (1ULL << r->n) * sizeof(u64), cudaMemcpyHostToDevice,
-                                    ln.up_stream));
+            for (int t = 0; t < r->ntab; t++) {
+                bool in_place = false;
+                SCK(effsc_internal_upload(s->device, r->in(t), r->htab[t], 1ULL << r->n, ln.up_stream, &in_place));
+                pageable |= in_place;
+            }
             r->up_ev = get_event(s);
             SCK(cudaEventRecord(r->up_ev, ln.up_stream));
             ln.uploading.push_back(r);
@@ -277,6 +286,8 @@ int admit(effsc_server* s, Lane& ln, Lane::Stage& st, u32* ntx, std::vector<Req*
         for (int t = 0; t < r->ntab; t++) launch_gen_uniform(r->seeds[t], 1ULL << r->n, r->in(t), cs);
         TRYS(activate(s, ln, r, st, ntx, fresh));
     }
+    // pageable tables are the caller's again once they are admitted
+    if (pageable) SCK(cudaStreamSynchronize(ln.up_stream));
     return EFFSC_OK;
 }
 
@@ -284,10 +295,11 @@ int admit(effsc_server* s, Lane& ln, Lane::Stage& st, u32* ntx, std::vector<Req*
 u64 req_len(const Req& r) { return r.round == 0 ? (1ULL << r.n) : (1ULL << (r.n - r.round + 1)); }
 
 // The request's remaining rounds fit one tail launch: its tables fit in one
-// block's shared memory (not in the middle of the two-pass start).
+// block's shared memory (not in the middle of a two-pass start).
 bool tail_eligible(const Req& r) {
     if (r.in_tail || r.round >= r.n) return false;
     if (r.two_pass && (r.round == 1 || r.round == 2)) return false;
+    if (r.tc && r.round == 4) return false;
     const int pol = r.kind == EFFSC_IP ? POL_IP : POL_ML, fw = r.field == EFFSC_FP3 ? 3 : 1;
     return req_len(r) <= tail_max_len(pol, fw, TAIL_SMEM_CAP);
 }
@@ -343,7 +355,7 @@ int step(effsc_server* s, Lane& ln) {
     const int maxb = max_grid();
     const u64 per_block = (u64)KERNEL_TPB * s->quads_per_thread;
     u32 first = 0, nseg = 0;
-    std::vector<Req*> finals, tails;
+    std::vector<Req*> finals, tails, tcs[2];
     for (Req* r : ln.active) {
         if (r->in_tail) {
             const cudaError_t q = cudaEventQuery(r->tail_ev);
@@ -354,6 +366,10 @@ int step(effsc_server* s, Lane& ln) {
             r->in_tail = false;                      // round == n: the final fold below
         } else if (tail_eligible(*r)) {
             tails.push_back(r);
+            continue;
+        }
+        if (r->tc && (r->round == 0 || r->round == 4)) {
+            tcs[r->round == 4].push_back(r);
             continue;
         }
         const bool f3 = r->field == EFFSC_FP3;
@@ -431,6 +447,57 @@ int step(effsc_server* s, Lane& ln) {
         SCK(cudaEventRecord(st.pre, cs));
         SCK(cudaStreamWaitEvent(ln.tail_stream, st.pre, 0));
     }
+    // the tensor-core start's two passes, a launch each for every request
+    // that is at them (their arguments staged behind the step's)
+    u32 staged = nseg;
+    for (int pass = 0; pass < 2; pass++) {
+        std::vector<Req*>& v = tcs[pass];
+        if (v.empty()) continue;
+        std::stable_sort(v.begin(), v.end(), [](const Req* x, const Req* y) { return x->n > y->n; });
+        u64 total = 0;
+        for (const Req* r : v) total += (1ULL << (r->n - 4)) / TC_TILE_ITEMS;
+        const u64 per_block = tc_many_tiles(total);
+        TcSeg* segs = reinterpret_cast<TcSeg*>(st.h_segs) + staged;
+        u32 blocks = 0;
+        for (size_t k = 0; k < v.size(); k++) {
+            const Req* r = v[k];
+            const u64 tiles = (1ULL << (r->n - 4)) / TC_TILE_ITEMS;
+            segs[k] = {blocks, (u32)((tiles + per_block - 1) / per_block), (u32)tiles, 0};
+            RoundArgs& a = st.h_args[staged + k];
+            memset(&a, 0, sizeof a);
+            const u32 rd = pass ? 4 : 0;
+            for (int t = 0; t < 2; t++) {
+                a.t[t].in[0] = r->in(t);
+                if (pass) for (int c = 0; c < 3; c++) a.t[t].out[c] = r->work(t) + c * (1ULL << (r->n - 1));
+            }
+            a.L = 1ULL << r->n;
+            a.chal_ptr = r->chal();
+            a.counter = r->counter();
+            a.status = s->d_status;
+            a.tx.tx = r->tx();
+            a.tx.proof_wire = r->wire() + (size_t)6 * rd;
+            a.tx.proof_chal = r->chal() + 3 * rd;
+            blocks += segs[k].nblocks;
+        }
+        if (blocks > ln.tc_blocks) {
+            if (ln.d_tc_partials) SCK(cudaFreeAsync(ln.d_tc_partials, cs));
+            ln.d_tc_partials = nullptr;
+            ln.tc_blocks = 0;
+            SCK(cudaMallocFromPoolAsync((void**)&ln.d_tc_partials, (size_t)blocks * 256 * sizeof(u64), s->pool, cs));
+            ln.tc_blocks = blocks;
+        }
+        for (size_t k = 0; k < v.size(); k++) st.h_args[staged + k].partials = ln.d_tc_partials + (size_t)segs[k].first_block * 256;
+        SCK(cudaMemcpyAsync(ln.d_segs + staged, st.h_segs + staged, v.size() * sizeof(TcSeg), cudaMemcpyHostToDevice, cs));
+        SCK(cudaMemcpyAsync(ln.d_args + staged, st.h_args + staged, v.size() * sizeof(RoundArgs), cudaMemcpyHostToDevice, cs));
+        const TcSeg* ds = reinterpret_cast<const TcSeg*>(ln.d_segs + staged);
+        const bool ok = pass ? launch_tc_fold_many(ds, (u32)v.size(), ln.d_args + staged, blocks, cs)
+                             : launch_ip_gram_many(ds, (u32)v.size(), ln.d_args + staged, blocks, cs);
+        cudaError_t e = cudaGetLastError();
+        if (!ok || e != cudaSuccess) return effsc_set_error(EFFSC_CUDA_ERROR, "serving start launch: %s", cudaGetErrorString(e));
+        s->kernels++;
+        effsc_internal_add_launches(1);
+        staged += (u32)v.size();
+    }
     if (nseg) {
         for (u32 k = 0; k < nseg; k++) st.h_args[k].partials = ln.d_partials + (size_t)st.h_segs[k].first_block * 12;
         SCK(cudaMemcpyAsync(ln.d_segs, st.h_segs, nseg * sizeof(ServeSeg), cudaMemcpyHostToDevice, cs));
@@ -501,7 +568,7 @@ int step(effsc_server* s, Lane& ln) {
         if (r->in_tail) {
             still.push_back(r);            // its final fold comes after the tail
         } else if (r->round < r->n) {
-            r->round += (r->two_pass && r->round == 0) ? 2 : 1;
+            r->round += r->round ? 1 : r->tc ? 4 : r->two_pass ? 2 : 1;
             still.push_back(r);
         }
     }
@@ -537,7 +604,8 @@ int submit_one(effsc_server* s, int kind, int field, uint32_t num_vars, const ui
     }
     effsc_internal_tx_state(t, &r->tx0);
     if ((int)r->tx0.deg != field) { delete r; return effsc_set_error(EFFSC_INVALID_ARG, "transcript: wrong field or kind"); }
-    r->two_pass = kind == EFFSC_IP && field == EFFSC_FP3 && num_vars >= 3;
+    r->tc = kind == EFFSC_IP && field == EFFSC_FP3 && num_vars >= TC_MIN_LOG;
+    r->two_pass = !r->tc && kind == EFFSC_IP && field == EFFSC_FP3 && num_vars >= 3;
     r->bytes = req_bytes(*r);
     if (r->bytes > s->budget) {
         size_t b = r->bytes;
@@ -665,6 +733,7 @@ int effsc_server_destroy(effsc_server* s) {
         if (ln.d_segs) cudaFree(ln.d_segs);
         if (ln.d_args) cudaFree(ln.d_args);
         if (ln.d_partials) cudaFree(ln.d_partials);
+        if (ln.d_tc_partials) cudaFreeAsync(ln.d_tc_partials, ln.stream);
         if (ln.tail_stream) cudaStreamDestroy(ln.tail_stream);
         if (ln.up_stream) cudaStreamDestroy(ln.up_stream);
         if (ln.own_stream) cudaStreamDestroy(ln.stream);
