@@ -32,7 +32,7 @@
 // with NV = 3, rounds 0-3 in 236 us with NV = 4 (~30 us of it the last block's
 // reduction and the four transcript steps) and 210 us with each tile asked into
 // L2 two tiles before its register loads (four ahead 216, eight 241) and
-// streaming loads.
+// streaming loads, 206 with two stages instead of three (more L1 for the loads).
 #include "ip012.cuh"
 #include "tc.cuh"
 
@@ -49,7 +49,7 @@ struct Gram {
     static constexpr int V = 1 << NV;
     static constexpr int UPW = Tile::UNITS / GR_LW;       // units per warp and tile
     static constexpr int AHEAD = NV == 3 ? 4 : 2;         // tiles in flight in registers
-    static constexpr int S = NV == 3 ? 6 : 3;             // stages of 32 (64) KB
+    static constexpr int S = NV == 3 ? 4 : 2;             // stages of 32 (64) KB: the rest is L1 for the loads in flight
     static constexpr u32 SMEM = S * Tile::BYTES + 1024;
     static constexpr u32 COLS = NV == 3 ? 128 : 512;      // tensor memory
     static constexpr int NQ = ((1 << (2 * NV)) - 1) / 3;  // entries of the rounds' matrices
@@ -67,35 +67,17 @@ struct Gram {
     };
 };
 
-// Digit sums of 32 accumulator rows -> G (added to sh.g).  Row r of the x
-// side is digit r mod 16 of value r / 16.
+// The accumulators -> G, a warp per 32 rows (two of x's words).
 template <bool LSB, int NV>
 __device__ __forceinline__ void gram_collect(u32 tmem, typename Gram<LSB, NV>::Shared& sh) {
     constexpr int V = 1 << NV;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const u32 d = lane & 15, sft = 4 * (d < 8 ? 2 * d : 2 * (d - 8) + 1);   // this row's weight 2^sft
     const u32 addr = tmem + ((u32)(32 * (warp & 3)) << 16) + (warp >> 2) * 256;
     const int i = 2 * warp + (lane >> 4);
 #pragma unroll 1
     for (int j = 0; j < V; j++) {
-        float f[16];
-        tc_ld16(f, addr + 16 * j);
-        tc_wait_ld(f);
-        u64 lo = 0, hi = 0;
-#pragma unroll
-        for (int b = 7; b >= 0; b--) {
-            // low and high digit of byte b: below 2^29
-            const u32 s = (u32)(f[b] * 262144.0f) + 16 * (u32)(f[8 + b] * 262144.0f);
-            if (b >= 4) hi = (hi << 8) + s;
-            else lo = (lo << 8) + s;
-        }
-        // lo + hi 2^32, below 2^86
-        const u64 mid = (lo >> 32) + (hi & 0xFFFFFFFFu);
-        u64 v = gl_reduce_limbs((u32)lo, (u32)mid, (u32)((hi >> 32) + (mid >> 32)), 0, 0);
-        v = gl_mul(v, 1ULL << sft);
-#pragma unroll
-        for (int o = 8; o; o >>= 1) v = gl_add(v, __shfl_xor_sync(0xffffffffu, v, o));
-        if (d == 0) sh.g[V * i + j] = gl_add(sh.g[V * i + j], v);
+        const u64 v = tc_row_sum(addr + 16 * j, lane);
+        if ((lane & 15) == 0) sh.g[V * i + j] = v;
     }
 }
 

@@ -23,8 +23,9 @@
 //
 // Measured, n = 26: the triple fold and round 3 on the integer pipes 373 us
 // (and round 4 another 120); the fourfold fold and round 4 here 280 us
-// (4.6 TB/s), 274 with tiles asked into L2 ahead.  Whole proof 1038 -> 857 us; LSB
-// n = 24 458 -> 416.  Not faster: a third group of epilogue warps (284 us, at
+// with three stages, 245 (5.2 TB/s) with two: the loads in flight need the L1
+// that the stages leave (asking tiles into L2 ahead, 268, then costs more than it
+// gives).  Not faster: a third group of epilogue warps (284 against 274 us, at
 // fewer registers), a third tile in registers (spills, 356), tensor-memory
 // loads one component ahead, streaming stores.
 #include "tc.cuh"
@@ -44,7 +45,7 @@ struct TcFold {
     static constexpr int UPW = Tile::UNITS / TF_LW;
     static constexpr int AHEAD = NV == 3 ? 4 : 2;
     static constexpr u32 WBYTES = 48 * 128 * Tile::ATOMS;
-    static constexpr int S = NV == 3 ? 6 : 3;
+    static constexpr int S = NV == 3 ? 4 : 2;      // stages: the rest is L1 for the loads in flight
     static constexpr u32 SMEM = S * Tile::BYTES + WBYTES + 1024;
     struct Shared {
         u64 full[S], empty[S], tfull[TF_BUFS], tempty[TF_BUFS], done;
@@ -176,9 +177,6 @@ __device__ __forceinline__ void tc_fold_body(const RoundArgs& a, u32 ntiles, u32
                 if (i + AHEAD < mine)
 #pragma unroll
                     for (int u = 0; u < UPW; u++) v[q][u] = __ldcs((const ulonglong2*)(X + word(i + AHEAD, u)));
-                if (lane == 0 && i + AHEAD + TC_PREFETCH < mine)
-#pragma unroll
-                    for (int u = 0; u < UPW; u++) l2_prefetch(X + word(i + AHEAD + TC_PREFETCH, u), 512);
                 fence_async_shared();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sh.full[s]);
