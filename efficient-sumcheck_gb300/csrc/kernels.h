@@ -324,6 +324,11 @@ int persist_max_grid(bool lsb);
 // Fp, Fp3 challenges): rounds 0 and 1 from 15 sums of one read (partials of
 // 48 words per block, so at most max_grid() / 4 blocks), then the fold with
 // r0 and r1 at once (a.chal_ptr, a.chal2_ptr) and round 2 from a second read.
+// The first of them on the tensor cores (k_c3gram.cu): tiles a.tile0 ..
+// a.tile0 + ntiles - 1 of TC_TILE_ITEMS quadruples, tables (every component)
+// 16-byte aligned, at most gram_max_tiles() tiles per block; partials of 108
+// words per block, a.acc of 108.
+bool launch_c3_gram(bool lsb, bool e0, const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s);
 bool launch_c3_r01(bool lsb, bool e0, const RoundArgs& a, int grid, cudaStream_t s);
 bool launch_c3_r2x(bool lsb, bool e0, const RoundArgs& a, int grid, cudaStream_t s);
 bool launch_ml01(const RoundArgs& a, int grid, cudaStream_t s);

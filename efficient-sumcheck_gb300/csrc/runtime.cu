@@ -807,11 +807,30 @@ int do_coef3_first(effsc_prover* P, const TxIO& tx0, const TxIO& tx2, const u64*
     a.tx = tx0;
     a.L = L;
     for (int i = 0; i < 3; i++) set_in(a, i, P->t[i]);
-    // partials of 48 words per block: max_grid() / 4 blocks at most
-    const int g1 = std::min<int>(grid_for(L), max_grid() / 4);   // a quadruple per group thread
-    if (!dry) TRY(timed_launch(P->ctx->stream, "coef_rounds_0_1", (uint64_t)L * (e0 ? 40 : 24), [&] {
-        return launch_c3_r01(lsb, e0, a, g1, P->ctx->stream);
-    }));
+    // on the tensor cores where the tables load 16 bytes at a time, in launches
+    // of as many tiles as the blocks' accumulators hold; else on the integer
+    // pipes (partials of 48 words per block: max_grid() / 4 blocks at most)
+    uintptr_t bits = 0;
+    for (int i = 0; i < 3; i++)
+        for (int c = 0; c < (P->t[i].ext ? 3 : 1); c++) bits |= (uintptr_t)a.t[i].in[c];
+    const size_t tiles = L / 4 / TC_TILE_ITEMS, sms = max_grid() / 8, most = sms * gram_max_tiles();
+    if ((bits & 15) == 0 && L / 4 % TC_TILE_ITEMS == 0 && tiles < (1u << 31)) {
+        if (!P->d_acc) CK(cudaMallocAsync((void**)&P->d_acc, 256 * sizeof(u64), P->ctx->stream));
+        a.acc = P->d_acc;
+        for (size_t at = 0; at < tiles && !dry; at += most) {
+            const size_t cnt = std::min(most, tiles - at);
+            a.tile0 = (u32)at;
+            a.acc_mode = cnt == tiles ? ACC_NONE : at == 0 ? ACC_FIRST : at + cnt == tiles ? ACC_LAST : ACC_MID;
+            TRY(timed_launch(P->ctx->stream, "coef_rounds_0_1", (uint64_t)cnt * TC_TILE_ITEMS * (e0 ? 160 : 96), [&] {
+                return launch_c3_gram(lsb, e0, a, (u32)cnt, (int)std::min(cnt, sms), P->ctx->stream);
+            }));
+        }
+    } else if (!dry) {
+        const int g1 = std::min<int>(grid_for(L), max_grid() / 4);   // a quadruple per group thread
+        TRY(timed_launch(P->ctx->stream, "coef_rounds_0_1", (uint64_t)L * (e0 ? 40 : 24), [&] {
+            return launch_c3_r01(lsb, e0, a, g1, P->ctx->stream);
+        }));
+    }
     int bi[3];
     for (int i = 0; i < 3; i++) TRY(out_buffer(P, P->t[i], true, L / 4, true, &bi[i]));
     RoundArgs b = base_args(P);

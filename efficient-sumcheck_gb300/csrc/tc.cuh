@@ -77,6 +77,32 @@ __device__ __forceinline__ void l2_prefetch(const void* p, u32 bytes) {
 __device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 
+// One word of digit products: 32 accumulator rows x 16 columns at `addr`, rows
+// 16 q .. 16 q + 15 (lanes of half q) the digits of one word, the columns
+// those of another; the two words' sum of products mod p in every lane of the
+// half.
+__device__ __forceinline__ u64 tc_row_sum(u32 addr, int lane) {
+    const u32 d = lane & 15, sft = 4 * (d < 8 ? 2 * d : 2 * (d - 8) + 1);   // this row's weight 2^sft
+    float f[16];
+    tc_ld16(f, addr);
+    tc_wait_ld(f);
+    u64 lo = 0, hi = 0;
+#pragma unroll
+    for (int b = 7; b >= 0; b--) {
+        // low and high digit of byte b: below 2^29
+        const u32 s = (u32)(f[b] * 262144.0f) + 16 * (u32)(f[8 + b] * 262144.0f);
+        if (b >= 4) hi = (hi << 8) + s;
+        else lo = (lo << 8) + s;
+    }
+    // lo + hi 2^32, below 2^86
+    const u64 mid = (lo >> 32) + (hi & 0xFFFFFFFFu);
+    u64 v = gl_reduce_limbs((u32)lo, (u32)mid, (u32)((hi >> 32) + (mid >> 32)), 0, 0);
+    v = gl_mul(v, 1ULL << sft);
+#pragma unroll
+    for (int o = 8; o; o >>= 1) v = gl_add(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
 // ---------------------------------------------------------------------------
 // Tiles of digit rows.  A tile is 128 items (groups of 2^NV table entries
 // that one entry of the NV times folded table comes from) of two tables, an
