@@ -94,8 +94,12 @@ void launch_eqf_fold_rows(bool ew, bool ep, Tab3 p, Tab3 e, u64 Lc, u64 rows, u6
     else if (ew) k_eqf_fold_rows<true, false><<<g, TPB, 0, s>>>(p, e, Lc, rows, per, tiles, part);
     else if (ep) k_eqf_fold_rows<false, true><<<g, TPB, 0, s>>>(p, e, Lc, rows, per, tiles, part);
     else k_eqf_fold_rows<false, false><<<g, TPB, 0, s>>>(p, e, Lc, rows, per, tiles, part);
-    const u64 blocks = (Lc + TPB - 1) / TPB;
-    k_eqf_fold_sum<<<(int)(blocks < (u64)max_grid() ? blocks : (u64)max_grid()), TPB, 0, s>>>(part, Lc, splits, fw, o0, o1, o2);
+    launch_eqf_sum(part, Lc, splits, fw, o0, o1, o2, s);
+}
+
+void launch_eqf_sum(const u64* part, u64 n, u64 splits, int fw, u64* o0, u64* o1, u64* o2, cudaStream_t s) {
+    const u64 blocks = (n + TPB - 1) / TPB;
+    k_eqf_fold_sum<<<(int)(blocks < (u64)max_grid() ? blocks : (u64)max_grid()), TPB, 0, s>>>(part, n, splits, fw, o0, o1, o2);
 }
 
 }  // namespace effsc

@@ -236,6 +236,17 @@ void launch_eqf_inner(bool ee, bool ep, Tab3 p, Tab3 er, u64 m, u64 rows, u64* s
 void launch_eqf_fold_rows(bool ew, bool ep, Tab3 p, Tab3 e, u64 Lc, u64 rows, u64 splits, u64* part, int fw, u64* o0,
                           u64* o1, u64* o2, cudaStream_t s);
 
+// Both sums over a base table on the tensor cores (k_eqf_tc.cu): out[m] = sum
+// over k < K of w[k] P(k, m), m < M, P(k, m) = p[m stride + k] (along) or
+// p[k stride + m]; ew: Fp3 weights and sums.  part: 3 M eqf_tc_splits(M, K)
+// words (with one split unused).
+bool eqf_tc_ok(u64 M, u64 K, u64 stride, const u64* p);
+u32 eqf_tc_splits(u64 M, u64 K);
+bool launch_eqf_tc(bool along, bool ew, const u64* p, u64 stride, Tab3 w, u64 M, u64 K, u64* part, u64* o0, u64* o1, u64* o2,
+                   u32* status, cudaStream_t s);
+void launch_eqf_sum(const u64* part, u64 n, u64 splits, int fw, u64* o0, u64* o1, u64* o2, cudaStream_t s);
+constexpr u64 EQF_TC_MIN = 1ULL << 18;
+
 int pol_ntables(int pol);
 int pol_nraw(int pol);
 int pol_nwire(int pol);

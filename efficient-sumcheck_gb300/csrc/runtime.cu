@@ -1248,7 +1248,13 @@ int do_eqf_left(effsc_prover* P, const TxIO& tx, bool dry) {
     const u64 rows2 = (u64)1 << (vl - 1), Lc = p.len >> (vl - 1);
     const u64 splits = rows2 < 64 ? rows2 : 64;
     cudaStream_t s = P->ctx->stream;
-    const size_t need = 3 * rows + 3 * rows2 + 3 * splits * Lc;
+    // large base tables: both passes over p on the tensor cores
+    const u64* pb = p.bufs[p.cur].p[0];
+    const bool tc_in = !p.ext && er.ext == (fw == 3) && eqf_tc_ok(rows, m, m, pb);
+    const bool tc_fold = !p.ext && eqf_tc_ok(Lc, rows2, Lc, pb);
+    const size_t part_words = std::max<size_t>({(size_t)(3 * splits * Lc), tc_in ? (size_t)(3 * rows * eqf_tc_splits(rows, m)) : 0,
+                                                tc_fold ? (size_t)(3 * Lc * eqf_tc_splits(Lc, rows2)) : 0});
+    const size_t need = 3 * rows + 3 * rows2 + part_words;
     if (P->eqf_cap < need) {
         if (P->eqf_scratch) CK(cudaFreeAsync(P->eqf_scratch, s));
         P->eqf_scratch = nullptr;
@@ -1272,6 +1278,7 @@ int do_eqf_left(effsc_prover* P, const TxIO& tx, bool dry) {
         u64* s2 = fw == 3 ? S + 2 * rows : nullptr;
         const uint64_t b1 = p.len * wbytes(p.ext) + m * wbytes(er.ext) + rows * wbytes(out_ext);
         TRY(timed_launch(s, "eqf_inner_sums", b1, [&] {
+            if (tc_in) return launch_eqf_tc(true, fw == 3, pb, m, ter, rows, m, part, S, s1, s2, P->status, s);
             launch_eqf_inner(er.ext, p.ext, tp, ter, m, rows, S, s1, s2, s);
             return true;
         }));
@@ -1309,6 +1316,7 @@ int do_eqf_left(effsc_prover* P, const TxIO& tx, bool dry) {
         const Buf& ob = p.bufs[bp];
         const uint64_t b2 = p.len * wbytes(p.ext) + Lc * wbytes(p.ext || out_ext) + 2 * splits * Lc * 24;
         TRY(timed_launch(s, "eqf_fold_left", b2, [&] {
+            if (tc_fold) return launch_eqf_tc(false, fw == 3, pb, Lc, te, Lc, rows2, part, ob.p[0], ob.p[1], ob.p[2], P->status, s);
             launch_eqf_fold_rows(fw == 3, p.ext, tp, te, Lc, rows2, splits, part, fw, ob.p[0], ob.p[1], ob.p[2], s);
             return true;
         }));
