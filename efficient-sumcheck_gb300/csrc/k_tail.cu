@@ -268,12 +268,23 @@ __device__ __forceinline__ void tail_tx_init(TailTx& x, const TailArgs& a, int l
     x.w = tx_load((const DevTranscript*)a.tx, lane);
     x.s = tx_stream<NW>(a.hook, a.hook_len, lane);
 }
+// The wire values (word FW e + c in that lane) times the scalar, by a whole warp.
+template <int POL, int FW>
+__device__ __forceinline__ u64 tail_scale(u64 wire, const TailArgs& a, int lane) {
+    constexpr int NW = TailRoles<POL, FW>::N;
+    if (FW == 1) return lane < NW ? gl_mul(wire, a.scalar[0][0]) : 0;
+    const int e = 3 * (lane / 3) < NW ? 3 * (lane / 3) : 0;
+    const F3 x = f3_make(shfl64(wire, e), shfl64(wire, e + 1), shfl64(wire, e + 2));
+    const F3 y = f3_mul<true, true>(x, ld_scalar(a.scalar));
+    return lane >= NW ? 0 : lane % 3 == 0 ? y.c0 : lane % 3 == 1 ? y.c1 : y.c2;
+}
 // The transcript step of a round: send the wire values (word i of them in
 // lane i), absorb the hook, squeeze the challenge into sh.chal, prepared.
 template <int POL, int FW>
 __device__ __forceinline__ void tail_transcript(TailTx& x, u64 wire, const TailArgs& a, TailShared& sh) {
     constexpr int NW = TailRoles<POL, FW>::N;
     const int lane = threadIdx.x & 31;
+    if (POL == POL_IP && a.scalar[0]) wire = tail_scale<POL, FW>(wire, a, lane);
     if (lane < NW) sh.tot[FW == 3 ? lane : 3 * lane] = wire;
     const u64 r = tx_step<NW, FW>(x.w, x.s, wire, a.hook, a.hook_len, lane, sh.tot, sh.raw, sh.scr);
     if (lane < 3) sh.chal[2 + lane] = r;

@@ -168,6 +168,7 @@ struct TailArgs {
                            // challenge) before the tables are written back
     u64* first_out;        // (optional) the tables' first entries, 3 words per table, 4 tables
     u32 lsb;               // LSB prover: pairs (2j, 2j+1); held bit-reversed in shared memory
+    const u64* scalar[3];  // EqFactored right phase: the wire times eq_l[0] (null: none; c1, c2 null if base)
 };
 // Largest table length (a power of two) the tail kernel holds for this
 // policy and field width (1: Fp, 3: Fp3), within `smem_cap` bytes.

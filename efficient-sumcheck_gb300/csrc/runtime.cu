@@ -1332,6 +1332,73 @@ int do_eqf_left(effsc_prover* P, const TxIO& tx, bool dry) {
     return EFFSC_OK;
 }
 
+// EqFactored right phase from round r on in one tail launch: the rounds are
+// InnerProduct rounds on (eq_r, p), the wire times eq_l[0]
+// (src/provers/eq_factored.rs:178-209).  The first of them folds p and eq_l
+// with the last left challenge before, the others are the tail's own folds.
+// Leaves the state the per-round path and finalize leave.
+bool eqf_tail_ok(const effsc_prover* P, size_t r, size_t num_rounds, const Chal& ch, bool* boundary, ClusterSplit* cl) {
+    if (P->kind != EFFSC_EQF || !P->tail_len || P->v == 0 || P->rounds < P->v_l) return false;
+    if (r >= num_rounds || num_rounds - r >= 63 || (ch.has && !ch.dev)) return false;
+    *boundary = ch.has && P->rounds - 1 < P->v_l;
+    const size_t L = *boundary ? P->t[0].len / 2 : P->t[0].len, rounds = num_rounds - r;
+    if (!is_pow2(P->t[0].len) || !is_pow2(L) || P->t[2].len != L || L > P->tail_len) return false;
+    const bool first = ch.has && !*boundary;
+    const int fw = P->field == EFFSC_FP3 ? 3 : 1;
+    if (tail_cluster_split(POL_IP, fw, L, (u32)rounds, first, &cl->cs_log, &cl->g_log)) return true;
+    const size_t folds = rounds - (first ? 0 : 1);
+    return L <= (size_t)tail_max_len(POL_IP, fw, TAIL_SMEM_CAP) && (L >> folds) >= 2;
+}
+
+int do_eqf_tail(effsc_prover* P, size_t r, size_t num_rounds, const Chal& ch, const TxIO& tx, bool boundary,
+                ClusterSplit cl, bool dry) {
+    const int fw = P->field == EFFSC_FP3 ? 3 : 1;
+    const bool ext = fw == 3, first = ch.has && !boundary;
+    if (boundary) {
+        const bool ech = ch.ext || P->t[0].ext || P->t[1].ext || P->t[2].ext;
+        TRY(fold_table(P, 0, SEM_MSB_PAD, ch, ech, dry));
+        TRY(fold_table(P, 1, SEM_MSB_PAD, ch, ech, dry));
+    }
+    const size_t L = P->t[0].len, rounds = num_rounds - r, folds = rounds + (first ? 1 : 0);   // the finalize included
+    TailArgs ta;
+    memset(&ta, 0, sizeof ta);
+    ta.L = L;
+    ta.nrounds = (u32)rounds;
+    ta.first_fold = first ? 1 : 0;
+    ta.chal_in = ch.dev;
+    ta.tx = tx.tx;
+    ta.hook = tx.hook;
+    ta.hook_len = tx.hook_len;
+    ta.proof_wire = tx.proof_wire;
+    ta.proof_chal = tx.proof_chal;
+    ta.final_fold = 1;
+    const Buf& sb = P->t[1].bufs[P->t[1].cur];
+    for (int c = 0; c < (P->t[1].ext ? 3 : 1); c++) ta.scalar[c] = sb.p[c];
+    const int tab[2] = {2, 0};
+    uint64_t bytes = 0;
+    int bi[2];
+    for (int i = 0; i < 2; i++) {
+        Table& T = P->t[tab[i]];
+        for (int c = 0; c < 3; c++) ta.in[i][c] = T.bufs[T.cur].p[c];
+        if (T.ext) ta.in_ext |= 1u << i;
+        bytes += L * wbytes(T.ext) + (L >> folds) * wbytes(ext);
+        TRY(out_buffer(P, T, ext, L >> folds, true, &bi[i]));
+        for (int c = 0; c < 3; c++) ta.out[i][c] = T.bufs[bi[i]].p[c];
+    }
+    if (!dry) TRY(timed_launch(P->ctx->stream, "eqf_right_tail", bytes, [&] {
+        return cl.cs_log ? launch_tail_cluster(POL_IP, fw, ta, cl.cs_log, cl.g_log, P->ctx->stream)
+                         : launch_tail(POL_IP, fw, nullptr, &ta, 1, L, P->ctx->stream);
+    }));
+    for (int i = 0; i < 2; i++) {
+        Table& T = P->t[tab[i]];
+        T.cur = bi[i];
+        T.len = L >> folds;
+        T.ext = ext;
+    }
+    P->rounds += rounds;
+    return EFFSC_OK;
+}
+
 // One round of EqFactoredProver (src/provers/eq_factored.rs:249-270).
 int round_eqf(effsc_prover* P, const Chal& ch, const TxIO& tx, bool dry) {
     Table &p = P->t[0], &el = P->t[1], &er = P->t[2];
@@ -2411,7 +2478,7 @@ int effsc_prove(effsc_prover* P, size_t num_rounds, effsc_transcript* T, const u
 
     auto launch_all = [&](bool dry) -> int {
         size_t r0 = 0;
-        bool tail_done = false;
+        bool tail_done = false, finalized = false;   // by a tail: with the read-back entries, without
         if (fuse3_ok(P, num_rounds)) {
             TxIO t0;
             memset(&t0, 0, sizeof t0);
@@ -2503,6 +2570,12 @@ int effsc_prove(effsc_prover* P, size_t num_rounds, effsc_transcript* T, const u
                 tail_done = true;
                 break;
             }
+            bool boundary = false;
+            if (eqf_tail_ok(P, r, num_rounds, ch, &boundary, &cl)) {
+                TRY(do_eqf_tail(P, r, num_rounds, ch, tx, boundary, cl, dry));
+                finalized = true;
+                break;
+            }
             if (gkr_tail_ok(P, r, num_rounds, ch)) {
                 TRY(do_gkr_tail(P, r, num_rounds, ch, tx, dry, P->d_first));
                 tail_done = true;
@@ -2517,7 +2590,7 @@ int effsc_prove(effsc_prover* P, size_t num_rounds, effsc_transcript* T, const u
             TRY(do_round(P, ch, tx, dry));
         }
         if (tail_done) return EFFSC_OK;
-        if (num_rounds) {
+        if (num_rounds && !finalized) {
             Chal ch;
             ch.has = true; ch.ext = P->field == EFFSC_FP3; ch.dev = P->d_chals + 3 * (num_rounds - 1);
             TRY(do_finalize(P, ch, dry));
