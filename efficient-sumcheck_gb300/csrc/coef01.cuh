@@ -208,6 +208,7 @@ static __device__ __noinline__ F3 cubic_at(F3 g0, F3 g1, F3 g2, F3 ginf, F3 r) {
 static __device__ __noinline__ void finalize_c301(const u64* S, const RoundArgs& a) {
     __shared__ u64 s_w[2][9];
     __shared__ u64 s_c[2][3];
+    __shared__ u64 s_gen[9], s_raw[3];
     __shared__ __align__(8) uint8_t s_scr[64];
     const int lane = threadIdx.x & 31;
     // round 0: h0(u) = P(u, 0) + P(u, 1); P(u, 0) is point u of column x = 0
@@ -220,6 +221,8 @@ static __device__ __noinline__ void finalize_c301(const u64* S, const RoundArgs&
     __syncwarp();
     DevTranscript* T = (DevTranscript*)a.tx.tx;
     WarpTx w = tx_load(T, lane);
+    const int deg = (int)w.deg, nw = 3 * deg;
+    const TxStream st = tx_stream(nw, a.tx.hook, a.tx.hook_len, lane);
     for (int rd = 0; rd < 2; rd++) {
         if (rd == 1 && lane < 3) {
             // column x = 0, inf, 2 (wire order) is points 4 xi .. 4 xi + 3 with
@@ -232,12 +235,10 @@ static __device__ __noinline__ void finalize_c301(const u64* S, const RoundArgs&
             s_w[1][3 * lane] = v.c0; s_w[1][3 * lane + 1] = v.c1; s_w[1][3 * lane + 2] = v.c2;
         }
         __syncwarp();
-        tx_send_elems(w, lane, s_w[rd], 3);
-        if (a.tx.hook_len) {
-            const uint8_t* hk = a.tx.hook;
-            tx_absorb(w, lane, a.tx.hook_len, [&](u32 k) -> uint8_t { return hk[k]; });
-        }
-        tx_challenge(w, lane, s_c[rd], s_scr);
+        const u64 wire = lane < nw ? s_w[rd][deg == 3 ? lane : 3 * lane] : 0;
+        const u64 r = tx_step(w, st, nw, deg, wire, a.tx.hook, a.tx.hook_len, lane, s_gen, s_raw, s_scr);
+        if (lane < 3) s_c[rd][lane] = r;
+        __syncwarp();
     }
     tx_store(T, w, lane);
     if (lane < 18) a.tx.proof_wire[lane] = s_w[lane / 9][lane % 9];

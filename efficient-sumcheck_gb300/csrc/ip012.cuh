@@ -250,6 +250,7 @@ static __device__ __noinline__ void finalize_ip012(const u64* S, const RoundArgs
     __shared__ u64 s_w[3][6];
     __shared__ u64 s_c[3][3];
     __shared__ u64 s_g[2][3][3];   // round 2: [P0 / Pd][v][component], the quadratics in r0 at r0
+    __shared__ u64 s_gen[9], s_raw[3];
     __shared__ __align__(8) uint8_t s_scr[64];
     const int lane = threadIdx.x & 31;
     if (lane == 0) {
@@ -261,6 +262,8 @@ static __device__ __noinline__ void finalize_ip012(const u64* S, const RoundArgs
     __syncwarp();
     DevTranscript* T = (DevTranscript*)a.tx.tx;
     WarpTx w = tx_load(T, lane);
+    const int deg = (int)w.deg, nw = 2 * deg;
+    const TxStream st = tx_stream(nw, a.tx.hook, a.tx.hook_len, lane);
     for (int rd = 0; rd < 3; rd++) {
         if (rd > 0 && lane < (rd == 1 ? 8 : 2)) {
             // this lane's quadratic: values at 0, 1 and its leading coefficient
@@ -296,12 +299,10 @@ static __device__ __noinline__ void finalize_ip012(const u64* S, const RoundArgs
             }
         }
         __syncwarp();
-        tx_send_elems(w, lane, s_w[rd], 2);
-        if (a.tx.hook_len) {
-            const uint8_t* hk = a.tx.hook;
-            tx_absorb(w, lane, a.tx.hook_len, [&](u32 k) -> uint8_t { return hk[k]; });
-        }
-        tx_challenge(w, lane, s_c[rd], s_scr);
+        const u64 wire = lane < nw ? s_w[rd][deg == 3 ? lane : 3 * lane] : 0;
+        const u64 r = tx_step(w, st, nw, deg, wire, a.tx.hook, a.tx.hook_len, lane, s_gen, s_raw, s_scr);
+        if (lane < 3) s_c[rd][lane] = r;
+        __syncwarp();
     }
     tx_store(T, w, lane);
     if (lane < 18) a.tx.proof_wire[lane] = s_w[lane / 6][lane % 6];

@@ -116,7 +116,7 @@ template <bool LSB, int NV>
 __device__ __noinline__ void gram_rounds(typename Gram<LSB, NV>::Shared& sh, const RoundArgs& a) {
     const int lane = threadIdx.x & 31;
     WarpTx w = tx_load((const DevTranscript*)a.tx.tx, lane);
-    const TxStream st = tx_stream<6>(a.tx.hook, a.tx.hook_len, lane);
+    const TxStream st = tx_stream(6, a.tx.hook, a.tx.hook_len, lane);
     if (lane < 3) sh.w[0][lane] = lane == 0 ? 1 : 0;
     __syncwarp();
     int off = 0;
@@ -144,7 +144,7 @@ __device__ __noinline__ void gram_rounds(typename Gram<LSB, NV>::Shared& sh, con
             for (int j = 0; j < n; j++) acc_add64(s, sh.v[lane / 3][j][lane % 3]);
             wire = acc_reduce(s);
         }
-        const u64 r = tx_step<6, 3>(w, st, wire, a.tx.hook, a.tx.hook_len, lane, sh.tot, sh.raw, sh.scr);
+        const u64 r = tx_step(w, st, 6, 3, wire, a.tx.hook, a.tx.hook_len, lane, sh.tot, sh.raw, sh.scr);
         if (lane < 6) a.tx.proof_wire[6 * k + lane] = wire;
         if (lane < 3) a.tx.proof_chal[3 * k + lane] = r;
         off += n * n;

@@ -68,22 +68,6 @@ struct TailTab {
     u32 stride, off, len;
 };
 
-// Sum of a warp's canonical values as three sums of 22-bit pieces (50 cycles
-// for the three; five levels of shuffles and modular adds take 300).
-__device__ __forceinline__ uint4 warp_sum_pieces(u64 v) {
-    uint4 p;
-    p.x = __reduce_add_sync(0xffffffffu, (u32)v & 0x3FFFFFu);
-    p.y = __reduce_add_sync(0xffffffffu, (u32)(v >> 22) & 0x3FFFFFu);
-    p.z = __reduce_add_sync(0xffffffffu, (u32)(v >> 44));
-    p.w = 0;
-    return p;
-}
-// x + y 2^22 + z 2^44 mod p (x, y, z < 2^32).
-__device__ __forceinline__ u64 join_pieces(const uint4& p) {
-    const u64 t = (u64)p.z << 44, lo = (u64)p.x + ((u64)p.y << 22) + t;
-    return gl_reduce_limbs((u32)lo, (u32)(lo >> 32), (p.z >> 20) + (lo < t ? 1u : 0u), 0, 0);
-}
-
 // Component c of lo + (hi - lo) r; ch = the prepared challenge.
 template <int FW>
 __device__ __forceinline__ u64 tail_fold_comp(const u64* row0, u32 stride, u32 j, u32 half, int c, const u64* ch) {
@@ -266,7 +250,7 @@ struct TailTx {
 template <int NW>
 __device__ __forceinline__ void tail_tx_init(TailTx& x, const TailArgs& a, int lane) {
     x.w = tx_load((const DevTranscript*)a.tx, lane);
-    x.s = tx_stream<NW>(a.hook, a.hook_len, lane);
+    x.s = tx_stream(NW, a.hook, a.hook_len, lane);
 }
 // The wire values (word FW e + c in that lane) times the scalar, by a whole warp.
 template <int POL, int FW>
@@ -286,7 +270,7 @@ __device__ __forceinline__ void tail_transcript(TailTx& x, u64 wire, const TailA
     const int lane = threadIdx.x & 31;
     if (POL == POL_IP && a.scalar[0]) wire = tail_scale<POL, FW>(wire, a, lane);
     if (lane < NW) sh.tot[FW == 3 ? lane : 3 * lane] = wire;
-    const u64 r = tx_step<NW, FW>(x.w, x.s, wire, a.hook, a.hook_len, lane, sh.tot, sh.raw, sh.scr);
+    const u64 r = tx_step(x.w, x.s, NW, FW, wire, a.hook, a.hook_len, lane, sh.tot, sh.raw, sh.scr);
     if (lane < 3) sh.chal[2 + lane] = r;
     if (FW == 3 && (lane == 1 || lane == 2)) sh.chal[lane - 1] = gl_mul_w(r);
 }

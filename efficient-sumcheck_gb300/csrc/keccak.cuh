@@ -247,9 +247,9 @@ __device__ __forceinline__ void tx_challenge(WarpTx& w, int lane, u64* out, uint
 }
 
 // One round's transcript step (src/runner.rs:39-55) as a stream of 64-bit
-// words: NW wire words (word i in lane i), the hook's, the padding byte.
+// words: nw wire words (word i in lane i), the hook's, the padding byte.
 // While wire, hook and padding fit the block they start in -- always so after
-// a squeeze, for hooks of whole words up to 136 - 8 NW bytes -- the step is
+// a squeeze, for hooks of whole words up to 136 - 8 nw bytes -- the step is
 // one xor per lane (shifted to the byte position an open absorb left off at),
 // the permutation, and the challenge straight from the lanes that hold it.
 struct TxStream {
@@ -257,25 +257,23 @@ struct TxStream {
     u32 words;       // wire and hook
     bool whole;      // the hook is whole, aligned words
 };
-template <int NW>
-__device__ __forceinline__ TxStream tx_stream(const uint8_t* hook, u32 hook_len, int lane) {
+__device__ __forceinline__ TxStream tx_stream(int nw, const uint8_t* hook, u32 hook_len, int lane) {
     TxStream s;
     s.whole = (hook_len & 7) == 0 && ((uintptr_t)hook & 7) == 0 && hook_len < TX_RATE;
     const int hw = s.whole ? (int)(hook_len >> 3) : 0;
-    s.words = NW + hw;
-    s.fixed = lane >= NW && lane < NW + hw ? ((const u64*)hook)[lane - NW] : lane == NW + hw ? 0x06 : 0;
+    s.words = nw + hw;
+    s.fixed = lane >= nw && lane < nw + hw ? ((const u64*)hook)[lane - nw] : lane == nw + hw ? 0x06 : 0;
     return s;
 }
-// Component `lane` of the challenge in lanes 0 .. DEG-1, 0 in the others; by
+// Component `lane` of the challenge in lanes 0 .. deg-1, 0 in the others; by
 // a whole converged warp.  `v`, `raw`, `scr`: shared memory for the general
-// form (NW / DEG elements of 3 words, 3 words, 48 bytes).
-template <int NW, int DEG>
-__device__ __forceinline__ u64 tx_step(WarpTx& w, const TxStream& s, u64 wire, const uint8_t* hook, u32 hook_len, int lane,
-                                       u64* v, u64* raw, uint8_t* scr) {
+// form (nw / deg elements of 3 words, 3 words, 48 bytes).
+__device__ __forceinline__ u64 tx_step(WarpTx& w, const TxStream& s, int nw, int deg, u64 wire, const uint8_t* hook,
+                                       u32 hook_len, int lane, u64* v, u64* raw, uint8_t* scr) {
     const u32 pos = w.squeezing ? 0 : w.pos;
     __syncwarp();
     if (s.whole && pos + 8 * s.words < TX_RATE) {
-        u64 x = (lane < NW ? wire : 0) | s.fixed;
+        u64 x = (lane < nw ? wire : 0) | s.fixed;
         if (pos) {
             const int q = (int)(pos >> 3);
             const u32 sh = 8 * (pos & 7);
@@ -284,15 +282,15 @@ __device__ __forceinline__ u64 tx_step(WarpTx& w, const TxStream& s, u64 wire, c
         }
         w.a ^= x ^ (lane == TX_RATE / 8 - 1 ? 0x80ULL << 56 : 0);
         keccak_f_warp(w.a, lane);
-        w.pos = 16 * DEG;
+        w.pos = 16 * deg;
         w.squeezing = 1;
         const u64 lo = shfl64(w.a, (2 * lane) & 31), hi = shfl64(w.a, (2 * lane + 1) & 31);
-        return lane < DEG ? gl_reduce128(lo, hi) : 0;
+        return lane < deg ? gl_reduce128(lo, hi) : 0;
     }
-    if (lane < NW) v[DEG == 3 ? lane : 3 * lane] = wire;
+    if (lane < nw) v[deg == 3 ? lane : 3 * lane] = wire;
     __syncwarp();
-    tx_send_elems(w, lane, v, NW / DEG);
+    tx_send_elems(w, lane, v, nw / deg);
     if (hook_len) tx_absorb(w, lane, hook_len, [&](u32 k) -> uint8_t { return hook[k]; });
     tx_challenge(w, lane, raw, scr);
-    return lane < DEG ? raw[lane] : 0;
+    return lane < deg ? raw[lane] : 0;
 }

@@ -50,6 +50,22 @@ template <u32 M>
 __device__ __forceinline__ F3 ldm(const u64* const* p, u64 i, int t) {
     return ((M >> t) & 1u) ? ld<true>(p, i) : ld<false>(p, i);
 }
+// Sum of a warp's canonical values as three sums of 22-bit pieces (50 cycles
+// for the three; five levels of shuffles and modular adds take 300).
+__device__ __forceinline__ uint4 warp_sum_pieces(u64 v) {
+    uint4 p;
+    p.x = __reduce_add_sync(0xffffffffu, (u32)v & 0x3FFFFFu);
+    p.y = __reduce_add_sync(0xffffffffu, (u32)(v >> 22) & 0x3FFFFFu);
+    p.z = __reduce_add_sync(0xffffffffu, (u32)(v >> 44));
+    p.w = 0;
+    return p;
+}
+// x + y 2^22 + z 2^44 mod p (x, y, z < 2^32).
+__device__ __forceinline__ u64 join_pieces(const uint4& p) {
+    const u64 t = (u64)p.z << 44, lo = (u64)p.x + ((u64)p.y << 22) + t;
+    return gl_reduce_limbs((u32)lo, (u32)(lo >> 32), (p.z >> 20) + (lo < t ? 1u : 0u), 0, 0);
+}
+
 __device__ __forceinline__ u64 next_pow2_dev(u64 n) {
     return n <= 1 ? 1 : (1ULL << (64 - __clzll(n - 1)));
 }
@@ -228,6 +244,7 @@ __device__ __forceinline__ int pol_nwire_dev(int pol) {
 static __device__ __noinline__ void finalize_ip01(const u64* raw, const RoundArgs& a) {
     __shared__ u64 s_w[2][6];
     __shared__ u64 s_c[2][3];
+    __shared__ u64 s_gen[9], s_raw[3];
     __shared__ __align__(8) uint8_t s_scr[64];
     const int lane = threadIdx.x & 31;
     if (lane == 0) {
@@ -237,6 +254,8 @@ static __device__ __noinline__ void finalize_ip01(const u64* raw, const RoundArg
     __syncwarp();
     DevTranscript* T = (DevTranscript*)a.tx.tx;
     WarpTx w = tx_load(T, lane);
+    const int deg = (int)w.deg, nw = 2 * deg;
+    const TxStream st = tx_stream(nw, a.tx.hook, a.tx.hook_len, lane);
     for (int rd = 0; rd < 2; rd++) {
         if (rd == 1 && lane == 0) {
             const F3 r = f3_make(s_c[0][0], s_c[0][1], s_c[0][2]);
@@ -249,12 +268,10 @@ static __device__ __noinline__ void finalize_ip01(const u64* raw, const RoundArg
             s_w[1][3] = qi.c0; s_w[1][4] = qi.c1; s_w[1][5] = qi.c2;
         }
         __syncwarp();
-        tx_send_elems(w, lane, s_w[rd], 2);
-        if (a.tx.hook_len) {
-            const uint8_t* hk = a.tx.hook;
-            tx_absorb(w, lane, a.tx.hook_len, [&](u32 k) -> uint8_t { return hk[k]; });
-        }
-        tx_challenge(w, lane, s_c[rd], s_scr);
+        const u64 wire = lane < nw ? s_w[rd][deg == 3 ? lane : 3 * lane] : 0;
+        const u64 r = tx_step(w, st, nw, deg, wire, a.tx.hook, a.tx.hook_len, lane, s_gen, s_raw, s_scr);
+        if (lane < 3) s_c[rd][lane] = r;
+        __syncwarp();
     }
     tx_store(T, w, lane);
     if (lane < 12) a.tx.proof_wire[lane] = s_w[lane / 6][lane % 6];
@@ -267,12 +284,15 @@ static __device__ __noinline__ void finalize_ip01(const u64* raw, const RoundArg
 static __device__ __noinline__ void finalize_ml01(const u64* raw, const RoundArgs& a) {
     __shared__ u64 s_w[2][3];
     __shared__ u64 s_c[2][3];
+    __shared__ u64 s_gen[9], s_raw[3];
     __shared__ __align__(8) uint8_t s_scr[64];
     const int lane = threadIdx.x & 31;
     if (lane == 0) { s_w[0][0] = gl_add(raw[0], raw[1]); s_w[0][1] = 0; s_w[0][2] = 0; }
     __syncwarp();
     DevTranscript* T = (DevTranscript*)a.tx.tx;
     WarpTx w = tx_load(T, lane);
+    const int deg = (int)w.deg, nw = 1 * deg;
+    const TxStream st = tx_stream(nw, a.tx.hook, a.tx.hook_len, lane);
     for (int rd = 0; rd < 2; rd++) {
         if (rd == 1 && lane == 0) {
             const F3 r = f3_make(s_c[0][0], s_c[0][1], s_c[0][2]);
@@ -280,12 +300,10 @@ static __device__ __noinline__ void finalize_ml01(const u64* raw, const RoundArg
             s_w[1][0] = v.c0; s_w[1][1] = v.c1; s_w[1][2] = v.c2;
         }
         __syncwarp();
-        tx_send_elems(w, lane, s_w[rd], 1);
-        if (a.tx.hook_len) {
-            const uint8_t* hk = a.tx.hook;
-            tx_absorb(w, lane, a.tx.hook_len, [&](u32 k) -> uint8_t { return hk[k]; });
-        }
-        tx_challenge(w, lane, s_c[rd], s_scr);
+        const u64 wire = lane < nw ? s_w[rd][deg == 3 ? lane : 3 * lane] : 0;
+        const u64 r = tx_step(w, st, nw, deg, wire, a.tx.hook, a.tx.hook_len, lane, s_gen, s_raw, s_scr);
+        if (lane < 3) s_c[rd][lane] = r;
+        __syncwarp();
     }
     tx_store(T, w, lane);
     if (lane < 6) a.tx.proof_wire[lane] = s_w[lane / 3][lane % 3];
@@ -304,31 +322,42 @@ static __device__ __noinline__ void finalize_warp(int pol, const u64* raw, const
     }
     __shared__ u64 s_wire[9];
     __shared__ u64 s_aux[6];
+    __shared__ u64 s_gen[9];
     __shared__ u64 s_chal[3];
     __shared__ __align__(8) uint8_t s_scratch[64];
     const int lane = threadIdx.x & 31;
-    int nwire = pol_nwire_dev(pol);
-    if (lane == 0) {
+    const int nwire = pol_nwire_dev(pol);
+    DevTranscript* T = (DevTranscript*)a.tx.tx;
+    WarpTx w;
+    if (T) w = tx_load(T, lane);       // on its way while the wire is formed
+    if (pol == POL_ML || pol == POL_C1 || pol == POL_IP || pol == POL_EQFL || pol == POL_GKR) {
+        // the raw values are the wire and the pair (GKR: q(0) and c2; q is
+        // quadratic, so the reference's q(inf) = (q(0) + q(2) - 2 q(1)) / 2,
+        // src/provers/gkr.rs:185-189, is c2)
+        if (lane < 3 * nwire) s_wire[lane] = raw[lane];
+        if (lane < 6) s_aux[lane] = raw[lane];
+    } else if (pol == POL_C3W) {
+        // raw = h(0), h(2), h(inf): wire [h(0), h(inf), h(2)]; no pair
+        if (lane < 9) s_wire[lane] = raw[lane < 3 ? lane : lane < 6 ? lane + 3 : lane - 3];
+        if (lane < 6) s_aux[lane] = lane < 3 ? raw[lane] : 0;
+    } else if (lane == 0) {
         F3 r[4];
         for (int i = 0; i < 4; i++) r[i] = f3_make(raw[3 * i], raw[3 * i + 1], raw[3 * i + 2]);
-        F3 w[3];
+        F3 o[3];
         if (pol == POL_EQFR) {
             F3 sc = ld_scalar(a.scalar);
             r[0] = f3_mul<true, true>(r[0], sc);
             r[1] = f3_mul<true, true>(r[1], sc);
         }
         switch (pol) {
-        case POL_ML: case POL_C1:
-            w[0] = r[0];
-            break;
         case POL_C2:
-            w[0] = r[0]; w[1] = r[2];
+            o[0] = r[0]; o[1] = r[2];
             break;
         case POL_C3: {
             // r = h(0), h(1), h(2), h(inf): wire [h(0), h(inf), h(2)]; the
             // aux pair is (c0, c1) of h = c0 + c1 x + c2 x^2 + c3 x^3:
             // A = h(1) - c0 - c3 = c1 + c2, B = h(2) - c0 - 8 c3 = 2 c1 + 4 c2
-            w[0] = r[0]; w[1] = r[3]; w[2] = r[2];
+            o[0] = r[0]; o[1] = r[3]; o[2] = r[2];
             const u64 inv2 = 0x7FFFFFFF80000001ULL;   // (p + 1) / 2
             const F3 c3x2 = f3_add<true>(r[3], r[3]), c3x4 = f3_add<true>(c3x2, c3x2);
             const F3 A = f3_sub<true>(f3_sub<true>(r[1], r[0]), r[3]);
@@ -338,35 +367,25 @@ static __device__ __noinline__ void finalize_warp(int pol, const u64* raw, const
             r[1] = f3_sub<true>(A, c2);
             break;
         }
-        case POL_C3W:
-            // r = h(0), h(2), h(inf): wire [h(0), h(inf), h(2)]; no aux pair
-            w[0] = r[0]; w[1] = r[2]; w[2] = r[1];
-            r[1] = f3_zero();
-            break;
         case POL_X1: case POL_X2: case POL_X3: {
             // r = the coefficients c0..c3 of h; the EvalsInfty wire
             // (src/provers/coefficient.rs:272-294): [h(0)] for degree 1,
             // [h(0), h(inf)] for 2, [h(0), h(inf), h(2)] for 3; aux (c0, c1)
-            w[0] = r[0];
-            if (pol == POL_X2) w[1] = r[2];
+            o[0] = r[0];
+            if (pol == POL_X2) o[1] = r[2];
             if (pol == POL_X3) {
-                w[1] = r[3];
+                o[1] = r[3];
                 const F3 two = f3_make(2, 0, 0);
-                w[2] = f3_add<true>(f3_mul<true, true>(f3_add<true>(f3_mul<true, true>(
+                o[2] = f3_add<true>(f3_mul<true, true>(f3_add<true>(f3_mul<true, true>(
                     f3_add<true>(f3_mul<true, true>(r[3], two), r[2]), two), r[1]), two), r[0]);
             }
             break;
         }
-        case POL_GKR:
-            // r = q(0), c2: q is quadratic, so the reference's
-            // q(inf) = (q(0) + q(2) - 2 q(1)) / 2 (src/provers/gkr.rs:185-189) is c2
-            w[0] = r[0]; w[1] = r[1];
-            break;
-        default:   // IP, EQF
-            w[0] = r[0]; w[1] = r[1];
+        default:   // EQFR
+            o[0] = r[0]; o[1] = r[1];
             break;
         }
-        for (int i = 0; i < nwire; i++) { s_wire[3 * i] = w[i].c0; s_wire[3 * i + 1] = w[i].c1; s_wire[3 * i + 2] = w[i].c2; }
+        for (int i = 0; i < nwire; i++) { s_wire[3 * i] = o[i].c0; s_wire[3 * i + 1] = o[i].c1; s_wire[3 * i + 2] = o[i].c2; }
         s_aux[0] = r[0].c0; s_aux[1] = r[0].c1; s_aux[2] = r[0].c2;
         s_aux[3] = r[1].c0; s_aux[4] = r[1].c1; s_aux[5] = r[1].c2;
     }
@@ -375,25 +394,17 @@ static __device__ __noinline__ void finalize_warp(int pol, const u64* raw, const
         for (int i = lane; i < 3 * nwire; i += 32) a.result[i] = s_wire[i];
         if (lane < 6) a.result[3 * nwire + lane] = s_aux[lane];
     }
-    if (a.tx.tx) {
-        DevTranscript* T = (DevTranscript*)a.tx.tx;
-        WarpTx w = tx_load(T, lane);
-        tx_send_elems(w, lane, s_wire, nwire);
-        if (a.tx.hook_len) {
-            const uint8_t* hk = a.tx.hook;
-            if (((w.pos & 7) == 0 || w.squeezing) && (a.tx.hook_len & 7) == 0 && ((uintptr_t)hk & 7) == 0) {
-                const u64* hw = (const u64*)hk;
-                tx_absorb_words(w, lane, a.tx.hook_len >> 3, [&](u32 k) -> u64 { return hw[k]; });
-            } else {
-                tx_absorb(w, lane, a.tx.hook_len, [&](u32 k) -> uint8_t { return hk[k]; });
-            }
-        }
-        tx_challenge(w, lane, s_chal, s_scratch);
-        tx_store(T, w, lane);
+    if (T) {
+        // the step on the wire's words (one per component of the field)
+        const int deg = (int)w.deg, nw = nwire * deg;
+        const TxStream st = tx_stream(nw, a.tx.hook, a.tx.hook_len, lane);
+        const u64 wire = lane < nw ? s_wire[deg == 3 ? lane : 3 * lane] : 0;
+        const u64 r = tx_step(w, st, nw, deg, wire, a.tx.hook, a.tx.hook_len, lane, s_gen, s_chal, s_scratch);
         if (lane < 3) {
-            if (a.tx.chal_next) a.tx.chal_next[lane] = s_chal[lane];
-            if (a.tx.proof_chal) a.tx.proof_chal[lane] = s_chal[lane];
+            if (a.tx.chal_next) a.tx.chal_next[lane] = r;
+            if (a.tx.proof_chal) a.tx.proof_chal[lane] = r;
         }
+        tx_store(T, w, lane);
         if (a.tx.proof_wire)
             for (int i = lane; i < 3 * nwire; i += 32) a.tx.proof_wire[i] = s_wire[i];
     }
@@ -402,29 +413,30 @@ static __device__ __noinline__ void finalize_warp(int pol, const u64* raw, const
 // Block + grid reduction of NRAW Fp3 values over the nb blocks of one round
 // (this block is number bid); the last block to finish finalises.
 template <int NRAW>
-__device__ __forceinline__ void reduce_and_finalize_seg(F3 (&v)[NRAW], const RoundArgs& a, int pol, u32 nb, u32 bid) {
-    __shared__ u64 s_red[NWARP][RAW_WORDS];
+__device__ __forceinline__ void reduce_and_finalize_in(F3 (&v)[NRAW], const RoundArgs& a, int pol, u32 nb, u32 bid) {
+    // sums in 22-bit pieces: three integer warp reductions per word (five
+    // levels of shuffles and modular adds took four times the issue slots, on
+    // every warp and again in the last block)
+    __shared__ uint4 s_red[NWARP][3 * NRAW];
     __shared__ u64 s_tot[RAW_WORDS];
     __shared__ int s_last;
+    constexpr int NW = 3 * NRAW;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int off = 16; off; off >>= 1) {
-#pragma unroll
-        for (int i = 0; i < NRAW; i++) {
-            v[i].c0 = gl_add(v[i].c0, __shfl_down_sync(0xffffffffu, v[i].c0, off));
-            v[i].c1 = gl_add(v[i].c1, __shfl_down_sync(0xffffffffu, v[i].c1, off));
-            v[i].c2 = gl_add(v[i].c2, __shfl_down_sync(0xffffffffu, v[i].c2, off));
-        }
+    for (int i = 0; i < NW; i++) {
+        const uint4 p = warp_sum_pieces(i % 3 == 0 ? v[i / 3].c0 : i % 3 == 1 ? v[i / 3].c1 : v[i / 3].c2);
+        if (lane == 0) s_red[warp][i] = p;
     }
-    if (lane == 0) {
-#pragma unroll
-        for (int i = 0; i < NRAW; i++) { s_red[warp][3 * i] = v[i].c0; s_red[warp][3 * i + 1] = v[i].c1; s_red[warp][3 * i + 2] = v[i].c2; }
-    }
+    if (threadIdx.x >= NW && threadIdx.x < RAW_WORDS) s_tot[threadIdx.x] = 0;
     __syncthreads();
-    if (threadIdx.x < 3 * NRAW) {
-        u64 s = 0;
+    if (threadIdx.x < NW) {
+        uint4 p = s_red[0][threadIdx.x];
 #pragma unroll
-        for (int w = 0; w < NWARP; w++) s = gl_add(s, s_red[w][threadIdx.x]);
+        for (int w = 1; w < NWARP; w++) {
+            const uint4 q = s_red[w][threadIdx.x];
+            p.x += q.x; p.y += q.y; p.z += q.z;
+        }
+        const u64 s = join_pieces(p);
         if (nb == 1) s_tot[threadIdx.x] = s;
         else a.partials[(u64)bid * RAW_WORDS + threadIdx.x] = s;
     }
@@ -438,33 +450,40 @@ __device__ __forceinline__ void reduce_and_finalize_seg(F3 (&v)[NRAW], const Rou
         __syncthreads();
         if (!s_last) return;
         __threadfence();
-        // every thread owns one of the 3*NRAW words and walks the partials
-        // (unrolled so that several blocks' loads are in flight at once)
-        u64 acc[RAW_WORDS];
-#pragma unroll
-        for (int i = 0; i < 3 * NRAW; i++) acc[i] = 0;
-#pragma unroll 4
-        for (u32 b = threadIdx.x; b < nb; b += TPB)
-#pragma unroll
-            for (int i = 0; i < 3 * NRAW; i++) acc[i] = gl_add(acc[i], __ldcg(&a.partials[(u64)b * RAW_WORDS + i]));
-#pragma unroll
-        for (int off = 16; off; off >>= 1)
-            for (int i = 0; i < 3 * NRAW; i++) acc[i] = gl_add(acc[i], __shfl_down_sync(0xffffffffu, acc[i], off));
-        __syncthreads();
-        if (lane == 0)
-            for (int i = 0; i < 3 * NRAW; i++) s_red[warp][i] = acc[i];
-        __syncthreads();
-        if (threadIdx.x < 3 * NRAW) {
-            u64 s = 0;
-            for (int w = 0; w < NWARP; w++) s = gl_add(s, s_red[w][threadIdx.x]);
-            s_tot[threadIdx.x] = s;
+        // a warp per word over the blocks' partials, several loads in flight
+        for (int i = warp; i < NW; i += NWARP) {
+            Acc s = acc_zero();
+#pragma unroll 8
+            for (u32 b = lane; b < nb; b += 32) acc_add64(s, __ldcg(&a.partials[(u64)b * RAW_WORDS + i]));
+            const uint4 p = warp_sum_pieces(acc_reduce(s));
+            if (lane == 0) s_tot[i] = join_pieces(p);
         }
         if (threadIdx.x == 0) *a.counter = 0;
     }
     __syncthreads();
-    if (NRAW < 4 && threadIdx.x < 3 * (4 - NRAW)) s_tot[3 * NRAW + threadIdx.x] = 0;
-    __syncthreads();
     if (warp == 0) finalize_warp(pol, s_tot, a);
+}
+
+// Three and more values are reduced out of line: inlined into the Coefficient
+// kernels, which hold 128 registers already, the reduction costs their main
+// loop 4 to 12% (the first fused round of 2^24 entries 145 us, called 131);
+// for one and two values the call costs more (GKR's rounds 83 us, called 88).
+template <int NRAW>
+struct RawSums { F3 v[NRAW]; };
+template <int NRAW>
+__device__ __noinline__ void reduce_and_finalize_out(RawSums<NRAW> s, const RoundArgs& a, int pol, u32 nb, u32 bid) {
+    reduce_and_finalize_in<NRAW>(s.v, a, pol, nb, bid);
+}
+template <int NRAW>
+__device__ __forceinline__ void reduce_and_finalize_seg(F3 (&v)[NRAW], const RoundArgs& a, int pol, u32 nb, u32 bid) {
+    if constexpr (NRAW >= 3) {
+        RawSums<NRAW> s;
+#pragma unroll
+        for (int i = 0; i < NRAW; i++) s.v[i] = v[i];
+        reduce_and_finalize_out<NRAW>(s, a, pol, nb, bid);
+    } else {
+        reduce_and_finalize_in<NRAW>(v, a, pol, nb, bid);
+    }
 }
 
 template <int NRAW>
