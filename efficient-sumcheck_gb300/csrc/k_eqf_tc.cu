@@ -10,6 +10,10 @@
 // three products per word and read the weights again for every entry (74 and
 // 87 us at 2^24 entries, HBM alone 20).
 //
+// At 2^24 entries 47 and 41 us (four stages; three 48 and 43), two tables of
+// that size in one launch 71: about 30 us are the loads (128 blocks, 16 KB a
+// tile), a sixth the MMAs (eight of 48 columns a tile), the rest start and
+// recombination.
 // One block per SM: sixteen warps load p (16 bytes per lane and load, four
 // tiles of 32 terms ahead), one warp loads the weights, one thread issues
 // the MMAs; then the sixteen warps recombine the digits.
@@ -20,7 +24,7 @@ namespace effsc {
 constexpr int ET_M = 64, ET_K = 32;            // entries of a block, terms of a tile
 constexpr int ET_LW = 16;
 constexpr int ET_TPB = 32 * (ET_LW + 2);
-constexpr int ET_S = 3, ET_AHEAD = 4;
+constexpr int ET_S = 4, ET_AHEAD = 4;
 constexpr u32 ET_ATOM = ET_K * 128;            // eight entries' digits
 constexpr u32 ET_BYTES = 9 * ET_ATOM;          // eight atoms of p, one of the weights
 constexpr u32 ET_SMEM = ET_S * ET_BYTES + 1024;
@@ -29,11 +33,12 @@ constexpr u32 ET_SMEM = ET_S * ET_BYTES + 1024;
 // sixteen: no bank conflicts).
 __device__ __forceinline__ u32 et_row(u32 q) { return q ^ ((q >> 3) & 1); }
 
+// Blocks of M / 64 groups of entries of p, then as many of p2 (null: none).
 // ALONG: P(k, m) = p[m s + k]; else P(k, m) = p[k s + m].  out: component c of
-// entry m at o[c][m] (splits = 1) or part[3 (split M + m) + c].
+// entry m at part[3 (split M + m) + c], or without part (one split) at o[c][m].
 template <bool ALONG, bool EW>
-__global__ void __launch_bounds__(ET_TPB, 1) k_eqf_tc(const u64* p, u64 stride, Tab3 w, u64 M, u64 K, u32 splits, u64* part,
-                                                      u64* o0, u64* o1, u64* o2, u32* status) {
+__global__ void __launch_bounds__(ET_TPB, 1) k_eqf_tc(const u64* p, const u64* p2, u64 stride, Tab3 w, u64 M, u64 K,
+                                                      u32 splits, u64* part, u64* o0, u64* o1, u64* o2, u32* status) {
     constexpr int NC = EW ? 3 : 1;
     extern __shared__ char et_dyn[];
     __shared__ u64 full[ET_S], empty[ET_S], done;
@@ -54,7 +59,13 @@ __global__ void __launch_bounds__(ET_TPB, 1) k_eqf_tc(const u64* p, u64 stride, 
     tc_fence_after();
     const u32 tmem = s_tmem;
     const u32 split = blockIdx.x % splits;
-    const u64 m0 = (u64)(blockIdx.x / splits) * ET_M, kk = K / splits, k0 = split * kk;
+    u64 m0 = (u64)(blockIdx.x / splits) * ET_M;
+    if (m0 >= M) {                               // the second table's blocks
+        m0 -= M;
+        p = p2;
+        part += 3 * M * splits;
+    }
+    const u64 kk = K / splits, k0 = split * kk;
     const u32 tiles = (u32)(kk / ET_K);
     bool abort = false;
     if (warp < ET_LW) {
@@ -154,7 +165,7 @@ __global__ void __launch_bounds__(ET_TPB, 1) k_eqf_tc(const u64* p, u64 stride, 
             const u64 v = tc_row_sum(tmem + ((u32)(32 * (warp & 3)) << 16) + 64 * blk + 16 * c, lane);
             const u64 m = m0 + 8 * blk + 2 * (warp & 3) + (lane >> 4);
             if ((lane & 15) == 0) {
-                if (splits > 1) part[3 * (split * M + m) + c] = v;
+                if (part) part[3 * (split * M + m) + c] = v;
                 else (c == 0 ? o0 : c == 1 ? o1 : o2)[m] = v;
             }
         }
@@ -179,23 +190,32 @@ bool eqf_tc_ok(u64 M, u64 K, u64 stride, const u64* p) {
     return M * K >= EQF_TC_MIN && K / eqf_tc_splits(M, K) <= 65536 && (K / eqf_tc_splits(M, K)) % ET_K == 0;
 }
 template <bool ALONG, bool EW>
-static bool eqf_tc_inst(const u64* p, u64 stride, Tab3 w, u64 M, u64 K, u32 splits, u64* part, u64* o0, u64* o1, u64* o2,
-                        u32* status, cudaStream_t s) {
+static bool eqf_tc_inst(const u64* p, const u64* p2, u64 stride, Tab3 w, u64 M, u64 K, u32 splits, u64* part, u64* o0, u64* o1,
+                        u64* o2, u32* status, cudaStream_t s) {
     static std::atomic<uint64_t> configured{0};
     if (!tc_allow_smem(k_eqf_tc<ALONG, EW>, ET_SMEM, configured)) return false;
-    k_eqf_tc<ALONG, EW><<<(int)(M / ET_M * splits), ET_TPB, ET_SMEM, s>>>(p, stride, w, M, K, splits, part, o0, o1, o2, status);
+    k_eqf_tc<ALONG, EW><<<(int)((p2 ? 2 : 1) * (M / ET_M) * splits), ET_TPB, ET_SMEM, s>>>(p, p2, stride, w, M, K, splits, part, o0,
+                                                                                       o1, o2, status);
     return true;
 }
 bool launch_eqf_tc(bool along, bool ew, const u64* p, u64 stride, Tab3 w, u64 M, u64 K, u64* part, u64* o0, u64* o1, u64* o2,
                    u32* status, cudaStream_t s) {
     const u32 splits = eqf_tc_splits(M, K);
+    u64* pt = splits > 1 ? part : nullptr;
     bool ok;
-    if (along) ok = ew ? eqf_tc_inst<true, true>(p, stride, w, M, K, splits, part, o0, o1, o2, status, s)
-                       : eqf_tc_inst<true, false>(p, stride, w, M, K, splits, part, o0, o1, o2, status, s);
-    else ok = ew ? eqf_tc_inst<false, true>(p, stride, w, M, K, splits, part, o0, o1, o2, status, s)
-                 : eqf_tc_inst<false, false>(p, stride, w, M, K, splits, part, o0, o1, o2, status, s);
+    if (along) ok = ew ? eqf_tc_inst<true, true>(p, nullptr, stride, w, M, K, splits, pt, o0, o1, o2, status, s)
+                       : eqf_tc_inst<true, false>(p, nullptr, stride, w, M, K, splits, pt, o0, o1, o2, status, s);
+    else ok = ew ? eqf_tc_inst<false, true>(p, nullptr, stride, w, M, K, splits, pt, o0, o1, o2, status, s)
+                 : eqf_tc_inst<false, false>(p, nullptr, stride, w, M, K, splits, pt, o0, o1, o2, status, s);
     if (ok && splits > 1) launch_eqf_sum(part, M, splits, ew ? 3 : 1, o0, o1, o2, s);
     return ok;
+}
+bool launch_eqf_tc_pair(bool along, bool ew, const u64* p, const u64* p2, u64 stride, Tab3 w, u64 M, u64 K, u64* part,
+                        u32* status, cudaStream_t s) {
+    const u32 splits = eqf_tc_splits(2 * M, K);
+    if (along) return ew && eqf_tc_inst<true, true>(p, p2, stride, w, M, K, splits, part, nullptr, nullptr, nullptr, status, s);
+    return ew ? eqf_tc_inst<false, true>(p, p2, stride, w, M, K, splits, part, nullptr, nullptr, nullptr, status, s)
+              : eqf_tc_inst<false, false>(p, p2, stride, w, M, K, splits, part, nullptr, nullptr, nullptr, status, s);
 }
 
 }  // namespace effsc

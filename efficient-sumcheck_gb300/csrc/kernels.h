@@ -208,6 +208,27 @@ struct GkrTailArgs {
 // Needs 8 * fw * (len[0] + .. + len[3]) bytes <= TAIL_SMEM_CAP.
 bool launch_gkr_tail(int fw, const GkrTailArgs& a, u64 smem_bytes, cudaStream_t s);
 
+// A whole GkrProver proof from two reads of the gate tables (k_gkr_phase.cu):
+// the sums launch_eqf_tc_pair leaves over n entries, and the tables of 2n
+// entries (planes of 2n words a component) that two InnerProduct tails run on.
+struct GkrSums {
+    const u64* p;
+    u64 n;
+    u32 splits;
+};
+struct GkrFinish {
+    u64* out[4][3];        // add, mult, W_b, W_c: one entry each
+    u64* first;            // 3 words per table
+};
+constexpr u32 GKR_SMALL = 1024;   // up to this many entries of w, by the first two kernels instead of GkrSums
+bool launch_gkr_rows(const u64* add, const u64* mult, const u64* W, u32 n, u64* F, u64* G, cudaStream_t s);
+bool launch_gkr_cols(int fw, const u64* add, const u64* mult, const u64* W, const u64* wb, const u64* chals, u32 k, u64* F,
+                     u64* G, cudaStream_t s);
+bool launch_gkr_terms_b(const GkrSums& add, const GkrSums& mult, const u64* W, u64* F, u64* G, cudaStream_t s);
+bool launch_gkr_terms_c(int fw, const GkrSums& add, const GkrSums& mult, const u64* W, const u64* wb, u64* F, u64* G,
+                        cudaStream_t s);
+bool launch_gkr_finish(int fw, const u64* fb, const u64* fc, const u64* gc, const GkrFinish& o, cudaStream_t s);
+
 // Serving steps: one entry per request in the step, sorted by first_block;
 // `code` = SERVE_IP (else ML) | SERVE_FP3 (else Fp) | phase << SERVE_PHASE_SHIFT.
 struct ServeSeg {
@@ -245,6 +266,11 @@ bool eqf_tc_ok(u64 M, u64 K, u64 stride, const u64* p);
 u32 eqf_tc_splits(u64 M, u64 K);
 bool launch_eqf_tc(bool along, bool ew, const u64* p, u64 stride, Tab3 w, u64 M, u64 K, u64* part, u64* o0, u64* o1, u64* o2,
                    u32* status, cudaStream_t s);
+// The same over two tables at once (along: Fp3 weights), the sums of the
+// eqf_tc_splits(2 M, K) splits left in part: component c of entry m of split i
+// of table t at part[3 ((t splits + i) M + m) + c].
+bool launch_eqf_tc_pair(bool along, bool ew, const u64* p, const u64* p2, u64 stride, Tab3 w, u64 M, u64 K, u64* part,
+                        u32* status, cudaStream_t s);
 void launch_eqf_sum(const u64* part, u64 n, u64 splits, int fw, u64* o0, u64* o1, u64* o2, cudaStream_t s);
 constexpr u64 EQF_TC_MIN = 1ULL << 18;
 

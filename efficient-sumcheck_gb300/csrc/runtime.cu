@@ -366,6 +366,10 @@ int grid_for(u64 work, u64 per_thread = 1) {
     return (int)(g < mg ? g : mg);
 }
 
+// Whole proofs from two reads of the gate tables (k_gkr_phase.cu) from k = 4
+// on: at k = 3 the one-block tail alone is as fast (79 us against 81), at
+// k = 4 92 against 82, at k = 8 205 against 129.
+constexpr size_t GKR_PHASES_MIN = 4;
 // GkrProver passes whose b-variable pairs run in groups sharing one W_b entry
 // (k_gkr.cu): from GKR_RUNS_MIN pairs on, a grid of a quarter of the threads
 // gives each lane a run of four.  At most one wave of two blocks per SM (the
@@ -1160,6 +1164,111 @@ int do_gkr_tail(effsc_prover* P, size_t r, size_t num_rounds, const Chal& ch, co
         T.ext = fw == 3;
     }
     P->rounds = num_rounds;
+    return EFFSC_OK;
+}
+
+// effsc_prove of a whole GkrProver proof (2k rounds) over base tables: two
+// reads of the gate tables and two InnerProduct tails (k_gkr_phase.cu).
+// Leaves the state the per-round path and finalize leave.
+bool gkr_phases_ok(const effsc_prover* P, size_t num_rounds) {
+    if (!P->fuse_first || P->kind != EFFSC_GKR || P->rounds != 0 || P->v_l < GKR_PHASES_MIN || num_rounds != 2 * P->v_l) return false;
+    const u64 n = (u64)1 << P->v_l;
+    for (int i = 0; i < 4; i++) {
+        const Table& T = P->t[i];
+        if (T.ext || T.cur != 0 || T.len != (i < 2 ? n * n : n)) return false;
+    }
+    if (n > GKR_SMALL)
+        for (int i = 0; i < 2; i++)
+            if (!eqf_tc_ok(n, n, n, P->t[i].bufs[0].p[0])) return false;
+    const int fw = P->field == EFFSC_FP3 ? 3 : 1;
+    u32 cs, g;
+    if (2 * n > P->tail_len) return false;
+    return tail_cluster_split(POL_IP, fw, 2 * n, (u32)P->v_l, false, &cs, &g) || 2 * n <= tail_max_len(POL_IP, fw, TAIL_SMEM_CAP);
+}
+
+int do_gkr_phases(effsc_prover* P, const TxIO& tx, bool dry, u64* first) {
+    const int fw = P->field == EFFSC_FP3 ? 3 : 1;
+    const u32 k = (u32)P->v_l;
+    const u64 n = (u64)1 << k;
+    cudaStream_t s = P->ctx->stream;
+    const bool tc = n > GKR_SMALL;
+    const u32 splits = tc ? eqf_tc_splits(2 * n, n) : 0;
+    // the weights 1, eq weights, F, G, the tails' last tables, the splits' sums
+    const size_t need = n + 3 * n + 6 * n + 6 * n + 24 + 6 * n * splits;
+    if (P->eqf_cap < need) {
+        if (P->eqf_scratch) CK(cudaFreeAsync(P->eqf_scratch, s));
+        P->eqf_scratch = nullptr;
+        CK(cudaMallocAsync((void**)&P->eqf_scratch, need * sizeof(u64), s));
+        P->eqf_cap = need;
+        const std::vector<u64> one(n, 1);
+        CK(cudaMemcpyAsync(P->eqf_scratch, one.data(), n * sizeof(u64), cudaMemcpyHostToDevice, s));
+        CK(cudaStreamSynchronize(s));
+    }
+    u64 *ones = P->eqf_scratch, *Ew = ones + n, *F = Ew + 3 * n, *G = F + 6 * n, *last = G + 6 * n;
+    u64 *pa = last + 24, *pm = pa + 3 * n * splits;
+    int bi[4];
+    for (int i = 0; i < 4; i++) TRY(out_buffer(P, P->t[i], fw == 3, 1, true, &bi[i]));
+    if (!dry) {
+        const u64 *add = P->t[0].bufs[0].p[0], *mult = P->t[1].bufs[0].p[0], *W = P->t[2].bufs[0].p[0];
+        const GkrSums sa = {pa, n, splits}, sm = {pm, n, splits};
+        const uint64_t gate = 8 * n * n, sums = 24 * n * splits;
+        // rounds r0 .. r0 + k - 1 on F and G, their last tables at `last` + 12 i
+        auto tail = [&](int i, u32 ext) -> int {
+            TailArgs ta;
+            memset(&ta, 0, sizeof ta);
+            for (int c = 0; c < 3; c++) {
+                ta.in[0][c] = F + 2 * n * c;
+                ta.in[1][c] = G + 2 * n * c;
+                ta.out[0][c] = last + 12 * i + 2 * c;
+                ta.out[1][c] = last + 12 * i + 6 + 2 * c;
+            }
+            ta.in_ext = ext;
+            ta.L = 2 * n;
+            ta.nrounds = k;
+            ta.tx = tx.tx;
+            ta.hook = tx.hook;
+            ta.hook_len = tx.hook_len;
+            ta.proof_wire = tx.proof_wire + (size_t)i * k * 6;
+            ta.proof_chal = tx.proof_chal + (size_t)i * k * 3;
+            ta.final_fold = 1;
+            ClusterSplit cl;
+            const bool clus = tail_cluster_split(POL_IP, fw, 2 * n, k, false, &cl.cs_log, &cl.g_log);
+            return timed_launch(s, i ? "gkr_c_tail" : "gkr_b_tail", 4 * n * wbytes(ext != 0), [&] {
+                return clus ? launch_tail_cluster(POL_IP, fw, ta, cl.cs_log, cl.g_log, s)
+                            : launch_tail(POL_IP, fw, nullptr, &ta, 1, 2 * n, s);
+            });
+        };
+        if (tc) {
+            const Tab3 w1 = {{W, ones, ones}};
+            TRY(timed_launch(s, "gkr_row_sums", 2 * (gate + sums), [&] { return launch_eqf_tc_pair(true, true, add, mult, n, w1, n, n, pa, P->status, s); }));
+            TRY(timed_launch(s, "gkr_terms_b", 2 * sums + 40 * n, [&] { return launch_gkr_terms_b(sa, sm, W, F, G, s); }));
+        } else {
+            TRY(timed_launch(s, "gkr_rows", 2 * gate + 40 * n, [&] { return launch_gkr_rows(add, mult, W, (u32)n, F, G, s); }));
+        }
+        TRY(tail(0, 0));
+        if (tc) {
+            const Tab3 we = {{Ew, Ew + n, Ew + 2 * n}};
+            TRY(timed_launch(s, "gkr_eq_weights", 8 * fw * n, [&] { return launch_build_eq(P->d_chals, k, fw == 3, Ew, Ew + n, Ew + 2 * n, s); }));
+            TRY(timed_launch(s, "gkr_column_sums", 2 * (gate + sums), [&] { return launch_eqf_tc_pair(false, fw == 3, add, mult, n, we, n, n, pa, P->status, s); }));
+            TRY(timed_launch(s, "gkr_terms_c", 2 * sums + 8 * n + 32 * fw * n, [&] { return launch_gkr_terms_c(fw, sa, sm, W, last, F, G, s); }));
+        } else {
+            TRY(timed_launch(s, "gkr_columns", 2 * gate + 32 * fw * n, [&] { return launch_gkr_cols(fw, add, mult, W, last, P->d_chals, k, F, G, s); }));
+        }
+        TRY(tail(1, fw == 3 ? 3u : 0u));
+        GkrFinish o;
+        memset(&o, 0, sizeof o);
+        for (int t = 0; t < 4; t++)
+            for (int c = 0; c < fw; c++) o.out[t][c] = P->t[t].bufs[bi[t]].p[c];
+        o.first = first;
+        TRY(timed_launch(s, "gkr_finish", 16 * 4 * fw, [&] { return launch_gkr_finish(fw, last, last + 12, last + 18, o, s); }));
+    }
+    for (int i = 0; i < 4; i++) {
+        Table& T = P->t[i];
+        T.cur = bi[i];
+        T.len = 1;
+        T.ext = fw == 3;
+    }
+    P->rounds = 2 * k;
     return EFFSC_OK;
 }
 
@@ -2527,6 +2636,16 @@ int effsc_prove(effsc_prover* P, size_t num_rounds, effsc_transcript* T, const u
             t2.proof_chal = P->d_chals + 3 * 2;
             TRY(do_ml_first(P, t0, t2, P->d_chals, dry));
             r0 = 3;
+        } else if (gkr_phases_ok(P, num_rounds)) {
+            TxIO t0;
+            memset(&t0, 0, sizeof t0);
+            t0.tx = P->d_tx;
+            t0.hook = P->d_hook;
+            t0.hook_len = (u32)hook_len;
+            t0.proof_wire = P->d_wire;
+            t0.proof_chal = P->d_chals;
+            TRY(do_gkr_phases(P, t0, dry, P->d_first));
+            return EFFSC_OK;
         } else if (gkr_first_ok(P, num_rounds)) {
             TxIO t0, t2;
             memset(&t0, 0, sizeof t0);
