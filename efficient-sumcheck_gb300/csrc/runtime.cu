@@ -2001,10 +2001,10 @@ cudaError_t effsc_internal_upload(int device, u64* dst, const uint64_t* host, si
     }
     return cudaMemcpyAsync(dst, host, words * sizeof(u64), cudaMemcpyHostToDevice, s);
 }
-void* effsc_internal_pinned_get(effsc_ctx* c, size_t bytes) { return pinned_get(c, bytes); }
-void effsc_internal_pinned_put(effsc_ctx* c, void* p, size_t bytes) { pinned_put(c, p, bytes); }
 int effsc_internal_ctx_device(const effsc_ctx* c) { return c->device; }
 cudaStream_t effsc_internal_ctx_stream(const effsc_ctx* c) { return c->stream; }
+void* effsc_internal_pinned_get(effsc_ctx* c, size_t bytes) { return pinned_get(c, bytes); }
+void effsc_internal_pinned_put(effsc_ctx* c, void* p, size_t bytes) { pinned_put(c, p, bytes); }
 uint64_t effsc_internal_add_launches(uint64_t k) { g_launches += k; return g_launches; }
 
 // ===========================================================================
