@@ -38,8 +38,17 @@ T_KECCAK, T_TEST = 0, 1
 P = 0xFFFFFFFF00000001
 
 
+_Words = ctypes.c_uint64 * 0
+
+
 def _p(a):
-    return a.ctypes.data_as(u64p)
+    """A pointer to the array's words, holding the array (through its buffer
+    0.7 us; the ndarray's own ctypes view, for what cannot lend a writable
+    one, 4.9)."""
+    try:
+        return _Words.from_buffer(a)
+    except (TypeError, ValueError):
+        return a.ctypes.data_as(u64p)
 
 
 def _bytes(b):
@@ -82,6 +91,8 @@ def launch_count_reset():
 
 def _elem(v, field):
     """Coerce one field element to a uint64 array of `field` words."""
+    if type(v) is np.ndarray and v.dtype == np.uint64 and v.shape == (field,) and v.flags.c_contiguous:
+        return v
     a = np.ascontiguousarray(np.asarray(v, dtype=np.uint64).reshape(-1))
     if a.size == field:
         return a
@@ -654,19 +665,25 @@ def sumcheck_verify_batch(claimed_sums, degree, round_polys, transcripts, hook=b
     ctx = ctx or Context.default()
     n = len(round_polys)
     nw = max(int(degree), 1)
-    rounds = [int(np.asarray(rp).shape[0]) for rp in round_polys]
-    flat = np.ascontiguousarray(np.concatenate(
-        [np.asarray(rp, dtype=np.uint64).reshape(-1) for rp in round_polys]) if n and sum(rounds)
-        else np.zeros(1, dtype=np.uint64))
+    polys = [rp if type(rp) is np.ndarray else np.asarray(rp, dtype=np.uint64) for rp in round_polys]
+    rounds = np.array([rp.shape[0] for rp in polys], dtype=np.uint32)
+    total = int(rounds.sum(dtype=np.int64))
+    if not total:
+        flat = np.zeros(1, dtype=np.uint64)
+    elif len({rp.shape[1:] for rp in polys}) == 1:     # whole rows: a third of the time of joining flat views
+        flat = np.concatenate(polys, dtype=np.uint64, casting="unsafe")
+    else:
+        flat = np.concatenate([np.asarray(rp, dtype=np.uint64).reshape(-1) for rp in polys])
     cs = np.ascontiguousarray(np.asarray(claimed_sums, dtype=np.uint64).reshape(n, field))
     fin = np.zeros((n, field), dtype=np.uint64)
-    ch = np.zeros((max(1, sum(rounds)), field), dtype=np.uint64)
+    ch = np.zeros((max(1, total), field), dtype=np.uint64)
     hb, hn = _bytes(hook)
-    check(load().effsc_verify_batch(ctx.h, field, n, _p(cs), int(degree), (ctypes.c_uint32 * max(n, 1))(*rounds),
+    check(load().effsc_verify_batch(ctx.h, field, n, _p(cs), int(degree),
+                                    (ctypes.c_uint32 * 0).from_buffer(rounds) if n else (ctypes.c_uint32 * 1)(),
                                     (vp * max(n, 1))(*[t.h for t in transcripts]), hb, hn, _p(flat), _p(ch),
                                     _p(fin)))
-    offs = np.concatenate([[0], np.cumsum(rounds)])
-    return fin, [ch[offs[i]:offs[i + 1]] for i in range(n)]
+    offs = np.cumsum(rounds, dtype=np.int64).tolist()
+    return fin, [ch[a:b] for a, b in zip([0] + offs[:-1], offs)]
 
 
 def fold(values, weight, field=FP3, repr=CANONICAL, ctx=None):
