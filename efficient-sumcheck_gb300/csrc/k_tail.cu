@@ -414,6 +414,7 @@ __global__ void __launch_bounds__(TAIL_TPB, 1) k_tail_cluster(TailArgs a, u32 cs
     __shared__ TailShared sh;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const u32 CS = 1u << cs_log, rank = cluster_rank();
+    chain_enter();
     const u32 Ll = (u32)(a.L >> cs_log);     // slice length (row stride)
     const u32 lgl = tail_lg(Ll);
     // this CTA's slice; base tables are embedded when the field is Fp3
@@ -527,13 +528,15 @@ static bool tail_cluster_inst(const TailArgs& a, u32 cs_log, u32 g_log, cudaStre
     cfg.blockDim = dim3(TAIL_TPB, 1, 1);
     cfg.dynamicSmemBytes = bytes;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = CS;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = pdl_on() ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, k_tail_cluster<POL, FW>, a, cs_log, g_log) == cudaSuccess;
 }
 

@@ -387,6 +387,16 @@ struct FirstSrc {
     const u64* p[4][3];
 };
 void launch_gather_first(const FirstSrc& src, u64* dst, cudaStream_t s);
+// A proof's ends: tx_words + hook_words words of the pinned block h into tx
+// and hook; wire | challenges | transcript | first entries into dst.
+struct ProofOut {
+    u64* dst;
+    const u64 *wire, *chals, *tx, *first;
+    u64 wire_words, chal_words;
+    u32 tx_words;
+};
+void launch_proof_in(const u64* h, u32 tx_words, u64* tx, u32 hook_words, u64* hook, cudaStream_t s);
+void launch_proof_out(const ProofOut& o, cudaStream_t s);
 void launch_fill(u64* dst, u64 n, u64 v, cudaStream_t s);
 bool launch_build_eq(const u64* w, u32 v, int ext, u64* c0, u64* c1, u64* c2, cudaStream_t s);
 void launch_gen_uniform(u64 seed, u64 n, u64* out, cudaStream_t s);

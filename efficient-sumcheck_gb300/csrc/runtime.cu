@@ -325,6 +325,7 @@ struct effsc_prover {
     // effsc_prove outputs: pinned staging (wire | challenges | transcript |
     // first entries of the tables) and the device copy of the first entries
     u64* h_out = nullptr;
+    u64* h_in = nullptr;                       // in the same block: the transcript's state and a short hook
     size_t h_out_bytes = 0;
     u64* d_first = nullptr;
 };
@@ -1691,6 +1692,7 @@ int do_finalize(effsc_prover* P, const Chal& ch, bool dry) {
 // effsc_prove (k_gather_first) so that the final value needs no extra copy.
 thread_local const u64* g_first = nullptr;
 constexpr size_t TX_OUT_WORDS = (sizeof(DevTranscript) + 7) / 8;
+constexpr size_t HOOK_IN_WORDS = 64;   // hooks up to this long travel with the transcript's state
 
 int read_first(effsc_prover* P, int ti, HF* out) {
     if (g_first) {
@@ -2555,11 +2557,12 @@ int effsc_prove(effsc_prover* P, size_t num_rounds, effsc_transcript* T, const u
     cudaStream_t s = P->ctx->stream;
     const int d = degree_of(P);
     // device buffers for the proof and the transcript
-    if (!P->d_tx) CK(cudaMallocAsync((void**)&P->d_tx, sizeof(DevTranscript), s));
+    if (!P->d_tx) CK(cudaMallocAsync((void**)&P->d_tx, TX_OUT_WORDS * 8, s));
     if (hook_len > P->hook_cap) {
         if (P->d_hook) CK(cudaFreeAsync(P->d_hook, s));
-        CK(cudaMallocAsync((void**)&P->d_hook, hook_len, s));
-        P->hook_cap = hook_len;
+        const size_t cap = (hook_len + 7) / 8 * 8;
+        CK(cudaMallocAsync((void**)&P->d_hook, cap, s));
+        P->hook_cap = cap;
         if (P->gexec) { cudaGraphExecDestroy(P->gexec); P->gexec = nullptr; }
     }
     if (num_rounds > P->rounds_cap || !P->d_wire) {
@@ -2571,21 +2574,30 @@ int effsc_prove(effsc_prover* P, size_t num_rounds, effsc_transcript* T, const u
         if (P->h_out) { CK(cudaStreamSynchronize(s)); pinned_put(P->ctx, P->h_out, P->h_out_bytes); P->h_out = nullptr; }
         // sized in steps of 64 rounds so that provers of similar size share blocks
         const size_t capr = (cap + 63) / 64 * 64;
-        P->h_out_bytes = (capr * 12 + TX_OUT_WORDS + 12) * sizeof(u64);
+        const size_t out_words = capr * 12 + TX_OUT_WORDS + 12;
+        P->h_out_bytes = (out_words + TX_OUT_WORDS + HOOK_IN_WORDS) * sizeof(u64);
         P->h_out = (u64*)pinned_get(P->ctx, P->h_out_bytes);
         if (!P->h_out) return fail(EFFSC_OOM, "pinned output block");
+        P->h_in = P->h_out + out_words;
         if (!P->d_first) CK(cudaMallocAsync((void**)&P->d_first, 12 * sizeof(u64), s));
         P->rounds_cap = cap;
         if (P->gexec) { cudaGraphExecDestroy(P->gexec); P->gexec = nullptr; }
     }
-    CK(cudaMemcpyAsync(P->d_tx, &T->st, sizeof(DevTranscript), cudaMemcpyHostToDevice, s));
-    if (hook_len) CK(cudaMemcpyAsync(P->d_hook, hook, hook_len, cudaMemcpyHostToDevice, s));
+    // the proof's ends are kernels of its chain, on the pinned block
+    const bool short_hook = hook_len <= HOOK_IN_WORDS * 8;
+    memcpy(P->h_in, &T->st, sizeof(DevTranscript));
+    if (hook_len && short_hook) memcpy(P->h_in + TX_OUT_WORDS, hook, hook_len);
+    if (hook_len && !short_hook) CK(cudaMemcpyAsync(P->d_hook, hook, hook_len, cudaMemcpyHostToDevice, s));
+    u64* const hw = P->h_out;
+    u64* const hc = hw + num_rounds * 3 * d;
+    u64* const ht = hc + num_rounds * 3;
+    u64* const hf_ = ht + TX_OUT_WORDS;
 
     bool at_reset = P->rounds == 0;
     for (int i = 0; i < 4; i++)
         if (!P->t[i].bufs.empty() && (P->t[i].cur != 0 || P->t[i].len != P->len0[i])) at_reset = false;
 
-    auto launch_all = [&](bool dry) -> int {
+    auto launch_proof = [&](bool dry) -> int {
         size_t r0 = 0;
         bool tail_done = false, finalized = false;   // by a tail: with the read-back entries, without
         if (fuse3_ok(P, num_rounds)) {
@@ -2728,6 +2740,16 @@ int effsc_prove(effsc_prover* P, size_t num_rounds, effsc_transcript* T, const u
         return EFFSC_OK;
     };
 
+    auto launch_all = [&](bool dry) -> int {
+        if (dry) return launch_proof(true);
+        launch_proof_in(P->h_in, TX_OUT_WORDS, (u64*)P->d_tx, short_hook ? (u32)((hook_len + 7) / 8) : 0, (u64*)P->d_hook, s);
+        TRY(launch_proof(false));
+        launch_proof_out({hw, P->d_wire, P->d_chals, (const u64*)P->d_tx, P->d_first, num_rounds * 3 * d, num_rounds * 3,
+                          (u32)TX_OUT_WORDS}, s);
+        g_launches += 2;
+        return EFFSC_OK;
+    };
+
     if (use_graph && at_reset && P->gexec && P->g_rounds == num_rounds && P->g_hook == hook_len) {
         CK(cudaGraphLaunch(P->gexec, s));
         g_launches += P->g_kernels;
@@ -2771,18 +2793,6 @@ int effsc_prove(effsc_prover* P, size_t num_rounds, effsc_transcript* T, const u
     } else {
         TRY(launch_all(false));
     }
-    // results: pinned copies of the wire values, challenges, transcript state
-    // and the tables' first entries, one synchronisation
-    u64* hw = P->h_out;
-    u64* hc = hw + num_rounds * 3 * d;
-    u64* ht = hc + num_rounds * 3;
-    u64* hf_ = ht + TX_OUT_WORDS;
-    if (num_rounds) {
-        CK(cudaMemcpyAsync(hw, P->d_wire, num_rounds * 3 * d * sizeof(u64), cudaMemcpyDeviceToHost, s));
-        CK(cudaMemcpyAsync(hc, P->d_chals, num_rounds * 3 * sizeof(u64), cudaMemcpyDeviceToHost, s));
-    }
-    CK(cudaMemcpyAsync(ht, P->d_tx, sizeof(DevTranscript), cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(hf_, P->d_first, 12 * sizeof(u64), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     TRY(check_status(P));
     memcpy(&T->st, ht, sizeof(DevTranscript));
