@@ -185,9 +185,9 @@ u32 eqf_tc_splits(u64 M, u64 K) {
     return (u32)s;
 }
 // Large sums over a base table that loads 16 bytes at a time.
-bool eqf_tc_ok(u64 M, u64 K, u64 stride, const u64* p) {
+bool eqf_tc_ok(bool along, u64 M, u64 K, u64 stride, const u64* p) {
     if (M % ET_M || K % ET_K || (stride & 1) || ((uintptr_t)p & 15) || M / ET_M > (1u << 20)) return false;
-    return M * K >= EQF_TC_MIN && K / eqf_tc_splits(M, K) <= 65536 && (K / eqf_tc_splits(M, K)) % ET_K == 0;
+    return M * K >= (along ? EQF_TC_MIN_ROWS : EQF_TC_MIN) && K / eqf_tc_splits(M, K) <= 65536 && (K / eqf_tc_splits(M, K)) % ET_K == 0;
 }
 template <bool ALONG, bool EW>
 static bool eqf_tc_inst(const u64* p, const u64* p2, u64 stride, Tab3 w, u64 M, u64 K, u32 splits, u64* part, u64* o0, u64* o1,

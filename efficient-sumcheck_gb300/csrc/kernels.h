@@ -229,6 +229,12 @@ bool launch_gkr_terms_c(int fw, const GkrSums& add, const GkrSums& mult, const u
                         cudaStream_t s);
 bool launch_gkr_finish(int fw, const u64* fb, const u64* fc, const u64* gc, const GkrFinish& o, cudaStream_t s);
 
+// A Multilinear proof from two reads of its base table (k_ml_phase.cu): the
+// sums of its rows of m entries, and of its m columns (splits, a power of two
+// up to rows, groups of rows; part: 3 m splits words).
+bool launch_ml_rows(const u64* p, u64 m, u64 rows, u64* T, cudaStream_t s);
+bool launch_ml_cols(const u64* p, u64 m, u64 rows, u64 splits, u64* part, u64* T, cudaStream_t s);
+
 // Serving steps: one entry per request in the step, sorted by first_block;
 // `code` = SERVE_IP (else ML) | SERVE_FP3 (else Fp) | phase << SERVE_PHASE_SHIFT.
 struct ServeSeg {
@@ -262,7 +268,7 @@ void launch_eqf_fold_rows(bool ew, bool ep, Tab3 p, Tab3 e, u64 Lc, u64 rows, u6
 // over k < K of w[k] P(k, m), m < M, P(k, m) = p[m stride + k] (along) or
 // p[k stride + m]; ew: Fp3 weights and sums.  part: 3 M eqf_tc_splits(M, K)
 // words (with one split unused).
-bool eqf_tc_ok(u64 M, u64 K, u64 stride, const u64* p);
+bool eqf_tc_ok(bool along, u64 M, u64 K, u64 stride, const u64* p);
 u32 eqf_tc_splits(u64 M, u64 K);
 bool launch_eqf_tc(bool along, bool ew, const u64* p, u64 stride, Tab3 w, u64 M, u64 K, u64* part, u64* o0, u64* o1, u64* o2,
                    u32* status, cudaStream_t s);
@@ -272,7 +278,9 @@ bool launch_eqf_tc(bool along, bool ew, const u64* p, u64 stride, Tab3 w, u64 M,
 bool launch_eqf_tc_pair(bool along, bool ew, const u64* p, const u64* p2, u64 stride, Tab3 w, u64 M, u64 K, u64* part,
                         u32* status, cudaStream_t s);
 void launch_eqf_sum(const u64* part, u64 n, u64 splits, int fw, u64* o0, u64* o1, u64* o2, cudaStream_t s);
-constexpr u64 EQF_TC_MIN = 1ULL << 18;
+// Sums along rows from 2^21 entries on (a block per row on the integer pipes
+// is 5 to 7 us faster below, over Fp3 and Fp), down columns from 2^18.
+constexpr u64 EQF_TC_MIN = 1ULL << 18, EQF_TC_MIN_ROWS = 1ULL << 21;
 
 int pol_ntables(int pol);
 int pol_nraw(int pol);
@@ -398,7 +406,8 @@ struct ProofOut {
 void launch_proof_in(const u64* h, u32 tx_words, u64* tx, u32 hook_words, u64* hook, cudaStream_t s);
 void launch_proof_out(const ProofOut& o, cudaStream_t s);
 void launch_fill(u64* dst, u64 n, u64 v, cudaStream_t s);
-bool launch_build_eq(const u64* w, u32 v, int ext, u64* c0, u64* c1, u64* c2, cudaStream_t s);
+// eq(w, .) over v variables, w[0] the index's highest bit (lsb: its lowest).
+bool launch_build_eq(const u64* w, u32 v, int ext, u64* c0, u64* c1, u64* c2, cudaStream_t s, bool lsb = false);
 void launch_gen_uniform(u64 seed, u64 n, u64* out, cudaStream_t s);
 bool diag_mulmod_rate(cudaStream_t s, double* mulmod_per_s, double* fp3_mul_per_s);
 bool diag_accumulate_rate(cudaStream_t s, double* mac_per_s, double* reduce_per_s);

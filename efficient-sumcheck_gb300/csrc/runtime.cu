@@ -371,6 +371,11 @@ int grid_for(u64 work, u64 per_thread = 1) {
 // on: at k = 3 the one-block tail alone is as fast (79 us against 81), at
 // k = 4 92 against 82, at k = 8 205 against 129.
 constexpr size_t GKR_PHASES_MIN = 4;
+// A Multilinear proof from two reads of its table (k_ml_phase.cu) from 2^18
+// entries on (LSB: 2^17), where a cluster alone holds the table: over Fp3
+// 2^17 110 us in the cluster against 121, 2^18 122 against 111; LSB 2^16 106
+// against 105, 2^17 125 against 109; 2^25 448 and 618 against 250 and 255.
+constexpr size_t ML_PHASES_MIN = 18, ML_PHASES_MIN_LSB = 17;
 // GkrProver passes whose b-variable pairs run in groups sharing one W_b entry
 // (k_gkr.cu): from GKR_RUNS_MIN pairs on, a grid of a quarter of the threads
 // gives each lane a run of four.  At most one wave of two blocks per SM (the
@@ -1101,6 +1106,87 @@ int do_ml_first(effsc_prover* P, const TxIO& tx0, const TxIO& tx2, const u64* ch
     return EFFSC_OK;
 }
 
+// effsc_prove of a Multilinear prover over a power-of-two base table on the
+// device: the first half of the variables from its sums over the others, the
+// rest from the table folded with all their challenges (k_ml_phase.cu).
+// *half: the rounds of the first phase.  Leaves that folded table, which the
+// next round takes as it is.
+bool ml_phases_ok(const effsc_prover* P, size_t num_rounds, size_t* half) {
+    if (!P->fuse_first || P->kind != EFFSC_ML) return false;
+    const Table& T = P->t[0];
+    if (T.ext || T.cur != 0 || T.bufs[0].host || !is_pow2(T.len)) return false;
+    size_t n = 0;
+    while (((size_t)1 << n) < T.len) n++;
+    const size_t a = n / 2;
+    if (n < (P->order == EFFSC_LSB ? ML_PHASES_MIN_LSB : ML_PHASES_MIN) || n > 40 || num_rounds <= a || num_rounds > n) return false;
+    *half = a;
+    const int fw = P->field == EFFSC_FP3 ? 3 : 1;
+    auto fits = [&](u64 L, size_t rounds) {
+        u32 cs, g;
+        return L <= P->tail_len && (tail_cluster_split(POL_ML, fw, L, (u32)rounds, false, &cs, &g) ||
+                                    (L <= tail_max_len(POL_ML, fw, TAIL_SMEM_CAP) && (L >> (rounds - 1)) >= 2));
+    };
+    return fits((u64)1 << a, a) && fits((u64)1 << (n - a), num_rounds - a);
+}
+
+int do_ml_phases(effsc_prover* P, size_t a, const TxIO& tx, bool dry) {
+    Table& T = P->t[0];
+    const int fw = P->field == EFFSC_FP3 ? 3 : 1;
+    const bool lsb = P->order == EFFSC_LSB;
+    const u64 A = (u64)1 << a, C = T.len >> a;      // entries of either half
+    const u64 m = lsb ? A : C, rows = lsb ? C : A;  // the table as rows of m entries
+    cudaStream_t s = P->ctx->stream;
+    const u64* p = T.bufs[0].p[0];
+    const bool tc = eqf_tc_ok(lsb, C, A, m, p);
+    const u64 splits = std::min<u64>(rows, 64);
+    const size_t need = A + 3 * A + std::max<size_t>(3 * m * splits, tc ? 3 * C * eqf_tc_splits(C, A) : 0);
+    if (P->eqf_cap < need) {
+        if (P->eqf_scratch) CK(cudaFreeAsync(P->eqf_scratch, s));
+        P->eqf_scratch = nullptr;
+        CK(cudaMallocAsync((void**)&P->eqf_scratch, need * sizeof(u64), s));
+        P->eqf_cap = need;
+    }
+    u64 *S = P->eqf_scratch, *Ew = S + A, *part = Ew + 3 * A;
+    int bi;
+    TRY(out_buffer(P, T, fw == 3, C, true, &bi));
+    if (!dry) {
+        TRY(timed_launch(s, "ml_sums", 8 * T.len, [&] {
+            return lsb ? launch_ml_cols(p, m, rows, splits, part, S, s) : launch_ml_rows(p, m, rows, S, s);
+        }));
+        if (lsb) g_launches++;
+        TailArgs ta;
+        memset(&ta, 0, sizeof ta);
+        ta.in[0][0] = S;
+        ta.L = A;
+        ta.nrounds = (u32)a;
+        ta.tx = tx.tx;
+        ta.hook = tx.hook;
+        ta.hook_len = tx.hook_len;
+        ta.proof_wire = tx.proof_wire;
+        ta.proof_chal = tx.proof_chal;
+        ta.lsb = lsb ? 1 : 0;
+        ClusterSplit cl;
+        const bool clus = tail_cluster_split(POL_ML, fw, A, (u32)a, false, &cl.cs_log, &cl.g_log);
+        TRY(timed_launch(s, "ml_first_tail", 8 * A, [&] {
+            return clus ? launch_tail_cluster(POL_ML, fw, ta, cl.cs_log, cl.g_log, s) : launch_tail(POL_ML, fw, nullptr, &ta, 1, A, s);
+        }));
+        TRY(timed_launch(s, "ml_eq_weights", 8 * fw * A, [&] { return launch_build_eq(P->d_chals, (u32)a, fw == 3, Ew, Ew + A, Ew + 2 * A, s, lsb); }));
+        const Tab3 tp = {{p, nullptr, nullptr}}, te = {{Ew, Ew + A, Ew + 2 * A}};
+        const Buf& o = T.bufs[bi];
+        TRY(timed_launch(s, "ml_fold", 8 * T.len + 8 * fw * C, [&] {
+            if (tc) return launch_eqf_tc(lsb, fw == 3, p, m, te, C, A, part, o.p[0], o.p[1], o.p[2], P->status, s);
+            if (lsb) launch_eqf_inner(fw == 3, false, tp, te, m, C, o.p[0], o.p[1], o.p[2], s);
+            else launch_eqf_fold_rows(fw == 3, false, tp, te, C, A, splits, part, fw, o.p[0], o.p[1], o.p[2], s);
+            return true;
+        }));
+        if (tc ? eqf_tc_splits(C, A) > 1 : !lsb) g_launches++;
+    }
+    T.cur = bi;
+    T.len = C;
+    T.ext = fw == 3;
+    return EFFSC_OK;
+}
+
 // GkrProver tail: from round r on, the four tables in one block's shared
 // memory (k_gkr_tail.cu) -- the remaining rounds, the finalize and the
 // read-back entries in one launch.  Leaves the state the per-round path and
@@ -1180,7 +1266,7 @@ bool gkr_phases_ok(const effsc_prover* P, size_t num_rounds) {
     }
     if (n > GKR_SMALL)
         for (int i = 0; i < 2; i++)
-            if (!eqf_tc_ok(n, n, n, P->t[i].bufs[0].p[0])) return false;
+            if (!eqf_tc_ok(true, n, n, n, P->t[i].bufs[0].p[0])) return false;
     const int fw = P->field == EFFSC_FP3 ? 3 : 1;
     u32 cs, g;
     if (2 * n > P->tail_len) return false;
@@ -1360,8 +1446,8 @@ int do_eqf_left(effsc_prover* P, const TxIO& tx, bool dry) {
     cudaStream_t s = P->ctx->stream;
     // large base tables: both passes over p on the tensor cores
     const u64* pb = p.bufs[p.cur].p[0];
-    const bool tc_in = !p.ext && er.ext == (fw == 3) && eqf_tc_ok(rows, m, m, pb);
-    const bool tc_fold = !p.ext && eqf_tc_ok(Lc, rows2, Lc, pb);
+    const bool tc_in = !p.ext && er.ext == (fw == 3) && eqf_tc_ok(true, rows, m, m, pb);
+    const bool tc_fold = !p.ext && eqf_tc_ok(false, Lc, rows2, Lc, pb);
     const size_t part_words = std::max<size_t>({(size_t)(3 * splits * Lc), tc_in ? (size_t)(3 * rows * eqf_tc_splits(rows, m)) : 0,
                                                 tc_fold ? (size_t)(3 * Lc * eqf_tc_splits(Lc, rows2)) : 0});
     const size_t need = 3 * rows + 3 * rows2 + part_words;
@@ -2598,7 +2684,8 @@ int effsc_prove(effsc_prover* P, size_t num_rounds, effsc_transcript* T, const u
         if (!P->t[i].bufs.empty() && (P->t[i].cur != 0 || P->t[i].len != P->len0[i])) at_reset = false;
 
     auto launch_proof = [&](bool dry) -> int {
-        size_t r0 = 0;
+        size_t r0 = 0, half = 0;
+        bool folded = false;                         // round r0's tables are folded with the challenge before it
         bool tail_done = false, finalized = false;   // by a tail: with the read-back entries, without
         if (fuse3_ok(P, num_rounds)) {
             TxIO t0;
@@ -2635,6 +2722,17 @@ int effsc_prove(effsc_prover* P, size_t num_rounds, effsc_transcript* T, const u
             t2.proof_chal = P->d_chals + 3 * 2;
             TRY(do_fuse_first(P, t0, t2, P->d_chals, dry));
             r0 = 3;
+        } else if (ml_phases_ok(P, num_rounds, &half)) {
+            TxIO t0;
+            memset(&t0, 0, sizeof t0);
+            t0.tx = P->d_tx;
+            t0.hook = P->d_hook;
+            t0.hook_len = (u32)hook_len;
+            t0.proof_wire = P->d_wire;
+            t0.proof_chal = P->d_chals;
+            TRY(do_ml_phases(P, half, t0, dry));
+            r0 = half;
+            folded = true;
         } else if (ml_first_ok(P, num_rounds)) {
             TxIO t0, t2;
             memset(&t0, 0, sizeof t0);
@@ -2684,7 +2782,7 @@ int effsc_prove(effsc_prover* P, size_t num_rounds, effsc_transcript* T, const u
         }
         for (size_t r = r0; r < num_rounds; r++) {
             Chal ch;
-            if (r > 0) { ch.has = true; ch.ext = P->field == EFFSC_FP3; ch.dev = P->d_chals + 3 * (r - 1); }
+            if (r > 0 && !(folded && r == r0)) { ch.has = true; ch.ext = P->field == EFFSC_FP3; ch.dev = P->d_chals + 3 * (r - 1); }
             TxIO tx;
             tx.tx = P->d_tx;
             tx.hook = P->d_hook;

@@ -290,8 +290,8 @@ class _Prover:
     def set_first_rounds(self, fused):
         """prove(): how the first rounds read the base tables.  False / 0: one
         pass per round; 1: rounds 0-2 of an InnerProduct, Multilinear or
-        partial GkrProver proof in two passes, a whole GkrProver proof from
-        two reads of add and mult; True / 2 (the default): as 1, and rounds
+        partial GkrProver proof in two passes, a whole GkrProver proof and a
+        Multilinear proof of more than half the variables from two reads; True / 2 (the default): as 1, and rounds
         0-4 of an InnerProduct proof in two passes where they apply (Fp3
         challenges, power-of-two base tables of 2^14 entries or more)."""
         level = 2 if fused is True else 0 if fused is False else int(fused)

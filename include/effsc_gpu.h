@@ -211,15 +211,18 @@ int effsc_prover_set_tail(effsc_prover* p, size_t max_len);
  * the base tables (round 1 from sums gathered during round 0; round 2 folds
  * with both challenges).  fused = 2 (the default) does the same and, for an
  * InnerProduct prover with base tables of 2^14 entries or more, computes
- * rounds 0-4 (of 4 rounds: 0-3) in two passes instead: the first rounds from the products of the entries a folded pair comes from, the
- * last with all their challenges folded at once.
+ * rounds 0-4 (of 4 rounds: 0-3) in two passes instead: the first
+ * rounds from the products of the entries a folded pair comes from, the last
+ * with all their challenges folded at once.
  * For a CoefficientProver with the degree-3 product evaluator over three
  * tables of 2^12 entries or more (table 0 in Fp or Fp3, tables 1-2 in Fp),
  * fused >= 1 computes rounds 0-2 in two passes (rounds 0 and 1 from the sums
  * of the products of one pass; round 2 folds with both challenges).  With
  * fused >= 1 a GkrProver with |w| >= 16 whose run is all its 2 log2 |w| rounds
  * proves them from two reads of add and mult and two tails (tables of 2 |w|
- * entries, which must be within max_len).
+ * entries, which must be within max_len), and a Multilinear prover (MSB or
+ * LSB) over 2^18 base entries or more (LSB 2^17) whose run is more than half
+ * of the variables from two reads of the table and two tails.
  * 0 runs one pass per round.  Proofs are identical. */
 int effsc_prover_set_first_rounds(effsc_prover* p, int fused);
 /* effsc_prove only (no reference counterpart; a tuning knob): for an
