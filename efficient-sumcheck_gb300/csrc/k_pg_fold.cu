@@ -105,6 +105,7 @@ template <bool E>
 __global__ void __launch_bounds__(PG_TPB) k_pg_group(const u64* __restrict__ in, u32 w, u32 g, u32 S,
                                                      const PgMul mul, u64* __restrict__ out) {
     extern __shared__ u64 sm[];
+    chain_enter();
     constexpr u32 EW = E ? 3 : 1;
     const u64* pairs = mul.q;
     const u32 R = 1u << g, P = 2 * S + 1;
@@ -168,6 +169,7 @@ template <bool E>
 __global__ void __launch_bounds__(PG_TPB) k_pg_warp(const u64* __restrict__ in, size_t trees, u32 w, u32 gw,
                                                     const PgMul mul, u64* __restrict__ out) {
     extern __shared__ u64 sm[];
+    chain_enter();
     constexpr u32 EW = E ? 3 : 1;
     const u64* pairs = mul.q;
     const u32 lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -220,6 +222,7 @@ __global__ void __launch_bounds__(PG_TPB) k_pg_warp(const u64* __restrict__ in, 
 template <bool E>
 __global__ void __launch_bounds__(PG_TPB) k_pg_level(const u64* __restrict__ in, size_t cnt, u32 w,
                                                      const PgMul mul, u64* __restrict__ out) {
+    chain_enter();
     const u64* pair = mul.q;
     const Mul3 ma = pg_mul3<E>(pair), mb = pg_mul3<E>(pair + 5);
     const u32 wo = w + 1;
@@ -321,6 +324,14 @@ extern "C" int effsc_protogalaxy_fold(effsc_ctx* ctx, int field, const uint64_t*
         res_fallback.assign(res_bytes / 8, 0);
         res = res_fallback.data();
     }
+    // the last pass writes the row there itself (a copy of a few hundred bytes
+    // and the gaps between plainly launched passes were a tenth of a call:
+    // 2^20 rows of 8, 114 -> 104 us)
+    u64* res_dev = nullptr;
+    if (!res_fallback.empty() || cudaHostGetDevicePointer((void**)&res_dev, res, 0) != cudaSuccess) {
+        cudaGetLastError();
+        res_dev = nullptr;
+    }
     int rc = EFFSC_OK;
     u64 *d_in = nullptr, *bufs[2] = {nullptr, nullptr};
     const u64* cur = nullptr;
@@ -342,6 +353,15 @@ extern "C" int effsc_protogalaxy_fold(effsc_ctx* ctx, int field, const uint64_t*
         u32 w = (u32)width, lvl = 0;
         int which = 0;
         size_t cap[2] = {0, 0};
+        auto buffer = [&](int b, size_t need) -> cudaError_t {
+            if (need <= cap[b]) return cudaSuccess;
+            if (bufs[b]) cudaFreeAsync(bufs[b], s);
+            bufs[b] = nullptr;
+            cap[b] = 0;
+            const cudaError_t e = cudaMallocAsync((void**)&bufs[b], need, s);
+            if (e == cudaSuccess) cap[b] = need;
+            return e;
+        };
         static std::atomic<uint64_t> attr_done{0};    // one bit per device
         const uint64_t bit = 1ull << (dev & 63);
         if (!(attr_done.load() & bit)) {
@@ -355,20 +375,18 @@ extern "C" int effsc_protogalaxy_fold(effsc_ctx* ctx, int field, const uint64_t*
             const u32 gw = pg_plan_warp(count, w, ew);
             if (gw) {
                 const size_t trees = count >> gw, need = trees * (w + gw) * ew * 8;
-                if (need > cap[which]) {
-                    if (bufs[which]) cudaFreeAsync(bufs[which], s);
-                    bufs[which] = nullptr;
-                    cap[which] = 0;
-                    PCK(cudaMallocAsync((void**)&bufs[which], need, s));
-                    cap[which] = need;
+                u64* dst = trees == 1 ? res_dev : nullptr;
+                if (!dst) {
+                    PCK(buffer(which, need));
+                    dst = bufs[which];
                 }
                 const size_t smem = (PG_TPB / 32) * pg_warp_smem(w, gw, ew);
                 const unsigned grid = (unsigned)((trees + PG_TPB / 32 - 1) / (PG_TPB / 32));
-                if (ew == 3) k_pg_warp<true><<<grid, PG_TPB, smem, s>>>(cur, trees, w, gw, muls(lvl, gw), bufs[which]);
-                else k_pg_warp<false><<<grid, PG_TPB, smem, s>>>(cur, trees, w, gw, muls(lvl, gw), bufs[which]);
+                if (ew == 3) launch_chain(k_pg_warp<true>, grid, PG_TPB, smem, s, cur, trees, w, gw, muls(lvl, gw), dst);
+                else launch_chain(k_pg_warp<false>, grid, PG_TPB, smem, s, cur, trees, w, gw, muls(lvl, gw), dst);
                 effsc_internal_add_launches(1);
                 PCK(cudaGetLastError());
-                cur = bufs[which];
+                cur = dst;
                 which ^= 1;
                 count = trees;
                 w += gw;
@@ -380,35 +398,33 @@ extern "C" int effsc_protogalaxy_fold(effsc_ctx* ctx, int field, const uint64_t*
             const size_t out_rows = g ? count >> g : count >> 1;
             const u32 out_w = w + (g ? g : 1);
             const size_t need = out_rows * out_w * ew * 8;
-            if (need > cap[which]) {
-                if (bufs[which]) cudaFreeAsync(bufs[which], s);
-                bufs[which] = nullptr;
-                cap[which] = 0;
-                PCK(cudaMallocAsync((void**)&bufs[which], need, s));
-                cap[which] = need;
+            u64* dst = out_rows == 1 ? res_dev : nullptr;
+            if (!dst) {
+                PCK(buffer(which, need));
+                dst = bufs[which];
             }
             if (g) {
                 const size_t smem = pg_group_smem(w, g, ew);
                 const u32 S = pg_stride(w, g);
-                if (ew == 3) k_pg_group<true><<<(unsigned)out_rows, PG_TPB, smem, s>>>(cur, w, g, S, muls(lvl, g), bufs[which]);
-                else k_pg_group<false><<<(unsigned)out_rows, PG_TPB, smem, s>>>(cur, w, g, S, muls(lvl, g), bufs[which]);
+                if (ew == 3) launch_chain(k_pg_group<true>, (unsigned)out_rows, PG_TPB, smem, s, cur, w, g, S, muls(lvl, g), dst);
+                else launch_chain(k_pg_group<false>, (unsigned)out_rows, PG_TPB, smem, s, cur, w, g, S, muls(lvl, g), dst);
                 lvl += g;
             } else {
                 const size_t items = out_rows * (w + 1);
                 const unsigned grid = (unsigned)std::min<size_t>((items + PG_TPB - 1) / PG_TPB, 152 * 16);
-                if (ew == 3) k_pg_level<true><<<grid, PG_TPB, 0, s>>>(cur, out_rows, w, muls(lvl, 1), bufs[which]);
-                else k_pg_level<false><<<grid, PG_TPB, 0, s>>>(cur, out_rows, w, muls(lvl, 1), bufs[which]);
+                if (ew == 3) launch_chain(k_pg_level<true>, grid, PG_TPB, 0, s, cur, out_rows, w, muls(lvl, 1), dst);
+                else launch_chain(k_pg_level<false>, grid, PG_TPB, 0, s, cur, out_rows, w, muls(lvl, 1), dst);
                 lvl += 1;
             }
             effsc_internal_add_launches(1);
             PCK(cudaGetLastError());
-            cur = bufs[which];
+            cur = dst;
             which ^= 1;
             count = out_rows;
             w = out_w;
         }
     }
-    if (final_w && width) PCK(cudaMemcpyAsync(res, cur, final_w * ew * 8, cudaMemcpyDefault, s));
+    if (final_w && width && cur != res_dev) PCK(cudaMemcpyAsync(res, cur, final_w * ew * 8, cudaMemcpyDefault, s));
     PCK(cudaStreamSynchronize(s));
     {
         size_t len = width ? final_w : 0;
