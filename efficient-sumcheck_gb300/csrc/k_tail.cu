@@ -1,5 +1,6 @@
-// k_tail.cu -- the last rounds of a Multilinear / InnerProduct proof in one
-// thread block or one thread-block cluster.
+// k_tail.cu -- the last rounds of a Multilinear, InnerProduct or Coefficient
+// (product of three Fp3 tables) proof in one thread block or one thread-block
+// cluster.
 //
 // Once a prover's tables are small, a round costs far more in kernel
 // boundaries (launch, grid-wide ticket, a lone last block running the
@@ -52,10 +53,10 @@ constexpr int TAIL_MAX_CS = 16;
 struct TailShared {
     uint4 part[3 * TAIL_NW];           // the warps' sums, in 22-bit pieces
     u64 chal[5];                       // W r1, W r2, r0, r1, r2 of the last challenge r
-    u64 tot[6];                        // wire values, component c of value e at 3 e + c
+    u64 tot[9];                        // wire values, component c of value e at 3 e + c
     u64 raw[3];
     __align__(8) uint8_t scr[64];
-    u64 cred[TAIL_MAX_CS][6];          // (cluster kernel, CTA 0) every CTA's sums
+    u64 cred[TAIL_MAX_CS][9];          // (cluster kernel, CTA 0) every CTA's sums
 };
 
 // Where a tail's tables are: component c of table t, entry i at
@@ -92,8 +93,9 @@ __device__ __forceinline__ void tail_fold(const TailTab& T, u32 out, bool base, 
         // a whole entry per thread
         Mul3 m;
         m.w1 = ch[0]; m.w2 = ch[1]; m.m0 = ch[2]; m.m1 = ch[3]; m.m2 = ch[4];
+        const u32 lg = tail_lg(half);
         for (u32 i = threadIdx.x; i < NT * half; i += TAIL_TPB) {
-            const int t = NT > 1 && i >= half ? 1 : 0;
+            const int t = NT > 1 ? i >> lg : 0;
             const u32 j = i - t * half;
             const u64* row = T.sm + t * 3 * T.stride + T.off;
             u64* dst = T.sm + t * 3 * T.stride + out;
@@ -116,7 +118,7 @@ __device__ __forceinline__ void tail_fold(const TailTab& T, u32 out, bool base, 
     const u32 lg = tail_lg(half);
     for (u32 i = threadIdx.x; i < NT * FW * half; i += TAIL_TPB) {
         const u32 r = i >> lg;                        // t FW + c
-        const int t = NT > 1 && r >= FW ? 1 : 0, c = (int)r - t * FW;
+        const int t = NT > 1 ? r / FW : 0, c = (int)r - t * FW;
         const u32 j = i & (half - 1);
         const u64 v = tail_fold_comp<FW>(T.sm + t * FW * T.stride + T.off, T.stride, j, half, c, ch);
         T.sm[r * T.stride + out + j] = v;
@@ -135,10 +137,13 @@ __device__ __forceinline__ void tail_fold(const TailTab& T, u32 out, bool base, 
 //   ROW   (IP over Fp3) x_k with all three y_m;
 //   VALUE (Fp, or Fp3 before base tables' first fold) a whole value; ML over
 //         Fp3: one component of it.
+// CoefficientProver's product of three Fp3 tables (POL_C3W): h(0), h(inf) and
+// h(2), sums of a product of three each (src/provers/coefficient.rs:272-294);
+// a role is a value, a lane a pair.
 // Every sum goes to sh.part, those of a wire word next to each other, wire word `word` is the sum of its TERMS x slots entries.
 template <int POL, int FW>
 struct TailRoles {
-    static constexpr int NWIRE = POL == POL_ML ? 1 : 2;
+    static constexpr int NWIRE = POL == POL_ML ? 1 : POL == POL_C3W ? 3 : 2;
     static constexpr int N = NWIRE * FW;                  // wire words
     static constexpr bool ROWS = POL == POL_IP && FW == 3;
     static constexpr int WPR = TAIL_NW / N, WPR_BASE = TAIL_NW / NWIRE;
@@ -172,11 +177,40 @@ __device__ __forceinline__ u32 tail_eval(const TailTab& T, bool base, TailShared
         }
         return 1;
     }
-    const u32 wpr = base ? R::WPR_BASE : R::WPR;
-    const u32 role = base ? warp / R::WPR_BASE : warp / R::WPR, slot = warp - role * wpr;
+    const bool whole = base || POL == POL_C3W;          // a role is a value, not a component or row of one
+    const u32 wpr = whole ? R::WPR_BASE : R::WPR;
+    const u32 role = whole ? warp / R::WPR_BASE : warp / R::WPR, slot = warp - role * wpr;
     const u32 slots = min(wpr, (half + 31) >> 5);
     if (slot >= slots) return slots;
     const u32 j0 = slot * 32 + lane, step = 32 * wpr;
+    if constexpr (POL == POL_C3W) {
+        // role = a point of the wire: lo (0), hi - lo (infinity), 2 hi - lo (2)
+        ProdAcc<true, true> s;
+        s.init();
+        for (u32 j = j0; j < half; j += step) {
+            F3 x[3];
+#pragma unroll
+            for (int t = 0; t < 3; t++) {
+                const u64* q = a + 3 * t * T.stride + j;
+                x[t] = f3_make(q[0], q[T.stride], q[2 * T.stride]);
+                if (role) {
+                    const F3 hi = f3_make(q[half], q[T.stride + half], q[2 * T.stride + half]);
+                    x[t] = f3_sub<true>(hi, x[t]);
+                    if (role == 2) x[t] = f3_add<true>(hi, x[t]);
+                }
+            }
+            s.mac(f3_mul<true, true>(x[0], x[1]), x[2]);
+        }
+        const F3 v = s.result();
+        const uint4 p0 = warp_sum_pieces(v.c0), p1 = warp_sum_pieces(v.c1), p2 = warp_sum_pieces(v.c2);
+        if (lane == 0) {
+            uint4* d = sh.part + 3 * role * slots + slot;
+            d[0] = p0;
+            d[slots] = p1;
+            d[2 * slots] = p2;
+        }
+        return slots;
+    }
     if (R::ROWS && !base) {
         const u32 which = role >= 3, k = role - 3 * which;
         AccF<0> s[3];
@@ -282,7 +316,7 @@ __device__ __forceinline__ void tail_record(const TailArgs& a, u32 k, const Tail
     constexpr u32 NW3 = 3 * TailRoles<POL, FW>::NWIRE;
     const u32 i = threadIdx.x - (TAIL_TPB - 32);
     if (i < NW3) a.proof_wire[k * NW3 + i] = FW == 3 || i % 3 == 0 ? sh.tot[i] : 0;
-    else if (i >= 8 && i < 11) a.proof_chal[3 * k + i - 8] = sh.chal[i - 6];
+    else if (i >= 16 && i < 19) a.proof_chal[3 * k + i - 16] = sh.chal[i - 14];
 }
 
 // The challenge before the first round, prepared (or zeros).
@@ -581,6 +615,7 @@ bool launch_tail_cluster(int pol, int fw, const TailArgs& a, u32 cs_log, u32 g_l
     case POL_ML * 4 + 3: return tail_cluster_inst<POL_ML, 3>(a, cs_log, g_log, s);
     case POL_IP * 4 + 1: return tail_cluster_inst<POL_IP, 1>(a, cs_log, g_log, s);
     case POL_IP * 4 + 3: return tail_cluster_inst<POL_IP, 3>(a, cs_log, g_log, s);
+    case POL_C3W * 4 + 3: return tail_cluster_inst<POL_C3W, 3>(a, cs_log, g_log, s);
     default: return false;
     }
 }
@@ -613,6 +648,7 @@ bool launch_tail(int pol, int fw, const TailArgs* dev_args, const TailArgs* one,
     case POL_ML * 4 + 3: return tail_inst<POL_ML, 3>(dev_args, one, n, smem_len, s);
     case POL_IP * 4 + 1: return tail_inst<POL_IP, 1>(dev_args, one, n, smem_len, s);
     case POL_IP * 4 + 3: return tail_inst<POL_IP, 3>(dev_args, one, n, smem_len, s);
+    case POL_C3W * 4 + 3: return tail_inst<POL_C3W, 3>(dev_args, one, n, smem_len, s);
     default: return false;
     }
 }

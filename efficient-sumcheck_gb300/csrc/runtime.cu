@@ -618,20 +618,25 @@ int round_std(effsc_prover* P, const Chal& ch, const TxIO& tx, bool dry) {
 // fit in shared memory, challenges in device memory, and every round still
 // folding to at least two entries (the length-1 cases stay on the per-round
 // path).
-// The tail kernels' policy for a prover: Multilinear and InnerProduct; -1
-// for the others.  (A tail for the Coefficient product evaluator of degree 3
-// over Fp3 measured slower than its per-round kernels: n = 24, 16 rounds,
-// 1.557 ms with the cluster tail from 2^14 entries, 1.533 ms with the
-// one-block tail from 2048, 1.519 ms without -- one SM folding and
-// evaluating 1024 triple products per round costs more than the launch it
-// saves.)
+// The tail kernels' policy for a prover: Multilinear, InnerProduct, and the
+// Coefficient product evaluator of degree 3 over Fp3; -1 for the others.
 int tail_pol(const effsc_prover* P) {
     if (P->kind == EFFSC_ML || P->kind == EFFSC_IP) return pol_of(P);
+    if (P->kind == EFFSC_COEF && !P->expr && P->ntab == 3 && P->field == EFFSC_FP3) return POL_C3W;
     return -1;
+}
+// The Coefficient tail takes tables that are Fp3 already, that is, folded, of
+// up to 2^14 entries: a cluster's first rounds on 2^15 take as long as the
+// round kernels' (2^24 entries, 16 rounds, a call: 863 us from 2^15 on, 855
+// from 2^14, 861 from 2^13, without 877; 2^16, 16 rounds: 150, 150, 156, 224).
+constexpr size_t COEF_TAIL_MAX = (size_t)1 << 14;
+bool tail_tables_ok(const effsc_prover* P, const Chal& ch) {
+    if (P->kind != EFFSC_COEF) return true;
+    return P->t[0].len <= COEF_TAIL_MAX && ch.has && P->t[0].ext && P->t[1].ext && P->t[2].ext;
 }
 
 bool tail_ok(const effsc_prover* P, size_t r, size_t num_rounds, const Chal& ch) {
-    if (tail_pol(P) < 0 || !P->tail_len) return false;
+    if (tail_pol(P) < 0 || !P->tail_len || !tail_tables_ok(P, ch)) return false;
     if (r >= num_rounds || (ch.has && !ch.dev)) return false;
     const size_t L = P->t[0].len;
     for (int i = 1; i < P->ntab; i++)
@@ -650,7 +655,7 @@ struct ClusterSplit {
     u32 cs_log = 0, g_log = 0;
 };
 bool cluster_tail_ok(const effsc_prover* P, size_t r, size_t num_rounds, const Chal& ch, ClusterSplit* cl) {
-    if (tail_pol(P) < 0 || !P->tail_len) return false;
+    if (tail_pol(P) < 0 || !P->tail_len || !tail_tables_ok(P, ch)) return false;
     if (r >= num_rounds || num_rounds - r >= 63 || (ch.has && !ch.dev)) return false;
     const size_t L = P->t[0].len;
     for (int i = 1; i < P->ntab; i++)
