@@ -168,25 +168,25 @@ __global__ void k_gkr_finish(const u64* fb, const u64* fc, const u64* gc, int fw
 }
 
 bool launch_gkr_terms_b(const GkrSums& add, const GkrSums& mult, const u64* W, u64* F, u64* G, cudaStream_t s) {
-    return launch_chain(k_gkr_terms_b, (int)((add.n + TPB - 1) / TPB), TPB, 0, s, add, mult, W, F, G);
+    return launch_dep(k_gkr_terms_b, (int)((add.n + TPB - 1) / TPB), TPB, 0, s, add, mult, W, F, G);
 }
 bool launch_gkr_rows(const u64* add, const u64* mult, const u64* W, u32 n, u64* F, u64* G, cudaStream_t s) {
-    return launch_chain(k_gkr_rows, (int)((n + NWARP - 1) / NWARP), TPB, 0, s, add, mult, W, n, F, G);
+    return launch_dep(k_gkr_rows, (int)((n + NWARP - 1) / NWARP), TPB, 0, s, add, mult, W, n, F, G);
 }
 bool launch_gkr_terms_c(int fw, const GkrSums& add, const GkrSums& mult, const u64* W, const u64* wb, u64* F, u64* G,
                         cudaStream_t s) {
     const int g = (int)((add.n + TPB - 1) / TPB);
-    return fw == 3 ? launch_chain(k_gkr_terms_c<3>, g, TPB, 0, s, add, mult, W, wb, F, G)
-                   : launch_chain(k_gkr_terms_c<1>, g, TPB, 0, s, add, mult, W, wb, F, G);
+    return fw == 3 ? launch_dep(k_gkr_terms_c<3>, g, TPB, 0, s, add, mult, W, wb, F, G)
+                   : launch_dep(k_gkr_terms_c<1>, g, TPB, 0, s, add, mult, W, wb, F, G);
 }
 bool launch_gkr_cols(int fw, const u64* add, const u64* mult, const u64* W, const u64* wb, const u64* chals, u32 k, u64* F,
                      u64* G, cudaStream_t s) {
     const int g = ((1 << k) + 7) / 8;
-    return fw == 3 ? launch_chain(k_gkr_cols<3>, g, TPB, 0, s, add, mult, W, wb, chals, k, F, G)
-                   : launch_chain(k_gkr_cols<1>, g, TPB, 0, s, add, mult, W, wb, chals, k, F, G);
+    return fw == 3 ? launch_dep(k_gkr_cols<3>, g, TPB, 0, s, add, mult, W, wb, chals, k, F, G)
+                   : launch_dep(k_gkr_cols<1>, g, TPB, 0, s, add, mult, W, wb, chals, k, F, G);
 }
 bool launch_gkr_finish(int fw, const u64* fb, const u64* fc, const u64* gc, const GkrFinish& o, cudaStream_t s) {
-    return launch_chain(k_gkr_finish, 1, 32, 0, s, fb, fc, gc, fw, o);
+    return launch_dep(k_gkr_finish, 1, 32, 0, s, fb, fc, gc, fw, o);
 }
 
 }  // namespace effsc

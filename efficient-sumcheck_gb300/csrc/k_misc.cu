@@ -30,15 +30,12 @@ static int sms_of(int device) {
 
 void kernels_init(int device) { sms_of(device); }
 
-// Programmatic dependent launch of the round kernels: off unless EFFSC_PDL=1
-// (measured at n = 26 in a CUDA graph: 1.273 ms per proof with it, 1.251
-// without).
-bool pdl_on(void) {
-    static const bool on = [] {
+bool pdl_on(bool few_blocks) {
+    static const int set = [] {
         const char* e = getenv("EFFSC_PDL");
-        return e && e[0] == '1';
+        return !e ? -1 : e[0] == '1' ? 1 : e[0] == '0' ? 0 : -1;
     }();
-    return on;
+    return set < 0 ? few_blocks : set == 1;
 }
 __global__ void k_gather_first(FirstSrc src, u64* dst) {
     chain_enter();
@@ -48,7 +45,7 @@ __global__ void k_gather_first(FirstSrc src, u64* dst) {
         dst[i] = p ? p[0] : 0;
     }
 }
-void launch_gather_first(const FirstSrc& src, u64* dst, cudaStream_t s) { launch_chain(k_gather_first, 1, 32, 0, s, src, dst); }
+void launch_gather_first(const FirstSrc& src, u64* dst, cudaStream_t s) { launch_dep(k_gather_first, 1, 32, 0, s, src, dst); }
 
 // The transcript state and a short hook from the caller's pinned block, and
 // the proof into it, as kernels of the proof's chain: five copies each cost a
@@ -75,11 +72,11 @@ __global__ void __launch_bounds__(256) k_proof_out(ProofOut o) {
     for (u64 i = t; i < 12; i += n) dst[i] = o.first[i];
 }
 void launch_proof_in(const u64* h, u32 tx_words, u64* tx, u32 hook_words, u64* hook, cudaStream_t s) {
-    launch_chain(k_proof_in, 1, 256, 0, s, h, tx_words, tx, hook_words, hook);
+    launch_dep(k_proof_in, 1, 256, 0, s, h, tx_words, tx, hook_words, hook);
 }
 void launch_proof_out(const ProofOut& o, cudaStream_t s) {
     const u64 blocks = (o.wire_words + 255) / 256;
-    launch_chain(k_proof_out, (int)(blocks < 1 ? 1 : blocks < 64 ? blocks : 64), 256, 0, s, o);
+    launch_dep(k_proof_out, (int)(blocks < 1 ? 1 : blocks < 64 ? blocks : 64), 256, 0, s, o);
 }
 
 int max_grid(void) {
@@ -249,8 +246,8 @@ bool launch_build_eq(const u64* w, u32 v, int ext, u64* c0, u64* c1, u64* c2, cu
     const int tpb = n <= (1u << 14) ? 64 : 256;
     const u64 blocks = (n + tpb - 1) / tpb;
     const int g = (int)(blocks < (u64)max_grid() * 2 ? blocks : (u64)max_grid() * 2);
-    return ext ? launch_chain(k_build_eq<true>, g, tpb, 0, s, w, v, lsb ? 1 : 0, c0, c1, c2)
-               : launch_chain(k_build_eq<false>, g, tpb, 0, s, w, v, lsb ? 1 : 0, c0, c1, c2);
+    return ext ? launch_dep(k_build_eq<true>, g, tpb, 0, s, w, v, lsb ? 1 : 0, c0, c1, c2)
+               : launch_dep(k_build_eq<false>, g, tpb, 0, s, w, v, lsb ? 1 : 0, c0, c1, c2);
 }
 
 }  // namespace effsc

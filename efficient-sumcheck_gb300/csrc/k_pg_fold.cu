@@ -324,9 +324,8 @@ extern "C" int effsc_protogalaxy_fold(effsc_ctx* ctx, int field, const uint64_t*
         res_fallback.assign(res_bytes / 8, 0);
         res = res_fallback.data();
     }
-    // the last pass writes the row there itself (a copy of a few hundred bytes
-    // and the gaps between plainly launched passes were a tenth of a call:
-    // 2^20 rows of 8, 114 -> 104 us)
+    // the last pass writes the row there itself (2^20 rows of 8, a call: 114 ->
+    // 104 us without the copy; 92 with the passes as dependent launches)
     u64* res_dev = nullptr;
     if (!res_fallback.empty() || cudaHostGetDevicePointer((void**)&res_dev, res, 0) != cudaSuccess) {
         cudaGetLastError();
@@ -382,8 +381,8 @@ extern "C" int effsc_protogalaxy_fold(effsc_ctx* ctx, int field, const uint64_t*
                 }
                 const size_t smem = (PG_TPB / 32) * pg_warp_smem(w, gw, ew);
                 const unsigned grid = (unsigned)((trees + PG_TPB / 32 - 1) / (PG_TPB / 32));
-                if (ew == 3) launch_chain(k_pg_warp<true>, grid, PG_TPB, smem, s, cur, trees, w, gw, muls(lvl, gw), dst);
-                else launch_chain(k_pg_warp<false>, grid, PG_TPB, smem, s, cur, trees, w, gw, muls(lvl, gw), dst);
+                if (ew == 3) launch_dep(k_pg_warp<true>, grid, PG_TPB, smem, s, cur, trees, w, gw, muls(lvl, gw), dst);
+                else launch_dep(k_pg_warp<false>, grid, PG_TPB, smem, s, cur, trees, w, gw, muls(lvl, gw), dst);
                 effsc_internal_add_launches(1);
                 PCK(cudaGetLastError());
                 cur = dst;
@@ -406,14 +405,14 @@ extern "C" int effsc_protogalaxy_fold(effsc_ctx* ctx, int field, const uint64_t*
             if (g) {
                 const size_t smem = pg_group_smem(w, g, ew);
                 const u32 S = pg_stride(w, g);
-                if (ew == 3) launch_chain(k_pg_group<true>, (unsigned)out_rows, PG_TPB, smem, s, cur, w, g, S, muls(lvl, g), dst);
-                else launch_chain(k_pg_group<false>, (unsigned)out_rows, PG_TPB, smem, s, cur, w, g, S, muls(lvl, g), dst);
+                if (ew == 3) launch_dep(k_pg_group<true>, (unsigned)out_rows, PG_TPB, smem, s, cur, w, g, S, muls(lvl, g), dst);
+                else launch_dep(k_pg_group<false>, (unsigned)out_rows, PG_TPB, smem, s, cur, w, g, S, muls(lvl, g), dst);
                 lvl += g;
             } else {
                 const size_t items = out_rows * (w + 1);
                 const unsigned grid = (unsigned)std::min<size_t>((items + PG_TPB - 1) / PG_TPB, 152 * 16);
-                if (ew == 3) launch_chain(k_pg_level<true>, grid, PG_TPB, 0, s, cur, out_rows, w, muls(lvl, 1), dst);
-                else launch_chain(k_pg_level<false>, grid, PG_TPB, 0, s, cur, out_rows, w, muls(lvl, 1), dst);
+                if (ew == 3) launch_dep(k_pg_level<true>, grid, PG_TPB, 0, s, cur, out_rows, w, muls(lvl, 1), dst);
+                else launch_dep(k_pg_level<false>, grid, PG_TPB, 0, s, cur, out_rows, w, muls(lvl, 1), dst);
                 lvl += 1;
             }
             effsc_internal_add_launches(1);

@@ -559,7 +559,7 @@ static bool tail_inst(const TailArgs* dev_args, const TailArgs* one, u32 n, u64 
     if (bytes > TAIL_SMEM_CAP) return false;
     if (one) {
         cudaFuncSetAttribute(k_tail_one<POL, FW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAIL_SMEM_CAP);
-        return launch_chain(k_tail_one<POL, FW>, 1, TAIL_TPB, bytes, s, *one);
+        return launch_dep(k_tail_one<POL, FW>, 1, TAIL_TPB, bytes, s, *one);
     } else {
         cudaFuncSetAttribute(k_tail_many<POL, FW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAIL_SMEM_CAP);
         k_tail_many<POL, FW><<<n, TAIL_TPB, bytes, s>>>(dev_args);
@@ -587,7 +587,7 @@ static bool tail_cluster_inst(const TailArgs& a, u32 cs_log, u32 g_log, cudaStre
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl_on() ? 2 : 1;
+    cfg.numAttrs = pdl_on(true) ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, k_tail_cluster<POL, FW>, a, cs_log, g_log) == cudaSuccess;
 }
 

@@ -12,15 +12,18 @@ namespace effsc {
 // Threads per block of every round kernel.
 constexpr int KERNEL_TPB = 256;
 
-// Kernels of a proof's chain are launched with programmatic dependent launch:
-// a kernel may be scheduled while the previous kernel on the stream drains
-// (its last block's reduction and transcript step), and waits on the device
-// (griddepcontrol.wait, the first statement of every such kernel) before it
-// touches memory.  EFFSC_PDL=0 in the environment launches them plainly.
-bool pdl_on(void);
+// Programmatic dependent launch: a kernel may be scheduled while the previous
+// kernel on the stream drains, and waits on the device (griddepcontrol.wait,
+// the first statement of every such kernel) before it touches memory.  Worth
+// it for kernels of a few blocks (launch_dep: the passes of the polynomial
+// fold, a proof's ends and tails); the grids of the rounds take SMs from the
+// kernel they wait for (2^26 entries 756 us a proof without, 763 with; LSB 2^24
+// 364 and 373), so launch_chain asks for it only under EFFSC_PDL=1.
+// EFFSC_PDL=0 launches all of them plainly.
+bool pdl_on(bool few_blocks);
 template <class... KArgs, class... Args>
-inline bool launch_chain(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                         Args... args) {
+inline bool launch_with(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                        Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -30,8 +33,16 @@ inline bool launch_chain(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = pdl_on() ? 1 : 0;
+    cfg.numAttrs = pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
+}
+template <class... KArgs, class... Args>
+inline bool launch_chain(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+    return launch_with(pdl_on(false), kernel, grid, block, smem, s, args...);
+}
+template <class... KArgs, class... Args>
+inline bool launch_dep(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+    return launch_with(pdl_on(true), kernel, grid, block, smem, s, args...);
 }
 int max_grid(void);
 // One wave of a grid-stride kernel: the blocks the SMs hold at once (the
