@@ -50,8 +50,8 @@ UNIT = "evals/s"
 # one full-size ncu capture of dram__bytes_read.sum / dram__bytes_write.sum
 # (a one-pass metric set) of `bench.py --only inner_product_msb --num-vars 26
 # --steps 1`; the fused rounds' figure is the average over their launches.
-NCU_TRAFFIC = {("ip_round_3_triple_fold", 26): 1449.9e6, ("ip_rounds_0_2", 26): 1077.2e6,
-               ("fused_round_fp3", 26): 144.4e6}
+NCU_TRAFFIC = {("ip_fold_and_round", 26): 1214.1e6, ("ip_first_rounds", 26): 1076.9e6,
+               ("fused_round_fp3", 26): 75.5e6}
 
 
 def parse():
@@ -444,7 +444,7 @@ def run_ours(args):
                 "algorithmic_bytes": 128 * n, "algorithmic_mulmods": 20 * n,
                 "equivalent_gbs": 128 * n / (ms_proof * 1e-3) / 1e9,
                 "note": "textbook schedule (one fold+evaluate pass per round), for comparison only: the proof "
-                        "computes rounds 0-3 in two passes over the base tables and moves 56N bytes, so this is "
+                        "computes rounds 0-4 in two passes over the base tables and moves 44N bytes, so this is "
                         "not its roofline"},
             "frac_of_lower_roofline": max(hbm_roof_ms, int_roof_ms) / ms_proof,
             "per_kernel": {k: {"launches": v["launches"], "ms": round(v["ms"], 4),
@@ -479,17 +479,17 @@ def batch_label(i):
 
 def ip_fp3_ops_as_run(n_vars):
     """64 x 64-bit products and 160-bit -> canonical reductions of one IP MSB
-    proof over Fp3 challenges as the device runs it (base tables of 2^n_vars,
-    n_vars >= 14): the first pass, 26 products per octet (N/8 octets, its
-    sums reduced once per thread); the triple fold, per item (two octets of
-    both tables, N/16 items) 4 x 21 products for the folds and 18 for round
-    3's two Fp3 x Fp3 sums, 12 reductions (the folded entries); every later
-    round (and the tail's rounds), per quadruple of the table being folded,
-    4 Fp3 folds of 9 products and 2 Fp3 x Fp3 sums of 9, 12 reductions."""
+    proof over Fp3 challenges as the integer pipes run it (base tables of
+    2^n_vars, n_vars >= 14): the first pass (rounds 0-3) and the fold by four
+    challenges are digit products on the tensor cores, which leave the integer
+    pipes 6 reductions per folded entry (both tables, N/16 entries) and round
+    4's two Fp3 x Fp3 sums, 18 products per folded pair; every later round
+    (and the tail's rounds), per quadruple of the table being folded, 4 Fp3
+    folds of 9 products and 2 Fp3 x Fp3 sums of 9, 12 reductions."""
     N = 1 << n_vars
-    prods = 26 * (N // 8) + (4 * 21 + 18) * (N // 16)
-    reds = 12 * (N // 16)
-    L = N // 8
+    prods = 18 * (N // 32)
+    reds = 6 * (N // 16)
+    L = N // 16
     while L >= 4:
         prods += 54 * (L // 4)
         reds += 12 * (L // 4)
@@ -499,16 +499,18 @@ def ip_fp3_ops_as_run(n_vars):
 
 def ip_fp3_bytes_as_run(n_vars):
     """Algorithmic HBM bytes of one IP MSB proof over Fp3 challenges as the
-    batched path runs it without the tail: rounds 0-1 read both base tables
-    (16 B per entry), round 2 reads them again and writes the Fp3 tables of
-    length N/4 (16 + 12 B per entry), round r >= 3 reads the Fp3 tables of
-    length N / 2^(r-1) and writes the halves (72 B per input entry);
+    batched path runs it without the tail.  From 2^14 entries: rounds 0-3 read
+    both base tables (16 B per entry), round 4 reads them again and writes the
+    Fp3 tables of length N/16 (16 + 3 B per entry), round r >= 5 reads the Fp3
+    tables of length N / 2^(r-1) and writes the halves (72 B per input entry).
+    Below: rounds 0-1 read the base tables, round 2 reads them again and
+    writes the tables of length N/4 (16 + 12 B per entry), then as above;
     num_vars < 3 runs one pass per round."""
     if n_vars < 3:
         return ip_fp3_bytes(n_vars)
     N = 1 << n_vars
-    tot = 16 * N + 28 * N
-    for r in range(3, n_vars):
+    start, tot = (5, 16 * N + 19 * N) if n_vars >= 14 else (3, 16 * N + 28 * N)
+    for r in range(start, n_vars):
         tot += 72 * (N >> (r - 1))
     return tot + 96
 

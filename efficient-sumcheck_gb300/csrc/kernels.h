@@ -143,13 +143,13 @@ struct RoundArgs {
     const u64* chal2_ptr;  // second challenge (InnerProduct double fold of round 2)
     u64 chal[3];
     const u64* scalar[3];  // EqFactored right phase: eq_l[0] (c1, c2 null if base)
-    u64* partials;         // gridDim * 12 words
+    u64* partials;         // 12 words a block (the tensor-core passes: 256)
     u32* counter;          // zero between launches (the last block resets it)
     u64* result;           // wire (d*3 words) then aux pair (6 words)
     u32* status;           // device status word (non-zero: error code)
     TxIO tx;
     // the first pass of the InnerProduct start over a chunk of the tables:
-    // its tiles start at tile0, and its 26 sums go to `acc` (ACC_FIRST),
+    // its tiles start at tile0, and its sums go to `acc` (ACC_FIRST),
     // are added there (ACC_MID) or are added and finalised (ACC_LAST)
     u32 tile0;
     u32 acc_mode;
