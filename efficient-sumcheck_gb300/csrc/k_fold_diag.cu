@@ -30,6 +30,7 @@ __global__ void k_diag_transcript(u32 iters, u64* out) {
     __shared__ __align__(8) uint8_t s_scr[64];
     const int lane = threadIdx.x;
     WarpTx w;
+    w.k = keccak_lane(lane);
     w.a = lane < 25 ? (u64)lane * 0x9E3779B97F4A7C15ULL : 0;
     w.pos = 0;
     w.squeezing = 0;
@@ -37,7 +38,7 @@ __global__ void k_diag_transcript(u32 iters, u64* out) {
     if (lane < 3) s_v[lane] = 1 + lane;
     __syncwarp();
     const u64 t0 = global_ns();
-    for (u32 k = 0; k < iters; k++) keccak_f_warp(w.a, lane);
+    for (u32 k = 0; k < iters; k++) w.a = keccak_f_warp(w.a, w.k);
     const u64 t1 = global_ns();
     for (u32 k = 0; k < iters; k++) {
         tx_send_elems(w, lane, s_v, 1);

@@ -26,13 +26,13 @@ struct DevTranscript {
     u32 reserved;
 };
 
-static __constant__ u64 c_keccak_rc[24] = {
+static __constant__ u64 c_keccak_rc[25] = {
     0x0000000000000001ULL, 0x0000000000008082ULL, 0x800000000000808AULL, 0x8000000080008000ULL,
     0x000000000000808BULL, 0x0000000080000001ULL, 0x8000000080008081ULL, 0x8000000000008009ULL,
     0x000000000000008AULL, 0x0000000000000088ULL, 0x0000000080008009ULL, 0x000000008000000AULL,
     0x000000008000808BULL, 0x800000000000008BULL, 0x8000000000008089ULL, 0x8000000000008003ULL,
     0x8000000000008002ULL, 0x8000000000000080ULL, 0x000000000000800AULL, 0x800000008000000AULL,
-    0x8000000080008081ULL, 0x8000000000008080ULL, 0x0000000080000001ULL, 0x8000000080008008ULL};
+    0x8000000080008081ULL, 0x8000000000008080ULL, 0x0000000080000001ULL, 0x8000000080008008ULL, 0};
 
 // rotation offsets (rho), indexed by lane x + 5y
 static __constant__ int c_keccak_rot[25] = {0, 1, 62, 28, 27, 36, 44, 6, 55, 20, 3, 10, 43,
@@ -63,32 +63,53 @@ __device__ __forceinline__ u64 rotl64_1(u64 v) {
 // shuffles, the parity of column x lands in lane x), then C[x-1] and C[x+1];
 // pi and chi take B[x, y], B[x+1, y] and B[x+2, y] straight from the lanes
 // that rho-rotate into them.  Eight 64-bit shuffles per round, ~8 cycles
-// each and ~24 of latency per dependent step.  The rest of the round is kept
-// off that chain: the rotation amount is split once, and a round's constant
-// is loaded a round ahead, masked to lane 0 and folded into chi (loading it
-// where it is used waited on the constant cache every round).  Measured on
-// one warp: 262 -> 205 cycles per round.  Also measured: column parities
-// from shared memory (296), five columns on five lanes (288), a 12-shuffle
-// parity with one dependent step fewer (255), the 24 rounds unrolled (248:
-// instruction fetch).
-static __device__ __noinline__ void keccak_f_warp(u64& a, int lane) {
-    const int i = lane < 25 ? lane : 0;
-    const int x = i % 5, y = i / 5;
-    const u32 rot = (u32)c_keccak_rot[i], my_rot = rot & 31;
-    const bool swap = rot >= 32;
+// each and ~24 of latency per dependent step.  The rest is kept off that
+// chain: a round's constant is loaded a round ahead (from a table with one
+// word more, so that its index needs no test), masked to lane 0 and folded
+// into chi; three rounds make a loop iteration, whose branch costs 50 cycles;
+// and what a lane needs to know -- its shuffles' sources, its rotation -- is
+// worked out once per kernel and handed over in two registers (KeccakLane):
+// worked out by every call it took 40 cycles a round.  Measured, a
+// permutation of a chain: 2.95 us with two rounds an iteration and the lane's
+// constants in the call, 2.60 with three, 2.21 with KeccakLane; the tail of
+// 2^12 entries 66 -> 58 us (four rounds an iteration 59, six 59, two 60).  Also
+// measured, in cycles a round against 262 -> 205 for the same change: column
+// parities from shared memory (296), five columns on five lanes (288), a
+// 12-shuffle parity with one dependent step fewer (255), the 24 rounds
+// unrolled (248: instruction fetch).
+// from: the shuffles' sources, five bits each; misc: C[x-1]'s and C[x+1]'s,
+// the rotation, and whether this is lane 0 or none of the 25.
+struct KeccakLane {
+    u32 from, misc;
+};
+__device__ __forceinline__ KeccakLane keccak_lane(int lane) {
+    const u32 i = lane < 25 ? lane : 0;
+    const u32 x = i % 5, y = i / 5;
     // pi: B[X, Y] = rho(A[x, y]) with X = y, Y = 2x + 3y; the source of lane
     // (X, Y) is x = (X + 3Y) mod 5, y = X.
-    const int xp1 = (x + 1) % 5, xp2 = (x + 2) % 5, xm1 = (x + 4) % 5;
-    const int src0 = ((x + 3 * y) % 5) + 5 * x;
-    const int src1 = ((xp1 + 3 * y) % 5) + 5 * xp1;
-    const int src2 = ((xp2 + 3 * y) % 5) + 5 * xp2;
-    const int l5 = min(i + 5, 31), l10 = min(i + 10, 31), l20 = min(i + 20, 31);
-    const u64 lane0 = lane == 0 ? ~0ULL : 0ULL;
+    const u32 xp1 = (x + 1) % 5, xp2 = (x + 2) % 5, xm1 = (x + 4) % 5;
+    const u32 src0 = ((x + 3 * y) % 5) + 5 * x;
+    const u32 src1 = ((xp1 + 3 * y) % 5) + 5 * xp1;
+    const u32 src2 = ((xp2 + 3 * y) % 5) + 5 * xp2;
+    const u32 rot = (u32)c_keccak_rot[i];
+    KeccakLane k;
+    k.from = src0 | src1 << 5 | src2 << 10 | min(i + 5, 31u) << 15 | min(i + 10, 31u) << 20 | min(i + 20, 31u) << 25;
+    k.misc = xm1 | xp1 << 5 | rot << 10 | (lane == 0 ? 1u << 16 : 0) | (lane >= 25 ? 1u << 17 : 0);
+    return k;
+}
+static __device__ __noinline__ u64 keccak_f_warp(u64 a, KeccakLane k) {
+    // a shuffle takes its source from the register's low five bits
+    const int src0 = k.from & 31, src1 = k.from >> 5 & 31, src2 = k.from >> 10 & 31;
+    const int l5 = k.from >> 15 & 31, l10 = k.from >> 20 & 31, l20 = k.from >> 25 & 31;
+    const int xm1 = k.misc & 31, xp1 = k.misc >> 5 & 31;
+    const u32 my_rot = k.misc >> 10 & 31;
+    const bool swap = k.misc >> 15 & 1;
+    const u64 lane0 = k.misc >> 16 & 1 ? ~0ULL : 0ULL;
     u64 next_rc = c_keccak_rc[0];
-#pragma unroll 2
+#pragma unroll 3
     for (int round = 0; round < 24; round++) {
         const u64 rc = next_rc & lane0;
-        next_rc = c_keccak_rc[round < 23 ? round + 1 : 0];
+        next_rc = c_keccak_rc[round + 1];
         u64 v = a ^ shfl64(a, l5);           // rows y, y+1
         const u64 a20 = shfl64(a, l20);      // row y+4 (used by lanes 0..4)
         v = v ^ shfl64(v, l10) ^ a20;        // rows y..y+3; lanes 0..4: C[x]
@@ -98,12 +119,13 @@ static __device__ __noinline__ void keccak_f_warp(u64& a, int lane) {
         const u64 b = shfl64(r, src0), b1 = shfl64(r, src1), b2 = shfl64(r, src2);
         a = b ^ (~b1 & b2) ^ rc;
     }
-    if (lane >= 25) a = 0;
+    return k.misc >> 17 & 1 ? 0 : a;
 }
 
 // Transcript state held by one warp: lane state word, byte position, mode.
 struct WarpTx {
     u64 a;
+    KeccakLane k;
     u32 pos;
     u32 squeezing;
     u32 deg;
@@ -112,6 +134,7 @@ struct WarpTx {
 __device__ __forceinline__ WarpTx tx_load(const DevTranscript* t, int lane) {
     WarpTx w;
     w.a = lane < 25 ? t->st[lane] : 0;
+    w.k = keccak_lane(lane);
     w.pos = t->pos;
     w.squeezing = t->squeezing;
     w.deg = t->deg;
@@ -128,7 +151,7 @@ __device__ __forceinline__ void tx_absorb(WarpTx& w, int lane, u32 len, Get get)
     if (w.squeezing) { w.pos = 0; w.squeezing = 0; }
     u32 done = 0;
     while (done < len) {
-        if (w.pos == TX_RATE) { keccak_f_warp(w.a, lane); w.pos = 0; }
+        if (w.pos == TX_RATE) { w.a = keccak_f_warp(w.a, w.k); w.pos = 0; }
         u32 chunk = min(len - done, (u32)TX_RATE - w.pos);
         if (lane < TX_RATE / 8) {
             u64 x = 0;
@@ -147,16 +170,16 @@ __device__ __forceinline__ void tx_absorb(WarpTx& w, int lane, u32 len, Get get)
 template <class Put>
 __device__ __forceinline__ void tx_squeeze(WarpTx& w, int lane, u32 len, Put put) {
     if (!w.squeezing) {
-        if (w.pos == TX_RATE) { keccak_f_warp(w.a, lane); w.pos = 0; }
+        if (w.pos == TX_RATE) { w.a = keccak_f_warp(w.a, w.k); w.pos = 0; }
         if (lane == (int)(w.pos >> 3)) w.a ^= (u64)0x06 << (8 * (w.pos & 7));
         if (lane == (TX_RATE - 1) / 8) w.a ^= (u64)0x80 << (8 * ((TX_RATE - 1) & 7));
-        keccak_f_warp(w.a, lane);
+        w.a = keccak_f_warp(w.a, w.k);
         w.pos = 0;
         w.squeezing = 1;
     }
     u32 done = 0;
     while (done < len) {
-        if (w.pos == TX_RATE) { keccak_f_warp(w.a, lane); w.pos = 0; }
+        if (w.pos == TX_RATE) { w.a = keccak_f_warp(w.a, w.k); w.pos = 0; }
         u32 chunk = min(len - done, (u32)TX_RATE - w.pos);
         if (lane < TX_RATE / 8) {
 #pragma unroll
@@ -177,7 +200,7 @@ __device__ __forceinline__ void tx_absorb_words(WarpTx& w, int lane, u32 nwords,
     if (w.squeezing) { w.pos = 0; w.squeezing = 0; }
     u32 done = 0;
     while (done < nwords) {
-        if (w.pos == TX_RATE) { keccak_f_warp(w.a, lane); w.pos = 0; }
+        if (w.pos == TX_RATE) { w.a = keccak_f_warp(w.a, w.k); w.pos = 0; }
         const u32 p8 = w.pos >> 3;
         const u32 chunk = min(nwords - done, (u32)(TX_RATE / 8) - p8);
         if ((u32)lane >= p8 && (u32)lane < p8 + chunk) w.a ^= getw(done + (u32)lane - p8);
@@ -188,16 +211,16 @@ __device__ __forceinline__ void tx_absorb_words(WarpTx& w, int lane, u32 nwords,
 template <class PutW>
 __device__ __forceinline__ void tx_squeeze_words(WarpTx& w, int lane, u32 nwords, PutW putw) {
     if (!w.squeezing) {
-        if (w.pos == TX_RATE) { keccak_f_warp(w.a, lane); w.pos = 0; }
+        if (w.pos == TX_RATE) { w.a = keccak_f_warp(w.a, w.k); w.pos = 0; }
         if (lane == (int)(w.pos >> 3)) w.a ^= (u64)0x06 << (8 * (w.pos & 7));
         if (lane == (TX_RATE - 1) / 8) w.a ^= (u64)0x80 << (8 * ((TX_RATE - 1) & 7));
-        keccak_f_warp(w.a, lane);
+        w.a = keccak_f_warp(w.a, w.k);
         w.pos = 0;
         w.squeezing = 1;
     }
     u32 done = 0;
     while (done < nwords) {
-        if (w.pos == TX_RATE) { keccak_f_warp(w.a, lane); w.pos = 0; }
+        if (w.pos == TX_RATE) { w.a = keccak_f_warp(w.a, w.k); w.pos = 0; }
         const u32 p8 = w.pos >> 3;
         const u32 chunk = min(nwords - done, (u32)(TX_RATE / 8) - p8);
         if ((u32)lane >= p8 && (u32)lane < p8 + chunk) putw(done + (u32)lane - p8, w.a);
@@ -281,7 +304,7 @@ __device__ __forceinline__ u64 tx_step(WarpTx& w, const TxStream& s, int nw, int
             x = (lane >= q ? x0 << sh : 0) | (sh && lane > q ? x1 >> (64 - sh) : 0);
         }
         w.a ^= x ^ (lane == TX_RATE / 8 - 1 ? 0x80ULL << 56 : 0);
-        keccak_f_warp(w.a, lane);
+        w.a = keccak_f_warp(w.a, w.k);
         w.pos = 16 * deg;
         w.squeezing = 1;
         const u64 lo = shfl64(w.a, (2 * lane) & 31), hi = shfl64(w.a, (2 * lane + 1) & 31);
