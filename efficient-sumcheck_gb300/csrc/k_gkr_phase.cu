@@ -18,7 +18,7 @@
 //
 // Folding the gate tables round by round moved 7.5 n^2 words (k = 12: 692 us
 // of kernels); this reads them twice, 71 us each on the tensor cores
-// (k_eqf_tc.cu), plus two tails of 70 us: 316 us.  The tails are one warp's
+// (k_eqf_tc.cu), plus two tails of 63 us: 294 us.  The tails are one warp's
 // latency, the reads two thirds of the copy rate.  Up to n = 1024 the sums run
 // here on the integer pipes, a warp per row and eight columns a block: their
 // tables fit L2 and a tensor-core block's start and end cost more than they do

@@ -11,9 +11,9 @@
 //
 // MSB: b is the high half of the index, T a sum along rows; LSB: the low half,
 // a sum down columns.  Memory bounds both reads from 2^24 entries on; below, the
-// two tails are three quarters of the time (20 rounds of 4.2 us).  A call, Fp,
-// 2^20 entries: 127 -> 111 us (LSB 143 -> 114); Fp3, 2^25: 448 -> 250 (LSB
-// 618 -> 255).
+// two tails are three quarters of the time (20 rounds of 3.4 us).  A call, Fp,
+// 2^20 entries: 127 -> 111 us (LSB 143 -> 114; 101 with the present
+// permutation); Fp3, 2^25: 448 -> 250 (LSB 618 -> 255).
 #include "round_common.cuh"
 
 namespace effsc {

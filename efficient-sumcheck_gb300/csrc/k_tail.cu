@@ -15,12 +15,13 @@
 // accessors see exactly what the per-round path would leave.  A batch
 // launches one block per instance.
 //
-// What bounds it is one warp's latency: of about 5.5 us a round (InnerProduct
-// over Fp3), 2.6 are the Keccak permutation, the rest the chain fold ->
+// What bounds it is one warp's latency: of 3.4 us a late round (InnerProduct
+// over Fp3), 2.2 are the Keccak permutation, the rest the chain fold ->
 // barrier -> sums -> barrier -> absorb, squeeze, reduce -> barrier.  n = 12:
 // 110.8 us when a thread carried whole quadruples and the words were summed
 // with shuffles, 74.8 in one block as split below, 66.6 in a cluster (whose
-// two barriers a round cost less than the first rounds' folds on one SM).
+// two barriers a round cost less than the first rounds' folds on one SM), 58
+// with the present permutation.
 #include "round_common.cuh"
 
 #include <atomic>
