@@ -75,7 +75,7 @@ __device__ __forceinline__ void verify_map(u32 d, const u64* w, const F3& r, F3&
                      f3_mul<true, true>(hinf, f3_mul<true, true>(f3_mul<true, true>(r, r), r)));
 }
 
-// What bounds it is the longest proof's chain of permutations (2.6 us each):
+// What bounds it is the longest proof's chain of permutations (2.2 us each):
 // so nothing else is on it.  The wire words are read a round ahead, the
 // transcript steps of 32 rounds run one after the other, and then each lane
 // forms one round's affine map and five levels of composition give the claim
