@@ -2562,6 +2562,7 @@ int effsc_prover_table_len(const effsc_prover* P, int table, size_t* out) {
     return EFFSC_OK;
 }
 
+constexpr size_t READ_PINNED_MAX = 64 << 10;
 int effsc_prover_read_table(effsc_prover* P, int table, uint64_t* out) {
     size_t n = 0;
     TRY(effsc_prover_table_len(P, table, &n));
@@ -2571,12 +2572,33 @@ int effsc_prover_read_table(effsc_prover* P, int table, uint64_t* out) {
     cudaStream_t s = P->ctx->stream;
     Table& T = P->t[table];
     const Buf& b = T.bufs[T.cur];
+    const size_t bytes = n * (size_t)P->field * sizeof(u64);
+    auto join = [&](u64* dst) {
+        launch_join_aos(b.p[0], T.ext ? b.p[1] : nullptr, T.ext ? b.p[2] : nullptr, n, P->field, dst,
+                        P->repr == EFFSC_MONTGOMERY, s);
+        g_launches++;
+    };
+    // a small table straight into a pinned block of the pool: no allocation,
+    // no pageable copy (an EqFactored
+    // proof of 2^24 entries and its three tables of 2^8: 271 -> 245 us)
+    if (bytes <= READ_PINNED_MAX) {
+        if (u64* h = (u64*)pinned_get(P->ctx, READ_PINNED_MAX)) {
+            u64* d = nullptr;
+            cudaError_t e = cudaHostGetDevicePointer((void**)&d, h, 0);
+            if (e == cudaSuccess) {
+                join(d);
+                e = cudaStreamSynchronize(s);
+                if (e == cudaSuccess) memcpy(out, h, bytes);
+            }
+            pinned_put(P->ctx, h, READ_PINNED_MAX);
+            CK(e);
+            return EFFSC_OK;
+        }
+    }
     u64* stage = nullptr;
-    CK(cudaMallocAsync((void**)&stage, n * (size_t)P->field * sizeof(u64), s));
-    launch_join_aos(b.p[0], T.ext ? b.p[1] : nullptr, T.ext ? b.p[2] : nullptr, n, P->field, stage,
-                    P->repr == EFFSC_MONTGOMERY, s);
-    g_launches++;
-    CK(cudaMemcpyAsync(out, stage, n * (size_t)P->field * sizeof(u64), cudaMemcpyDeviceToHost, s));
+    CK(cudaMallocAsync((void**)&stage, bytes, s));
+    join(stage);
+    CK(cudaMemcpyAsync(out, stage, bytes, cudaMemcpyDeviceToHost, s));
     CK(cudaFreeAsync(stage, s));
     CK(cudaStreamSynchronize(s));
     return EFFSC_OK;
