@@ -1785,18 +1785,39 @@ thread_local const u64* g_first = nullptr;
 constexpr size_t TX_OUT_WORDS = (sizeof(DevTranscript) + 7) / 8;
 constexpr size_t HOOK_IN_WORDS = 64;   // hooks up to this long travel with the transcript's state
 
-int read_first(effsc_prover* P, int ti, HF* out) {
-    if (g_first) {
-        *out = hf(g_first[3 * ti], g_first[3 * ti + 1], g_first[3 * ti + 2]);
-        return EFFSC_OK;
+// The tables' current first entries, for k_gather_first.
+FirstSrc first_entries(const effsc_prover* P) {
+    FirstSrc src;
+    memset(&src, 0, sizeof src);
+    for (int i = 0; i < 4; i++) {
+        if (P->t[i].bufs.empty() || !P->t[i].len) continue;
+        const Buf& b = P->t[i].bufs[P->t[i].cur];
+        for (int c = 0; c < (P->t[i].ext ? 3 : 1); c++) src.p[i][c] = b.p[c];
     }
-    Table& T = P->t[ti];
-    const Buf& b = T.bufs[T.cur];
-    u64 w[3] = {0, 0, 0};
-    for (int c = 0; c < (T.ext ? 3 : 1); c++)
-        CK(cudaMemcpyAsync(&w[c], b.p[c], sizeof(u64), cudaMemcpyDefault, P->ctx->stream));
-    CK(cudaStreamSynchronize(P->ctx->stream));
-    *out = hf(w[0], w[1], w[2]);
+    return src;
+}
+// Outside effsc_prove: all of them at once into the prover's mapped result
+// block (12 of its words), read there while this object lives (a copy for
+// every component and a synchronisation for every table before: GKR's witness
+// values after a proof of k = 12, PLACEHOLDER us for both).
+struct FirstEntries {
+    int rc = EFFSC_OK;
+    explicit FirstEntries(effsc_prover* P, bool want = true) {
+        if (g_first || !want) return;
+        launch_gather_first(first_entries(P), P->d_res, P->ctx->stream);
+        g_launches++;
+        const cudaError_t e = cudaStreamSynchronize(P->ctx->stream);
+        if (e != cudaSuccess) rc = fail(EFFSC_CUDA_ERROR, "reading the tables' first entries: %s", cudaGetErrorString(e));
+        else { g_first = P->h_res; own = true; }
+    }
+    ~FirstEntries() { if (own) g_first = nullptr; }
+    bool own = false;
+};
+
+int read_first(effsc_prover* P, int ti, HF* out) {
+    FirstEntries f(P);
+    TRY(f.rc);
+    *out = hf(g_first[3 * ti], g_first[3 * ti + 1], g_first[3 * ti + 2]);
     return EFFSC_OK;
 }
 
@@ -2438,6 +2459,8 @@ int effsc_gkr_claimed_w_values(effsc_prover* P, uint64_t* out) {
     CK(cudaSetDevice(P->ctx->device));
     HF wb = hf(0), wc = hf(0);
     if (P->t[0].len == 1) {
+        FirstEntries f(P);
+        TRY(f.rc);
         TRY(read_first(P, 2, &wb));
         TRY(read_first(P, 3, &wc));
     }
@@ -2549,6 +2572,10 @@ int effsc_prover_final_value(effsc_prover* P, uint64_t* out) {
     if (!P || !out) return fail(EFFSC_INVALID_ARG, "NULL argument");
     CK(cudaSetDevice(P->ctx->device));
     HF v;
+    bool single = false;
+    for (const Table& T : P->t) single |= !T.bufs.empty() && T.len == 1;
+    FirstEntries f(P, single);
+    TRY(f.rc);
     TRY(final_value(P, &v));
     store_elem(out, v, P->field, P->repr);
     return EFFSC_OK;
@@ -2852,14 +2879,7 @@ int effsc_prove(effsc_prover* P, size_t num_rounds, effsc_transcript* T, const u
             TRY(do_finalize(P, ch, dry));
         }
         if (!dry) {
-            FirstSrc src;
-            memset(&src, 0, sizeof src);
-            for (int i = 0; i < 4; i++) {
-                if (P->t[i].bufs.empty()) continue;
-                const Buf& b = P->t[i].bufs[P->t[i].cur];
-                for (int c = 0; c < (P->t[i].ext ? 3 : 1); c++) src.p[i][c] = b.p[c];
-            }
-            launch_gather_first(src, P->d_first, s);
+            launch_gather_first(first_entries(P), P->d_first, s);
             g_launches++;
         }
         return EFFSC_OK;
