@@ -44,10 +44,13 @@ _Words = ctypes.c_uint64 * 0
 def _p(a):
     """A pointer to the array's words, holding the array (through its buffer
     0.7 us; the ndarray's own ctypes view, for what cannot lend a writable
-    one, 4.9)."""
+    one, 4.9).  The words have to lie in C order: the library reads them as
+    they are in memory."""
     try:
         return _Words.from_buffer(a)
     except (TypeError, ValueError):
+        if not a.flags.c_contiguous:
+            raise ValueError("the array's words are not in C order") from None
         return a.ctypes.data_as(u64p)
 
 
@@ -670,8 +673,10 @@ def sumcheck_verify_batch(claimed_sums, degree, round_polys, transcripts, hook=b
     total = int(rounds.sum(dtype=np.int64))
     if not total:
         flat = np.zeros(1, dtype=np.uint64)
-    elif len({rp.shape[1:] for rp in polys}) == 1:     # whole rows: a third of the time of joining flat views
-        flat = np.concatenate(polys, dtype=np.uint64, casting="unsafe")
+    elif len({rp.shape[1:] for rp in polys}) == 1:
+        # whole rows: a third of the time of joining flat views.  The result
+        # keeps a memory order that all of them share, so C order is asked for.
+        flat = np.ascontiguousarray(np.concatenate(polys, dtype=np.uint64, casting="unsafe"))
     else:
         flat = np.concatenate([np.asarray(rp, dtype=np.uint64).reshape(-1) for rp in polys])
     cs = np.ascontiguousarray(np.asarray(claimed_sums, dtype=np.uint64).reshape(n, field))
