@@ -38,7 +38,7 @@ __device__ __forceinline__ u32 et_row(u32 q) { return q ^ ((q >> 3) & 1); }
 // entry m at part[3 (split M + m) + c], or without part (one split) at o[c][m].
 template <bool ALONG, bool EW>
 __global__ void __launch_bounds__(ET_TPB, 1) k_eqf_tc(const u64* p, const u64* p2, u64 stride, Tab3 w, u64 M, u64 K,
-                                                      u32 splits, u64* part, u64* o0, u64* o1, u64* o2, u32* status) {
+                                                      u32 splits, u64* part, u64* o0, u64* o1, u64* o2, TcWaits tw) {
     constexpr int NC = EW ? 3 : 1;
     extern __shared__ char et_dyn[];
     __shared__ u64 full[ET_S], empty[ET_S], done;
@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(ET_TPB, 1) k_eqf_tc(const u64* p, const u64* p
                 const u32 i = i0 + q;
                 if (i >= tiles || abort) break;
                 const u32 s = i % ET_S;
-                if (!mbar_wait_bounded(&empty[s], ((i / ET_S) & 1u) ^ 1u)) { abort = true; break; }
+                if (!mbar_wait_warp(&empty[s], ((i / ET_S) & 1u) ^ 1u, tw.no_wait)) { abort = true; break; }
                 char* st = stages + s * ET_BYTES;
 #pragma unroll
                 for (int u = 0; u < 2; u++) {
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(ET_TPB, 1) k_eqf_tc(const u64* p, const u64* p
                 const u32 i = i0 + q;
                 if (i >= tiles || abort) break;
                 const u32 s = i % ET_S;
-                if (!mbar_wait_bounded(&empty[s], ((i / ET_S) & 1u) ^ 1u)) { abort = true; break; }
+                if (!mbar_wait_warp(&empty[s], ((i / ET_S) & 1u) ^ 1u, tw.no_wait)) { abort = true; break; }
                 char* st = stages + s * ET_BYTES + 8 * ET_ATOM;
 #pragma unroll
                 for (int c = 0; c < NC; c++) *(uint4*)(st + swz128(et_row(lane), c)) = digits_of(x[q][c]);
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(ET_TPB, 1) k_eqf_tc(const u64* p, const u64* p
     } else if (lane == 0) {
         for (u32 i = 0; i < tiles; i++) {
             const u32 s = i % ET_S;
-            if (!mbar_wait_bounded(&full[s], (i / ET_S) & 1u)) { abort = true; break; }
+            if (!mbar_wait_step(&full[s], (i / ET_S) & 1u, tw.no_wait)) { abort = true; break; }
             tc_fence_after();
             const u32 base = smem_u32(stages) + s * ET_BYTES;
             const u64 b = tc_desc(base + 8 * ET_ATOM, ET_ATOM, 1024);
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(ET_TPB, 1) k_eqf_tc(const u64* p, const u64* p
     tc_fence_before();
     __syncthreads();
     if (warp == ET_LW + 1) tc_dealloc(tmem, 512);
-    if (bad && threadIdx.x == 0 && status) *(volatile u32*)status = EFFSC_STATUS_TIMEOUT;
+    if (bad && threadIdx.x == 0 && tw.status) *(volatile u32*)tw.status = EFFSC_STATUS_TIMEOUT;
 }
 
 // Blocks for M entries: splits of K until about a wave of blocks, at least
@@ -191,31 +191,31 @@ bool eqf_tc_ok(bool along, u64 M, u64 K, u64 stride, const u64* p) {
 }
 template <bool ALONG, bool EW>
 static bool eqf_tc_inst(const u64* p, const u64* p2, u64 stride, Tab3 w, u64 M, u64 K, u32 splits, u64* part, u64* o0, u64* o1,
-                        u64* o2, u32* status, cudaStream_t s) {
+                        u64* o2, TcWaits tw, cudaStream_t s) {
     static std::atomic<uint64_t> configured{0};
     if (!tc_allow_smem(k_eqf_tc<ALONG, EW>, ET_SMEM, configured)) return false;
     k_eqf_tc<ALONG, EW><<<(int)((p2 ? 2 : 1) * (M / ET_M) * splits), ET_TPB, ET_SMEM, s>>>(p, p2, stride, w, M, K, splits, part, o0,
-                                                                                       o1, o2, status);
+                                                                                       o1, o2, tw);
     return true;
 }
 bool launch_eqf_tc(bool along, bool ew, const u64* p, u64 stride, Tab3 w, u64 M, u64 K, u64* part, u64* o0, u64* o1, u64* o2,
-                   u32* status, cudaStream_t s) {
+                   TcWaits tw, cudaStream_t s) {
     const u32 splits = eqf_tc_splits(M, K);
     u64* pt = splits > 1 ? part : nullptr;
     bool ok;
-    if (along) ok = ew ? eqf_tc_inst<true, true>(p, nullptr, stride, w, M, K, splits, pt, o0, o1, o2, status, s)
-                       : eqf_tc_inst<true, false>(p, nullptr, stride, w, M, K, splits, pt, o0, o1, o2, status, s);
-    else ok = ew ? eqf_tc_inst<false, true>(p, nullptr, stride, w, M, K, splits, pt, o0, o1, o2, status, s)
-                 : eqf_tc_inst<false, false>(p, nullptr, stride, w, M, K, splits, pt, o0, o1, o2, status, s);
+    if (along) ok = ew ? eqf_tc_inst<true, true>(p, nullptr, stride, w, M, K, splits, pt, o0, o1, o2, tw, s)
+                       : eqf_tc_inst<true, false>(p, nullptr, stride, w, M, K, splits, pt, o0, o1, o2, tw, s);
+    else ok = ew ? eqf_tc_inst<false, true>(p, nullptr, stride, w, M, K, splits, pt, o0, o1, o2, tw, s)
+                 : eqf_tc_inst<false, false>(p, nullptr, stride, w, M, K, splits, pt, o0, o1, o2, tw, s);
     if (ok && splits > 1) launch_eqf_sum(part, M, splits, ew ? 3 : 1, o0, o1, o2, s);
     return ok;
 }
 bool launch_eqf_tc_pair(bool along, bool ew, const u64* p, const u64* p2, u64 stride, Tab3 w, u64 M, u64 K, u64* part,
-                        u32* status, cudaStream_t s) {
+                        TcWaits tw, cudaStream_t s) {
     const u32 splits = eqf_tc_splits(2 * M, K);
-    if (along) return ew && eqf_tc_inst<true, true>(p, p2, stride, w, M, K, splits, part, nullptr, nullptr, nullptr, status, s);
-    return ew ? eqf_tc_inst<false, true>(p, p2, stride, w, M, K, splits, part, nullptr, nullptr, nullptr, status, s)
-              : eqf_tc_inst<false, false>(p, p2, stride, w, M, K, splits, part, nullptr, nullptr, nullptr, status, s);
+    if (along) return ew && eqf_tc_inst<true, true>(p, p2, stride, w, M, K, splits, part, nullptr, nullptr, nullptr, tw, s);
+    return ew ? eqf_tc_inst<false, true>(p, p2, stride, w, M, K, splits, part, nullptr, nullptr, nullptr, tw, s)
+              : eqf_tc_inst<false, false>(p, p2, stride, w, M, K, splits, part, nullptr, nullptr, nullptr, tw, s);
 }
 
 }  // namespace effsc

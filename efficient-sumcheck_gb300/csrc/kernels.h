@@ -138,6 +138,7 @@ struct RoundArgs {
     TabIO t[4];
     u64 L;                 // length before folding (fold/fused) or current length (eval)
     u32 m_shift;           // EqFactored left phase: log2 |eq_r|; GkrProver: k = log2 |W|
+    u32 no_wait;           // the tensor-core passes' waits give up at once (self-test of that route)
     u64 el_len;            // EqFactored left phase: current |eq_l|
     const u64* chal_ptr;   // challenge in device memory, or null to use `chal`
     const u64* chal2_ptr;  // second challenge (InnerProduct double fold of round 2)
@@ -275,6 +276,12 @@ void launch_eqf_inner(bool ee, bool ep, Tab3 p, Tab3 er, u64 m, u64 rows, u64* s
 void launch_eqf_fold_rows(bool ew, bool ep, Tab3 p, Tab3 e, u64 Lc, u64 rows, u64 splits, u64* part, int fw, u64* o0,
                           u64* o1, u64* o2, cudaStream_t s);
 
+// What a pass's bounded waits take: the status word a timeout goes to, and
+// RoundArgs::no_wait.
+struct TcWaits {
+    u32* status;
+    u32 no_wait;
+};
 // Both sums over a base table on the tensor cores (k_eqf_tc.cu): out[m] = sum
 // over k < K of w[k] P(k, m), m < M, P(k, m) = p[m stride + k] (along) or
 // p[k stride + m]; ew: Fp3 weights and sums.  part: 3 M eqf_tc_splits(M, K)
@@ -282,12 +289,12 @@ void launch_eqf_fold_rows(bool ew, bool ep, Tab3 p, Tab3 e, u64 Lc, u64 rows, u6
 bool eqf_tc_ok(bool along, u64 M, u64 K, u64 stride, const u64* p);
 u32 eqf_tc_splits(u64 M, u64 K);
 bool launch_eqf_tc(bool along, bool ew, const u64* p, u64 stride, Tab3 w, u64 M, u64 K, u64* part, u64* o0, u64* o1, u64* o2,
-                   u32* status, cudaStream_t s);
+                   TcWaits tw, cudaStream_t s);
 // The same over two tables at once (along: Fp3 weights), the sums of the
 // eqf_tc_splits(2 M, K) splits left in part: component c of entry m of split i
 // of table t at part[3 ((t splits + i) M + m) + c].
 bool launch_eqf_tc_pair(bool along, bool ew, const u64* p, const u64* p2, u64 stride, Tab3 w, u64 M, u64 K, u64* part,
-                        u32* status, cudaStream_t s);
+                        TcWaits tw, cudaStream_t s);
 void launch_eqf_sum(const u64* part, u64 n, u64 splits, int fw, u64* o0, u64* o1, u64* o2, cudaStream_t s);
 // Sums along rows from 2^21 entries on (a block per row on the integer pipes
 // is 5 to 7 us faster below, over Fp3 and Fp), down columns from 2^18.

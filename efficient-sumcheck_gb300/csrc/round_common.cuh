@@ -695,6 +695,12 @@ __device__ __forceinline__ u64 global_ns() {
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
 }
+__device__ __forceinline__ bool mbar_test(u64* bar, u32 phase) {
+    u32 ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(phase) : "memory");
+    return ok != 0;
+}
 // Wait for phase `phase` of `bar`; false after `limit_ns` (default 1 s).
 __device__ __forceinline__ bool mbar_wait_bounded(u64* bar, u32 phase, u64 limit_ns = 1000000000ULL) {
     if (mbar_try_wait(bar, phase)) return true;
@@ -702,6 +708,20 @@ __device__ __forceinline__ bool mbar_wait_bounded(u64* bar, u32 phase, u64 limit
     while (!mbar_try_wait(bar, phase))
         if (global_ns() - t0 > limit_ns) return false;
     return true;
+}
+// One thread's wait in a pipeline's loop.  no_wait: a limit of zero, the phase
+// is complete or the wait gives up (RoundArgs::no_wait).
+__device__ __forceinline__ bool mbar_wait_step(u64* bar, u32 phase, u32 no_wait) {
+    return no_wait ? mbar_test(bar, phase) : mbar_wait_bounded(bar, phase);
+}
+// The same wait by a whole warp: the lanes poll on their own, so near the limit
+// some could give up where others go on, and on success they may leave the
+// loop one by one.  The vote gives all of them one answer, together: what
+// follows may be an instruction of the whole warp (tcgen05.ld, a full-mask
+// shuffle), and no lane arrives for words that another did not store.
+__device__ __forceinline__ bool mbar_wait_warp(u64* bar, u32 phase, u32 no_wait) {
+    const bool ok = mbar_wait_step(bar, phase, no_wait);
+    return __all_sync(0xffffffffu, ok);
 }
 
 template <u32 M, int NT>
@@ -790,7 +810,7 @@ __global__ void __launch_bounds__(TPB, 2) k_fused_tma(RoundArgs a, u32 ntiles) {
     u32 i = 0;
     for (u32 tile = blockIdx.x; tile < ntiles; tile += G, i++) {
         const int s = i % S;
-        if (!mbar_wait_bounded(&full_bar[s], (i / S) & 1u)) { abort = true; break; }
+        if (!mbar_wait_warp(&full_bar[s], (i / S) & 1u, 0)) { abort = true; break; }
         const u64* st_ = tma_smem + (size_t)s * SW;
         const u64 k = (u64)tile * TQ + threadIdx.x;
 #pragma unroll

@@ -291,6 +291,7 @@ struct effsc_prover {
     u64* d_acc = nullptr;
     u32* counter = nullptr;
     u32* status = nullptr;
+    u32 no_wait = 0;                           // effsc_diag_prover_no_wait
     u64* h_res = nullptr;                      // mapped pinned: wire (9 words) + aux (6 words)
     u64* d_res = nullptr;
     DevTranscript* d_tx = nullptr;
@@ -421,9 +422,11 @@ RoundArgs base_args(effsc_prover* P) {
     a.partials = P->partials;
     a.counter = P->counter;
     a.status = P->status;
+    a.no_wait = P->no_wait;
     a.result = P->d_res;
     return a;
 }
+TcWaits tc_waits(const effsc_prover* P) { return {P->status, P->no_wait}; }
 void set_in(RoundArgs& a, int slot, const Table& T) {
     const Buf& b = T.bufs[T.cur];
     for (int c = 0; c < 3; c++) a.t[slot].in[c] = b.p[c];
@@ -1179,7 +1182,7 @@ int do_ml_phases(effsc_prover* P, size_t a, const TxIO& tx, bool dry) {
         const Tab3 tp = {{p, nullptr, nullptr}}, te = {{Ew, Ew + A, Ew + 2 * A}};
         const Buf& o = T.bufs[bi];
         TRY(timed_launch(s, "ml_fold", 8 * T.len + 8 * fw * C, [&] {
-            if (tc) return launch_eqf_tc(lsb, fw == 3, p, m, te, C, A, part, o.p[0], o.p[1], o.p[2], P->status, s);
+            if (tc) return launch_eqf_tc(lsb, fw == 3, p, m, te, C, A, part, o.p[0], o.p[1], o.p[2], tc_waits(P), s);
             if (lsb) launch_eqf_inner(fw == 3, false, tp, te, m, C, o.p[0], o.p[1], o.p[2], s);
             else launch_eqf_fold_rows(fw == 3, false, tp, te, C, A, splits, part, fw, o.p[0], o.p[1], o.p[2], s);
             return true;
@@ -1332,7 +1335,7 @@ int do_gkr_phases(effsc_prover* P, const TxIO& tx, bool dry, u64* first) {
         };
         if (tc) {
             const Tab3 w1 = {{W, ones, ones}};
-            TRY(timed_launch(s, "gkr_row_sums", 2 * (gate + sums), [&] { return launch_eqf_tc_pair(true, true, add, mult, n, w1, n, n, pa, P->status, s); }));
+            TRY(timed_launch(s, "gkr_row_sums", 2 * (gate + sums), [&] { return launch_eqf_tc_pair(true, true, add, mult, n, w1, n, n, pa, tc_waits(P), s); }));
             TRY(timed_launch(s, "gkr_terms_b", 2 * sums + 40 * n, [&] { return launch_gkr_terms_b(sa, sm, W, F, G, s); }));
         } else {
             TRY(timed_launch(s, "gkr_rows", 2 * gate + 40 * n, [&] { return launch_gkr_rows(add, mult, W, (u32)n, F, G, s); }));
@@ -1341,7 +1344,7 @@ int do_gkr_phases(effsc_prover* P, const TxIO& tx, bool dry, u64* first) {
         if (tc) {
             const Tab3 we = {{Ew, Ew + n, Ew + 2 * n}};
             TRY(timed_launch(s, "gkr_eq_weights", 8 * fw * n, [&] { return launch_build_eq(P->d_chals, k, fw == 3, Ew, Ew + n, Ew + 2 * n, s); }));
-            TRY(timed_launch(s, "gkr_column_sums", 2 * (gate + sums), [&] { return launch_eqf_tc_pair(false, fw == 3, add, mult, n, we, n, n, pa, P->status, s); }));
+            TRY(timed_launch(s, "gkr_column_sums", 2 * (gate + sums), [&] { return launch_eqf_tc_pair(false, fw == 3, add, mult, n, we, n, n, pa, tc_waits(P), s); }));
             TRY(timed_launch(s, "gkr_terms_c", 2 * sums + 8 * n + 32 * fw * n, [&] { return launch_gkr_terms_c(fw, sa, sm, W, last, F, G, s); }));
         } else {
             TRY(timed_launch(s, "gkr_columns", 2 * gate + 32 * fw * n, [&] { return launch_gkr_cols(fw, add, mult, W, last, P->d_chals, k, F, G, s); }));
@@ -1479,7 +1482,7 @@ int do_eqf_left(effsc_prover* P, const TxIO& tx, bool dry) {
         u64* s2 = fw == 3 ? S + 2 * rows : nullptr;
         const uint64_t b1 = p.len * wbytes(p.ext) + m * wbytes(er.ext) + rows * wbytes(out_ext);
         TRY(timed_launch(s, "eqf_inner_sums", b1, [&] {
-            if (tc_in) return launch_eqf_tc(true, fw == 3, pb, m, ter, rows, m, part, S, s1, s2, P->status, s);
+            if (tc_in) return launch_eqf_tc(true, fw == 3, pb, m, ter, rows, m, part, S, s1, s2, tc_waits(P), s);
             launch_eqf_inner(er.ext, p.ext, tp, ter, m, rows, S, s1, s2, s);
             return true;
         }));
@@ -1517,7 +1520,7 @@ int do_eqf_left(effsc_prover* P, const TxIO& tx, bool dry) {
         const Buf& ob = p.bufs[bp];
         const uint64_t b2 = p.len * wbytes(p.ext) + Lc * wbytes(p.ext || out_ext) + 2 * splits * Lc * 24;
         TRY(timed_launch(s, "eqf_fold_left", b2, [&] {
-            if (tc_fold) return launch_eqf_tc(false, fw == 3, pb, Lc, te, Lc, rows2, part, ob.p[0], ob.p[1], ob.p[2], P->status, s);
+            if (tc_fold) return launch_eqf_tc(false, fw == 3, pb, Lc, te, Lc, rows2, part, ob.p[0], ob.p[1], ob.p[2], tc_waits(P), s);
             launch_eqf_fold_rows(fw == 3, p.ext, tp, te, Lc, rows2, splits, part, fw, ob.p[0], ob.p[1], ob.p[2], s);
             return true;
         }));
@@ -2650,6 +2653,14 @@ int effsc_diag_bounded_wait(effsc_ctx* ctx, uint64_t limit_ns, int arrive, uint3
     cudaFreeHost(h);
     if (e != cudaSuccess) return fail(EFFSC_CUDA_ERROR, "bounded-wait self-test: %s", cudaGetErrorString(e));
     *status_out = v;
+    return EFFSC_OK;
+}
+
+int effsc_diag_prover_no_wait(effsc_prover* P, int on) {
+    if (!P) return fail(EFFSC_INVALID_ARG, "prover is NULL");
+    const u32 v = on ? 1 : 0;
+    if (v != P->no_wait && P->gexec) { cudaGraphExecDestroy(P->gexec); P->gexec = nullptr; }
+    P->no_wait = v;
     return EFFSC_OK;
 }
 

@@ -74,6 +74,7 @@ SIGNATURES = {
                                 u64p, u64p, u64p]),
     "effsc_gkr_create": (ci, [vp, ci, ci, u64p, u64p, u64p, sz, ci, ctypes.POINTER(vp)]),
     "effsc_gkr_claimed_w_values": (ci, [vp, u64p]),
+    "effsc_diag_prover_no_wait": (ci, [vp, ci]),
     "effsc_diag_bounded_wait": (ci, [vp, ctypes.c_uint64, ci, ctypes.POINTER(ctypes.c_uint32)]),
     "effsc_prover_set_tail": (ci, [vp, sz]),
     "effsc_prover_set_first_rounds": (ci, [vp, ci]),
