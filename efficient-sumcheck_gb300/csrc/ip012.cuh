@@ -104,7 +104,9 @@ __device__ __forceinline__ void load_octet(u64 (&v)[8], const u64* X, u64 m, u64
         v[1] = e45.x; v[5] = e45.y; v[3] = e67.x; v[7] = e67.y;
     } else {
         // eight slices of the table per octet: read-only loads with a 128-byte
-        // L2 fetch hint (the second pass measured 0.404 -> 0.375 ms at n = 26)
+        // L2 fetch hint (the second pass measured 0.404 -> 0.375 ms at n = 26;
+        // coherent ones 6 % slower).  Nothing may write the table while the
+        // kernel runs: launch_ip3x is never dependent on the pass that copied it.
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             u64 r;

@@ -26,8 +26,9 @@ bool launch_ip012_mirror(bool lsb, const RoundArgs& a, int grid, cudaStream_t s)
 bool launch_ip012(bool lsb, const RoundArgs& a, int grid, cudaStream_t s) {
     return lsb ? launch_chain(k_ip_r012<true>, grid, TPB, 0, s, a) : launch_chain(k_ip_r012<false>, grid, TPB, 0, s, a);
 }
-bool launch_ip3x(bool lsb, const RoundArgs& a, int grid, cudaStream_t s) {
-    return lsb ? launch_chain(k_ip_r3x<true>, grid, TPB, 0, s, a) : launch_chain(k_ip_r3x<false>, grid, TPB, 0, s, a);
+bool launch_ip3x(bool lsb, bool copied, const RoundArgs& a, int grid, cudaStream_t s) {
+    const bool dep = pdl_on(false) && !copied;
+    return lsb ? launch_with(dep, k_ip_r3x<true>, grid, TPB, 0, s, a) : launch_with(dep, k_ip_r3x<false>, grid, TPB, 0, s, a);
 }
 
 }  // namespace effsc

@@ -101,8 +101,11 @@ __device__ __forceinline__ void pg_cp8(u64* dst, const u64* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
 }
 
+// The kernels' `in` may be the output of the pass before, whose end a dependent
+// launch overlaps: not __restrict__, which would promise that nothing writes
+// it while the kernel runs.
 template <bool E>
-__global__ void __launch_bounds__(PG_TPB) k_pg_group(const u64* __restrict__ in, u32 w, u32 g, u32 S,
+__global__ void __launch_bounds__(PG_TPB) k_pg_group(const u64* in, u32 w, u32 g, u32 S,
                                                      const PgMul mul, u64* __restrict__ out) {
     extern __shared__ u64 sm[];
     chain_enter();
@@ -166,7 +169,7 @@ __global__ void __launch_bounds__(PG_TPB) k_pg_group(const u64* __restrict__ in,
 // lanes read neighbouring words.  Per warp: A holds the R input rows, B the
 // R/2 rows of level 1; the levels then alternate.
 template <bool E>
-__global__ void __launch_bounds__(PG_TPB) k_pg_warp(const u64* __restrict__ in, size_t trees, u32 w, u32 gw,
+__global__ void __launch_bounds__(PG_TPB) k_pg_warp(const u64* in, size_t trees, u32 w, u32 gw,
                                                     const PgMul mul, u64* __restrict__ out) {
     extern __shared__ u64 sm[];
     chain_enter();
@@ -220,7 +223,7 @@ __global__ void __launch_bounds__(PG_TPB) k_pg_warp(const u64* __restrict__ in, 
 // One level on global memory: cnt output rows of width w + 1 from 2 cnt
 // input rows of width w.
 template <bool E>
-__global__ void __launch_bounds__(PG_TPB) k_pg_level(const u64* __restrict__ in, size_t cnt, u32 w,
+__global__ void __launch_bounds__(PG_TPB) k_pg_level(const u64* in, size_t cnt, u32 w,
                                                      const PgMul mul, u64* __restrict__ out) {
     chain_enter();
     const u64* pair = mul.q;

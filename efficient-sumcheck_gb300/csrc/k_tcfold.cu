@@ -310,11 +310,11 @@ __global__ void __launch_bounds__(TF_TPB, 1) k_tc_fold_many(const TcSeg* segs, u
 }
 
 template <bool LSB, int NV>
-static bool fold_inst(const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s) {
+static bool fold_inst(bool copied, const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s) {
     constexpr u32 SMEM = TcFold<LSB, NV>::SMEM;
     static std::atomic<uint64_t> configured{0};
     if (!tc_allow_smem(k_tc_fold<LSB, NV>, SMEM, configured)) return false;
-    return launch_chain(k_tc_fold<LSB, NV>, grid, TF_TPB, SMEM, s, a, ntiles);
+    return launch_with(pdl_on(false) && !copied, k_tc_fold<LSB, NV>, grid, TF_TPB, SMEM, s, a, ntiles);
 }
 bool launch_tc_fold_many(const TcSeg* segs, u32 nsegs, const RoundArgs* args, u32 grid, cudaStream_t s) {
     constexpr u32 SMEM = TcFold<false, 4>::SMEM;
@@ -323,9 +323,9 @@ bool launch_tc_fold_many(const TcSeg* segs, u32 nsegs, const RoundArgs* args, u3
     k_tc_fold_many<<<grid, TF_TPB, SMEM, s>>>(segs, nsegs, args);
     return true;
 }
-bool launch_tc_fold(bool lsb, int nv, const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s) {
-    if (nv == 3) return lsb ? fold_inst<true, 3>(a, ntiles, grid, s) : fold_inst<false, 3>(a, ntiles, grid, s);
-    if (nv == 4) return lsb ? fold_inst<true, 4>(a, ntiles, grid, s) : fold_inst<false, 4>(a, ntiles, grid, s);
+bool launch_tc_fold(bool lsb, int nv, bool copied, const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s) {
+    if (nv == 3) return lsb ? fold_inst<true, 3>(copied, a, ntiles, grid, s) : fold_inst<false, 3>(copied, a, ntiles, grid, s);
+    if (nv == 4) return lsb ? fold_inst<true, 4>(copied, a, ntiles, grid, s) : fold_inst<false, 4>(copied, a, ntiles, grid, s);
     return false;
 }
 

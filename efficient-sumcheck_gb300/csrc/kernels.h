@@ -332,25 +332,27 @@ bool launch_ip2x(bool lsb, const RoundArgs& a, int grid, cudaStream_t s);
 // 26 base-field sums of one read of the tables (launch_ip012; partials of 32
 // words per block, grid at most max_grid() * 3 / 8 blocks), then the fold with r0,
 // r1, r2 at once and round 3 from a second read (launch_ip3x; a.chal_ptr
-// holds r0, r1, r2 as 9 consecutive words).
+// holds r0, r1, r2 as 9 consecutive words).  copied: the tables are the copy
+// that the first pass wrote, so the second is launched plainly, never
+// dependent: it loads them as read-only data.
 bool launch_ip012(bool lsb, const RoundArgs& a, int grid, cudaStream_t s);
 // The first pass over tables in host memory that also copies them to the
 // device buffers a.t[0].out[0], a.t[1].out[0] (L words each, 16-byte aligned)
 // for the second pass.
 bool launch_ip012_mirror(bool lsb, const RoundArgs& a, int grid, cudaStream_t s);
-bool launch_ip3x(bool lsb, const RoundArgs& a, int grid, cudaStream_t s);
+bool launch_ip3x(bool lsb, bool copied, const RoundArgs& a, int grid, cudaStream_t s);
 // InnerProduct rounds 0 .. nv (nv = 3 or 4) in two passes on the tensor cores,
 // tables 16-byte aligned.  First pass (k_gram.cu): rounds 0 .. nv - 1 from
 // tiles a.tile0 .. a.tile0 + ntiles - 1 of TC_TILE_ITEMS groups of 2^nv
 // entries, at most gram_max_tiles() per block (with `mirror` the words are
 // also copied to the device buffers a.t[i].out[0]); partials of 4^nv words per
 // block, a.acc of as many.  Second pass (k_tcfold.cu): the fold with r_0 ..
-// r_{nv-1} (a.chal_ptr: 3 nv words) and round nv, over all
+// r_{nv-1} (a.chal_ptr: 3 nv words; copied as for launch_ip3x) and round nv, over all
 // (L >> nv) / TC_TILE_ITEMS tiles.
 constexpr u32 TC_TILE_ITEMS = 128;
 bool launch_ip_gram(bool lsb, int nv, bool mirror, const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s);
 u32 gram_max_tiles(void);
-bool launch_tc_fold(bool lsb, int nv, const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s);
+bool launch_tc_fold(bool lsb, int nv, bool copied, const RoundArgs& a, u32 ntiles, int grid, cudaStream_t s);
 // The same passes (MSB, nv = 4) of many proofs in one launch each: segment k
 // has nblocks blocks for the ntiles = (L >> 4) / TC_TILE_ITEMS tiles of
 // args[k] (at most gram_max_tiles() per block).

@@ -1036,9 +1036,9 @@ int do_fuse3(effsc_prover* P, size_t num_rounds, const TxIO& tx0, const u64* cha
     }
     // the general form: one wave (two blocks per SM, the kernel's residency)
     if (!dry) TRY(timed_launch(P->ctx->stream, "ip_fold_and_round", 16 * (uint64_t)L + 48 * (uint64_t)N, [&] {
-        if (!tc) return launch_ip3x(lsb, b, std::min<int>(grid_for(L / 16), two_per_sm), P->ctx->stream);
+        if (!tc) return launch_ip3x(lsb, mirror, b, std::min<int>(grid_for(L / 16), two_per_sm), P->ctx->stream);
         const size_t tiles = N / TC_TILE_ITEMS;
-        return launch_tc_fold(lsb, nv, b, (u32)tiles, (int)std::min<size_t>(tiles, sms), P->ctx->stream);
+        return launch_tc_fold(lsb, nv, mirror, b, (u32)tiles, (int)std::min<size_t>(tiles, sms), P->ctx->stream);
     }));
     for (int i = 0; i < 2; i++) {
         Table& T = P->t[i];
