@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(CG_TPB, 1) k_c3_gram(RoundArgs a, u32 ntiles) 
             for (int q = 0; q < 9; q++) f[q] = gl_mul(f[q], g[q]);
             if (i + CG_FGG < mine) c3_load_fg<LSB>(t, a, tile_k0(i + CG_FGG) + quad, Q);
             const u32 s = i % CG_S;
-            if (!mbar_wait_warp(&sh.empty[s], ((i / CG_S) & 1u) ^ 1u, a.no_wait)) { abort = true; break; }
+            abort |= !mbar_wait_step(&sh.empty[s], ((i / CG_S) & 1u) ^ 1u, a.no_wait | abort);
             char* rows = stages + s * CG_BYTES + CG_ATOM;
 #pragma unroll
             for (int q = 0; q < 9; q++)
@@ -193,13 +193,13 @@ __global__ void __launch_bounds__(CG_TPB, 1) k_c3_gram(RoundArgs a, u32 ntiles) 
 #pragma unroll
                 for (int u = 0; u < U::UPW; u++)
                     v[q][u] = __ldcs((const ulonglong2*)U::at(a, w * U::UPW + u, lane, tile_k0(q), Q));
-        for (u32 i0 = 0; i0 < mine && !abort; i0 += CG_AHEAD) {
+        for (u32 i0 = 0; i0 < mine; i0 += CG_AHEAD) {
 #pragma unroll
             for (int q = 0; q < CG_AHEAD; q++) {
                 const u32 i = i0 + q;
-                if (i >= mine || abort) break;
+                if (i >= mine) break;
                 const u32 s = i % CG_S;
-                if (!mbar_wait_warp(&sh.empty[s], ((i / CG_S) & 1u) ^ 1u, a.no_wait)) { abort = true; break; }
+                abort |= !mbar_wait_step(&sh.empty[s], ((i / CG_S) & 1u) ^ 1u, a.no_wait | abort);
 #pragma unroll
                 for (int u = 0; u < U::UPW; u++) U::store(stages + s * CG_BYTES, w * U::UPW + u, lane, v[q][u]);
                 if (i + CG_AHEAD < mine)
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(CG_TPB, 1) k_c3_gram(RoundArgs a, u32 ntiles) 
     } else if (lane == 0) {
         for (u32 i = 0; i < mine; i++) {
             const u32 s = i % CG_S;
-            if (!mbar_wait_step(&sh.full[s], (i / CG_S) & 1u, a.no_wait)) { abort = true; break; }
+            if (!mbar_wait_bounded(&sh.full[s], (i / CG_S) & 1u)) { abort = true; break; }
             tc_fence_after();
             const u32 xb = smem_u32(stages) + s * CG_BYTES, yb = xb + CG_ATOM;
 #pragma unroll

@@ -82,13 +82,13 @@ __global__ void __launch_bounds__(ET_TPB, 1) k_eqf_tc(const u64* p, const u64* p
             if ((u32)q < tiles)
 #pragma unroll
                 for (int u = 0; u < 2; u++) v[q][u] = __ldcs(at(q, u));
-        for (u32 i0 = 0; i0 < tiles && !abort; i0 += ET_AHEAD) {
+        for (u32 i0 = 0; i0 < tiles; i0 += ET_AHEAD) {
 #pragma unroll
             for (int q = 0; q < ET_AHEAD; q++) {
                 const u32 i = i0 + q;
-                if (i >= tiles || abort) break;
+                if (i >= tiles) break;
                 const u32 s = i % ET_S;
-                if (!mbar_wait_warp(&empty[s], ((i / ET_S) & 1u) ^ 1u, tw.no_wait)) { abort = true; break; }
+                abort |= !mbar_wait_step(&empty[s], ((i / ET_S) & 1u) ^ 1u, tw.no_wait | abort);
                 char* st = stages + s * ET_BYTES;
 #pragma unroll
                 for (int u = 0; u < 2; u++) {
@@ -120,13 +120,13 @@ __global__ void __launch_bounds__(ET_TPB, 1) k_eqf_tc(const u64* p, const u64* p
             if ((u32)q < tiles)
 #pragma unroll
                 for (int c = 0; c < NC; c++) x[q][c] = w.c[c][k0 + (u64)q * ET_K + lane];
-        for (u32 i0 = 0; i0 < tiles && !abort; i0 += 2) {
+        for (u32 i0 = 0; i0 < tiles; i0 += 2) {
 #pragma unroll
             for (int q = 0; q < 2; q++) {
                 const u32 i = i0 + q;
-                if (i >= tiles || abort) break;
+                if (i >= tiles) break;
                 const u32 s = i % ET_S;
-                if (!mbar_wait_warp(&empty[s], ((i / ET_S) & 1u) ^ 1u, tw.no_wait)) { abort = true; break; }
+                abort |= !mbar_wait_step(&empty[s], ((i / ET_S) & 1u) ^ 1u, tw.no_wait | abort);
                 char* st = stages + s * ET_BYTES + 8 * ET_ATOM;
 #pragma unroll
                 for (int c = 0; c < NC; c++) *(uint4*)(st + swz128(et_row(lane), c)) = digits_of(x[q][c]);
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(ET_TPB, 1) k_eqf_tc(const u64* p, const u64* p
     } else if (lane == 0) {
         for (u32 i = 0; i < tiles; i++) {
             const u32 s = i % ET_S;
-            if (!mbar_wait_step(&full[s], (i / ET_S) & 1u, tw.no_wait)) { abort = true; break; }
+            if (!mbar_wait_bounded(&full[s], (i / ET_S) & 1u)) { abort = true; break; }
             tc_fence_after();
             const u32 base = smem_u32(stages) + s * ET_BYTES;
             const u64 b = tc_desc(base + 8 * ET_ATOM, ET_ATOM, 1024);

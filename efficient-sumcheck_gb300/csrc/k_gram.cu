@@ -205,13 +205,13 @@ __device__ __forceinline__ void gram_body(const RoundArgs& a, u32 ntiles, u32 bi
             if ((u32)q < mine)
 #pragma unroll
                 for (int u = 0; u < UPW; u++) v[q][u] = __ldcs((const ulonglong2*)(X + word(q, u)));
-        for (u32 i0 = 0; i0 < mine && !abort; i0 += AHEAD) {
+        for (u32 i0 = 0; i0 < mine; i0 += AHEAD) {
 #pragma unroll
             for (int q = 0; q < AHEAD; q++) {
                 const u32 i = i0 + q;
-                if (i >= mine || abort) break;
+                if (i >= mine) break;
                 const u32 s = i % S, ph = (i / S) & 1u;
-                if (!mbar_wait_warp(&sh.empty[s], ph ^ 1u, a.no_wait)) { abort = true; break; }
+                abort |= !mbar_wait_step(&sh.empty[s], ph ^ 1u, a.no_wait | abort);
 #pragma unroll
                 for (int u = 0; u < UPW; u++) Tile::store(stages + s * Tile::BYTES, warp * UPW + u, lane, v[q][u]);
                 if (MIRROR)
@@ -231,7 +231,7 @@ __device__ __forceinline__ void gram_body(const RoundArgs& a, u32 ntiles, u32 bi
     } else if (lane == 0) {
         for (u32 i = 0; i < mine; i++) {
             const u32 s = i % S, ph = (i / S) & 1u;
-            if (!mbar_wait_step(&sh.full[s], ph, a.no_wait)) { abort = true; break; }
+            if (!mbar_wait_bounded(&sh.full[s], ph)) { abort = true; break; }
             tc_fence_after();
             const u32 xb = smem_u32(stages) + s * Tile::BYTES, yb = xb + Tile::ATOMS * Tile::ATOM;
 #pragma unroll

@@ -165,13 +165,13 @@ __device__ __forceinline__ void tc_fold_body(const RoundArgs& a, u32 ntiles, u32
             if ((u32)q < mine)
 #pragma unroll
                 for (int u = 0; u < UPW; u++) v[q][u] = __ldcs((const ulonglong2*)(X + word(q, u)));
-        for (u32 i0 = 0; i0 < mine && !abort; i0 += AHEAD) {
+        for (u32 i0 = 0; i0 < mine; i0 += AHEAD) {
 #pragma unroll
             for (int q = 0; q < AHEAD; q++) {
                 const u32 i = i0 + q;
-                if (i >= mine || abort) break;
+                if (i >= mine) break;
                 const u32 s = i % S, ph = (i / S) & 1u;
-                if (!mbar_wait_warp(&sh.empty[s], ph ^ 1u, a.no_wait)) { abort = true; break; }
+                abort |= !mbar_wait_step(&sh.empty[s], ph ^ 1u, a.no_wait | abort);
 #pragma unroll
                 for (int u = 0; u < UPW; u++) Tile::store(stages + s * Tile::BYTES, warp * UPW + u, lane, v[q][u]);
                 if (i + AHEAD < mine)
@@ -187,8 +187,8 @@ __device__ __forceinline__ void tc_fold_body(const RoundArgs& a, u32 ntiles, u32
             const u32 wb = smem_u32(wmat);
             for (u32 i = 0; i < mine; i++) {
                 const u32 s = i % S, b = i % TF_BUFS;
-                if (!mbar_wait_step(&sh.full[s], (i / S) & 1u, a.no_wait) ||
-                    !mbar_wait_step(&sh.tempty[b], ((i / TF_BUFS) & 1u) ^ 1u, a.no_wait)) { abort = true; break; }
+                if (!mbar_wait_bounded(&sh.full[s], (i / S) & 1u) ||
+                    !mbar_wait_bounded(&sh.tempty[b], ((i / TF_BUFS) & 1u) ^ 1u)) { abort = true; break; }
                 tc_fence_after();
                 const u32 base = smem_u32(stages) + s * Tile::BYTES;
 #pragma unroll
@@ -213,7 +213,8 @@ __device__ __forceinline__ void tc_fold_body(const RoundArgs& a, u32 ntiles, u32
         const bool high = lane >= 16;
         for (u32 i = group; i < mine; i += TF_EG) {
             const u32 b = i % TF_BUFS;
-            if (!mbar_wait_warp(&sh.tfull[b], (i / TF_BUFS) & 1u, a.no_wait)) { abort = true; break; }
+            abort |= !mbar_wait_step(&sh.tfull[b], (i / TF_BUFS) & 1u, a.no_wait | abort);
+            __syncwarp();          // the loads are instructions of the whole warp
             tc_fence_after();
             const u64 m = Tile::entry(quad, lane, (bid + (u64)i * G) * (LSB ? 128 : 64), H);
             F3 x[2];

@@ -709,18 +709,26 @@ __device__ __forceinline__ bool mbar_wait_bounded(u64* bar, u32 phase, u64 limit
         if (global_ns() - t0 > limit_ns) return false;
     return true;
 }
-// One thread's wait in a pipeline's loop.  no_wait: a limit of zero, the phase
-// is complete or the wait gives up (RoundArgs::no_wait).
+// A pipeline's waits by all lanes of a warp.  The lanes poll on their own, so
+// near the limit some could give up where others go on, and on success they
+// may leave the poll one by one; what follows may need all of them (a
+// full-mask barrier or shuffle, tcgen05.ld).  Two ways to keep them together:
+//  - in the tensor-core passes a lane that gave up stays in the loop: it
+//    notes it and goes through the remaining steps without waiting
+//    (mbar_wait_step with no_wait = 1).  What it stores and reads is within
+//    its stage and thrown away: the block's vote after the loop sees the note.
+//    A vote or a break on the wait itself changes nothing when all is well;
+//    this costs nothing either (GKR's two reads 71 + 72 us with all three).
+//  - in the TMA-staged round kernel a vote (mbar_wait_warp): no lane may reach
+//    the refill of a stage that another has left.
+// no_wait: a limit of zero, the phase is complete or the wait gives up
+// (RoundArgs::no_wait sets it from the first step; the thread that issues the
+// MMAs has no such test, which would cost 2 us a read there).
 __device__ __forceinline__ bool mbar_wait_step(u64* bar, u32 phase, u32 no_wait) {
     return no_wait ? mbar_test(bar, phase) : mbar_wait_bounded(bar, phase);
 }
-// The same wait by a whole warp: the lanes poll on their own, so near the limit
-// some could give up where others go on, and on success they may leave the
-// loop one by one.  The vote gives all of them one answer, together: what
-// follows may be an instruction of the whole warp (tcgen05.ld, a full-mask
-// shuffle), and no lane arrives for words that another did not store.
-__device__ __forceinline__ bool mbar_wait_warp(u64* bar, u32 phase, u32 no_wait) {
-    const bool ok = mbar_wait_step(bar, phase, no_wait);
+__device__ __forceinline__ bool mbar_wait_warp(u64* bar, u32 phase) {
+    const bool ok = mbar_wait_bounded(bar, phase);
     return __all_sync(0xffffffffu, ok);
 }
 
@@ -810,7 +818,7 @@ __global__ void __launch_bounds__(TPB, 2) k_fused_tma(RoundArgs a, u32 ntiles) {
     u32 i = 0;
     for (u32 tile = blockIdx.x; tile < ntiles; tile += G, i++) {
         const int s = i % S;
-        if (!mbar_wait_warp(&full_bar[s], (i / S) & 1u, 0)) { abort = true; break; }
+        if (!mbar_wait_warp(&full_bar[s], (i / S) & 1u)) { abort = true; break; }
         const u64* st_ = tma_smem + (size_t)s * SW;
         const u64 k = (u64)tile * TQ + threadIdx.x;
 #pragma unroll

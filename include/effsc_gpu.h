@@ -350,8 +350,8 @@ int effsc_diag_transcript_latency(effsc_ctx* ctx, double* ns_per_permutation, do
 int effsc_diag_bounded_wait(effsc_ctx* ctx, uint64_t limit_ns, int arrive, uint32_t* status);
 /* The same for the pipelines of the tensor-core passes (no reference
  * counterpart): on = 1 gives the prover's passes a limit of zero for the
- * waits between their warps, so that they give up where a stage is not there
- * yet and effsc_prove returns EFFSC_TIMEOUT; on = 0 (as created) the limit of
+ * waits of their loading and epilogue warps, so that they give up where a
+ * stage is not ready yet and effsc_prove returns EFFSC_TIMEOUT; on = 0 (as created) the limit of
  * 1 s.  After a timeout the prover is reset with effsc_prover_reset and proves
  * again. */
 int effsc_diag_prover_no_wait(effsc_prover* p, int on);

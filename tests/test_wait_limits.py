@@ -1,11 +1,12 @@
 """The tensor-core passes' waits run out, without a fault.
 
 Their pipelines (k_ip_gram, k_tc_fold, k_c3_gram, k_eqf_tc) wait between their
-warps with a limit.  Here the limit is zero, so that the issuing thread gives up
-where the first stage is not loaded yet and the other warps follow: the pass
-has to end by itself (its tensor memory given back, every warp out of its loop
-together), the call has to say EFFSC_TIMEOUT, and the same prover's next
-proof, with the usual limit, has to be the oracle's, word for word."""
+warps with a limit.  Here the limit is zero for the loading and the epilogue
+warps, so that they give up where a stage is not free, or its sums are not there,
+yet (the sizes give every block more tiles than stages): the pass has to end by
+itself, its tensor memory given back and its warps together, the call has to
+say EFFSC_TIMEOUT, and the same prover's next proof, with the usual limit, has
+to be the oracle's, word for word."""
 import os
 
 import numpy as np
@@ -32,17 +33,17 @@ def cases(E, what):
     def words(*shape):
         return g.integers(0, O.P, size=shape, dtype=np.uint64)
     if what.startswith("ip"):
-        lsb, rounds = "lsb" in what, 4 if "four" in what else 18
-        tabs = [words(1 << 18) for _ in range(2)]
+        lsb, rounds = "lsb" in what, 4 if "four" in what else 21
+        tabs = [words(1 << 21) for _ in range(2)]
         return (E.InnerProductProverLSB if lsb else E.InnerProductProver)(*tabs), rounds, O.Prover(O.IP, O.LSB if lsb else O.MSB, 3, tabs)
     if what.startswith("ml"):
-        lsb, n = "lsb" in what, 21           # LSB: the sums along rows start there
+        lsb, n = "lsb" in what, 21
         t = words(1 << n)
         return (E.MultilinearProverLSB if lsb else E.MultilinearProver)(t), n, O.Prover(O.ML, O.LSB if lsb else O.MSB, 3, [t])
     if what.startswith("coef"):
         lsb = "lsb" in what
-        tabs = [words(1 << 16, 3), words(1 << 16), words(1 << 16)]
-        return (E.CoefficientProverLSB if lsb else E.CoefficientProver)(tabs), 16, O.Prover(O.COEF, O.LSB if lsb else O.MSB, 3, tabs)
+        tabs = [words(1 << 20, 3), words(1 << 20), words(1 << 20)]
+        return (E.CoefficientProverLSB if lsb else E.CoefficientProver)(tabs), 20, O.Prover(O.COEF, O.LSB if lsb else O.MSB, 3, tabs)
     if what == "eqf":
         w, p = words(21, 3), words(1 << 21)
         return E.EqFactoredProver(w, p), 21, O.Prover.eq_factored(3, w, p)
