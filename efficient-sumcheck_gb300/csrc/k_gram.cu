@@ -34,14 +34,15 @@
 // L2 two tiles before its register loads (four ahead 216, eight 241) and
 // streaming loads, 206 with two stages instead of three (more L1 for the loads).
 #include "ip012.cuh"
+#include "residency.h"
 #include "tc.cuh"
 
 namespace effsc {
 
 constexpr int GR_LW = 16;                     // loading warps
 constexpr int GR_TPB = 32 * (GR_LW + 1);
+constexpr u64 GR_LIMIT_NS = tc_wait_ns(false), GR_HOST_LIMIT_NS = tc_wait_ns(true);
 constexpr u32 GR_MAX_TILES = 65536 / 128;     // tiles per accumulator: 2^16 groups (2^16 * 225 < 2^24)
-constexpr u64 GR_LIMIT_NS = 1000000000ULL;
 
 template <bool LSB, int NV>
 struct Gram {
@@ -170,6 +171,7 @@ __device__ __forceinline__ void gram_body(const RoundArgs& a, u32 ntiles, u32 bi
     using GT = Gram<LSB, NV>;
     using Tile = TcTile<LSB, NV>;
     constexpr int S = GT::S, UPW = GT::UPW, AHEAD = GT::AHEAD, V = GT::V;
+    constexpr u64 LIMIT = MIRROR ? GR_HOST_LIMIT_NS : GR_LIMIT_NS;
     extern __shared__ char gram_dyn[];
     __shared__ typename GT::Shared sh;
     char* stages = gram_dyn + ((1024 - (smem_u32(gram_dyn) & 1023)) & 1023);
@@ -211,7 +213,7 @@ __device__ __forceinline__ void gram_body(const RoundArgs& a, u32 ntiles, u32 bi
                 const u32 i = i0 + q;
                 if (i >= mine) break;
                 const u32 s = i % S, ph = (i / S) & 1u;
-                abort |= !mbar_wait_step(&sh.empty[s], ph ^ 1u, a.no_wait | abort);
+                abort |= !mbar_wait_step(&sh.empty[s], ph ^ 1u, a.no_wait | abort, LIMIT);
 #pragma unroll
                 for (int u = 0; u < UPW; u++) Tile::store(stages + s * Tile::BYTES, warp * UPW + u, lane, v[q][u]);
                 if (MIRROR)
@@ -231,7 +233,7 @@ __device__ __forceinline__ void gram_body(const RoundArgs& a, u32 ntiles, u32 bi
     } else if (lane == 0) {
         for (u32 i = 0; i < mine; i++) {
             const u32 s = i % S, ph = (i / S) & 1u;
-            if (!mbar_wait_bounded(&sh.full[s], ph)) { abort = true; break; }
+            if (!mbar_wait_bounded(&sh.full[s], ph, LIMIT)) { abort = true; break; }
             tc_fence_after();
             const u32 xb = smem_u32(stages) + s * Tile::BYTES, yb = xb + Tile::ATOMS * Tile::ATOM;
 #pragma unroll
@@ -247,7 +249,7 @@ __device__ __forceinline__ void gram_body(const RoundArgs& a, u32 ntiles, u32 bi
     // the accumulators are final once `done` completes (the MMA thread's
     // commit covers everything it issued, an abort included)
     if (warp < GR_LW || lane == 0) {
-        if (!mbar_wait_bounded(&sh.done, 0, 4 * GR_LIMIT_NS)) abort = true;
+        if (!mbar_wait_bounded(&sh.done, 0, 4 * LIMIT)) abort = true;
     }
     __syncwarp();
     tc_fence_after();

@@ -1,0 +1,53 @@
+// residency.h -- where a caller's table is, and how passes may read it there.
+// Plain C++, so that the rules are compiled and tested without a GPU.
+#pragma once
+#include <cstddef>
+#include <cstdint>
+#include <sys/mman.h>
+#include <unistd.h>
+
+namespace effsc {
+
+enum class Residency {
+    device,     // device memory
+    managed,    // managed memory: its pages may be on their way
+    pinned,     // pinned or registered host memory
+    pageable    // host memory as malloc or mmap gives it, a mapped file included
+};
+
+// Reads that arrive within the link's latency.  A pageable (or managed) page may
+// first have to be brought in, from a file at worst.
+constexpr bool prompt_reads(Residency r) { return r == Residency::device || r == Residency::pinned; }
+
+// The limit of a tensor-core pass's waits on its own loads.  The pass that copies
+// host tables (from_host) may meet pages that are not there yet.  Its blocks
+// have at most some 400 tiles in flight, 1 KB in each of 32 places of two MSB
+// tables (LSB: 16 KB in each table): 3200 pages of 4 KB, so 100 s are 30 ms for
+// each of them one after the other, a disk's slowest.
+constexpr uint64_t tc_wait_ns(bool from_host) { return from_host ? 100000000000ULL : 1000000000ULL; }
+
+// Rounds that the first pass of the InnerProduct start runs on the tensor
+// cores (k_gram.cu): 4 where the proof has five, else 3; 0: the general form
+// of direct loads without waits (k_ip012.cu, 3 rounds).  `addresses`: the
+// tables' and their copies', or-ed (16-byte loads and stores).  Tables that are
+// not prompt are read once, by the first pass, when it also copies them
+// (`copied`, with the limit above); where they are read in place by both, the
+// direct loads do it.
+constexpr int ip_start_rounds(size_t L, size_t num_rounds, uintptr_t addresses, bool prompt, bool copied, size_t tile_items) {
+    const int nv = num_rounds >= 5 ? 4 : 3;
+    const size_t items = L >> nv;
+    return (!prompt && !copied) || (addresses & 15) || items % tile_items || items / tile_items >= ((size_t)1 << 31) ? 0 : nv;
+}
+
+// Bring the pages of pageable memory in before a kernel reads them: on the host
+// a missing page is a microsecond, from the GPU ten.  False where the system
+// cannot (the kernel then brings them in).
+inline bool populate_pages(const void* p, size_t bytes) {
+    if (!bytes) return true;
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t lo = (uintptr_t)p & ~(page - 1), hi = ((uintptr_t)p + bytes + page - 1) & ~(page - 1);
+    constexpr int populate_read = 22;      // MADV_POPULATE_READ (Linux 5.14)
+    return madvise((void*)lo, hi - lo, populate_read) == 0;
+}
+
+}  // namespace effsc

@@ -724,8 +724,8 @@ __device__ __forceinline__ bool mbar_wait_bounded(u64* bar, u32 phase, u64 limit
 // no_wait: a limit of zero, the phase is complete or the wait gives up
 // (RoundArgs::no_wait sets it from the first step; the thread that issues the
 // MMAs has no such test, which would cost 2 us a read there).
-__device__ __forceinline__ bool mbar_wait_step(u64* bar, u32 phase, u32 no_wait) {
-    return no_wait ? mbar_test(bar, phase) : mbar_wait_bounded(bar, phase);
+__device__ __forceinline__ bool mbar_wait_step(u64* bar, u32 phase, u32 no_wait, u64 limit_ns = 1000000000ULL) {
+    return no_wait ? mbar_test(bar, phase) : mbar_wait_bounded(bar, phase, limit_ns);
 }
 __device__ __forceinline__ bool mbar_wait_warp(u64* bar, u32 phase) {
     const bool ok = mbar_wait_bounded(bar, phase);

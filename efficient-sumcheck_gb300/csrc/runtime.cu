@@ -8,6 +8,7 @@
 #include "effsc_gpu.h"
 #include "kernels.h"
 #include "keccak.cuh"
+#include "residency.h"
 
 #include <algorithm>
 #include <cstdarg>
@@ -252,6 +253,8 @@ struct Buf {
     bool ext = false;
     bool owned = true;
     bool host = false;      // the caller's host memory, read in place (never bulk-copied)
+    bool prompt = true;     // prompt_reads (residency.h)
+    bool populated = false; // populate_pages was called for it
 };
 struct Table {
     std::vector<Buf> bufs;  // bufs[0]: the input table, never written by a round
@@ -829,10 +832,13 @@ int do_coef3_first(effsc_prover* P, const TxIO& tx0, const TxIO& tx2, const u64*
     // of as many tiles as the blocks' accumulators hold; else on the integer
     // pipes (partials of 48 words per block: max_grid() / 4 blocks at most)
     uintptr_t bits = 0;
-    for (int i = 0; i < 3; i++)
+    bool prompt = true;
+    for (int i = 0; i < 3; i++) {
         for (int c = 0; c < (P->t[i].ext ? 3 : 1); c++) bits |= (uintptr_t)a.t[i].in[c];
+        prompt &= P->t[i].bufs[0].prompt;
+    }
     const size_t tiles = L / 4 / TC_TILE_ITEMS, sms = max_grid() / 8, most = sms * gram_max_tiles();
-    if ((bits & 15) == 0 && L / 4 % TC_TILE_ITEMS == 0 && tiles < (1u << 31)) {
+    if (prompt && (bits & 15) == 0 && L / 4 % TC_TILE_ITEMS == 0 && tiles < (1u << 31)) {
         if (!P->d_acc) CK(cudaMallocAsync((void**)&P->d_acc, 256 * sizeof(u64), P->ctx->stream));
         a.acc = P->d_acc;
         for (size_t at = 0; at < tiles && !dry; at += most) {
@@ -917,16 +923,17 @@ bool mirror_ok(effsc_prover* P, size_t L) {
 }
 
 // The tensor-core start takes every two-pass start whose tables it can load
-// 16 bytes at a time: rounds 0-4 when the proof has them (one pass over the
+// 16 bytes at a time and whose words come in time (residency.h): rounds 0-4 when the proof has them (one pass over the
 // tables fewer bytes of folded tables: 2 x 24 L/16 instead of 2 x 24 L/8),
 // else rounds 0-3.  0: the general form (k_ip012.cu, rounds 0-3).
-int tc_rounds(size_t L, size_t num_rounds, const RoundArgs& a) {
+int tc_rounds(const effsc_prover* P, size_t L, size_t num_rounds, bool copied, const RoundArgs& a) {
     uintptr_t bits = 0;
-    for (int i = 0; i < 2; i++) bits |= (uintptr_t)a.t[i].in[0] | (uintptr_t)a.t[i].out[0];
-    const int nv = num_rounds >= 5 ? 4 : 3;
-    const size_t items = L >> nv;
-    if ((bits & 15) || items % TC_TILE_ITEMS || items / TC_TILE_ITEMS >= (1u << 31)) return 0;
-    return nv;
+    bool prompt = true;
+    for (int i = 0; i < 2; i++) {
+        bits |= (uintptr_t)a.t[i].in[0] | (uintptr_t)a.t[i].out[0];
+        prompt &= P->t[i].bufs[P->t[i].cur].prompt;
+    }
+    return ip_start_rounds(L, num_rounds, bits, prompt, copied, TC_TILE_ITEMS);
 }
 // The first pass over tiles lo .. lo + n - 1: one launch while a block's
 // accumulators hold its tiles, else several, the sums carried from one to the
@@ -1006,7 +1013,15 @@ int do_fuse3(effsc_prover* P, size_t num_rounds, const TxIO& tx0, const u64* cha
             a.t[i].out[0] = P->t[i].bufs[mi[i]].p[0];
         }
     const bool mirror = mi[0] >= 0;
-    const int tc = tc_rounds(L, num_rounds, a), nv = tc ? tc : 3;
+    const int tc = tc_rounds(P, L, num_rounds, mirror, a), nv = tc ? tc : 3;
+    // bring in pages that are not there yet, once for the prover (a first proof
+    // of 2^24 entries, MSB and LSB: of a newly mapped file 2.0 and 21 ms
+    // without, 1.9 and 1.9 with; of untouched memory 136 and 131, 2.1 and 2.1)
+    for (int i = 0; i < 2 && mirror; i++) {
+        Buf& h = P->t[i].bufs[0];
+        if (!h.prompt && !h.populated) populate_pages(h.p[0], L * sizeof(u64));
+        h.populated = true;
+    }
     const char* name = mirror ? "ip_first_rounds_from_host" : "ip_first_rounds";
     if (tc) {
         if (!P->d_acc) CK(cudaMallocAsync((void**)&P->d_acc, 256 * sizeof(u64), P->ctx->stream));
@@ -1145,7 +1160,7 @@ int do_ml_phases(effsc_prover* P, size_t a, const TxIO& tx, bool dry) {
     const u64 m = lsb ? A : C, rows = lsb ? C : A;  // the table as rows of m entries
     cudaStream_t s = P->ctx->stream;
     const u64* p = T.bufs[0].p[0];
-    const bool tc = eqf_tc_ok(lsb, C, A, m, p);
+    const bool tc = T.bufs[0].prompt && eqf_tc_ok(lsb, C, A, m, p);
     const u64 splits = std::min<u64>(rows, 64);
     const size_t need = A + 3 * A + std::max<size_t>(3 * m * splits, tc ? 3 * C * eqf_tc_splits(C, A) : 0);
     if (P->eqf_cap < need) {
@@ -2084,6 +2099,14 @@ void effsc_internal_tx_state(const effsc_transcript* t, void* out) {
     if (t->kind != EFFSC_T_KECCAK) st.deg = 0;   // marks a transcript the device cannot run
     memcpy(out, &st, sizeof st);
 }
+namespace {
+Residency residency(const uint64_t* ptr) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, ptr) != cudaSuccess) { cudaGetLastError(); return Residency::pageable; }
+    return at.type == cudaMemoryTypeDevice ? Residency::device : at.type == cudaMemoryTypeManaged ? Residency::managed
+         : at.type == cudaMemoryTypeHost ? Residency::pinned : Residency::pageable;
+}
+}  // namespace
 const u64* effsc_internal_device_view(int device, const uint64_t* ptr, bool* is_host) {
     cudaPointerAttributes at;
     *is_host = false;
@@ -2391,6 +2414,7 @@ static int create_in_place(effsc_ctx* ctx, int kind, int order, int field, int n
         b.cap = lens[i];
         b.ext = ncomp[i] == 3;
         b.p[0] = (u64*)dev_tables[i];
+        b.prompt = prompt_reads(residency(dev_tables[i]));
         if (host) {
             bool is_host = false;
             const u64* v = device_view(ctx->device, dev_tables[i], &is_host);
