@@ -39,6 +39,13 @@ constexpr int ip_start_rounds(size_t L, size_t num_rounds, uintptr_t addresses, 
     return (!prompt && !copied) || (addresses & 15) || items % tile_items || items / tile_items >= ((size_t)1 << 31) ? 0 : nv;
 }
 
+// Copying host words by a kernel that reads them in place: pageable memory that
+// the GPU reads through the host's own page tables (elsewhere each page
+// faults or moves to the GPU), from 64 KB on (below, latency either way).
+constexpr bool kernel_copies(Residency r, bool host_page_tables, size_t words, uintptr_t address) {
+    return r == Residency::pageable && host_page_tables && words >= ((size_t)1 << 13) && (address & 7) == 0;
+}
+
 // Bring the pages of pageable memory in before a kernel reads them: on the host
 // a missing page is a microsecond, from the GPU ten.  False where the system
 // cannot (the kernel then brings them in).
@@ -49,5 +56,21 @@ inline bool populate_pages(const void* p, size_t bytes) {
     constexpr int populate_read = 22;      // MADV_POPULATE_READ (Linux 5.14)
     return madvise((void*)lo, hi - lo, populate_read) == 0;
 }
+
+// The caller's memory while kernels read it: once `pending`, the scope is not
+// left without having waited for them, on the errors' ways out as well.
+template <class Wait>
+struct ReadsInPlace {
+    Wait wait;               // returns an error code, 0 for none
+    bool pending = false;
+    explicit ReadsInPlace(Wait w) : wait(w) {}
+    ReadsInPlace(const ReadsInPlace&) = delete;
+    int finish() {
+        const bool p = pending;
+        pending = false;
+        return p ? (int)wait() : 0;
+    }
+    ~ReadsInPlace() { finish(); }
+};
 
 }  // namespace effsc

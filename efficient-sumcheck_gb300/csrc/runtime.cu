@@ -204,8 +204,6 @@ HF tx_h_challenge(effsc_transcript* t) {
 }
 }  // namespace
 
-cudaError_t effsc_internal_upload(int device, u64* dst, const uint64_t* host, size_t words, cudaStream_t s, bool* in_place);
-
 // ===========================================================================
 // context
 // ===========================================================================
@@ -1945,15 +1943,9 @@ int prover_common_init(effsc_prover* P) {
 int upload_table(effsc_prover* P, Table& T, const uint64_t* host, size_t len, int ncomp, int repr) {
     cudaStream_t s = P->ctx->stream;
     Buf b;
-    auto upload = [&](u64* dst) -> int {
-        bool in_place = false;
-        CK(effsc_internal_upload(P->ctx->device, dst, host, len * ncomp, s, &in_place));
-        if (in_place) CK(cudaStreamSynchronize(s));
-        return EFFSC_OK;
-    };
     if (ncomp == 1) {
         TRY(alloc_buf(P, b, len, false));
-        if (len) TRY(upload(b.p[0]));
+        if (len) CK(cudaMemcpyAsync(b.p[0], host, len * sizeof(u64), cudaMemcpyHostToDevice, s));
         if (repr == EFFSC_MONTGOMERY && len) {
             launch_split_aos(b.p[0], len, 1, b.p[0], nullptr, nullptr, 1, nullptr, s);
             g_launches++;
@@ -1966,7 +1958,7 @@ int upload_table(effsc_prover* P, Table& T, const uint64_t* host, size_t len, in
         CK(cudaMallocAsync((void**)&flag, sizeof(u32), s));
         CK(cudaMemsetAsync(flag, 0, sizeof(u32), s));
         if (len) {
-            TRY(upload(stage));
+            CK(cudaMemcpyAsync(stage, host, len * 3 * sizeof(u64), cudaMemcpyHostToDevice, s));
             launch_split_aos(stage, len, 3, b.p[0], b.p[1], b.p[2], repr == EFFSC_MONTGOMERY, flag, s);
             g_launches++;
         }
@@ -2117,29 +2109,6 @@ const u64* effsc_internal_device_view(int device, const uint64_t* ptr, bool* is_
     int pageable = 0;
     cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, device);
     return pageable ? (const u64*)ptr : nullptr;
-}
-// Copy host words to the device on `s`.  Pageable memory that the GPU can read
-// in place (its page tables are the host's) goes by a copy kernel: the driver
-// stages pageable copies through a pinned buffer at a fifth of the link's
-// rate (161 MB of tables: 35 GB/s against ~180).  *in_place = true: the
-// source is read until `s` reaches this point, so the caller synchronises
-// before it gives the memory back (cudaMemcpyAsync returns with a pageable
-// source already read).  From 64 KB on; smaller copies are latency either way.
-cudaError_t effsc_internal_upload(int device, u64* dst, const uint64_t* host, size_t words, cudaStream_t s, bool* in_place) {
-    *in_place = false;
-    if (words >= ((size_t)1 << 13) && ((uintptr_t)host & 7) == 0) {
-        cudaPointerAttributes at;
-        int direct = 0;
-        if (cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type == cudaMemoryTypeUnregistered &&
-            cudaDeviceGetAttribute(&direct, cudaDevAttrPageableMemoryAccess, device) == cudaSuccess && direct) {
-            launch_copy((const u64*)host, dst, words, s);
-            g_launches++;
-            *in_place = true;
-            return cudaGetLastError();
-        }
-        cudaGetLastError();
-    }
-    return cudaMemcpyAsync(dst, host, words * sizeof(u64), cudaMemcpyHostToDevice, s);
 }
 int effsc_internal_ctx_device(const effsc_ctx* c) { return c->device; }
 cudaStream_t effsc_internal_ctx_stream(const effsc_ctx* c) { return c->stream; }

@@ -75,6 +75,58 @@ def test_rules(tmp_path):
     assert out[11:] == want
 
 
+HARNESS_COPY = r"""
+#include <cstdio>
+#include "residency.h"
+using namespace effsc;
+static int waits = 0;
+static int leave(int at, bool in_place) {     // a scope with three ways out
+    ReadsInPlace reads([] { waits++; return at_error; });
+    if (at == 0) return 10;
+    reads.pending |= in_place;
+    if (at == 1) return 11;                    // an error after the reads began
+    if (reads.finish()) return 12;
+    return 0;
+}
+int main() {
+    for (int in_place = 0; in_place < 2; in_place++)
+        for (int at = 0; at < 3; at++) {
+            waits = 0;
+            const int rc = leave(at, in_place);
+            std::printf("%d %d ", rc, waits);
+        }
+    at_error = 7;
+    waits = 0;
+    const int rc = leave(2, true);
+    std::printf("%d %d ", rc, waits);
+    const Residency all[4] = {Residency::device, Residency::managed, Residency::pinned, Residency::pageable};
+    for (Residency r : all)
+        for (int tables = 0; tables < 2; tables++)
+            for (size_t words : {(size_t)8191, (size_t)8192})
+                for (uintptr_t address : {(uintptr_t)4096, (uintptr_t)4100})
+                    std::printf("%d", (int)kernel_copies(r, tables != 0, words, address));
+}
+"""
+
+
+def test_copies_in_place(tmp_path):
+    """Who copies by a kernel, and that a scope with reads in flight is never left
+    before they are done: not by an error's way out, not twice, not for nothing."""
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if cxx is None:
+        pytest.skip("no C++ compiler")
+    src, exe = tmp_path / "c.cpp", tmp_path / "c"
+    src.write_text("#include <initializer_list>\nstatic int at_error = 0;\n" + HARNESS_COPY)
+    subprocess.check_call([cxx, "-std=c++17", "-O1", "-I", CSRC, str(src), "-o", str(exe)])
+    out = subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout.split()
+    assert [int(x) for x in out[:14]] == [10, 0, 11, 0, 0, 0, 10, 0, 11, 1, 0, 1, 12, 1]
+    assert out[14] == "0" * 30 + "10"          # pageable, host page tables, 64 KB, aligned
+    serve = open(os.path.join(CSRC, "serve.cu")).read()
+    body = serve[serve.index("int admit("):]
+    body = body[:body.index("\n}")]
+    assert body.index("ReadsInPlace reads(") < body.index("TRYS(") and "&reads.pending" in body
+
+
 @pytest.fixture(scope="module")
 def E():
     import effsc_gpu
