@@ -36,6 +36,7 @@
 #include "ip012.cuh"
 #include "residency.h"
 #include "tc.cuh"
+#include "tc_plan.h"
 
 namespace effsc {
 
@@ -320,9 +321,7 @@ __global__ void __launch_bounds__(GR_TPB, 1) k_ip_gram_many(const TcSeg* segs, u
 
 u32 gram_max_tiles(void) { return GR_MAX_TILES; }
 u32 tc_many_tiles(u64 total) {
-    const u64 blocks = (u64)(max_grid() / 8) * 5 / 2;
-    const u64 t = (total + blocks - 1) / blocks;
-    return (u32)(t < 16 ? 16 : t > GR_MAX_TILES ? GR_MAX_TILES : t);
+    return (u32)tc_tiles_per_block(total, (u64)(max_grid() / 8), GR_MAX_TILES);
 }
 
 template <bool LSB, int NV, bool MIRROR>

@@ -27,6 +27,7 @@
 #include "effsc_gpu.h"
 #include "kernels.h"
 #include "residency.h"
+#include "tc_plan.h"
 #include "keccak.cuh"
 
 #include <algorithm>
@@ -143,8 +144,7 @@ struct Lane {
     ServeSeg* d_segs = nullptr;
     RoundArgs* d_args = nullptr;
     u64* d_partials = nullptr;
-    u64* d_tc_partials = nullptr;   // from the pool, grown in the lane stream's order
-    u32 tc_blocks = 0;
+    u64* d_tc_partials = nullptr;   // 256 words for each of tc_blocks
 };
 
 struct effsc_server {
@@ -161,7 +161,7 @@ struct effsc_server {
     std::deque<Done> done;
     u32* h_status = nullptr;
     u32* d_status = nullptr;
-    size_t partial_blocks = 0;
+    size_t partial_blocks = 0, tc_blocks = 0;
     // pinned result slots
     u64* h_results = nullptr;
     std::vector<int> free_slots;
@@ -497,13 +497,7 @@ int step(effsc_server* s, Lane& ln) {
             a.tx.proof_chal = r->chal() + 3 * rd;
             blocks += segs[k].nblocks;
         }
-        if (blocks > ln.tc_blocks) {
-            if (ln.d_tc_partials) SCK(cudaFreeAsync(ln.d_tc_partials, cs));
-            ln.d_tc_partials = nullptr;
-            ln.tc_blocks = 0;
-            SCK(cudaMallocFromPoolAsync((void**)&ln.d_tc_partials, (size_t)blocks * 256 * sizeof(u64), s->pool, cs));
-            ln.tc_blocks = blocks;
-        }
+        if (blocks > s->tc_blocks) return effsc_set_error(EFFSC_CUDA_ERROR, "serving: %u blocks of the start", blocks);
         for (size_t k = 0; k < v.size(); k++) st.h_args[staged + k].partials = ln.d_tc_partials + (size_t)segs[k].first_block * 256;
         SCK(cudaMemcpyAsync(ln.d_segs + staged, st.h_segs + staged, v.size() * sizeof(TcSeg), cudaMemcpyHostToDevice, cs));
         SCK(cudaMemcpyAsync(ln.d_args + staged, st.h_args + staged, v.size() * sizeof(RoundArgs), cudaMemcpyHostToDevice, cs));
@@ -678,6 +672,14 @@ int effsc_server_create(effsc_ctx* ctx, uint64_t hbm_budget_bytes, uint32_t max_
     uint64_t keep = ~0ULL;   // keep freed memory in the pool for the next admissions
     cudaMemPoolSetAttribute(s->pool, cudaMemPoolAttrReleaseThreshold, &keep);
     s->partial_blocks = (size_t)max_active * max_grid();
+    // no step allocates: the start's blocks for whatever the budget (or the
+    // device) holds at once, an InnerProduct request's tables and work buffers
+    // being 40 bytes an entry and a tile 16 x TC_TILE_ITEMS entries (64 GB, 64
+    // requests: 3.5 MB a lane)
+    size_t fr = 0, total = 0;
+    if (cudaMemGetInfo(&fr, &total) != cudaSuccess) return bail(effsc_set_error(EFFSC_CUDA_ERROR, "cudaMemGetInfo"));
+    s->tc_blocks = tc_blocks_most(std::min<uint64_t>(hbm_budget_bytes, total) / (40 * 16 * TC_TILE_ITEMS), max_active,
+                                  (uint64_t)(max_grid() / 8), gram_max_tiles());
     for (int l = 0; l < SERVE_LANES; l++) {
         Lane& ln = s->lane[l];
         if (l == 0) ln.stream = effsc_internal_ctx_stream(ctx);
@@ -701,7 +703,8 @@ int effsc_server_create(effsc_ctx* ctx, uint64_t hbm_budget_bytes, uint32_t max_
         }
         if (cudaMalloc((void**)&ln.d_segs, max_active * sizeof(ServeSeg)) != cudaSuccess ||
             cudaMalloc((void**)&ln.d_args, max_active * sizeof(RoundArgs)) != cudaSuccess ||
-            cudaMalloc((void**)&ln.d_partials, s->partial_blocks * 12 * sizeof(u64)) != cudaSuccess)
+            cudaMalloc((void**)&ln.d_partials, s->partial_blocks * 12 * sizeof(u64)) != cudaSuccess ||
+            cudaMalloc((void**)&ln.d_tc_partials, s->tc_blocks * 256 * sizeof(u64)) != cudaSuccess)
             return bail(effsc_set_error(EFFSC_OOM, "serving: allocation failed"));
     }
     const size_t nslots = (size_t)2 * max_active * SERVE_INFLIGHT;
@@ -753,7 +756,7 @@ int effsc_server_destroy(effsc_server* s) {
         if (ln.d_segs) cudaFree(ln.d_segs);
         if (ln.d_args) cudaFree(ln.d_args);
         if (ln.d_partials) cudaFree(ln.d_partials);
-        if (ln.d_tc_partials) cudaFreeAsync(ln.d_tc_partials, ln.stream);
+        if (ln.d_tc_partials) cudaFree(ln.d_tc_partials);
         if (ln.tail_stream) cudaStreamDestroy(ln.tail_stream);
         if (ln.up_stream) cudaStreamDestroy(ln.up_stream);
         if (ln.own_stream) cudaStreamDestroy(ln.stream);
