@@ -364,11 +364,15 @@ int step(effsc_server* s, Lane& ln) {
     u32 ntx = 0;
     std::vector<Req*> fresh;
     int rc = admit(s, ln, st, &ntx, fresh);
-    if (rc != EFFSC_OK) return rc;
     // initial transcript states of the admitted requests: one H2D each from
-    // the pinned stage (they are small and few)
+    // the pinned stage (they are small and few); also where a later request's
+    // admission failed, since these are active
     for (u32 k = 0; k < ntx; k++)
         SCK(cudaMemcpyAsync(fresh[k]->tx(), &st.h_tx[k], sizeof(DevTranscript), cudaMemcpyHostToDevice, cs));
+    if (rc != EFFSC_OK) {
+        SCK(cudaStreamSynchronize(cs));      // the next call fills this stage again
+        return rc;
+    }
     if (ln.active.empty()) return EFFSC_OK;
     const int maxb = max_grid();
     const u64 per_block = (u64)KERNEL_TPB * s->quads_per_thread;
