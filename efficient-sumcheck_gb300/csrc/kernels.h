@@ -144,7 +144,7 @@ struct RoundArgs {
     const u64* chal2_ptr;  // second challenge (InnerProduct double fold of round 2)
     u64 chal[3];
     const u64* scalar[3];  // EqFactored right phase: eq_l[0] (c1, c2 null if base)
-    u64* partials;         // 12 words a block (the tensor-core passes: 256)
+    u64* partials;         // the blocks' sums (partial_words, tc_plan.h)
     u32* counter;          // zero between launches (the last block resets it)
     u64* result;           // wire (d*3 words) then aux pair (6 words)
     u32* status;           // device status word (non-zero: error code)

@@ -9,6 +9,7 @@
 #include "kernels.h"
 #include "keccak.cuh"
 #include "residency.h"
+#include "tc_plan.h"
 
 #include <algorithm>
 #include <cstdarg>
@@ -1926,8 +1927,7 @@ int final_value(effsc_prover* P, HF* out) {
 
 int prover_common_init(effsc_prover* P) {
     cudaStream_t s = P->ctx->stream;
-    // 12 words per block of the round kernels, 256 per SM of the tensor-core passes
-    CK(cudaMallocAsync((void**)&P->partials, (size_t)max_grid() * 32 * sizeof(u64), s));
+    CK(cudaMallocAsync((void**)&P->partials, partial_words(P->kind == EFFSC_IP, P->kind == EFFSC_COEF, max_grid()) * sizeof(u64), s));
     CK(cudaMallocAsync((void**)&P->counter, 2 * sizeof(u32), s));
     CK(cudaMemsetAsync(P->counter, 0, 2 * sizeof(u32), s));
     P->h_res = (u64*)pinned_get(P->ctx, 16 * sizeof(u64));

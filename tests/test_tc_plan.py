@@ -60,6 +60,49 @@ def test_blocks_fit(tmp_path):
     assert len(out) == len(lines) + 1
 
 
+def test_partials_hold_every_pass(tmp_path):
+    """The words that each kind's passes write, from the kernels' sources, fit."""
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if cxx is None:
+        pytest.skip("no C++ compiler")
+    src, exe = tmp_path / "p.cpp", tmp_path / "p"
+    src.write_text("""#include <cstdio>
+#include "tc_plan.h"
+int main() { for (int s = 1; s <= 200; s++) std::printf("%zu %zu %zu\\n", effsc::partial_words(true, false, 8 * s), effsc::partial_words(false, true, 8 * s),
+    effsc::partial_words(false, false, 8 * s)); }""")
+    subprocess.check_call([cxx, "-std=c++17", "-O1", "-I", CSRC, str(src), "-o", str(exe)])
+    rows = [[int(x) for x in r.split()] for r in subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout.split("\n") if r]
+    assert len(rows) == 200
+    for sms, (ip, coef, other) in enumerate(rows, 1):
+        rounds = 8 * sms * 12                        # round_common.cuh: RAW_WORDS a block
+        # k_ip_gram: 16 x 16 words a block, one an SM; ip012.cuh: 32, two an SM
+        assert ip >= max(rounds, sms * 256, 2 * sms * 32)
+        # k_c3_gram: 12 x 9, one an SM; coef01.cuh: 48, a quarter of the grid
+        assert coef >= max(rounds, sms * 108, 2 * sms * 48)
+        assert other == rounds
+
+
+@pytest.mark.gpu
+def test_small_provers_stay_small():
+    """What a prover without tables of a size holds on the device."""
+    import ctypes
+    import numpy as np
+    import effsc_gpu as E
+    E.MultilinearProver(np.arange(8, dtype=np.uint64))
+    rt = ctypes.CDLL("libcudart.so.13")
+    pool, used = ctypes.c_void_p(), ctypes.c_uint64()
+    assert rt.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+
+    def now():
+        E.Context.default().synchronize()
+        assert rt.cudaMemPoolGetAttribute(pool, 7, ctypes.byref(used)) == 0       # cudaMemPoolAttrUsedMemCurrent
+        return used.value
+    at = now()
+    keep = [E.MultilinearProver(np.arange(8, dtype=np.uint64)) for _ in range(32)]
+    assert now() - at < 32 * (200 << 10)
+    del keep
+
+
 def test_a_step_allocates_nothing():
     text = open(os.path.join(CSRC, "serve.cu")).read()
     body = text[text.index("\nint step("):]
