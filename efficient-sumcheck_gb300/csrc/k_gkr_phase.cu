@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(TPB) k_gkr_terms_c(GkrSums add, GkrSums mult, 
 }
 
 // The same from the gate tables: eight columns a block, thread = (column, one
-// of 32 groups of rows); each block forms the n <= 256 weights itself.
+// of 32 groups of rows); each block forms the n <= GKR_SMALL weights itself.
 template <int FW>
 __global__ void __launch_bounds__(TPB) k_gkr_cols(const u64* add, const u64* mult, const u64* W, const u64* wb,
                                                   const u64* chals, u32 k, u64* F, u64* G) {

@@ -8,7 +8,7 @@
 // product: the digit rows of the tables (tc.cuh; 128 items to a tile, the
 // digits contiguous: K) times a constant matrix of 48 columns, column
 // 16 c + d the 4-bit digit d of component c of E_v 16^w(e) mod p.  Sums stay
-// below 256 * 225 < 2^16, exact in f32.  What is left for the integer pipes is
+// at most 256 * 225 < 2^16, exact in f32.  What is left for the integer pipes is
 // to put sixteen digit sums back together per component (two per
 // multiply-add in float, then four 32-bit pieces per 64-bit sum) instead of
 // 3 (2^NV - 1) products with their differences per entry.

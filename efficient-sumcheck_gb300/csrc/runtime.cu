@@ -314,7 +314,8 @@ struct effsc_prover {
     // effsc_prove: 0 = one pass per round; 1 = InnerProduct rounds 0-2 in
     // two passes (k_ip01.cu), the Multilinear and GkrProver starts, the
     // EqFactored left phase from the inner sums (k_eqf.cu); 2 = as 1, with
-    // InnerProduct rounds 0-3 in two passes (k_ip012.cu) where they apply
+    // InnerProduct rounds 0-4 in two passes (k_gram.cu and k_tcfold.cu; rounds
+    // 0-3 in k_ip012.cu's general form) where they apply
     int fuse_first = 2;
     // CoefficientProver with a declarative evaluator: the term program over
     // the columns (pairwise tables, then the tablewise tables' columns);
@@ -895,9 +896,10 @@ bool fuse_first_ok(const effsc_prover* P, size_t num_rounds) {
     return !whole_in_tail(P, num_rounds);
 }
 
-// Rounds 0-3 in two passes (k_ip012.cu) from num_vars = 14 on (below, the
-// one-block tail takes the proof within a few rounds): leaves the state the
-// per-round path leaves after round 3.
+// Rounds 0-4 in two passes on the tensor cores (k_gram.cu, k_tcfold.cu; 0-3 in
+// a run of four rounds, and for tables that tc_rounds refuses, in k_ip012.cu)
+// from num_vars = 14 on (below, the tail takes the proof within a few rounds):
+// leaves the state the per-round path leaves after the last of them.
 constexpr size_t FUSE3_MIN_LEN = 1 << 14;
 bool fuse3_ok(const effsc_prover* P, size_t num_rounds) {
     if (P->fuse_first < 2 || num_rounds < 4 || !fuse_first_ok(P, num_rounds)) return false;
@@ -922,9 +924,10 @@ bool mirror_ok(effsc_prover* P, size_t L) {
 }
 
 // The tensor-core start takes every two-pass start whose tables it can load
-// 16 bytes at a time and whose words come in time (residency.h): rounds 0-4 when the proof has them (one pass over the
-// tables fewer bytes of folded tables: 2 x 24 L/16 instead of 2 x 24 L/8),
-// else rounds 0-3.  0: the general form (k_ip012.cu, rounds 0-3).
+// 16 bytes at a time and whose words come in time (residency.h): rounds 0-4
+// when the proof has them (fewer bytes of folded tables written: 2 x 24 L/16
+// instead of 2 x 24 L/8), else rounds 0-3.  0: the general form (k_ip012.cu,
+// rounds 0-3).
 int tc_rounds(const effsc_prover* P, size_t L, size_t num_rounds, bool copied, const RoundArgs& a) {
     uintptr_t bits = 0;
     bool prompt = true;

@@ -4,7 +4,7 @@
 // A 64-bit word is sixteen 4-bit digits.  As the low bits of an e4m3 byte a
 // digit n in 0..15 is the number n 2^-9 (0..7 subnormal, 8..15 normal with the
 // smallest exponent), so splitting a word takes a mask and a shift, no
-// conversion.  A product of two digits is below 225 in units of 2^-18, and a
+// conversion.  A product of two digits is at most 225 in units of 2^-18, and a
 // float accumulator of such sums is exact below 2^24 of them: 74565 terms.
 // A chunk is a word's sixteen digit bytes: the low digits of bytes 0..7, then
 // the high digits (digit e < 8 weighs 16^(2 e), digit 8 + b 16^(2 b + 1)).

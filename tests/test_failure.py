@@ -1,10 +1,11 @@
 """Failure handling without a GPU fault.
 
-The only waits in the library's kernels are the TMA-staged round kernel's
-waits on its own mbarriers; each gives up after a time limit, records
-EFFSC_STATUS_TIMEOUT and returns.  The self-test entry point runs that wait on
+The waits of the library's kernels on their own mbarriers (the TMA-staged
+round kernel's and the tensor-core passes') give up after a time limit, record
+EFFSC_STATUS_TIMEOUT and return.  The self-test entry point runs that wait on
 a barrier nothing completes (short limit) and on one that completes: the
-status must say so and the context must stay usable.  Host-side failures
+status must say so and the context must stay usable (the tensor-core passes'
+route after it: test_wait_limits.py).  Host-side failures
 (bad arguments, requests larger than the serving budget, reference panics)
 are covered beside the features they guard."""
 import time

@@ -1,8 +1,8 @@
-"""Tables from pageable host memory are copied by a kernel from 64 KB on:
-lengths around that limit, odd lengths, sources 8 but not 16 bytes aligned,
-memory the caller changes as soon as the call returns, and served requests
-from such tables of every size around the tensor-core start's and the tail's
-limits -- against the oracle."""
+"""Tables from pageable host memory (a served request's are copied by a kernel
+from 64 KB on): lengths around that limit, odd lengths, sources 8 but not 16
+bytes aligned, memory the caller changes as soon as the call returns, and
+served requests from such tables of every size around the tensor-core start's
+and the tail's limits -- against the oracle."""
 import os
 
 import numpy as np
