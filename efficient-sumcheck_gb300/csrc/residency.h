@@ -3,7 +3,6 @@
 #pragma once
 #include <cstddef>
 #include <cstdint>
-#include <sys/mman.h>
 #include <unistd.h>
 
 namespace effsc {
@@ -46,15 +45,13 @@ constexpr bool kernel_copies(Residency r, bool host_page_tables, size_t words, u
     return r == Residency::pageable && host_page_tables && words >= ((size_t)1 << 13) && (address & 7) == 0;
 }
 
-// Bring the pages of pageable memory in before a kernel reads them: on the host
-// a missing page is a microsecond, from the GPU ten.  False where the system
-// cannot (the kernel then brings them in).
-inline bool populate_pages(const void* p, size_t bytes) {
-    if (!bytes) return true;
-    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
-    const uintptr_t lo = (uintptr_t)p & ~(page - 1), hi = ((uintptr_t)p + bytes + page - 1) & ~(page - 1);
-    constexpr int populate_read = 22;      // MADV_POPULATE_READ (Linux 5.14)
-    return madvise((void*)lo, hi - lo, populate_read) == 0;
+// Bring the pages of pageable memory in before a kernel reads them, by a read
+// in each: on the host a missing page is a microsecond, from the GPU ten.
+// (Resident pages: 20 us for 128 MB of 64 KB pages, madvise(MADV_POPULATE_READ) 73.)
+inline void touch_pages(const void* p, size_t bytes) {
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    const volatile char* c = (const volatile char*)p;
+    for (size_t at = 0; at < bytes; at += page - ((uintptr_t)(c + at) & (page - 1))) (void)c[at];
 }
 
 // The caller's memory while kernels read it: once `pending`, the scope is not

@@ -43,6 +43,7 @@ void effsc_internal_tx_state(const effsc_transcript* t, void* out);
 int effsc_internal_ctx_device(const effsc_ctx* c);
 cudaStream_t effsc_internal_ctx_stream(const effsc_ctx* c);
 uint64_t effsc_internal_add_launches(uint64_t k);
+cudaError_t effsc_internal_upload(int device, u64* dst, const uint64_t* host, size_t words, cudaStream_t s, bool* in_place);
 
 #define SCK(call)                                                                                           \
     do {                                                                                                    \
@@ -144,7 +145,7 @@ struct Lane {
     ServeSeg* d_segs = nullptr;
     RoundArgs* d_args = nullptr;
     u64* d_partials = nullptr;
-    u64* d_tc_partials = nullptr;   // 256 words for each of tc_blocks
+    u64* d_tc_partials = nullptr;   // 256 words for each of tc_blocks, behind d_partials
 };
 
 struct effsc_server {
@@ -154,7 +155,6 @@ struct effsc_server {
     uint64_t budget = 0, reserved = 0;
     u32 max_active = 0, n_active = 0;
     int quads_per_thread = 8;
-    bool host_page_tables = false;   // the GPU reads pageable memory through the host's page tables
     uint64_t next_id = 0;
     Lane lane[SERVE_LANES];
     std::deque<Req*> finishing;
@@ -244,25 +244,6 @@ int join_uploaded(effsc_server* s, Lane& ln, Lane::Stage& st, u32* ntx, std::vec
     return EFFSC_OK;
 }
 
-// Host words to the device on `up`.  Pageable memory goes by a copy kernel: the
-// driver's pageable copies keep the host in the call, one after the other,
-// where the kernels queue (48 requests of 14 to 20 variables, 161 MB: 3.00 ms
-// against 3.69).  *in_place: the source is read until `up` gets here.  Pages
-// that are not there are brought in first; where that fails the driver copies.
-cudaError_t upload(effsc_server* s, u64* dst, const uint64_t* host, size_t words, cudaStream_t up, bool* in_place) {
-    cudaPointerAttributes at;
-    const bool known = cudaPointerGetAttributes(&at, host) == cudaSuccess;
-    if (!known) cudaGetLastError();
-    const Residency r = known && at.type == cudaMemoryTypeUnregistered ? Residency::pageable : Residency::pinned;
-    if (kernel_copies(r, s->host_page_tables, words, (uintptr_t)host) && populate_pages(host, words * sizeof(u64))) {
-        *in_place = true;
-        launch_copy((const u64*)host, dst, words, up);
-        effsc_internal_add_launches(1);
-        return cudaGetLastError();
-    }
-    return cudaMemcpyAsync(dst, host, words * sizeof(u64), cudaMemcpyHostToDevice, up);
-}
-
 int admit(effsc_server* s, Lane& ln, Lane::Stage& st, u32* ntx, std::vector<Req*>& fresh) {
     cudaStream_t cs = ln.stream;
     // pageable tables are the caller's again once they are admitted, or the call failed
@@ -295,7 +276,7 @@ int admit(effsc_server* s, Lane& ln, Lane::Stage& st, u32* ntx, std::vector<Req*
             SCK(cudaStreamWaitEvent(ln.up_stream, e, 0));
             s->free_events.push_back(e);
             for (int t = 0; t < r->ntab; t++) {
-                SCK(upload(s, r->in(t), r->htab[t], 1ULL << r->n, ln.up_stream, &reads.pending));
+                SCK(effsc_internal_upload(s->device, r->in(t), r->htab[t], 1ULL << r->n, ln.up_stream, &reads.pending));
             }
             r->up_ev = get_event(s);
             SCK(cudaEventRecord(r->up_ev, ln.up_stream));
@@ -664,8 +645,6 @@ int effsc_server_create(effsc_ctx* ctx, uint64_t hbm_budget_bytes, uint32_t max_
     s->budget = hbm_budget_bytes;
     s->max_active = max_active;
     auto bail = [&](int rc) { effsc_server_destroy(s); return rc; };
-    int tables = 0;
-    s->host_page_tables = cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, s->device) == cudaSuccess && tables;
     cudaMemPoolProps props;
     memset(&props, 0, sizeof props);
     props.allocType = cudaMemAllocationTypePinned;
@@ -676,13 +655,11 @@ int effsc_server_create(effsc_ctx* ctx, uint64_t hbm_budget_bytes, uint32_t max_
     uint64_t keep = ~0ULL;   // keep freed memory in the pool for the next admissions
     cudaMemPoolSetAttribute(s->pool, cudaMemPoolAttrReleaseThreshold, &keep);
     s->partial_blocks = (size_t)max_active * max_grid();
-    // no step allocates: the start's blocks for whatever the budget (or the
-    // device) holds at once, an InnerProduct request's tables and work buffers
-    // being 40 bytes an entry and a tile 16 x TC_TILE_ITEMS entries (64 GB, 64
-    // requests: 3.5 MB a lane)
-    size_t fr = 0, total = 0;
-    if (cudaMemGetInfo(&fr, &total) != cudaSuccess) return bail(effsc_set_error(EFFSC_CUDA_ERROR, "cudaMemGetInfo"));
-    s->tc_blocks = tc_blocks_most(std::min<uint64_t>(hbm_budget_bytes, total) / (40 * 16 * TC_TILE_ITEMS), max_active,
+    // no step allocates: the start's blocks for whatever the budget (or a
+    // device of 288 GB) holds at once, an InnerProduct request's tables and work
+    // buffers being 40 bytes an entry and a tile 16 x TC_TILE_ITEMS entries
+    // (64 GB, 64 requests: 3.5 MB a lane)
+    s->tc_blocks = tc_blocks_most(std::min<uint64_t>(hbm_budget_bytes, 288ULL << 30) / (40 * 16 * TC_TILE_ITEMS), max_active,
                                   (uint64_t)(max_grid() / 8), gram_max_tiles());
     for (int l = 0; l < SERVE_LANES; l++) {
         Lane& ln = s->lane[l];
@@ -707,9 +684,9 @@ int effsc_server_create(effsc_ctx* ctx, uint64_t hbm_budget_bytes, uint32_t max_
         }
         if (cudaMalloc((void**)&ln.d_segs, max_active * sizeof(ServeSeg)) != cudaSuccess ||
             cudaMalloc((void**)&ln.d_args, max_active * sizeof(RoundArgs)) != cudaSuccess ||
-            cudaMalloc((void**)&ln.d_partials, s->partial_blocks * 12 * sizeof(u64)) != cudaSuccess ||
-            cudaMalloc((void**)&ln.d_tc_partials, s->tc_blocks * 256 * sizeof(u64)) != cudaSuccess)
+            cudaMalloc((void**)&ln.d_partials, (s->partial_blocks * 12 + s->tc_blocks * 256) * sizeof(u64)) != cudaSuccess)
             return bail(effsc_set_error(EFFSC_OOM, "serving: allocation failed"));
+        ln.d_tc_partials = ln.d_partials + s->partial_blocks * 12;
     }
     const size_t nslots = (size_t)2 * max_active * SERVE_INFLIGHT;
     if (cudaHostAlloc((void**)&s->h_results, nslots * RES_WORDS * sizeof(u64), cudaHostAllocDefault) != cudaSuccess ||
@@ -760,7 +737,6 @@ int effsc_server_destroy(effsc_server* s) {
         if (ln.d_segs) cudaFree(ln.d_segs);
         if (ln.d_args) cudaFree(ln.d_args);
         if (ln.d_partials) cudaFree(ln.d_partials);
-        if (ln.d_tc_partials) cudaFree(ln.d_tc_partials);
         if (ln.tail_stream) cudaStreamDestroy(ln.tail_stream);
         if (ln.up_stream) cudaStreamDestroy(ln.up_stream);
         if (ln.own_stream) cudaStreamDestroy(ln.stream);
