@@ -159,8 +159,8 @@ struct RoundArgs {
 enum AccMode { ACC_NONE = 0, ACC_FIRST = 1, ACC_MID = 2, ACC_LAST = 3 };
 
 
-// The last rounds of an MSB Multilinear / InnerProduct proof run by one block
-// with the tables in shared memory: rounds r0 .. r0 + nrounds - 1, each a
+// The last rounds of a Multilinear, InnerProduct or Coefficient proof run by one
+// block or cluster with the tables in shared memory: rounds r0 .. r0 + nrounds - 1, each a
 // fold with the previous challenge (except a first round 0) plus evaluation,
 // block reduction and the transcript step, without a kernel boundary.
 struct TailArgs {

@@ -310,8 +310,8 @@ struct effsc_prover {
     uint64_t g_kernels = 0;                    // kernel nodes in the graph
     TabState g_post[4];
     size_t g_post_rounds = 0;
-    // effsc_prove: tables of at most this length finish in the one-block tail
-    // kernel (SIZE_MAX: as large as shared memory allows; 0: never)
+    // effsc_prove: tables of at most this length finish in a tail kernel, a
+    // cluster or one block (SIZE_MAX: as large as shared memory allows; 0: never)
     size_t tail_len = SIZE_MAX;
     // effsc_prove: 0 = one pass per round; 1 = InnerProduct rounds 0-2 in
     // two passes (k_ip01.cu), the Multilinear and GkrProver starts, the
@@ -1020,7 +1020,7 @@ int do_fuse3(effsc_prover* P, size_t num_rounds, const TxIO& tx0, const u64* cha
     const int tc = tc_rounds(P, L, num_rounds, mirror, a), nv = tc ? tc : 3;
     // bring in pages that are not there yet, once for the prover (a first proof
     // of 2^24 entries, MSB and LSB: of a newly mapped file 2.0 and 21 ms
-    // without, 1.9 and 1.9 with; of untouched memory 136 and 131, 2.1 and 2.1)
+    // without, 1.8 and 1.8 with; of untouched memory 136 and 131, 2.7 and 2.7)
     for (int i = 0; i < 2 && mirror; i++) {
         Buf& h = P->t[i].bufs[0];
         if (!h.prompt && !h.touched) touch_pages(h.p[0], L * sizeof(u64));

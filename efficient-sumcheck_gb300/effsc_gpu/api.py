@@ -301,8 +301,8 @@ class _Prover:
         check(load().effsc_prover_set_first_rounds(self.h, level))
 
     def set_tail(self, max_len):
-        """prove(): tables of at most max_len entries finish in the one-block
-        tail kernel (None: as large as shared memory allows, 0: never)."""
+        """prove(): tables of at most max_len entries finish in a tail kernel,
+        one block or a cluster (None: as large as shared memory allows, 0: never)."""
         check(load().effsc_prover_set_tail(self.h, (1 << 64) - 1 if max_len is None else int(max_len)))
 
     def set_persistent(self, max_len):

@@ -194,12 +194,13 @@ int effsc_prover_final_value(effsc_prover* p, uint64_t* out);
  * Writes table_len() elements of `field` words each (AoS). */
 int effsc_prover_table_len(const effsc_prover* p, int table, size_t* out_len);
 int effsc_prover_read_table(effsc_prover* p, int table, uint64_t* out);
-/* effsc_prove only (no reference counterpart; a tuning knob): once an MSB
- * Multilinear / InnerProduct prover's power-of-two tables are at most
- * max_len long, the remaining rounds run in one launch with the tables in
- * shared memory: one thread block, or (Multilinear, tables up to 16 times
- * one block's capacity, entered mid-proof) a thread-block cluster that hands
- * over to one block.  A GkrProver's rounds move into one block once add,
+/* effsc_prove only (no reference counterpart; a tuning knob): once a
+ * Multilinear or InnerProduct prover's power-of-two tables (MSB or LSB; a
+ * degree-3 Coefficient prover's folded Fp3 tables, up to 2^14 entries; an
+ * EqFactored prover's in its right phase) are at most max_len long, the
+ * remaining rounds run in one launch with the tables in shared memory: one
+ * thread block, or, from 2^11 entries and up to 16 times one block's capacity,
+ * a thread-block cluster that hands over to one block.  A GkrProver's rounds move into one block once add,
  * mult, W_b and W_c fit in shared memory together and add is at most max_len
  * long.  Default SIZE_MAX: as long as shared memory allows; 0 disables.
  * Proofs are identical. */
