@@ -328,7 +328,7 @@ extern "C" int effsc_protogalaxy_fold(effsc_ctx* ctx, int field, const uint64_t*
         res = res_fallback.data();
     }
     // the last pass writes the row there itself (2^20 rows of 8, a call: 114 ->
-    // 104 us without the copy; 92 with the passes as dependent launches)
+    // 104 us without the copy; 98-102 with the passes as dependent launches)
     u64* res_dev = nullptr;
     if (!res_fallback.empty() || cudaHostGetDevicePointer((void**)&res_dev, res, 0) != cudaSuccess) {
         cudaGetLastError();

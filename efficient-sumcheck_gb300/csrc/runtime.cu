@@ -2122,8 +2122,8 @@ const u64* effsc_internal_device_view(int device, const uint64_t* ptr, bool* is_
     return pageable ? (const u64*)ptr : nullptr;
 }
 // Host words to the device on `s`.  Pageable memory goes by a copy kernel, its
-// missing pages brought in first: the driver's pageable copies keep the host in
-// the call, one after the other, where the kernels queue (48 served requests of
+// missing pages brought in first: CUDA's pageable copies keep the host in the
+// call, one after the other, where the kernels queue (48 served requests of
 // 14 to 20 variables, 161 MB: 3.05 ms against 3.69), and a table of 2^24 words
 // that nothing has touched takes them 5.8 ms against 1.3 (written before: 0.95
 // and 0.86).  *in_place: the source is read until `s` gets here.
